@@ -392,18 +392,10 @@ __global__ void __launch_bounds__(KPT) k_kzm_step_pair(const float* __restrict__
                               vfma(P.iy2, at(sc, ROW) + at(sc, -ROW),
                                    vfma(P.iz2, at(pp + m * KPS, 0) + at(pm + m * KPS, 0), P.lap_c * c[m])));
             }
-            F2 h[6];
-            bulk_field_pair(c, P.A, P.B, P.C, h);
-            h[0] = vfma(-P.kappa, lap[0], h[0]);
-            h[1] = vfma(-P.kappa, lap[3], h[1]);
-            h[2] = vfma(P.kappa, lap[0] + lap[3], h[2]);
-            h[3] = vfma(-P.kappa, lap[1], h[3]);
-            h[4] = vfma(-P.kappa, lap[2], h[4]);
-            h[5] = vfma(-P.kappa, lap[4], h[5]);
-            const F2 corr = (1.0f / 3.0f) * (h[0] + h[1] + h[2]);
-            const float nmd = -P.mob_dt;
-            F2 u[5] = {vfma(nmd, h[0] - corr, c[0]), vfma(nmd, h[3], c[1]), vfma(nmd, h[4], c[2]),
-                       vfma(nmd, h[1] - corr, c[3]), vfma(nmd, h[5], c[4])};
+            F2 h[5], u[5];
+            bulk_field5<F2>(c, P.A, P.B, P.C, h);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) u[m] = vfma(-P.mob_dt, vfma(-P.kappa, lap[m], h[m]), c[m]);
             float v[2][5];
 #pragma unroll
             for (int m = 0; m < 5; ++m) {

@@ -52,6 +52,10 @@ struct QsrConst {
     float L2i2x, L2i2y, L2i2z;  // L2/(2d)
     float l3m[6];               // (L3/2) / (4 da db) for M_ab from undivided central differences (xx yy zz xy xz yz)
     float l2w[6];               // L2 / (4 da db) for d_a D_b from undivided second differences (xx yy zz xy xz yz)
+    float lx, ly, lz;           // Liso/da^2: pure second differences of the L1 term
+    float l3s[3];               // L3/da^2: pure second differences of the L3 contraction
+    float l3c[3];               // L3/(2 da db): mixed second differences of the L3 contraction (xy xz yz)
+    float l3d[6];               // L3/(4 da db): products of first differences in the L3 terms (xx yy zz xy xz yz)
 };
 
 // ---------------------------------------------------------------------------------------
@@ -335,170 +339,9 @@ __device__ __forceinline__ void chem_potential(const Acc& A, const DAcc& DA, con
 }
 
 // ---------------------------------------------------------------------------------------
-// Packed-pair form of the interior chemical potential. Blackwell issues one FFMA2 / FADD2 /
-// FMUL2 for two FP32 lanes, so the stencil arithmetic runs on component pairs: X = (xx, yy),
-// Y = (xy, xz); yz stays scalar and zz = -(xx + yy). Same terms and weights as
-// chem_potential<kL2, kL3, false>; only the rounding order differs.
-// ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float2 bc2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-// a - b as b * (-1) + a (the product is exact, so this is the rounded difference)
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-
-// Interior cells (2 <= i, j, k <= N - 3 when L2 is on, else 1 <= .. <= N - 2) read only Q:
-//  * the column divergence D_b = d_k Q_kb at the centre (the L3 term's D . grad) from the face
-//    neighbours' central differences, as the reference's interior D;
-//  * the L2 term d_a D_b (QSR.cu:436-460), the central difference of the reference's central D,
-//    which for an interior cell is exactly sum_k S_ak(Q_kb) / (4 da dk): S_ak the undivided
-//    mixed (four-corner) second difference for k != a and the wide second difference
-//    Q(+2a) - 2 Q + Q(-2a) for k = a. The corner sums are the ones the L3 term needs anyway, so
-//    no divergence field is staged.
-template <bool kL2, bool kL3, class Acc>
-__device__ __forceinline__ void chem_potential_interior_x2(const Acc& A, const QsrConst& P, int i, int j, int k,
-                                                           const float q[5], bool anchor, float mu[5], float lap[5]) {
-    constexpr bool kMixed = kL2 || kL3;
-    auto X = [&](int di, int dj, int dk) { return make_float2(A(0, di, dj, dk), A(3, di, dj, dk)); };
-    auto Y = [&](int di, int dj, int dk) { return make_float2(A(1, di, dj, dk), A(2, di, dj, dk)); };
-    auto Z = [&](int di, int dj, int dk) { return A(4, di, dj, dk); };  // yz
-    const float2 qX = make_float2(q[0], q[3]), qY = make_float2(q[1], q[2]);
-    const float qZ = q[4];
-    // face neighbours, their sums (Laplacian, pure second derivatives) and undivided central
-    // differences (first derivatives)
-    const float2 Xpx = X(1, 0, 0), Xmx = X(-1, 0, 0), Xpy = X(0, 1, 0), Xmy = X(0, -1, 0), Xpz = X(0, 0, 1),
-                 Xmz = X(0, 0, -1);
-    const float2 Ypx = Y(1, 0, 0), Ymx = Y(-1, 0, 0), Ypy = Y(0, 1, 0), Ymy = Y(0, -1, 0), Ypz = Y(0, 0, 1),
-                 Ymz = Y(0, 0, -1);
-    const float Zpx = Z(1, 0, 0), Zmx = Z(-1, 0, 0), Zpy = Z(0, 1, 0), Zmy = Z(0, -1, 0), Zpz = Z(0, 0, 1),
-                Zmz = Z(0, 0, -1);
-    const float2 sxX = add2(Xpx, Xmx), syX = add2(Xpy, Xmy), szX = add2(Xpz, Xmz);
-    const float2 sxY = add2(Ypx, Ymx), syY = add2(Ypy, Ymy), szY = add2(Ypz, Ymz);
-    const float sxZ = Zpx + Zmx, syZ = Zpy + Zmy, szZ = Zpz + Zmz;
-    const float2 lapX = fma2(bc2(P.ix2), sxX, fma2(bc2(P.iy2), syX, fma2(bc2(P.iz2), szX, mul2(bc2(P.lap_c), qX))));
-    const float2 lapY = fma2(bc2(P.ix2), sxY, fma2(bc2(P.iy2), syY, fma2(bc2(P.iz2), szY, mul2(bc2(P.lap_c), qY))));
-    const float lapZ = fmaf(P.ix2, sxZ, fmaf(P.iy2, syZ, fmaf(P.iz2, szZ, P.lap_c * qZ)));
-    lap[0] = lapX.x; lap[3] = lapX.y; lap[1] = lapY.x; lap[2] = lapY.y; lap[4] = lapZ;
-    float h[6];
-    bulk_field(q, P.cQ, P.cQ2, P.cQ3, h);
-    // elastic (one-constant or L1): hX = (h_xx, h_yy), hY = (h_xy, h_xz), h_zz, h_yz
-    float2 hX = fma2(bc2(-P.Liso), lapX, make_float2(h[0], h[1]));
-    float2 hY = fma2(bc2(-P.Liso), lapY, make_float2(h[3], h[4]));
-    float hzz = fmaf(P.Liso, lapX.x + lapX.y, h[2]);  // - Liso lap_zz, lap_zz = -(lap_xx + lap_yy)
-    float hyz = fmaf(-P.Liso, lapZ, h[5]);
-    // undivided mixed second differences (four corners) of every component: (xx, yy), (xy, xz), yz
-    float2 mxyX{}, mxzX{}, myzX{}, mxyY{}, mxzY{}, myzY{};
-    float mxyZ = 0.0f, mxzZ = 0.0f, myzZ = 0.0f;
-    if (kMixed) {
-        mxyX = sub2(sub2(X(1, 1, 0), X(1, -1, 0)), sub2(X(-1, 1, 0), X(-1, -1, 0)));
-        mxzX = sub2(sub2(X(1, 0, 1), X(1, 0, -1)), sub2(X(-1, 0, 1), X(-1, 0, -1)));
-        myzX = sub2(sub2(X(0, 1, 1), X(0, 1, -1)), sub2(X(0, -1, 1), X(0, -1, -1)));
-        mxyY = sub2(sub2(Y(1, 1, 0), Y(1, -1, 0)), sub2(Y(-1, 1, 0), Y(-1, -1, 0)));
-        mxzY = sub2(sub2(Y(1, 0, 1), Y(1, 0, -1)), sub2(Y(-1, 0, 1), Y(-1, 0, -1)));
-        myzY = sub2(sub2(Y(0, 1, 1), Y(0, 1, -1)), sub2(Y(0, -1, 1), Y(0, -1, -1)));
-        mxyZ = (Z(1, 1, 0) - Z(1, -1, 0)) - (Z(-1, 1, 0) - Z(-1, -1, 0));
-        mxzZ = (Z(1, 0, 1) - Z(1, 0, -1)) - (Z(-1, 0, 1) - Z(-1, 0, -1));
-        myzZ = (Z(0, 1, 1) - Z(0, 1, -1)) - (Z(0, -1, 1) - Z(0, -1, -1));
-    }
-    if (kL2) {
-        // wide second differences Q(+2a) - 2 Q + Q(-2a) of the components d_a D_b needs
-        const float q2xx = 2.0f * q[0], q2xy = 2.0f * q[1], q2xz = 2.0f * q[2], q2yy = 2.0f * q[3],
-                    q2yz = 2.0f * q[4];
-        const float wx_xx = (A(0, 2, 0, 0) + A(0, -2, 0, 0)) - q2xx;
-        const float wx_xy = (A(1, 2, 0, 0) + A(1, -2, 0, 0)) - q2xy;
-        const float wx_xz = (A(2, 2, 0, 0) + A(2, -2, 0, 0)) - q2xz;
-        const float wy_yy = (A(3, 0, 2, 0) + A(3, 0, -2, 0)) - q2yy;
-        const float wy_xy = (A(1, 0, 2, 0) + A(1, 0, -2, 0)) - q2xy;
-        const float wy_yz = (A(4, 0, 2, 0) + A(4, 0, -2, 0)) - q2yz;
-        const float wz_xx = (A(0, 0, 0, 2) + A(0, 0, 0, -2)) - q2xx;
-        const float wz_yy = (A(3, 0, 0, 2) + A(3, 0, 0, -2)) - q2yy;
-        const float wz_xz = (A(2, 0, 0, 2) + A(2, 0, 0, -2)) - q2xz;
-        const float wz_yz = (A(4, 0, 0, 2) + A(4, 0, 0, -2)) - q2yz;
-        const float wz_zz = -(wz_xx + wz_yy);
-        const float mxz_zz = -(mxzX.x + mxzX.y), myz_zz = -(myzX.x + myzX.y);
-        const float cxx = P.l2w[0], cyy = P.l2w[1], czz = P.l2w[2], cxy = P.l2w[3], cxz = P.l2w[4], cyz = P.l2w[5];
-        // d_x D_x, d_y D_y, d_z D_z
-        const float dxDx = fmaf(cxx, wx_xx, fmaf(cxy, mxyY.x, cxz * mxzY.y));
-        const float dyDy = fmaf(cxy, mxyY.x, fmaf(cyy, wy_yy, cyz * myzZ));
-        const float dzDz = fmaf(cxz, mxzY.y, fmaf(cyz, myzZ, czz * wz_zz));
-        // mixed: d_x D_y + d_y D_x, d_x D_z + d_z D_x, d_y D_z + d_z D_y
-        const float sxy = fmaf(cxx, wx_xy, fmaf(cxy, mxyX.y, fmaf(cxz, mxzZ,
-                          fmaf(cxy, mxyX.x, fmaf(cyy, wy_xy, cyz * myzY.y)))));
-        const float sxz = fmaf(cxx, wx_xz, fmaf(cxy, mxyZ, fmaf(cxz, mxz_zz,
-                          fmaf(cxz, mxzX.x, fmaf(cyz, myzY.x, czz * wz_xz)))));
-        const float syz = fmaf(cxy, mxyY.y, fmaf(cyy, wy_yz, fmaf(cyz, myz_zz,
-                          fmaf(cxz, mxzY.x, fmaf(cyz, myzX.y, czz * wz_yz)))));
-        hX = fma2(bc2(-1.0f), make_float2(dxDx, dyDy), hX);
-        hY = fma2(bc2(-1.0f), make_float2(sxy, sxz), hY);
-        hzz -= dzDz;
-        hyz -= syz;
-    }
-    float corr = (hX.x + hX.y + hzz) * (1.0f / 3.0f);
-    float2 muX = add2(hX, bc2(-corr));  // (mu_xx, mu_yy)
-    float2 muY = hY;                    // (mu_xy, mu_xz)
-    float muZ = hyz;                    // mu_yz
-    if (kL3) {
-        // undivided central differences per axis
-        const float2 dXx = sub2(Xpx, Xmx), dXy = sub2(Xpy, Xmy), dXz = sub2(Xpz, Xmz);
-        const float2 dYx = sub2(Ypx, Ymx), dYy = sub2(Ypy, Ymy), dYz = sub2(Ypz, Ymz);
-        const float dZx = Zpx - Zmx, dZy = Zpy - Zmy, dZz = Zpz - Zmz;
-        const float d5x = -(dXx.x + dXx.y), d5y = -(dXy.x + dXy.y), d5z = -(dXz.x + dXz.y);  // zz
-        // M_ab = dQ_kl/da dQ_kl/db over all nine entries: xx, yy, zz once, off-diagonals twice
-        const float2 dYx2 = add2(dYx, dYx), dYy2 = add2(dYy, dYy), dYz2 = add2(dYz, dYz);
-        auto M = [&](float2 xa, float2 xb, float2 ya, float2 yb2, float za, float zb, float va, float vb) {
-            const float2 t = fma2(ya, yb2, mul2(xa, xb));
-            return fmaf(2.0f * za, zb, fmaf(va, vb, t.x + t.y));
-        };
-        float hxx = fmaf(P.l3m[0], M(dXx, dXx, dYx, dYx2, dZx, dZx, d5x, d5x), muX.x);
-        float hyy = fmaf(P.l3m[1], M(dXy, dXy, dYy, dYy2, dZy, dZy, d5y, d5y), muX.y);
-        float hz = fmaf(P.l3m[2], M(dXz, dXz, dYz, dYz2, dZz, dZz, d5z, d5z), -(muX.x + muX.y));
-        float hxy = fmaf(P.l3m[3], M(dXx, dXy, dYx, dYy2, dZx, dZy, d5x, d5y), muY.x);
-        float hxz = fmaf(P.l3m[4], M(dXx, dXz, dYx, dYz2, dZx, dZz, d5x, d5z), muY.y);
-        float hyz3 = fmaf(P.l3m[5], M(dXy, dXz, dYy, dYz2, dZy, dZz, d5y, d5z), muZ);
-        // column divergence at the centre: D_x = d_x Q_xx + d_y Q_xy + d_z Q_xz, ... (QSR.cu:325-371)
-        const float Dx = fmaf(P.i2x, dXx.x, fmaf(P.i2y, dYy.x, P.i2z * dYz.y));
-        const float Dy = fmaf(P.i2x, dYx.x, fmaf(P.i2y, dXy.y, P.i2z * dZz));
-        const float Dz = fmaf(P.i2x, dYx.y, fmaf(P.i2y, dZy, P.i2z * d5z));
-        // B(Q_c) = D . grad Q_c + Q_ab d_a d_b Q_c (QSR.cu:580-603) on all components at once:
-        // weights of the six second derivatives, shared by every component
-        const float Qzz = -q[0] - q[3];
-        const float2 wxx = bc2(q[0] * P.ix2), wyy = bc2(q[3] * P.iy2), wzz = bc2(Qzz * P.iz2);
-        const float2 wxy = bc2(2.0f * q[1] * P.i4xy), wxz = bc2(2.0f * q[2] * P.i4xz), wyz = bc2(2.0f * q[4] * P.i4yz);
-        const float2 Dc0 = bc2(Dx * P.i2x), Dc1 = bc2(Dy * P.i2y), Dc2 = bc2(Dz * P.i2z);
-        const float2 q2X = add2(qX, qX), q2Y = add2(qY, qY);
-        const float2 cX = fma2(wxx, sub2(sxX, q2X), fma2(wyy, sub2(syX, q2X), fma2(wzz, sub2(szX, q2X),
-                          fma2(wxy, mxyX, fma2(wxz, mxzX, mul2(wyz, myzX))))));
-        const float2 cY = fma2(wxx, sub2(sxY, q2Y), fma2(wyy, sub2(syY, q2Y), fma2(wzz, sub2(szY, q2Y),
-                          fma2(wxy, mxyY, fma2(wxz, mxzY, mul2(wyz, myzY))))));
-        const float q2Z = 2.0f * qZ;
-        const float cZ = fmaf(wxx.x, sxZ - q2Z, fmaf(wyy.x, syZ - q2Z, fmaf(wzz.x, szZ - q2Z,
-                         fmaf(wxy.x, mxyZ, fmaf(wxz.x, mxzZ, wyz.x * myzZ)))));
-        const float2 BX = fma2(Dc0, dXx, fma2(Dc1, dXy, fma2(Dc2, dXz, cX)));  // (B_xx, B_yy)
-        const float2 BY = fma2(Dc0, dYx, fma2(Dc1, dYy, fma2(Dc2, dYz, cY)));  // (B_xy, B_xz)
-        const float BZ = fmaf(Dc0.x, dZx, fmaf(Dc1.x, dZy, fmaf(Dc2.x, dZz, cZ)));  // B_yz
-        // h -= L3 B, B_zz = -(B_xx + B_yy); re-projected traceless (QSR.cu:611-619)
-        const float2 hdX = fma2(bc2(-P.L3), BX, make_float2(hxx, hyy));
-        const float2 hdY = fma2(bc2(-P.L3), BY, make_float2(hxy, hxz));
-        hz = fmaf(P.L3, BX.x + BX.y, hz);
-        hyz3 = fmaf(-P.L3, BZ, hyz3);
-        corr = (hdX.x + hdX.y + hz) * (1.0f / 3.0f);
-        muX = add2(hdX, bc2(-corr));
-        muY = hdY;
-        muZ = hyz3;
-    }
-    mu[0] = muX.x; mu[3] = muX.y; mu[1] = muY.x; mu[2] = muY.y; mu[4] = muZ;
-    if (anchor) {
-        float Q0[5];
-        surface_q0(P, i, j, k, Q0);
-#pragma unroll
-        for (int c = 0; c < 5; ++c) mu[c] += P.Weff * (q[c] - Q0[c]);
-    }
-}
-
-// ---------------------------------------------------------------------------------------
 // Two cells at once: F2 holds one value of two different cells, and every operation on it is
-// one packed instruction (FFMA2 / FADD2 / FMUL2) for both cells. chem_interior_pair is the
-// interior chemical potential of chem_potential_interior_x2 written on F2.
+// one packed instruction (FFMA2 / FADD2 / FMUL2) for both cells. The routines below are written
+// on a value type F, which is F2 (two cells) or float (one cell).
 // ---------------------------------------------------------------------------------------
 struct F2 {
     float2 v;
@@ -511,145 +354,269 @@ __device__ __forceinline__ F2 operator*(float s, F2 b) { return F2{__fmul2_rn(ma
 __device__ __forceinline__ F2 operator-(F2 a) { return F2{__fmul2_rn(a.v, make_float2(-1.0f, -1.0f))}; }
 __device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) { return F2{__ffma2_rn(a.v, b.v, c.v)}; }
 __device__ __forceinline__ F2 vfma(float a, F2 b, F2 c) { return F2{__ffma2_rn(make_float2(a, a), b.v, c.v)}; }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+template <class F>
+__device__ __forceinline__ F vset(float a);
+template <>
+__device__ __forceinline__ F2 vset<F2>(float a) { return mk2(a, a); }
+template <>
+__device__ __forceinline__ float vset<float>(float a) { return a; }
 
-__device__ __forceinline__ void bulk_field_pair(const F2 q[5], float cQ, float cQ2, float cQ3, F2 h[6]) {
-    const F2 Qxx = q[0], Qxy = q[1], Qxz = q[2], Qyy = q[3], Qyz = q[4];
-    const F2 Qzz = -(Qxx + Qyy);
-    const F2 trQ2 = vfma(Qxx, Qxx, vfma(Qyy, Qyy, Qzz * Qzz)) +
-                    2.0f * vfma(Qxy, Qxy, vfma(Qxz, Qxz, Qyz * Qyz));
-    const F2 q2xx = vfma(Qxx, Qxx, vfma(Qxy, Qxy, Qxz * Qxz));
-    const F2 q2xy = vfma(Qxx, Qxy, vfma(Qxy, Qyy, Qxz * Qyz));
-    const F2 q2xz = vfma(Qxx, Qxz, vfma(Qxy, Qyz, Qxz * Qzz));
-    const F2 q2yy = vfma(Qxy, Qxy, vfma(Qyy, Qyy, Qyz * Qyz));
-    const F2 q2yz = vfma(Qxy, Qxz, vfma(Qyy, Qyz, Qyz * Qzz));
-    const F2 q2zz = vfma(Qxz, Qxz, vfma(Qyz, Qyz, Qzz * Qzz));
-    const F2 t3 = (1.0f / 3.0f) * trQ2;
-    const F2 cg = vfma(cQ3, trQ2, mk2(cQ, cQ));
-    h[0] = vfma(-cQ2, q2xx - t3, cg * Qxx);
-    h[1] = vfma(-cQ2, q2yy - t3, cg * Qyy);
-    h[2] = vfma(-cQ2, q2zz - t3, cg * Qzz);
-    h[3] = vfma(-cQ2, q2xy, cg * Qxy);
-    h[4] = vfma(-cQ2, q2xz, cg * Qxz);
-    h[5] = vfma(-cQ2, q2yz, cg * Qyz);
+// Bulk molecular field of the five stored components (xx, xy, xz, yy, yz). It is traceless as
+// written (tr(Q^2 - I tr Q^2 / 3) = 0 and Qzz = -(Qxx + Qyy)), so the zz entry is never formed;
+// with Qzz eliminated the off-diagonal entries of Q^2 are two products each.
+template <class F>
+__device__ __forceinline__ void bulk_field5(const F q[5], float cQ, float cQ2, float cQ3, F h[5]) {
+    const F Qxx = q[0], Qxy = q[1], Qxz = q[2], Qyy = q[3], Qyz = q[4];
+    const F s = Qxx + Qyy;  // -Qzz
+    const F q2xx = vfma(Qxx, Qxx, vfma(Qxy, Qxy, Qxz * Qxz));
+    const F q2yy = vfma(Qyy, Qyy, vfma(Qxy, Qxy, Qyz * Qyz));
+    const F t = vfma(Qyz, Qyz, vfma(Qyy, s, q2xx));         // tr(Q^2) / 2
+    const F cg = vfma(2.0f * cQ3, t, vset<F>(cQ));          // cQ + cQ3 tr(Q^2)
+    const F c23 = (2.0f / 3.0f * cQ2) * t;                  // cQ2 tr(Q^2) / 3
+    h[0] = vfma(cg, Qxx, vfma(-cQ2, q2xx, c23));
+    h[3] = vfma(cg, Qyy, vfma(-cQ2, q2yy, c23));
+    h[1] = vfma(cg, Qxy, -cQ2 * vfma(Qxy, s, Qxz * Qyz));
+    h[2] = vfma(cg, Qxz, cQ2 * vfma(Qxz, Qyy, -(Qxy * Qyz)));
+    h[4] = vfma(cg, Qyz, cQ2 * vfma(Qyz, Qxx, -(Qxy * Qxz)));
 }
 
-// A(c, di, dj, dk) returns an F2 (component c of both cells at that offset; c = 5 is Qzz).
-// The terms are formed one stored component at a time (components 0 xx, 1 xy, 2 xz, 3 yy, 4 yz),
-// so that only the first differences of every component stay live for M_ab and the divergence:
-//  * its face neighbours give its Laplacian and first differences;
-//  * its four-corner and wide second differences go straight into the L2 term d_a D_b, which for
-//    an interior cell is sum_k S_ak(Q_kb) / (4 da dk) (wide second difference for k = a, four
-//    corners for k != a), and into its L3 contraction Q_ab d_a d_b Q_c;
-//  * h is projected traceless once at the end (the projection is linear, so projecting after the
-//    L1/L2 terms and again after L3, as QSR.cu:462-469 and 611-619 do, gives the same result).
-template <bool kL2, bool kL3, class Acc>
-__device__ __forceinline__ void chem_interior_pair(const Acc& A, const QsrConst& P, const F2 q[5], F2 mu[5],
-                                                   F2 lap[5]) {
-    F2 h[6];
-    bulk_field_pair(q, P.cQ, P.cQ2, P.cQ3, h);
+// What one component contributes to the stencil terms of a cell: undivided first differences
+// Q[+1] - Q[-1], sums Q[+1] + Q[-1] (interior) or whole second differences (face stencils), mixed
+// second differences of the four corners, and the L2 term's wide second differences, again as sums
+// Q[+2] + Q[-2] (interior) or whole (face stencils).
+template <class F>
+struct Sten {
+    F d[3], s[3], mxy, mxz, myz, wx, wy, wz;
+};
+
+// Chemical potential (bulk, L1, L2, L3) of one or two cells; S(c, o) fills the stencil of stored
+// component c (0 xx, 1 xy, 2 xz, 3 yy, 4 yz). The FMA pipe and the issue slots bound it, so it is
+// arranged to need few operations rather than to follow the reference term by term:
+//  * the L1 Laplacian and the L3 contraction Q_ab d_a d_b Q_c use the same second differences, so
+//    they share one weight per axis, Liso/da^2 + L3 Q_aa/da^2, formed once for all components;
+//  * bulk, L1 and L3 D.grad + contraction terms are traceless, so only the L2 term and the
+//    (L3/2) M_ab term (kept apart in ax, ay, az) need the traceless projection, and no zz entry
+//    of the others is formed (the reference projects after the L1/L2 terms and again after L3,
+//    QSR.cu:462-469 and 611-619; the projection is linear);
+//  * M_ab is summed over the five stored components: dQ_zz = -(dQ_xx + dQ_yy) turns the three
+//    diagonal products into two;
+//  * the centre terms -2 Q of the sums are collected per entry.
+// The L2 term d_a D_b is sum_k S_ak(Q_kb) / (4 da dk): the wide second difference for k = a, four
+// corners for k != a. With kFace the stencils hold the reference's one-sided forms (QSR.cu:245-371)
+// in the same undivided units and l3on is 0 for a cell on a face (no L3 term there, QSR.cu:474-621).
+// lap is formed for the IMEX right-hand side only.
+template <bool kL2, bool kL3, bool kLap, bool kFace, class F, class St>
+__device__ __forceinline__ void chem_core(const St& S, const QsrConst& P, const F q[5], F l3on, F mu[5], F lap[5]) {
+    F* h = mu;
+    bulk_field5<F>(q, P.cQ, P.cQ2, P.cQ3, h);
     const float cxx = P.l2w[0], cyy = P.l2w[1], czz = P.l2w[2], cxy = P.l2w[3], cxz = P.l2w[4], cyz = P.l2w[5];
-    // second-derivative weights of the L3 contraction, shared by every component
-    const F2 Qzz = -(q[0] + q[3]);
-    const F2 wxx = P.ix2 * q[0], wyy = P.iy2 * q[3], wzz = P.iz2 * Qzz;
-    const F2 wxy = (2.0f * P.i4xy) * q[1], wxz = (2.0f * P.i4xz) * q[2], wyz = (2.0f * P.i4yz) * q[4];
-    F2 d[5][3], contract[5];
+    F gx = vset<F>(P.lx), gy = vset<F>(P.ly), gz = vset<F>(P.lz);
+    F gxy{}, gxz{}, gyz{};
+    if (kL3) {
+        const F q0 = kFace ? l3on * q[0] : q[0], q3 = kFace ? l3on * q[3] : q[3];
+        gx = vfma(P.l3s[0], q0, gx);
+        gy = vfma(P.l3s[1], q3, gy);
+        gz = vfma(-P.l3s[2], q0 + q3, gz);
+        gxy = P.l3c[0] * q[1];
+        gxz = P.l3c[1] * q[2];
+        gyz = P.l3c[2] * q[4];
+        if (kFace) { gxy = l3on * gxy; gxz = l3on * gxz; gyz = l3on * gyz; }
+    }
+    F g0{};
+    if (!kFace) g0 = -2.0f * (gx + gy + gz);
+    F ax = vset<F>(0.0f), ay = ax, az = ax;  // xx, yy, zz entries that need the projection
+    if (kL2 && !kFace) {
+        ax = (2.0f * cxx) * q[0];
+        ay = (2.0f * cyy) * q[3];
+        az = (-2.0f * czz) * (q[0] + q[3]);
+        h[1] = vfma(2.0f * (cxx + cyy), q[1], h[1]);
+        h[2] = vfma(2.0f * (cxx + czz), q[2], h[2]);
+        h[4] = vfma(2.0f * (cyy + czz), q[4], h[4]);
+    }
+    F d[5][3];
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-        const F2 px = A(c, 1, 0, 0), mx = A(c, -1, 0, 0), py = A(c, 0, 1, 0), my = A(c, 0, -1, 0);
-        const F2 pz = A(c, 0, 0, 1), mz = A(c, 0, 0, -1);
-        const F2 sx = px + mx, sy = py + my, sz = pz + mz;
-        d[c][0] = px - mx;
-        d[c][1] = py - my;
-        d[c][2] = pz - mz;
-        lap[c] = vfma(P.ix2, sx, vfma(P.iy2, sy, vfma(P.iz2, sz, P.lap_c * q[c])));
-        // -Liso lap into h (h_zz takes -Liso lap_zz = Liso (lap_xx + lap_yy))
-        if (c == 0) { h[0] = vfma(-P.Liso, lap[c], h[0]); h[2] = vfma(P.Liso, lap[c], h[2]); }
-        if (c == 3) { h[1] = vfma(-P.Liso, lap[c], h[1]); h[2] = vfma(P.Liso, lap[c], h[2]); }
-        if (c == 1) h[3] = vfma(-P.Liso, lap[c], h[3]);
-        if (c == 2) h[4] = vfma(-P.Liso, lap[c], h[4]);
-        if (c == 4) h[5] = vfma(-P.Liso, lap[c], h[5]);
-        if (kL2 || kL3) {
-            const F2 mxy = (A(c, 1, 1, 0) - A(c, 1, -1, 0)) - (A(c, -1, 1, 0) - A(c, -1, -1, 0));
-            const F2 mxz = (A(c, 1, 0, 1) - A(c, 1, 0, -1)) - (A(c, -1, 0, 1) - A(c, -1, 0, -1));
-            const F2 myz = (A(c, 0, 1, 1) - A(c, 0, 1, -1)) - (A(c, 0, -1, 1) - A(c, 0, -1, -1));
-            if (kL2) {
-                const F2 q2 = 2.0f * q[c];
-                if (c == 0) {  // xx
-                    h[0] = vfma(-cxx, (A(0, 2, 0, 0) + A(0, -2, 0, 0)) - q2, h[0]);
-                    h[2] = vfma(czz, (A(0, 0, 0, 2) + A(0, 0, 0, -2)) - q2, h[2]);
-                    h[3] = vfma(-cxy, mxy, h[3]);
-                    h[5] = vfma(cyz, myz, h[5]);
-                } else if (c == 3) {  // yy
-                    h[1] = vfma(-cyy, (A(3, 0, 2, 0) + A(3, 0, -2, 0)) - q2, h[1]);
-                    h[2] = vfma(czz, (A(3, 0, 0, 2) + A(3, 0, 0, -2)) - q2, h[2]);
-                    h[3] = vfma(-cxy, mxy, h[3]);
-                    h[4] = vfma(cxz, mxz, h[4]);
-                } else if (c == 1) {  // xy
-                    h[0] = vfma(-cxy, mxy, h[0]);
-                    h[1] = vfma(-cxy, mxy, h[1]);
-                    h[3] = vfma(-cxx, (A(1, 2, 0, 0) + A(1, -2, 0, 0)) - q2, h[3]);
-                    h[3] = vfma(-cyy, (A(1, 0, 2, 0) + A(1, 0, -2, 0)) - q2, h[3]);
-                    h[4] = vfma(-cyz, myz, h[4]);
-                    h[5] = vfma(-cxz, mxz, h[5]);
-                } else if (c == 2) {  // xz
-                    h[0] = vfma(-cxz, mxz, h[0]);
-                    h[2] = vfma(-cxz, mxz, h[2]);
-                    h[3] = vfma(-cyz, myz, h[3]);
-                    h[4] = vfma(-cxx, (A(2, 2, 0, 0) + A(2, -2, 0, 0)) - q2, h[4]);
-                    h[4] = vfma(-czz, (A(2, 0, 0, 2) + A(2, 0, 0, -2)) - q2, h[4]);
-                    h[5] = vfma(-cxy, mxy, h[5]);
-                } else {  // yz
-                    h[1] = vfma(-cyz, myz, h[1]);
-                    h[2] = vfma(-cyz, myz, h[2]);
-                    h[3] = vfma(-cxz, mxz, h[3]);
-                    h[4] = vfma(-cxy, mxy, h[4]);
-                    h[5] = vfma(-cyy, (A(4, 0, 2, 0) + A(4, 0, -2, 0)) - q2, h[5]);
-                    h[5] = vfma(-czz, (A(4, 0, 0, 2) + A(4, 0, 0, -2)) - q2, h[5]);
-                }
-            }
-            if (kL3) {
-                const F2 q2 = 2.0f * q[c];
-                contract[c] = vfma(wxx, sx - q2, vfma(wyy, sy - q2, vfma(wzz, sz - q2,
-                              vfma(wxy, mxy, vfma(wxz, mxz, wyz * myz)))));
+        Sten<F> o;
+        S(c, o);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) d[c][a] = o.d[a];
+        F e = vfma(gx, o.s[0], vfma(gy, o.s[1], gz * o.s[2]));
+        if (!kFace) e = vfma(g0, q[c], e);
+        if (kLap) {
+            lap[c] = vfma(P.ix2, o.s[0], vfma(P.iy2, o.s[1], P.iz2 * o.s[2]));
+            if (!kFace) lap[c] = vfma(P.lap_c, q[c], lap[c]);
+        }
+        if (kL3) e = vfma(gxy, o.mxy, vfma(gxz, o.mxz, vfma(gyz, o.myz, e)));
+        if (kL2) {
+            if (c == 0) {  // xx
+                ax = vfma(-cxx, o.wx, ax);
+                az = vfma(czz, o.wz, az);
+                h[1] = vfma(-cxy, o.mxy, h[1]);
+                h[4] = vfma(cyz, o.myz, h[4]);
+            } else if (c == 3) {  // yy
+                ay = vfma(-cyy, o.wy, ay);
+                az = vfma(czz, o.wz, az);
+                h[1] = vfma(-cxy, o.mxy, h[1]);
+                h[2] = vfma(cxz, o.mxz, h[2]);
+            } else if (c == 1) {  // xy
+                ax = vfma(-cxy, o.mxy, ax);
+                ay = vfma(-cxy, o.mxy, ay);
+                h[1] = vfma(-cxx, o.wx, vfma(-cyy, o.wy, h[1]));
+                h[2] = vfma(-cyz, o.myz, h[2]);
+                h[4] = vfma(-cxz, o.mxz, h[4]);
+            } else if (c == 2) {  // xz
+                ax = vfma(-cxz, o.mxz, ax);
+                az = vfma(-cxz, o.mxz, az);
+                h[1] = vfma(-cyz, o.myz, h[1]);
+                h[2] = vfma(-cxx, o.wx, vfma(-czz, o.wz, h[2]));
+                h[4] = vfma(-cxy, o.mxy, h[4]);
+            } else {  // yz
+                ay = vfma(-cyz, o.myz, ay);
+                az = vfma(-cyz, o.myz, az);
+                h[1] = vfma(-cxz, o.mxz, h[1]);
+                h[2] = vfma(-cxy, o.mxy, h[2]);
+                h[4] = vfma(-cyy, o.wy, vfma(-czz, o.wz, h[4]));
             }
         }
+        h[c] = h[c] - e;
     }
     if (kL3) {
-        F2 d5[3];
+        // the face form drops the whole term through its first differences (each term has two)
+        if (kFace) {
 #pragma unroll
-        for (int a = 0; a < 3; ++a) d5[a] = -(d[0][a] + d[3][a]);
-        auto M = [&](int a, int b) {
-            const F2 diag = vfma(d[0][a], d[0][b], vfma(d[3][a], d[3][b], d5[a] * d5[b]));
-            const F2 off = vfma(d[1][a], d[1][b], vfma(d[2][a], d[2][b], d[4][a] * d[4][b]));
-            return vfma(2.0f, off, diag);
+            for (int c = 0; c < 5; ++c)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) d[c][a] = l3on * d[c][a];
+        }
+        // (L3/2) M_ab, M_ab = dQ_kl/da dQ_kl/db over all nine entries
+        F ex[3], ey[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            ex[a] = vfma(0.5f, d[3][a], d[0][a]);
+            ey[a] = vfma(0.5f, d[0][a], d[3][a]);
+        }
+        auto M = [&](int a, int b) {  // M_ab / 2 (undivided)
+            return vfma(d[0][a], ex[b], vfma(d[3][a], ey[b], vfma(d[1][a], d[1][b], vfma(d[2][a], d[2][b],
+                        d[4][a] * d[4][b]))));
         };
-        // (L3 / 2) M_ab: h_zz first, as -(hx_xx + hx_yy) of the projected field gets it below
-        h[0] = vfma(P.l3m[0], M(0, 0), h[0]);
-        h[1] = vfma(P.l3m[1], M(1, 1), h[1]);
-        h[2] = vfma(P.l3m[2], M(2, 2), h[2]);
-        h[3] = vfma(P.l3m[3], M(0, 1), h[3]);
-        h[4] = vfma(P.l3m[4], M(0, 2), h[4]);
-        h[5] = vfma(P.l3m[5], M(1, 2), h[5]);
-        // centre divergence D_x = d_x Q_xx + d_y Q_xy + d_z Q_xz, ... (QSR.cu:325-371), times 1/(2 da)
-        const F2 Dc0 = P.i2x * vfma(P.i2x, d[0][0], vfma(P.i2y, d[1][1], P.i2z * d[2][2]));
-        const F2 Dc1 = P.i2y * vfma(P.i2x, d[1][0], vfma(P.i2y, d[3][1], P.i2z * d[4][2]));
-        const F2 Dc2 = P.i2z * vfma(P.i2x, d[2][0], vfma(P.i2y, d[4][1], P.i2z * d5[2]));
-        F2 B[5];
+        ax = vfma(P.l3d[0], M(0, 0), ax);
+        ay = vfma(P.l3d[1], M(1, 1), ay);
+        az = vfma(P.l3d[2], M(2, 2), az);
+        h[1] = vfma(P.l3d[3], M(0, 1), h[1]);
+        h[2] = vfma(P.l3d[4], M(0, 2), h[2]);
+        h[4] = vfma(P.l3d[5], M(1, 2), h[4]);
+        // -L3 D_a / (2 da) with the centre divergence D_x = d_x Q_xx + d_y Q_xy + d_z Q_xz, ... (QSR.cu:325-371)
+        const F Dx = vfma(-P.l3d[0], d[0][0], vfma(-P.l3d[3], d[1][1], -P.l3d[4] * d[2][2]));
+        const F Dy = vfma(-P.l3d[3], d[1][0], vfma(-P.l3d[1], d[3][1], -P.l3d[5] * d[4][2]));
+        const F Dz = vfma(-P.l3d[4], d[2][0], vfma(-P.l3d[5], d[4][1], P.l3d[2] * (d[0][2] + d[3][2])));
 #pragma unroll
-        for (int c = 0; c < 5; ++c) B[c] = vfma(Dc0, d[c][0], vfma(Dc1, d[c][1], vfma(Dc2, d[c][2], contract[c])));
-        h[0] = vfma(-P.L3, B[0], h[0]);
-        h[1] = vfma(-P.L3, B[3], h[1]);
-        h[2] = vfma(P.L3, B[0] + B[3], h[2]);  // - L3 B_zz, B_zz = -(B_xx + B_yy)
-        h[3] = vfma(-P.L3, B[1], h[3]);
-        h[4] = vfma(-P.L3, B[2], h[4]);
-        h[5] = vfma(-P.L3, B[4], h[5]);
+        for (int c = 0; c < 5; ++c) h[c] = vfma(Dx, d[c][0], vfma(Dy, d[c][1], vfma(Dz, d[c][2], h[c])));
     }
-    const F2 corr = (1.0f / 3.0f) * (h[0] + h[1] + h[2]);
-    mu[0] = h[0] - corr;
-    mu[1] = h[3];
-    mu[2] = h[4];
-    mu[3] = h[1] - corr;
-    mu[4] = h[5];
+    if (kL2 || kL3) {
+        const F corr = (1.0f / 3.0f) * (ax + ay + az);
+        h[0] = h[0] + (ax - corr);
+        h[3] = h[3] + (ay - corr);
+    }
+}
+
+// Interior stencil of two cells, rows j and j + 1 of one column. V(c, di, dj, dk) returns component
+// c at that offset from row j (so dj runs over -2 .. 3). Differences along j are formed per row: the
+// two rows overlap (row j is a neighbour of row j + 1), and a packed operand would have to be
+// assembled from them with register moves.
+template <bool kL2, bool kL3, class Val>
+struct InteriorPair {
+    const Val& V;
+    __device__ __forceinline__ void operator()(int c, Sten<F2>& o) const {
+        auto pair = [&](int di, int dk) { return mk2(V(c, di, 0, dk), V(c, di, 1, dk)); };
+        auto dj = [&](int di, int dk) {  // Q(j + 1) - Q(j - 1) of both rows
+            return mk2(V(c, di, 1, dk) - V(c, di, -1, dk), V(c, di, 2, dk) - V(c, di, 0, dk));
+        };
+        const F2 px = pair(1, 0), mx = pair(-1, 0), pz = pair(0, 1), mz = pair(0, -1);
+        o.s[0] = px + mx;
+        o.s[1] = mk2(V(c, 0, 1, 0) + V(c, 0, -1, 0), V(c, 0, 2, 0) + V(c, 0, 0, 0));
+        o.s[2] = pz + mz;
+        o.d[0] = px - mx;
+        o.d[1] = dj(0, 0);
+        o.d[2] = pz - mz;
+        if (kL2 || kL3) {
+            o.mxy = dj(1, 0) - dj(-1, 0);
+            o.mxz = (pair(1, 1) - pair(1, -1)) - (pair(-1, 1) - pair(-1, -1));
+            o.myz = dj(0, 1) - dj(0, -1);
+        }
+        if (kL2) {
+            if (c == 0 || c == 1 || c == 2) o.wx = pair(2, 0) + pair(-2, 0);
+            if (c == 1 || c == 3 || c == 4)
+                o.wy = mk2(V(c, 0, 2, 0) + V(c, 0, -2, 0), V(c, 0, 3, 0) + V(c, 0, -1, 0));
+            if (c != 1) o.wz = pair(0, 2) + pair(0, -2);
+        }
+    }
+};
+
+// The reference's stencils next to a grid face along one axis, as offsets from a cell at position
+// `pos` of n: first differences are one-sided at the faces (QSR.cu:245-273), which is the central
+// form with its neighbours clamped to the grid and twice the weight (r, relative to 1/(2 d)); second
+// differences are the inner neighbour's (QSR.cu:296-320); the derivative of the divergence takes
+// the clamped first difference of clamped first differences.
+struct FaceAxis {
+    int hi, lo, s;           // clamped neighbours; shift of the second difference's centre
+    int hh, hl, lh, ll;      // the clamped neighbours' own neighbours
+    float r, rh, rl;         // weights of the first differences at the cell and at its neighbours
+    __device__ __forceinline__ FaceAxis(int pos, int n) {
+        const int h = min(pos + 1, n - 1), l = max(pos - 1, 0);
+        hi = h - pos;
+        lo = l - pos;
+        s = min(max(pos, 1), n - 2) - pos;
+        hh = min(h + 1, n - 1) - pos;
+        hl = max(h - 1, 0) - pos;
+        lh = min(l + 1, n - 1) - pos;
+        ll = max(l - 1, 0) - pos;
+        r = (pos == 0 || pos == n - 1) ? 2.0f : 1.0f;
+        rh = (h == n - 1) ? 2.0f : 1.0f;
+        rl = (l == 0) ? 2.0f : 1.0f;
+    }
+};
+
+// Stencil of one cell of the grid with the face forms along every axis (equal to the interior one
+// away from the faces). V(c, di, dj, dk) takes runtime offsets.
+template <bool kL2, bool kL3, class Val>
+struct FaceOne {
+    const Val& V;
+    const FaceAxis &x, &y, &z;
+    __device__ __forceinline__ void operator()(int c, Sten<float>& o) const {
+        o.d[0] = V(c, x.hi, 0, 0) - V(c, x.lo, 0, 0);
+        o.d[1] = V(c, 0, y.hi, 0) - V(c, 0, y.lo, 0);
+        o.d[2] = V(c, 0, 0, z.hi) - V(c, 0, 0, z.lo);
+        o.s[0] = (V(c, x.s + 1, 0, 0) + V(c, x.s - 1, 0, 0)) - 2.0f * V(c, x.s, 0, 0);
+        o.s[1] = (V(c, 0, y.s + 1, 0) + V(c, 0, y.s - 1, 0)) - 2.0f * V(c, 0, y.s, 0);
+        o.s[2] = (V(c, 0, 0, z.s + 1) + V(c, 0, 0, z.s - 1)) - 2.0f * V(c, 0, 0, z.s);
+        if (kL2 || kL3) {
+            o.mxy = (x.r * y.r) * ((V(c, x.hi, y.hi, 0) - V(c, x.hi, y.lo, 0)) - (V(c, x.lo, y.hi, 0) - V(c, x.lo, y.lo, 0)));
+            o.mxz = (x.r * z.r) * ((V(c, x.hi, 0, z.hi) - V(c, x.hi, 0, z.lo)) - (V(c, x.lo, 0, z.hi) - V(c, x.lo, 0, z.lo)));
+            o.myz = (y.r * z.r) * ((V(c, 0, y.hi, z.hi) - V(c, 0, y.hi, z.lo)) - (V(c, 0, y.lo, z.hi) - V(c, 0, y.lo, z.lo)));
+        }
+        if (kL2) {
+            if (c == 0 || c == 1 || c == 2)
+                o.wx = x.r * (x.rh * (V(c, x.hh, 0, 0) - V(c, x.hl, 0, 0)) - x.rl * (V(c, x.lh, 0, 0) - V(c, x.ll, 0, 0)));
+            if (c == 1 || c == 3 || c == 4)
+                o.wy = y.r * (y.rh * (V(c, 0, y.hh, 0) - V(c, 0, y.hl, 0)) - y.rl * (V(c, 0, y.lh, 0) - V(c, 0, y.ll, 0)));
+            if (c != 1)
+                o.wz = z.r * (z.rh * (V(c, 0, 0, z.hh) - V(c, 0, 0, z.hl)) - z.rl * (V(c, 0, 0, z.lh) - V(c, 0, 0, z.ll)));
+        }
+    }
+};
+
+// Frobenius-norm cap of the explicit update (QSR.cu:719-731).
+__device__ __forceinline__ void cap_norm(float qcap, float out[5]) {
+    const float zz = -out[0] - out[3];
+    const float tr = out[0] * out[0] + out[3] * out[3] + zz * zz +
+                     2.0f * (out[1] * out[1] + out[2] * out[2] + out[4] * out[4]);
+    const float qn = sqrtf(tr > 0.0f ? tr : 0.0f);
+    if (qn > qcap && qn > 0.0f) {
+        const float s = qcap / qn;
+#pragma unroll
+        for (int c = 0; c < 5; ++c) out[c] *= s;
+    }
 }
 
 // Explicit update with compensated storage: a cell holds hi + lo (two FP32 words). The
@@ -701,17 +668,7 @@ __device__ __forceinline__ void euler_update(const QsrConst& P, const float q[5]
 #pragma unroll
         for (int c = 0; c < 5; ++c) out[c] += P.sigma * g[c];
     }
-    if (P.qcap > 0.0f) {
-        const float zz = -out[0] - out[3];
-        const float tr = out[0] * out[0] + out[3] * out[3] + zz * zz +
-                         2.0f * (out[1] * out[1] + out[2] * out[2] + out[4] * out[4]);
-        const float qn = sqrtf(tr > 0.0f ? tr : 0.0f);
-        if (qn > P.qcap && qn > 0.0f) {
-            const float s = P.qcap / qn;
-#pragma unroll
-            for (int c = 0; c < 5; ++c) out[c] *= s;
-        }
-    }
+    if (P.qcap > 0.0f) cap_norm(P.qcap, out);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -748,6 +705,13 @@ __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, 
     if (nz < -1e-10) { r.nx = -nx; r.ny = -ny; r.nz = -nz; }
     return r;
 }
+
+// Programmatic dependent launch (launch_pdl): a kernel is put on the SMs while its predecessor in the
+// stream drains, sets itself up, and waits in pdl_wait until the predecessor's writes are complete;
+// pdl_trigger then lets its own successor be put in place. Every access to data that an earlier
+// kernel writes comes after pdl_wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Warp and block reductions (fixed order: deterministic for a fixed launch shape).
 __device__ __forceinline__ double warp_sum(double v) {

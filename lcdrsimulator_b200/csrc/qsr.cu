@@ -684,6 +684,11 @@ QsrConst make_const(const qsr_handle* h, double T, double S_shell, double dt) {
     const int ab[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {0, 2}, {1, 2}};
     for (int m = 0; m < 6; ++m) P.l3m[m] = (float)(0.5 * p.L3 * i2[ab[m][0]] * i2[ab[m][1]]);
     for (int m = 0; m < 6; ++m) P.l2w[m] = (float)(p.L2 * i2[ab[m][0]] * i2[ab[m][1]]);
+    const double Liso = all_zero ? p.kappa : p.L1;
+    P.lx = (float)(Liso * ix2); P.ly = (float)(Liso * iy2); P.lz = (float)(Liso * iz2);
+    P.l3s[0] = (float)(p.L3 * ix2); P.l3s[1] = (float)(p.L3 * iy2); P.l3s[2] = (float)(p.L3 * iz2);
+    for (int m = 0; m < 3; ++m) P.l3c[m] = (float)(2.0 * p.L3 * i2[ab[3 + m][0]] * i2[ab[3 + m][1]]);
+    for (int m = 0; m < 6; ++m) P.l3d[m] = (float)(p.L3 * i2[ab[m][0]] * i2[ab[m][1]]);
     return P;
 }
 
@@ -922,7 +927,8 @@ int qsr_create(const qsr_params* params, qsr_handle** out) {
         qsr_destroy(h);
         return LDG_ERR_CUDA;
     }
-    rc = tiled_plan_build(h->tiled, p.Nx, p.Ny, p.Nz, h->sj, h->si, fl.data(), h->q[0], h->q[1], h->sc);
+    rc = tiled_plan_build(h->tiled, p.Nx, p.Ny, p.Nz, h->sj, h->si, fl.data(), h->flags, h->q[0], h->q[1],
+                          h->sc, p.L2 != 0.0, p.L3 != 0.0);
     if (rc != LDG_OK) {
         qsr_destroy(h);
         return rc;
@@ -1097,7 +1103,7 @@ int qsr_step(qsr_handle* h, int n_steps, const qsr_step_args* a) {
         float* outb = h->q[1 - h->cur];
         if (!imex) {
             if (choice == 1 && h->tiled.ok) {
-                int rc = tiled_step(h->tiled, in, outb, h->flags, P, L2, L3, noise, false, h->stream, h->lo[h->cur],
+                int rc = tiled_step(h->tiled, in, outb, P, L2, L3, noise, false, h->stream, h->lo[h->cur],
                                     h->lo[1 - h->cur]);
                 if (rc) return rc;
             } else {
@@ -1108,7 +1114,7 @@ int qsr_step(qsr_handle* h, int n_steps, const qsr_step_args* a) {
             h->cur = 1 - h->cur;
         } else {
             if (choice == 1 && h->tiled.ok) {
-                int rc = tiled_step(h->tiled, in, h->rhs, h->flags, P, L2, L3, noise, true, h->stream);
+                int rc = tiled_step(h->tiled, in, h->rhs, P, L2, L3, noise, true, h->stream);
                 if (rc) return rc;
             } else {
                 dispatch_direct<true>(h, in, h->rhs, P, L2, L3, noise);
@@ -1270,7 +1276,8 @@ struct ens_handle {
     std::vector<tiled::EnsInstDev> host_inst;
     CUtensorMap* d_tms = nullptr;          // 2 per instance: input buffer q[0] / q[1]
     tiled::EnsInstDev* d_inst = nullptr;
-    tiled::EnsItem* d_items = nullptr;
+    tiled::TileItem* d_items = nullptr;
+    tiled::RowMask* d_masks = nullptr;
     int n_items = 0;
     tiled::EnsCtl* d_ctl = nullptr;
     int* d_err = nullptr;
@@ -1290,30 +1297,23 @@ namespace {
 
 constexpr int kEnsGraphSteps = 32;
 
-using EnsKernel = void (*)(const CUtensorMap*, const tiled::EnsInstDev*, const tiled::EnsItem*, int, tiled::EnsCtl*,
-                           int*);
+using EnsKernel = void (*)(const CUtensorMap*, const tiled::EnsInstDev*, const tiled::TileItem*,
+                           const tiled::RowMask*, int, tiled::EnsCtl*, int*);
 
-template <bool kPair>
-EnsKernel ens_kernel_t(bool L2, bool L3, bool N) {
+EnsKernel ens_kernel(bool L2, bool L3, bool N) {
     using namespace tiled;
     const int key = (L2 ? 1 : 0) | (L3 ? 2 : 0) | (N ? 4 : 0);
     switch (key) {
-        case 0: return k_step_ensemble<false, false, false, kPair>;
-        case 1: return k_step_ensemble<true, false, false, kPair>;
-        case 2: return k_step_ensemble<false, true, false, kPair>;
-        case 3: return k_step_ensemble<true, true, false, kPair>;
-        case 4: return k_step_ensemble<false, false, true, kPair>;
-        case 5: return k_step_ensemble<true, false, true, kPair>;
-        case 6: return k_step_ensemble<false, true, true, kPair>;
-        default: return k_step_ensemble<true, true, true, kPair>;
+        case 0: return k_step_ensemble<false, false, false>;
+        case 1: return k_step_ensemble<true, false, false>;
+        case 2: return k_step_ensemble<false, true, false>;
+        case 3: return k_step_ensemble<true, true, false>;
+        case 4: return k_step_ensemble<false, false, true>;
+        case 5: return k_step_ensemble<true, false, true>;
+        case 6: return k_step_ensemble<false, true, true>;
+        default: return k_step_ensemble<true, true, true>;
     }
 }
-
-// The ensemble runs the two-cell routine unless LDG_QSR_PAIR=0.
-EnsKernel ens_kernel(bool L2, bool L3, bool N) {
-    return tiled_pair_enabled() ? ens_kernel_t<true>(L2, L3, N) : ens_kernel_t<false>(L2, L3, N);
-}
-int ens_threads() { return tiled_pair_enabled() ? tiled::PAIR_THREADS : tiled::THREADS; }
 
 void ens_drop_graph(ens_handle* h) {
     if (h->graph) cudaGraphExecDestroy(h->graph);
@@ -1323,23 +1323,38 @@ void ens_drop_graph(ens_handle* h) {
 
 // Work list of all instances split into chunks of `chunk` planes (instance-major, so CTAs that
 // run together share halo planes of one droplet in L2), and the persistent grid size.
-int ens_rechunk(ens_handle* h, int chunk) {
-    std::vector<tiled::EnsItem> items;
+int ens_rechunk(ens_handle* h, int cap) {
+    std::vector<const TiledPlan*> plans;
+    for (const qsr_handle* q : h->inst) plans.push_back(&q->tiled);
+    const int chunk = tiled_length(plans, cap, h->L2 || h->L3);
+    std::vector<tiled::TileItem> items;
+    std::vector<int> first;   // first item of every instance
     long long active = 0;
+    int recs = 0;
     for (size_t n = 0; n < h->inst.size(); ++n) {
         long long a = 0;
-        for (const int4& t : tiled_items(h->inst[n]->tiled, chunk, &a))
-            items.push_back(tiled::EnsItem{t.x, t.y, t.z, t.w, (int)n, 0, 0, 0});
+        int nr = 0;
+        first.push_back((int)items.size());
+        tiled_device_items(tiled_items(h->inst[n]->tiled, chunk, &a), (int)n, recs, items, &nr);
+        recs += nr;
         active += a;
     }
+    first.push_back((int)items.size());
     h->active = active;
     if (h->d_items) cudaFree(h->d_items);
+    if (h->d_masks) cudaFree(h->d_masks);
     h->d_items = nullptr;
+    h->d_masks = nullptr;
     h->n_items = (int)items.size();
     if (h->n_items > 0) {
-        int rc = alloc_or_fail((void**)&h->d_items, items.size() * sizeof(tiled::EnsItem));
+        int rc = alloc_or_fail((void**)&h->d_items, items.size() * sizeof(items[0]));
+        if (!rc) rc = alloc_or_fail((void**)&h->d_masks, (size_t)recs * tiled::MASK_BYTES);
         if (rc) return rc;
-        LDG_CUDA(cudaMemcpy(h->d_items, items.data(), items.size() * sizeof(tiled::EnsItem), cudaMemcpyHostToDevice));
+        LDG_CUDA(cudaMemcpy(h->d_items, items.data(), items.size() * sizeof(items[0]), cudaMemcpyHostToDevice));
+        for (size_t n = 0; n < h->inst.size(); ++n)
+            if ((rc = tiled_masks(h->inst[n]->tiled, h->d_items + first[n], first[n + 1] - first[n], h->L2, h->d_masks)))
+                return rc;
+        LDG_CUDA(cudaStreamSynchronize(nullptr));
     }
     h->chunk = chunk;
     const EnsKernel k = ens_kernel(h->L2, h->L3, h->noise);
@@ -1347,7 +1362,7 @@ int ens_rechunk(ens_handle* h, int chunk) {
     int dev = 0, sms = 0, per_sm = 0;
     LDG_CUDA(cudaGetDevice(&dev));
     LDG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    LDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, ens_threads(), h->smem));
+    LDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tiled::THREADS, h->smem));
     LDG_REQUIRE(per_sm > 0, LDG_ERR_CUDA, "ensemble: step kernel does not fit on an SM");
     h->grid = std::max(1, std::min(sms * per_sm, h->n_items));
     ens_drop_graph(h);
@@ -1356,9 +1371,8 @@ int ens_rechunk(ens_handle* h, int chunk) {
 
 int ens_launch(ens_handle* h) {
     const EnsKernel k = ens_kernel(h->L2, h->L3, h->noise);
-    k<<<h->grid, ens_threads(), h->smem, h->stream>>>(h->d_tms, h->d_inst, h->d_items, h->n_items, h->d_ctl,
-                                                      h->d_err);
-    LDG_LAUNCHED("k_step_ensemble");
+    LDG_CUDA(launch_pdl(k, dim3((unsigned)h->grid), tiled::THREADS, h->smem, h->stream, h->d_tms, h->d_inst, h->d_items, h->d_masks,
+                        h->n_items, h->d_ctl, h->d_err));
     return LDG_OK;
 }
 
@@ -1529,23 +1543,27 @@ int ens_create(const ens_params* params, int n_instances, const ens_instance* in
         D.P.instance = 0;
         D.q[0] = qh->q[0];
         D.q[1] = qh->q[1];
-        D.flags = qh->flags;
         D.T_high = d.T_high; D.T_low = d.T_low;
         D.pre = d.pre_equil_iters; D.ramp = d.ramp_iters;
         D.protocol = p.protocol;
         D.custom_shell = p.boundary_custom ? 1 : 0;
         D.S_custom = p.boundary_S;
         D.a3 = a3; D.T_star = p.T_star; D.B = B; D.C = Cc;
-        tms[2 * n] = qh->tiled.tmap[0];
-        tms[2 * n + 1] = qh->tiled.tmap[1];
+        // the ensemble's kernel reads every droplet with the same halo
+        for (int b = 0; b < 2 && rc == LDG_OK; ++b)
+            rc = tiled_encode(&tms[2 * n + b], qh->q[b], qh->p.Nx, qh->p.Ny, qh->p.Nz, qh->sj, qh->si, qh->sc, h->L2);
         h->cells += qh->ncells;
         h->active += qh->active_cells;
         h->written += qh->written_cells;
     }
     using namespace tiled;
-    h->smem = tiled_pair_enabled() ? h->inst[0]->tiled.smem_bytes[2]
-              : (h->L2 || h->L3)   ? h->inst[0]->tiled.smem_bytes[1]
-                                   : h->inst[0]->tiled.smem_bytes[0];
+    if (rc != LDG_OK) {
+        const std::string msg = ldg_last_error();
+        ens_destroy(h);
+        set_error(msg);
+        return rc;
+    }
+    h->smem = h->L2 ? tile_smem_bytes<true>() : tile_smem_bytes<false>();
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if ((rc = alloc_or_fail((void**)&h->d_tms, tms.size() * sizeof(CUtensorMap))) ||
         (rc = alloc_or_fail((void**)&h->d_inst, h->host_inst.size() * sizeof(EnsInstDev))) ||
@@ -1799,7 +1817,7 @@ int ens_destroy(ens_handle* h) {
     for (qsr_handle* q : h->inst) qsr_destroy(q);
     cudaFree(h->stage);
     if (h->obs_host) cudaFreeHost(h->obs_host);
-    cudaFree(h->d_tms); cudaFree(h->d_inst); cudaFree(h->d_items); cudaFree(h->d_ctl); cudaFree(h->d_err);
+    cudaFree(h->d_tms); cudaFree(h->d_inst); cudaFree(h->d_items); cudaFree(h->d_masks); cudaFree(h->d_ctl); cudaFree(h->d_err);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return LDG_OK;

@@ -2,22 +2,29 @@
 //
 // A CTA owns a (TJ x TK) column tile of the (j, k) plane and marches along i over a chunk
 // of planes. Each plane of the input field arrives in shared memory through one TMA load
-// of a 4-D box (k, j, i, component) covering the tile plus a halo of 2 rows and 4 columns
-// (the k start stays on a 16-byte boundary), so every Q value is read from HBM about once.
-// The ring holds the planes i-2 .. i+2 that the cells of plane i read, plus planes in flight.
-// Interior cells read only Q: the L2 term's derivatives of the column divergence are
-// evaluated from Q directly (wide and four-corner second differences, which for an interior
-// cell equal the reference's central differences of its central divergence), so no divergence
-// field is staged and the warps share nothing but the plane ring. Each warp (one tile row)
+// of a 4-D box (k, j, i, component) covering the tile plus its halo (the k start stays on a 16-byte
+// boundary), so every Q value is read from HBM about once. The ring holds the planes that the cells
+// of plane i read, plus planes in flight. Interior cells read only Q: the L2 term's derivatives of
+// the column divergence are evaluated from Q directly (wide and four-corner second differences,
+// which for an interior cell equal the reference's central differences of its central divergence),
+// so no divergence field is staged and the warps share nothing but the plane ring. Each warp
 // therefore marches on its own: it waits only for the TMA of the planes it reads, and when it
 // is done with a plane it arrives on that slot's counter; the warp whose arrival completes the
 // count issues the load of the plane that reuses the slot. There is no CTA barrier per plane.
-// Cells next to a grid face take the reference's face stencils with the divergence evaluated on
-// the fly. Per cell the kernel evaluates the chemical potential and the update from shared memory
-// and writes only the cells that change (moving and strongly anchored cells): frozen exterior
-// cells hold identical values in both ping-pong buffers. Tiles that contain no changing cell are
-// never visited (host-built work list). The same per-tile routine drives a persistent,
-// work-stealing ensemble kernel over many droplets.
+// Rows with cells next to a grid face take the reference's face stencils in the same undivided
+// form with neighbours clamped to the grid. Per cell the kernel evaluates the chemical potential and
+// the update from shared memory and writes only the cells that change (moving and strongly anchored
+// cells): frozen exterior cells hold identical values in both ping-pong buffers. Tiles that contain
+// no changing cell are never visited (host-built work list). The same per-tile routine drives a
+// persistent, work-stealing ensemble kernel over many droplets.
+//
+// What bounds it. With L2 and L3 the issue slots and the FMA pipe: 418 instructions per visited
+// cell at 65 % issue efficiency, 184 of them on the FMA pipe. L1 only: the loads and stores (a 256^3
+// step with its arithmetic left out takes 87 of 89 us). A grid of few tiles: the serial march of one
+// item (about 1 us per plane), hence tiled_length, and the launch gap, hence the programmatic
+// dependent launches (2 us a step). Per step, one work-list length for all before -> now, 256^3 with
+// all terms 168 -> 142 us, 64^3 L1 only 16.4 -> 4.7 us, 32^3 15.3 -> 4.1 us, 101 x 90 x 117 touching
+// its faces with all terms 68 -> 21 us.
 //
 // mbarrier waits are bounded: on timeout the kernel records LDG_ERR_TIMEOUT in a device
 // word, waits (bounded) for its own TMA loads and returns.
@@ -30,7 +37,9 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdint>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -42,30 +51,53 @@ namespace ldg {
 namespace tiled {
 
 constexpr int TK = 32;               // tile width along k (one warp per row)
-constexpr int TJ = 8;                // tile rows along j (one warp each)
-constexpr int THREADS = TK * TJ;
+constexpr int TJ = 8;                // tile rows along j
+constexpr int THREADS = TK * TJ / 2;  // two cells per thread: rows 2w and 2w + 1 of warp w
 constexpr int NWARP = THREADS / 32;
-// Halo rows / columns loaded with each plane: the stencils reach two cells out. The TMA box
-// starts at column k0 - HK, which must be a multiple of 4 floats (16 bytes), so tiles start at
-// k0 = 2 (mod 4) (the first may start at k0 = -2: its two columns outside the grid are zero
-// fill and compute nothing).
-constexpr int HJ = 2, HK = 2;
+// Halo columns loaded with each plane: the TMA box starts at column k0 - HK, which must be a
+// multiple of 4 floats (16 bytes), so tiles start at k0 = 2 (mod 4) (the first may start at
+// k0 = -2: its two columns outside the grid are zero fill and compute nothing).
+constexpr int HK = 2;
 constexpr int RW = TK + 2 * HK;      // 36 floats per smem row
-constexpr int ROWS = TJ + 2 * HJ;    // 12 rows
-constexpr int CSTR = RW * ROWS;      // floats per component plane
-constexpr int PLANE = 5 * CSTR;      // floats per plane (all components)
-constexpr int SLOT = (PLANE + 31) / 32 * 32;  // floats per ring slot (TMA destinations 128-byte aligned)
-constexpr int LOOK = 2;              // the cells of plane i read planes i-2 .. i+2
-// Q ring slots: planes i-2 .. i+2 are read at plane i, the rest are in flight. The L1-only step
-// runs three CTAs (24 warps) per SM: 7 slots (~67 KB) and at most 80 registers a thread. The
-// L2/L3 steps need more registers (the mixed and wide second differences) and run two CTAs per
-// SM with 9 slots (~86 KB, four planes in flight).
-// (two cells per thread: 128-thread CTAs, four per SM, 6 slots ~ 52 KB)
-template <bool kD, bool kPair = false>
-__host__ __device__ constexpr int nq() { return kPair ? 6 : (kD ? 9 : 7); }
-constexpr uint32_t PLANE_BYTES = PLANE * 4;
-constexpr int CHUNK = 16;            // planes per work item (default; tunable)
-constexpr unsigned long long WAIT_NS = 2000000000ull;  // 2 s per wait
+
+// What a step with / without the L2 term keeps in shared memory. The L2 term reads two cells out
+// (wide second differences): two halo rows and the planes i-2 .. i+2. Without it the stencil reaches
+// one cell: one halo row and the planes i-1 .. i+1, so the same ring has three planes in flight
+// instead of one, and a plane is 7.2 instead of 8.6 KB (five 128-thread CTAs per SM instead of
+// four): 256^3, R = 115, L1 only 95 -> 88 us a step, 128^3 17 -> 15 us.
+template <bool kL2>
+struct Tile {
+    static constexpr int H = kL2 ? 2 : 1;             // halo rows and planes read on each side
+    static constexpr int ROWS = TJ + 2 * H;
+    static constexpr int CSTR = RW * ROWS;            // floats per component plane
+    static constexpr int PLANE = 5 * CSTR;            // floats per plane (all components)
+    // floats per ring slot: the plane, then its row masks; 128-byte aligned
+    static constexpr int SLOT = (PLANE + 4 * TJ + 31) / 32 * 32;
+    static constexpr uint32_t BYTES = PLANE * 4;
+};
+constexpr int NQ = 6;  // ring slots: planes i-H .. i+H are read at plane i, the rest are in flight
+// CTAs per SM the register budget is set for.
+template <bool kL2, bool kL3>
+__host__ __device__ constexpr int ctas() { return kL2 || kL3 ? 4 : 5; }
+
+// What a warp does with one row of 32 cells of one plane, one bit per cell. They are formed once per
+// work list from the cell classes and travel through the ring with their plane (one bulk copy on
+// the plane's mbarrier): the classes themselves, one global byte load per cell and plane, had to
+// be fetched a plane ahead by every thread, and their latency was exposed at every plane of a march.
+struct RowMask {
+    uint32_t move, fixed, anchor;  // kMove; kFixed; kMove && kAnchor
+    uint32_t face;                 // kMove next to a grid face: the row takes the face stencils
+};
+constexpr uint32_t MASK_BYTES = TJ * sizeof(RowMask);
+
+// One work item: the tile at (j0, k0) over planes [ib, ie) of droplet `inst`; `rec` is the index of
+// its first plane's masks.
+struct TileItem {
+    int j0, k0, ib, ie, inst, rec, pad0, pad1;
+};
+constexpr int CHUNK = 12;            // planes per work item of a full work list (tiled_length)
+constexpr long long WAIT_CLK = 4000000000ll;  // about 2 s per wait
+constexpr long long DRAIN_CLK = 40000000ll;   // about 20 ms per slot after an abort
 
 __device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -90,19 +122,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-// Waits for the phase with the given parity, giving up after WAIT_NS of wall time.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* b, uint32_t parity) {
+// Waits for the phase with the given parity, giving up after WAIT_CLK cycles or when another warp
+// of the CTA gave up.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* b, uint32_t parity, const int* abort) {
     if (mbar_try_wait(b, parity)) return true;
-    const unsigned long long t0 = global_ns();
+    const long long t0 = clock64();
     while (true) {
         if (mbar_try_wait(b, parity)) return true;
-        if (global_ns() - t0 > WAIT_NS) return false;
+        if (*(const volatile int*)abort || clock64() - t0 > WAIT_CLK) return false;
     }
+}
+// After an abort: waits for a copy that may be in flight, for a bounded time.
+__device__ __forceinline__ void drain_bounded(uint64_t* b, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait(b, parity))
+        if (clock64() - t0 > DRAIN_CLK) return;
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3,
@@ -114,54 +148,94 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* tm, in
         : "memory");
 }
 
-// Shared-memory Q accessor centred on local cell (jl, kl) of plane i; planes i-2..i+2.
+// 16-byte shared load that is not merged with an earlier one of the same address.
+__device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+// Untiled bulk copy (16-byte aligned addresses, size a multiple of 16).
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     su32(dst)),
+                 "l"(src), "r"(bytes), "r"(su32(bar))
+                 : "memory");
+}
+
+// Shared-memory Q accessor centred on a cell of plane i; planes i-2..i+2 (i-1..i+1 without the L2 term).
+template <bool kL2>
 struct SmemQ {
     const float* pl[5];
     int off;
     __device__ __forceinline__ float operator()(int c, int di, int dj, int dk) const {
-        const float* s = pl[di + 2] + off + dj * RW + dk;
-        if (c < 5) return s[c * CSTR];
-        return -(s[0] + s[3 * CSTR]);
+        return pl[di + 2][off + dj * RW + dk + c * Tile<kL2>::CSTR];
+    }
+};
+// The same with runtime offsets (face cells): the plane is picked from the five by selects.
+struct SmemQRt {
+    const float* pl[5];
+    int off;
+    __device__ __forceinline__ float operator()(int c, int di, int dj, int dk) const {
+        const float* s = di == 0 ? pl[2] : (di > 0 ? (di == 1 ? pl[3] : pl[4]) : (di == -1 ? pl[1] : pl[0]));
+        return s[off + dj * RW + dk + c * Tile<true>::CSTR];
+    }
+};
+// Face cells without the L2 term read the field itself: the shifted second difference of a cell on
+// a face reaches two cells in, one more than the one-cell halo holds.
+struct GlobQRt {
+    const float* q;  // component 0 of the cell
+    long long sc, si;
+    int sj;
+    __device__ __forceinline__ float operator()(int c, int di, int dj, int dk) const {
+        return __ldg(q + c * sc + di * si + (long long)dj * sj + dk);
     }
 };
 
-// Column divergence D_comp at offset (di, dj, dk) of cell (i, j, k), evaluated on the fly from a
-// Q accessor with the reference's face stencils (QSR.cu:325-371): the face path of the tiled kernel.
-template <class Acc>
-struct FlyD {
-    const Acc* A;
-    const QsrConst* P;
-    int i, j, k;
-    __device__ __forceinline__ float operator()(int comp, int di, int dj, int dk) const {
-        float D[3];
-        dcol_at(*A, *P, i, j, k, di, dj, dk, D);
-        return D[comp];
+// Chemical potential of one cell of a row that has cells next to a grid face. The cell is in the
+// grid: every stencil position is clamped to it. One cell at a time: the packed form of both rows
+// needs about twice the registers for the runtime offsets and spilled (101 x 90 x 117 box, default
+// radius: 23.5 against 21.5 us a step).
+template <bool kL2, bool kL3, bool kLap>
+__device__ __forceinline__ void chem_face(const SmemQ<kL2>& A, int row, const float* qin, const QsrConst& P, int i, int j,
+                                          int k, const float q[5], float mu[5], float lap[5]) {
+    const FaceAxis x(i, P.Nx), y(j, P.Ny), z(k, P.Nz);
+    const bool inner = i > 0 && i < P.Nx - 1 && j > 0 && j < P.Ny - 1 && k > 0 && k < P.Nz - 1;
+    if constexpr (kL2) {
+        SmemQRt R;
+#pragma unroll
+        for (int d = 0; d < 5; ++d) R.pl[d] = A.pl[d];
+        R.off = A.off + row * RW;
+        const FaceOne<kL2, kL3, SmemQRt> S{R, x, y, z};
+        chem_core<kL2, kL3, kLap, true, float>(S, P, q, inner ? 1.0f : 0.0f, mu, lap);
+    } else {
+        const GlobQRt R{qin + (long long)i * P.si + (long long)j * P.sj + k, P.sc, P.si, P.sj};
+        const FaceOne<kL2, kL3, GlobQRt> S{R, x, y, z};
+        chem_core<kL2, kL3, kLap, true, float>(S, P, q, inner ? 1.0f : 0.0f, mu, lap);
     }
-};
+}
 
 // Shared-memory layout of one CTA of the tiled kernels.
 struct TileSmem {
-    float* sq;          // nq planes of Q (tile + halo, 5 components)
-    uint64_t* bar;      // nq mbarriers, one per Q slot (TMA completion)
-    unsigned* freed;    // nq counters of warps done with the slot's plane
+    float* sq;          // NQ slots: a plane of Q (tile + halo, 5 components) and its row masks
+    uint64_t* bar;      // NQ mbarriers, one per slot (copy completion)
+    unsigned* freed;    // NQ counters of warps done with the slot's plane
     int* s_abort;       // set when a bounded wait gave up
     int* s_item;        // work item broadcast (persistent kernel)
 };
 
-template <bool kD, bool kPair = false>
+template <bool kL2>
 __device__ __forceinline__ TileSmem tile_smem(unsigned char* raw) {
-    constexpr int NQ = nq<kD, kPair>();
     TileSmem S;
     S.sq = reinterpret_cast<float*>(raw);
-    S.bar = reinterpret_cast<uint64_t*>(S.sq + NQ * SLOT);
+    S.bar = reinterpret_cast<uint64_t*>(S.sq + NQ * Tile<kL2>::SLOT);
     S.freed = reinterpret_cast<unsigned*>(S.bar + NQ);
     S.s_abort = reinterpret_cast<int*>(S.freed + NQ);
     S.s_item = S.s_abort + 1;
     return S;
 }
-template <bool kD, bool kPair = false>
+template <bool kL2>
 __host__ __device__ constexpr size_t tile_smem_bytes() {
-    return (size_t)nq<kD, kPair>() * SLOT * 4 + nq<kD, kPair>() * 8 + nq<kD, kPair>() * 4 + 16;
+    return (size_t)NQ * (Tile<kL2>::SLOT * 4 + 8 + 4) + 16;
 }
 
 // A warp's arrival on a slot counter: returns the count before it (acquire-release at CTA
@@ -172,366 +246,188 @@ __device__ __forceinline__ unsigned arrive_freed(unsigned* ctr) {
     return old;
 }
 
-// One work item: the (TJ x TK) column tile at (j0, k0) over planes [ib, ie). `phase` holds the
-// parity of the next phase of every slot barrier (bit s for slot s), so a CTA can run many
-// items in a row; every load the item issues is waited for by every warp before it returns.
-// Returns false when a bounded wait gave up (the CTA must stop). The caller synchronises the CTA
-// before and after an item.
-// kComp: compensated storage (explicit steps only): the low words of the input cells are read
-// from lo_in and the new low words written to lo_out.
+// One work item: the (TJ x TK) column tile at (j0, k0) over planes [ib, ie), `masks` the RowMasks of
+// its planes. `phase` holds the parity of the next phase of every slot barrier (bit s for slot s),
+// so a CTA can run many items in a row; every copy the item issues is waited for by every warp
+// before it returns. Returns false when a bounded wait gave up (the CTA must stop). The caller
+// synchronises the CTA before and after an item.
+// Each thread updates two cells (rows 2w and 2w + 1 of warp w): their chemical potential runs as one
+// packed (FFMA2 / FADD2 / FMUL2) instruction stream, and adjacent rows share operands (the centre of
+// one is a j-neighbour of the other). kComp: compensated storage (explicit steps only): the low words
+// of the input cells are read from lo_in and the new low words written to lo_out.
 template <bool kL2, bool kL3, bool kNoise, bool kRHS, bool kComp = false>
-__device__ __forceinline__ bool process_tile(const CUtensorMap* tm, float* __restrict__ qout,
-                                             const uint8_t* __restrict__ flags, int j0, int k0, int ib, int ie,
-                                             const QsrConst& P, const TileSmem& S, uint32_t& phase,
-                                             int* __restrict__ err, const float* __restrict__ lo_in = nullptr,
+__device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float* __restrict__ qin,
+                                             float* __restrict__ qout, const RowMask* __restrict__ masks, int j0,
+                                             int k0, int ib, int ie, const QsrConst& P, const TileSmem& S,
+                                             uint32_t& phase, int* __restrict__ err,
+                                             const float* __restrict__ lo_in = nullptr,
                                              float* __restrict__ lo_out = nullptr) {
-    constexpr int NQ = nq<kL2 || kL3>();
+    constexpr int H = Tile<kL2>::H, SLOT = Tile<kL2>::SLOT, PLANE = Tile<kL2>::PLANE;
+    static_assert(NQ > 2 * H + 1, "the ring holds planes i - H .. i + H and at least one in flight");
     float* sq = S.sq;
     uint64_t* bar = S.bar;
-    const int base = ib - 2;  // first plane this item loads; slots and phases count from it
-    const int tid = threadIdx.x;
-    const int kl = tid & 31, jl = tid >> 5;
-
-    // Plane p (p >= base) lives in slot (p - base) % NQ and completes that slot's barrier phase
-    // number (p - base) / NQ of this item (every caller has p >= base: unsigned arithmetic).
-    auto slot = [&](int p) { return (uint32_t)(p - base) % (uint32_t)NQ; };
-    auto parity = [&](int p) { return ((phase >> slot(p)) & 1u) ^ (((uint32_t)(p - base) / (uint32_t)NQ) & 1u); };
-
-    // Planes outside the grid, and planes past the last one this item reads (ie - 1 + LOOK),
-    // complete their phase with a plain arrive (no data).
-    auto issue = [&](int p) {
-        uint64_t* b = &bar[slot(p)];
-        if (p >= 0 && p < P.Nx && p < ie + LOOK) {
-            fence_proxy_async();
-            mbar_expect_tx(b, PLANE_BYTES);
-            tma_load_4d(sq + slot(p) * SLOT, tm, k0 - HK, j0 - HJ, p, 0, b);
-        } else {
-            mbar_arrive(b);
-        }
-    };
-    if (tid == 0)
-        for (int p = base; p < base + NQ; ++p) issue(p);
-    bool ok = true;
-    auto wait_plane = [&](int p) {
-        if (!mbar_wait_bounded(&bar[slot(p)], parity(p))) {
-            atomicExch(err, LDG_ERR_TIMEOUT);
-            *(volatile int*)S.s_abort = 1;
-            ok = false;
-        }
-    };
-    // Planes [base, ie + NQ - 2) are issued: the first NQ here, then plane p + NQ when the last
-    // warp is done with plane p (after its plane p + 2), for every p <= ie - 3.
-    const int issued_end = ie + NQ - 2;
-
-    const int j = j0 + jl, k = k0 + kl;
-    const bool in_grid = (j < P.Ny) && (k >= 0) && (k < P.Nz);
-    // Interior cells take the Q-only path: every stencil position within the grid away from the
-    // faces (the L2 term reaches two cells out: 2 <= pos <= N - 3; otherwise 1 <= pos <= N - 2).
-    constexpr int kLo = kL2 ? 2 : 1;
-    const bool jk_interior = j >= kLo && j <= P.Ny - 1 - kLo && k >= kLo && k <= P.Nz - 1 - kLo;
-    const long long cell0 = (long long)j * P.sj + k;
-    uint8_t f_next = in_grid ? __ldg(flags + (long long)ib * P.si + cell0) : 0;
-    // Shared-memory planes i-2 .. i+2 of the current step, rolled forward by one plane per step.
-    const float* qpl[5];
-#pragma unroll
-    for (int d = 0; d < 5; ++d) qpl[d] = sq + slot(ib + d - 2) * SLOT;
-    int waited_end = base;
-    for (int p = base; p <= ib + LOOK - 1; ++p) wait_plane(p);
-    waited_end = ib + LOOK;
-    for (int i = ib; i < ie; ++i) {
-        if (*(volatile int*)S.s_abort) { ok = false; break; }  // another warp gave up
-        const uint8_t f = f_next;
-        if (in_grid && i + 1 < ie) f_next = __ldg(flags + (long long)(i + 1) * P.si + cell0);
-        wait_plane(i + LOOK);
-        waited_end = i + LOOK + 1;
-        if (!ok) break;
-        const bool fixed = in_grid && !kRHS && (f & kFixed);
-        const bool move = in_grid && (f & kMove) != 0;
-        // The Q-only interior form is taken by a whole warp when none of its computing cells is
-        // near a face (exterior cells of a droplet compute nothing, so small droplets use it too).
-        const bool warp_interior =
-            __all_sync(0xffffffffu, !move || (jk_interior && i >= kLo && i <= P.Nx - 1 - kLo)) != 0;
-        if (fixed || move) {
-            const long long id = (long long)i * P.si + cell0;
-            SmemQ A;
-#pragma unroll
-            for (int d = 0; d < 5; ++d) A.pl[d] = qpl[d];
-            A.off = (jl + HJ) * RW + (kl + HK);
-            float c[5], o[5];
-#pragma unroll
-            for (int m = 0; m < 5; ++m) c[m] = A(m, 0, 0, 0);
-            if (fixed) {
-                surface_q0(P, i, j, k, o);
-                if (kComp) {
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) lo_out[m * P.sc + id] = 0.0f;
-                }
-            } else {
-                float mu[5], lap[5];
-                if (warp_interior) {
-                    chem_potential_interior_x2<kL2, kL3>(A, P, i, j, k, c, (f & kAnchor) != 0, mu, lap);
-                } else {
-                    const FlyD<SmemQ> DA{&A, &P, i, j, k};
-                    chem_potential<kL2, kL3, true>(A, DA, P, i, j, k, c, (f & kAnchor) != 0, mu, lap);
-                }
-                const uint32_t cell = (uint32_t)(k + P.Nz * (j + P.Ny * i));
-                if (kRHS) {
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) o[m] = c[m] - P.mob_dt * mu[m] - P.alpha * lap[m];
-                    if (kNoise) {
-                        float g[5];
-                        normals5(cell, P.instance, P.step, P.key0, P.key1, g);
-#pragma unroll
-                        for (int m = 0; m < 5; ++m) o[m] += P.sigma * g[m];
-                    }
-                } else if (kComp) {
-                    float lo[5];
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) lo[m] = __ldg(lo_in + m * P.sc + id);
-                    euler_update_comp(P, c, lo, mu, cell, kNoise, o);
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) lo_out[m * P.sc + id] = lo[m];
-                } else {
-                    euler_update(P, c, mu, cell, kNoise, o);
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < 5; ++m) qout[m * P.sc + id] = o[m];
-        }
-        // This warp is done with plane i-2: arrive on its slot; the last warp refills the slot with
-        // plane i-2+NQ.
-        __syncwarp();
-        if (kl == 0) {
-            const uint32_t s = slot(i - 2);
-            if (arrive_freed(&S.freed[s]) % (unsigned)NWARP == (unsigned)NWARP - 1u) issue(i - 2 + NQ);
-        }
-#pragma unroll
-        for (int d = 0; d < 4; ++d) qpl[d] = qpl[d + 1];
-        qpl[4] = sq + slot(i + 3) * SLOT;
-    }
-    // Drain: every load this item issues lands before the slots are reused or released. After
-    // an abort some refills are never issued; those waits give up after their bound.
-    if (ok) {
-        for (int p = waited_end; p < issued_end; ++p) wait_plane(p);
-    } else {
-        for (int p = waited_end; p < issued_end; ++p)
-            if (!mbar_wait_bounded(&bar[slot(p)], parity(p))) break;
-    }
-    // Advance the per-slot phase parities by the number of loads each slot received.
-    const int n_issued = issued_end - base;
-#pragma unroll
-    for (int s = 0; s < NQ; ++s) {
-        const int uses = (n_issued > s) ? (n_issued - s + NQ - 1) / NQ : 0;
-        phase ^= (uint32_t)(uses & 1) << s;
-    }
-    return ok;
-}
-
-// Rows of the two cells of a thread in the two-cell kernels: warp w updates tile rows
-// PAIR_R0 * w and PAIR_R0 * w + PAIR_DR. Adjacent rows share operands: the centre of one cell
-// is a j-neighbour of the other, and their j +- 1 and j +- 2 rows overlap, so the compiler loads
-// those shared values once.
-constexpr int PAIR_R0 = 2, PAIR_DR = 1;
-
-// Shared-memory accessor of two cells of one plane: local (jl, kl) and (jl + PAIR_DR, kl).
-struct SmemQ2 {
-    const float* pl[5];
-    int off;
-    __device__ __forceinline__ F2 operator()(int c, int di, int dj, int dk) const {
-        const float* s = pl[di + 2] + off + dj * RW + dk;
-        if (c < 5) return mk2(s[c * CSTR], s[c * CSTR + PAIR_DR * RW]);
-        return mk2(-(s[0] + s[3 * CSTR]), -(s[PAIR_DR * RW] + s[3 * CSTR + PAIR_DR * RW]));
-    }
-};
-constexpr int PAIR_THREADS = TK * TJ / 2;  // 128: each thread updates two rows of the tile
-constexpr int PAIR_NWARP = PAIR_THREADS / 32;
-
-// process_tile for 128 threads, two cells per thread (rows 2w and 2w + 1 of warp w): the interior
-// chemical potential of both cells runs as one packed (FFMA2 / FADD2 / FMUL2) instruction stream;
-// face cells, the strong-anchoring rewrite and the update run per cell.
-template <bool kL2, bool kL3, bool kNoise, bool kRHS, bool kComp = false>
-__device__ __forceinline__ bool process_tile_pair(const CUtensorMap* tm, float* __restrict__ qout,
-                                                  const uint8_t* __restrict__ flags, int j0, int k0, int ib, int ie,
-                                                  const QsrConst& P, const TileSmem& S, uint32_t& phase,
-                                                  int* __restrict__ err, const float* __restrict__ lo_in = nullptr,
-                                                  float* __restrict__ lo_out = nullptr) {
-    constexpr int NQ = nq<kL2 || kL3, true>();
-    static_assert(NQ > 2 * LOOK && LOOK == 2, "the ring holds planes i - 2 .. i + 2 and at least one in flight");
-    float* sq = S.sq;
-    uint64_t* bar = S.bar;
-    const int base = ib - 2;
+    const int base = ib - H;  // first plane this item loads; slots and phases count from it
     const int tid = threadIdx.x;
     const int kl = tid & 31, w = tid >> 5;
+    // Plane p (p >= base) lives in slot (p - base) % NQ.
     auto slot = [&](int p) { return (uint32_t)(p - base) % (uint32_t)NQ; };
-    auto parity = [&](int p) { return ((phase >> slot(p)) & 1u) ^ (((uint32_t)(p - base) / (uint32_t)NQ) & 1u); };
-    auto issue = [&](int p) {
-        uint64_t* b = &bar[slot(p)];
-        if (p >= 0 && p < P.Nx && p < ie + LOOK) {
+    // Planes outside the grid, and planes past the last one this item reads (ie - 1 + H), complete
+    // their phase with a plain arrive (no data). The planes of the item bring their row masks.
+    auto issue = [&](int p, uint32_t sl) {
+        uint64_t* b = &bar[sl];
+        if (p >= 0 && p < P.Nx && p < ie + H) {
+            const bool own = p >= ib && p < ie;
+            float* dst = sq + sl * SLOT;
             fence_proxy_async();
-            mbar_expect_tx(b, PLANE_BYTES);
-            tma_load_4d(sq + slot(p) * SLOT, tm, k0 - HK, j0 - HJ, p, 0, b);
+            mbar_expect_tx(b, Tile<kL2>::BYTES + (own ? MASK_BYTES : 0u));
+            tma_load_4d(dst, tm, k0 - HK, j0 - H, p, 0, b);
+            if (own) bulk_load(dst + PLANE, masks + (size_t)(p - ib) * TJ, MASK_BYTES, b);
         } else {
             mbar_arrive(b);
         }
     };
     if (tid == 0)
-        for (int p = base; p < base + NQ; ++p) issue(p);
+        for (int p = base; p < base + NQ; ++p) issue(p, slot(p));
     bool ok = true;
     // Waits run in increasing plane order, so each slot's expected parity is tracked by toggling
     // its bit of `par` after every wait on it (no division per plane).
     uint32_t par = phase;
     auto wait_slot = [&](uint32_t sl) {
-        if (!mbar_wait_bounded(&bar[sl], (par >> sl) & 1u)) {
+        if (!mbar_wait_bounded(&bar[sl], (par >> sl) & 1u, S.s_abort)) {
             atomicExch(err, LDG_ERR_TIMEOUT);
             *(volatile int*)S.s_abort = 1;
             ok = false;
         }
         par ^= 1u << sl;
     };
-    auto wait_plane = [&](int p) { wait_slot(slot(p)); };
-    const int issued_end = ie + NQ - 2;
-    constexpr int kLo = kL2 ? 2 : 1;
-    const int k = k0 + kl;
-    int jr[2];
-    bool in_grid[2], jk_int[2];
-    long long cell0[2];
-    uint8_t f_next[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        jr[r] = j0 + PAIR_R0 * w + PAIR_DR * r;
-        in_grid[r] = (jr[r] < P.Ny) && (k >= 0) && (k < P.Nz);
-        jk_int[r] = jr[r] >= kLo && jr[r] <= P.Ny - 1 - kLo && k >= kLo && k <= P.Nz - 1 - kLo;
-        cell0[r] = (long long)jr[r] * P.sj + k;
-        f_next[r] = in_grid[r] ? __ldg(flags + (long long)ib * P.si + cell0[r]) : 0;
-    }
+    // Planes [base, ie + NQ - H) are issued: the first NQ here, then plane p + NQ when the last
+    // warp is done with plane p (after its plane p + H), for every p <= ie - H - 1.
+    const int issued_end = ie + NQ - H;
+    const int j = j0 + 2 * w, k = k0 + kl;
+    const uint32_t bit = 1u << kl;
+    const int off = (2 * w + H) * RW + kl + HK;
+    long long id = (long long)ib * P.si + (long long)j * P.sj + k;  // row j; row j + 1 is P.sj further
+    // Shared-memory planes i-H .. i+H of the current step, rolled forward by one plane per step.
     const float* qpl[5];
 #pragma unroll
-    for (int d = 0; d < 5; ++d) qpl[d] = sq + slot(ib + d - 2) * SLOT;
-    int waited_end = base;
-    for (int p = base; p <= ib + LOOK - 1; ++p) wait_plane(p);
-    waited_end = ib + LOOK;
-    uint32_t s_w = slot(ib + LOOK);  // slot of plane i + LOOK, advanced by one per plane
-    for (int i = ib; i < ie; ++i) {
-        if (*(volatile int*)S.s_abort) { ok = false; break; }
-        uint8_t f[2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            f[r] = f_next[r];
-            if (in_grid[r] && i + 1 < ie) f_next[r] = __ldg(flags + (long long)(i + 1) * P.si + cell0[r]);
-        }
+    for (int d = 2 - H; d <= 2 + H; ++d) qpl[d] = sq + slot(ib + d - 2) * SLOT;
+    for (int p = base; p < ib + H; ++p) wait_slot(slot(p));
+    int waited_end = ib + H;
+    uint32_t s_w = slot(ib + H);  // slot of plane i + H, advanced by one per plane
+    for (int i = ib; i < ie; ++i, id += P.si) {
         wait_slot(s_w);
-        waited_end = i + LOOK + 1;
-        if (!ok) break;
-        bool fixed[2], move[2];
-        bool interior = true;
+        waited_end = i + H + 1;
+        if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp stops or none of it
+        // The masks are read again after the chemical potential: eight registers fewer live across it.
+        const uint32_t mk = su32(qpl[2] + PLANE) + 2 * w * sizeof(RowMask);
+        uint4 m0 = lds_u4(mk), m1 = lds_u4(mk + sizeof(RowMask));
+        if ((m0.x | m1.x) != 0u || (!kRHS && (m0.y | m1.y) != 0u)) {
+            SmemQ<kL2> A;
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            fixed[r] = in_grid[r] && !kRHS && (f[r] & kFixed);
-            move[r] = in_grid[r] && (f[r] & kMove) != 0;
-            interior = interior && (!move[r] || (jk_int[r] && i >= kLo && i <= P.Nx - 1 - kLo));
-        }
-        const bool warp_interior = __all_sync(0xffffffffu, interior) != 0;
-        const bool any_move = __any_sync(0xffffffffu, move[0] || move[1]) != 0;
-        float mu[2][5], lap[2][5], c[2][5];
-        if (any_move) {
-            SmemQ A[2];
+            for (int d = 2 - H; d <= 2 + H; ++d) A.pl[d] = qpl[d];
+            A.off = off;
+            F2 c[5], mu[5], lap[5];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) c[m] = mk2(A(m, 0, 0, 0), A(m, 0, 1, 0));
+            if ((m0.w | m1.w) == 0u) {
+                const InteriorPair<kL2, kL3, SmemQ<kL2>> St{A};
+                chem_core<kL2, kL3, kRHS, false, F2>(St, P, c, F2{}, mu, lap);
+            } else {
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    float cr[5], mr[5], lr[5];
+#pragma unroll
+                    for (int m = 0; m < 5; ++m) cr[m] = mr[m] = lr[m] = r ? c[m].v.y : c[m].v.x;
+                    if ((r ? m1.x : m0.x) & bit) chem_face<kL2, kL3, kRHS>(A, r, qin, P, i, j + r, k, cr, mr, lr);
+#pragma unroll
+                    for (int m = 0; m < 5; ++m) {
+                        (r ? mu[m].v.y : mu[m].v.x) = mr[m];
+                        if (kRHS) (r ? lap[m].v.y : lap[m].v.x) = lr[m];
+                    }
+                }
+            }
+            m0 = lds_u4(mk);
+            m1 = lds_u4(mk + sizeof(RowMask));
+            if ((m0.z | m1.z) != 0u) {  // weak-anchoring penalty (QSR.cu:623-652)
+                float Qa[5], Qb[5];
+                surface_q0(P, i, j, k, Qa);
+                surface_q0(P, i, j + 1, k, Qb);
+                const F2 wf = mk2((m0.z & bit) ? P.Weff : 0.0f, (m1.z & bit) ? P.Weff : 0.0f);
+#pragma unroll
+                for (int m = 0; m < 5; ++m) mu[m] = vfma(wf, c[m] - mk2(Qa[m], Qb[m]), mu[m]);
+            }
+            F2 u[5];
+            if (kRHS) {
+#pragma unroll
+                for (int m = 0; m < 5; ++m) u[m] = vfma(-P.alpha, lap[m], vfma(-P.mob_dt, mu[m], c[m]));
+            } else if (!kComp) {
+#pragma unroll
+                for (int m = 0; m < 5; ++m) u[m] = vfma(-P.mob_dt, mu[m], c[m]);
+            }
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
+                const uint32_t mv = r ? m1.x : m0.x, fx = r ? m1.y : m0.y;
+                const bool fixed = !kRHS && (fx & bit), move = (mv & bit) != 0u;
+                if (!(fixed || move)) continue;
+                const long long ir = id + (r ? P.sj : 0);
+                float o[5];
 #pragma unroll
-                for (int d = 0; d < 5; ++d) A[r].pl[d] = qpl[d];
-                A[r].off = (PAIR_R0 * w + PAIR_DR * r + HJ) * RW + (kl + HK);
+                for (int m = 0; m < 5; ++m) o[m] = r ? u[m].v.y : u[m].v.x;
+                if (fixed) {
+                    surface_q0(P, i, j + r, k, o);
+                    if (kComp) {
 #pragma unroll
-                for (int m = 0; m < 5; ++m) c[r][m] = A[r](m, 0, 0, 0);
-            }
-            if (warp_interior) {
-                SmemQ2 A2;
-#pragma unroll
-                for (int d = 0; d < 5; ++d) A2.pl[d] = qpl[d];
-                A2.off = A[0].off;
-                F2 q2[5], mu2[5], lap2[5];
-#pragma unroll
-                for (int m = 0; m < 5; ++m) q2[m] = mk2(c[0][m], c[1][m]);
-                chem_interior_pair<kL2, kL3>(A2, P, q2, mu2, lap2);
-#pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    mu[0][m] = mu2[m].v.x; mu[1][m] = mu2[m].v.y;
-                    lap[0][m] = lap2[m].v.x; lap[1][m] = lap2[m].v.y;
-                }
-                const bool anch0 = move[0] && (f[0] & kAnchor), anch1 = move[1] && (f[1] & kAnchor);
-                if (__any_sync(0xffffffffu, anch0 || anch1)) {
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        if (r == 0 ? anch0 : anch1) {
-                            float Q0[5];
-                            surface_q0(P, i, jr[r], k, Q0);
-#pragma unroll
-                            for (int m = 0; m < 5; ++m) mu[r][m] += P.Weff * (c[r][m] - Q0[m]);
-                        }
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-                    if (move[r]) {
-                        const FlyD<SmemQ> DA{&A[r], &P, i, jr[r], k};
-                        chem_potential<kL2, kL3, true>(A[r], DA, P, i, jr[r], k, c[r], (f[r] & kAnchor) != 0, mu[r],
-                                                       lap[r]);
-                    }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            if (!(fixed[r] || move[r])) continue;
-            const long long id = (long long)i * P.si + cell0[r];
-            float o[5];
-            if (fixed[r]) {
-                surface_q0(P, i, jr[r], k, o);
-                if (kComp) {
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) lo_out[m * P.sc + id] = 0.0f;
-                }
-            } else {
-                const uint32_t cell = (uint32_t)(k + P.Nz * (jr[r] + P.Ny * i));
-                if (kRHS) {
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) o[m] = c[r][m] - P.mob_dt * mu[r][m] - P.alpha * lap[r][m];
-                    if (kNoise) {
-                        float g[5];
-                        normals5(cell, P.instance, P.step, P.key0, P.key1, g);
-#pragma unroll
-                        for (int m = 0; m < 5; ++m) o[m] += P.sigma * g[m];
+                        for (int m = 0; m < 5; ++m) lo_out[m * P.sc + ir] = 0.0f;
                     }
                 } else if (kComp) {
-                    float lo[5];
+                    float lo[5], cr[5], mr[5];
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) lo[m] = __ldg(lo_in + m * P.sc + id);
-                    euler_update_comp(P, c[r], lo, mu[r], cell, kNoise, o);
+                    for (int m = 0; m < 5; ++m) {
+                        lo[m] = __ldg(lo_in + m * P.sc + ir);
+                        cr[m] = r ? c[m].v.y : c[m].v.x;
+                        mr[m] = r ? mu[m].v.y : mu[m].v.x;
+                    }
+                    euler_update_comp(P, cr, lo, mr, (uint32_t)(k + P.Nz * (j + r + P.Ny * i)), kNoise, o);
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) lo_out[m * P.sc + id] = lo[m];
+                    for (int m = 0; m < 5; ++m) lo_out[m * P.sc + ir] = lo[m];
                 } else {
-                    euler_update(P, c[r], mu[r], cell, kNoise, o);
-                }
-            }
+                    if (kNoise) {
+                        float g[5];
+                        normals5((uint32_t)(k + P.Nz * (j + r + P.Ny * i)), P.instance, P.step, P.key0, P.key1, g);
 #pragma unroll
-            for (int m = 0; m < 5; ++m) qout[m * P.sc + id] = o[m];
+                        for (int m = 0; m < 5; ++m) o[m] = fmaf(P.sigma, g[m], o[m]);
+                    }
+                    if (!kRHS && P.qcap > 0.0f) cap_norm(P.qcap, o);
+                }
+#pragma unroll
+                for (int m = 0; m < 5; ++m) qout[m * P.sc + ir] = o[m];
+            }
         }
+        // This warp is done with plane i-H: arrive on its slot; the last warp refills the slot with
+        // plane i-H+NQ.
         __syncwarp();
         if (kl == 0) {
-            // slot of plane i - 2 = slot of plane i + 2 minus four
-            const uint32_t sl = s_w + (NQ - 4) >= (uint32_t)NQ ? s_w - 4 : s_w + (NQ - 4);
-            if (arrive_freed(&S.freed[sl]) % (unsigned)PAIR_NWARP == (unsigned)PAIR_NWARP - 1u) issue(i - 2 + NQ);
+            // slot of plane i - H = slot of plane i + H minus 2 H
+            const uint32_t sl = s_w >= 2u * H ? s_w - 2 * H : s_w + (NQ - 2 * H);
+            if (arrive_freed(&S.freed[sl]) % (unsigned)NWARP == (unsigned)NWARP - 1u) issue(i - H + NQ, sl);
         }
-        s_w = (s_w + 1 == (uint32_t)NQ) ? 0u : s_w + 1;  // now the slot of plane i + 3
+        s_w = (s_w + 1 == (uint32_t)NQ) ? 0u : s_w + 1;  // now the slot of plane i + H + 1
 #pragma unroll
-        for (int d = 0; d < 4; ++d) qpl[d] = qpl[d + 1];
-        qpl[4] = sq + s_w * SLOT;
+        for (int d = 2 - H; d < 2 + H; ++d) qpl[d] = qpl[d + 1];
+        qpl[2 + H] = sq + s_w * SLOT;
     }
-    if (ok) {
-        for (int p = waited_end; p < issued_end; ++p) wait_plane(p);
-    } else {
-        for (int p = waited_end; p < issued_end; ++p)
-            if (!mbar_wait_bounded(&bar[slot(p)], parity(p))) break;
+    // Drain: every copy this item issues lands before the slots are reused or released. After
+    // an abort some refills are never issued; those waits give up at once.
+    for (int p = waited_end; p < issued_end; ++p) {
+        if (ok) {
+            wait_slot(slot(p));
+        } else {
+            const uint32_t sl = slot(p);
+            drain_bounded(&bar[sl], (par >> sl) & 1u);
+            par ^= 1u << sl;
+        }
     }
+    // Advance the per-slot phase parities by the number of copies each slot received.
     const int n_issued = issued_end - base;
 #pragma unroll
     for (int sl = 0; sl < NQ; ++sl) {
@@ -541,10 +437,10 @@ __device__ __forceinline__ bool process_tile_pair(const CUtensorMap* tm, float* 
     return ok;
 }
 
-template <bool kD, bool kPair = false>
+template <bool kL2>
 __device__ __forceinline__ void tile_smem_init(const TileSmem& S) {
     if (threadIdx.x == 0) {
-        for (int s = 0; s < nq<kD, kPair>(); ++s) {
+        for (int s = 0; s < NQ; ++s) {
             mbar_init(&S.bar[s], 1);
             S.freed[s] = 0;
         }
@@ -554,50 +450,53 @@ __device__ __forceinline__ void tile_smem_init(const TileSmem& S) {
     __syncthreads();
 }
 
-// Single grid, two cells per thread (128 threads): four CTAs per SM.
+// Single grid: one work item per CTA.
 template <bool kL2, bool kL3, bool kNoise, bool kRHS, bool kComp = false>
-__global__ void __launch_bounds__(PAIR_THREADS, 4)
-    k_step_tiled_pair(const __grid_constant__ CUtensorMap tm_in, float* __restrict__ qout,
-                      const uint8_t* __restrict__ flags, const int4* __restrict__ items, QsrConst P,
-                      int* __restrict__ err, const float* __restrict__ lo_in, float* __restrict__ lo_out) {
+__global__ void __launch_bounds__(THREADS, ctas<kL2, kL3>())
+    k_step_tiled(const __grid_constant__ CUtensorMap tm_in, const float* __restrict__ qin, float* __restrict__ qout,
+                 const RowMask* __restrict__ masks, const TileItem* __restrict__ items, QsrConst P,
+                 int* __restrict__ err, const float* __restrict__ lo_in, float* __restrict__ lo_out) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const TileSmem S = tile_smem<kL2 || kL3, true>(smem_raw);
-    tile_smem_init<kL2 || kL3, true>(S);
-    const int4 item = items[blockIdx.x];
+    const TileSmem S = tile_smem<kL2>(smem_raw);
+    tile_smem_init<kL2>(S);
+    const TileItem e = items[blockIdx.x];
     uint32_t phase = 0;
-    process_tile_pair<kL2, kL3, kNoise, kRHS, kComp>(&tm_in, qout, flags, item.x, item.y, item.z, item.w, P, S, phase,
-                                                     err, lo_in, lo_out);
+    pdl_wait();
+    pdl_trigger();
+    process_tile<kL2, kL3, kNoise, kRHS, kComp>(&tm_in, qin, qout, masks + (size_t)e.rec * TJ, e.j0, e.k0, e.ib, e.ie,
+                                                P, S, phase, err, lo_in, lo_out);
 }
 
-// Single grid: one work item per CTA; two CTAs per SM with the L2/L3 terms, three without.
-template <bool kL2, bool kL3, bool kNoise, bool kRHS, bool kComp = false>
-__global__ void __launch_bounds__(THREADS, (kL2 || kL3) ? 2 : 3)
-    k_step_tiled(const __grid_constant__ CUtensorMap tm_in, float* __restrict__ qout, const uint8_t* __restrict__ flags,
-                 const int4* __restrict__ items, QsrConst P, int* __restrict__ err, const float* __restrict__ lo_in,
-                 float* __restrict__ lo_out) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const TileSmem S = tile_smem<kL2 || kL3>(smem_raw);
-    tile_smem_init<kL2 || kL3>(S);
-    const int4 item = items[blockIdx.x];
-    uint32_t phase = 0;
-    process_tile<kL2, kL3, kNoise, kRHS, kComp>(&tm_in, qout, flags, item.x, item.y, item.z, item.w, P, S, phase, err,
-                                                lo_in, lo_out);
+// Row masks of a work list: one block per item, one warp per tile row, a ballot per plane. `lo` is
+// the distance from a face from which the interior stencils hold (2 with the L2 term, else 1).
+inline __global__ void __launch_bounds__(TK* TJ) k_tile_masks(const TileItem* __restrict__ items,
+                                                              const uint8_t* __restrict__ flags, int Nx, int Ny, int Nz,
+                                                              int sj, long long si, int lo, RowMask* __restrict__ masks) {
+    const TileItem e = items[blockIdx.x];
+    const int kl = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int j = e.j0 + row, k = e.k0 + kl;
+    const bool in = j < Ny && k >= 0 && k < Nz;
+    const bool jk = j >= lo && j <= Ny - 1 - lo && k >= lo && k <= Nz - 1 - lo;
+    for (int i = e.ib; i < e.ie; ++i) {
+        const uint8_t f = in ? flags[(long long)i * si + (long long)j * sj + k] : 0;
+        RowMask m;
+        m.move = __ballot_sync(0xffffffffu, f & kMove);
+        m.fixed = __ballot_sync(0xffffffffu, f & kFixed);
+        m.anchor = __ballot_sync(0xffffffffu, (f & kMove) && (f & kAnchor));
+        m.face = __ballot_sync(0xffffffffu, (f & kMove) && !(jk && i >= lo && i <= Nx - 1 - lo));
+        if (kl == 0) masks[(size_t)(e.rec + i - e.ib) * TJ + row] = m;
+    }
 }
 
 // ---------------------------------------------------------------------------------------
 // Ensemble: many independent droplets, one persistent work-stealing launch per step.
 // ---------------------------------------------------------------------------------------
-struct EnsItem {
-    int j0, k0, ib, ie, inst, pad0, pad1, pad2;
-};
-
 // Per-instance descriptor. The step index lives on the device (EnsCtl), so the temperature of
 // the protocol, the shell order and the noise counter are formed in the kernel and one captured
 // CUDA graph can be replayed for any number of steps.
 struct EnsInstDev {
     QsrConst P;            // static parts (noise key and stream included); cQ, S_shell, step set per step
     float* q[2];           // ping-pong buffers: input of step s is q[s & 1]
-    const uint8_t* flags;
     double T_high, T_low;  // protocol (QSR.cu:2679-2687)
     long long pre, ramp;
     int protocol;          // 1 step, 2 linear ramp
@@ -640,14 +539,16 @@ __host__ __device__ __forceinline__ double ens_S_eq(double A, double B, double C
     return best_S;
 }
 
-// kPair: the two-cell routine (128 threads, four CTAs per SM), else one cell per thread.
-template <bool kL2, bool kL3, bool kNoise, bool kPair>
-__global__ void __launch_bounds__(kPair ? PAIR_THREADS : THREADS, kPair ? 4 : ((kL2 || kL3) ? 2 : 3))
+template <bool kL2, bool kL3, bool kNoise>
+__global__ void __launch_bounds__(THREADS, ctas<kL2, kL3>())
     k_step_ensemble(const CUtensorMap* __restrict__ tms, const EnsInstDev* __restrict__ inst,
-                    const EnsItem* __restrict__ items, int n_items, EnsCtl* __restrict__ ctl, int* __restrict__ err) {
+                    const TileItem* __restrict__ items, const RowMask* __restrict__ masks, int n_items,
+                    EnsCtl* __restrict__ ctl, int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const TileSmem S = tile_smem<kL2 || kL3, kPair>(smem_raw);
-    tile_smem_init<kL2 || kL3, kPair>(S);
+    const TileSmem S = tile_smem<kL2>(smem_raw);
+    tile_smem_init<kL2>(S);
+    pdl_wait();
+    pdl_trigger();
     // Every CTA reads the step index before any CTA of this launch finishes (the last CTA to
     // finish advances it).
     const long long step = *((volatile long long*)&ctl->step);
@@ -661,7 +562,7 @@ __global__ void __launch_bounds__(kPair ? PAIR_THREADS : THREADS, kPair ? 4 : ((
         const bool stop = (it >= n_items) || (*S.s_abort != 0);
         __syncthreads();
         if (stop) break;
-        const EnsItem e = items[it];
+        const TileItem e = items[it];
         const EnsInstDev& D = inst[e.inst];
         QsrConst P = D.P;
         const double T = ens_temperature(D, step);
@@ -674,12 +575,8 @@ __global__ void __launch_bounds__(kPair ? PAIR_THREADS : THREADS, kPair ? 4 : ((
             P.S_shell = (float)D.S_custom;
         }
         P.step = step;
-        if constexpr (kPair)
-            process_tile_pair<kL2, kL3, kNoise, false>(tms + 2 * e.inst + which, D.q[1 - which], D.flags, e.j0, e.k0,
-                                                       e.ib, e.ie, P, S, phase, err);
-        else
-            process_tile<kL2, kL3, kNoise, false>(tms + 2 * e.inst + which, D.q[1 - which], D.flags, e.j0, e.k0, e.ib,
-                                                  e.ie, P, S, phase, err);
+        process_tile<kL2, kL3, kNoise, false>(tms + 2 * e.inst + which, D.q[which], D.q[1 - which],
+                                              masks + (size_t)e.rec * TJ, e.j0, e.k0, e.ib, e.ie, P, S, phase, err);
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -699,6 +596,7 @@ __global__ void __launch_bounds__(kPair ? PAIR_THREADS : THREADS, kPair ? 4 : ((
 // of its changing cells (kmin > kmax: none).
 struct TiledBand {
     int j0 = 0, rows = 0, ib = 0, ie = 0;
+    bool face = false;            // changing cells next to a j face
     std::vector<int> kmin, kmax;
 };
 
@@ -708,7 +606,13 @@ struct TiledPlan {
     long long written_cells = 0;  // cells written per step (moving + strongly anchored)
     int n_items = 0;
     int chunk = 0;                // planes per work item (the longest item)
-    int4* items = nullptr;        // device work list (j0, k0, i_begin, i_end)
+    tiled::TileItem* items = nullptr;   // device work list
+    tiled::RowMask* masks = nullptr;    // row masks of the items' planes
+    const uint8_t* flags = nullptr;     // device cell classes
+    int Nx = 0, Ny = 0, sj = 0;
+    long long si = 0;
+    bool L2 = false;              // the kernels take the L2 term (halo, interior distance)
+    bool deep = false;            // the L2 or the L3 term
     int n_plane_items = 0;
     int4* plane_items = nullptr;  // the same tiles one plane each (j0, k0, i, i + 1): IMEX sweeps
     int Nz = 0;
@@ -716,20 +620,17 @@ struct TiledPlan {
     int* err = nullptr;           // device error word
     CUtensorMap tmap[2];
     const float* bufs[2] = {nullptr, nullptr};
-    size_t smem_bytes[3] = {0, 0, 0};  // [L1 only, with L2/L3, with L2/L3 two cells per thread]
 };
 
-// Work items for chunks of `chunk` planes. In each row band and plane chunk the k tiles start at
-// the first changing cell (rounded down to the 4-float TMA alignment) instead of at multiples of
-// TK, and each tile's plane range is cut to the planes whose changing cells reach it: every
-// changing cell lies in exactly one item, and fewer idle lanes are visited than with a fixed tile
-// grid. Items are ordered longest first, and among items of one length with the plane chunk
-// slowest (CTAs resident together share halo planes in L2). *active: the cells of the grid inside
-// the items' tiles (read once per step).
-inline std::vector<int4> tiled_items(const TiledPlan& plan, int chunk, long long* active) {
+// Calls emit(j0, k0, first, last + 1, face) for every work item of chunks of `chunk` planes. In each
+// row band and plane chunk the k tiles start at the first changing cell (rounded down to the 4-float
+// TMA alignment) instead of at multiples of TK, and each tile's plane range is cut to the planes
+// whose changing cells reach it: every changing cell lies in exactly one item, and fewer idle lanes
+// are visited than with a fixed tile grid. `face`: the item has changing cells next to a grid face.
+template <class Emit>
+inline void tiled_each_item(const TiledPlan& plan, int chunk, Emit emit) {
     using namespace tiled;
-    std::vector<int4> items;
-    long long act = 0;
+    const int lo_d = plan.L2 ? 2 : 1;
     for (const TiledBand& b : plan.bands) {
         for (int ib = b.ib; ib < b.ie; ib += chunk) {
             const int ie = std::min(b.ie, ib + chunk);
@@ -742,66 +643,102 @@ inline std::vector<int4> tiled_items(const TiledPlan& plan, int chunk, long long
             if (kmax < 0) continue;
             for (int k0 = ((kmin - 2) & ~3) + 2; k0 <= kmax; k0 += TK) {
                 int first = -1, last = -1;
+                bool face = false;
                 for (int p = ib; p < ie; ++p) {
                     const int lo = b.kmin[p - b.ib], hi = b.kmax[p - b.ib];
                     if (lo <= hi && lo <= k0 + TK - 1 && hi >= k0) {
                         if (first < 0) first = p;
                         last = p;
+                        face = face || p < lo_d || p > plan.Nx - 1 - lo_d || (lo < lo_d && k0 <= lo) ||
+                               (hi > plan.Nz - 1 - lo_d && k0 + TK > hi);
                     }
                 }
                 if (first < 0) continue;
-                items.push_back(make_int4(b.j0, k0, first, last + 1));
-                act += (long long)b.rows * (std::min(plan.Nz, k0 + TK) - std::max(0, k0)) * (last + 1 - first);
+                emit(b.j0, k0, first, last + 1, face || b.face, b.rows);
             }
         }
     }
-    std::stable_sort(items.begin(), items.end(), [](const int4& a, const int4& b) {
-        if (a.z != b.z) return a.z < b.z;
-        if (a.x != b.x) return a.x < b.x;
-        return a.y < b.y;
-    });
-    // Longest items first (ties keep the order above): CTAs are dispatched in item order, so
-    // the short items of the droplet's poles fill the last wave instead of trailing it.
-    std::stable_sort(items.begin(), items.end(),
-                     [](const int4& a, const int4& b) { return (a.w - a.z) > (b.w - b.z); });
-    if (active) *active = act;
-    return items;
 }
 
-// Kernel choice: LDG_QSR_PAIR=0 always takes one cell per thread, LDG_QSR_PAIR=1 always two;
-// otherwise (the default) the ensemble takes two and a single grid chooses by its work list.
-inline int tiled_pair_mode() {
-    static const int mode = [] {
-        const char* e = getenv("LDG_QSR_PAIR");
-        return (e && e[0] == '0') ? 0 : ((e && e[0] == '1') ? 1 : 2);
-    }();
-    return mode;
-}
-inline bool tiled_pair_enabled() { return tiled_pair_mode() != 0; }
-
-// A single grid takes the two-cell kernel when its work list fills the GPU at least twice over
-// (two waves of four 128-thread CTAs per SM); a smaller list finishes sooner with one cell per
-// thread, whose 256-thread CTAs bring twice the warps to each item (64^3, R = 28: 0.0102 against
-// 0.0123 ms per step).
-inline bool tiled_use_pair(const TiledPlan& plan) {
-    if (tiled_pair_mode() != 2) return tiled_pair_mode() == 1;
+// Planes per work item. `cap` is the length asked for (the default, or a length the autotuner
+// tries); a list too short to fill the GPU at that length is cut further, by this estimate of a
+// step's time in microseconds: with n items on `slots` CTA slots,
+//     waves(n) * (kItem + c * kPlane),
+// kItem the first planes' way to shared memory, kPlane a plane of a CTA while its SM is shared (L1
+// only: 0.95 us alone to 1.75 us with five CTAs; with L2 / L3 2.6 us), waves fractional from the
+// fifth on (longest items first evens them out). An item on a face takes twice as long per plane.
+// Measured against it (64^3, R = 28, L1: 4.8 us at 1 plane, 17.1 at 16; 128^3: 13.9 us at 6, 20.2
+// at 16; 96^3 with L2 and L3: 15.1 us at 4, 24.8 at 16; 256^3: 8 to 16 within 2 %).
+inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, bool deep) {
     static const int sms = [] {
         int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) !=
-                                                      cudaSuccess)
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return 148;
         return n;
     }();
-    return plan.n_items >= 2 * 4 * sms;
+    if (cap < 8) return cap;
+    const int per_sm = deep ? 4 : 5;
+    const double kItem = deep ? 1.3 : 1.0, face_plane = deep ? 5.3 : 2.0;
+    int best = cap;
+    double best_t = std::numeric_limits<double>::infinity();
+    for (int c : {cap, 6, 4, 3, 2, 1}) {
+        long long n = 0;
+        bool faces = false;
+        for (const TiledPlan* p : plans)
+            tiled_each_item(*p, c, [&](int, int, int, int, bool f, int) {
+                ++n;
+                faces = faces || f;
+            });
+        const double full = (double)n / ((double)sms * per_sm);
+        const int m = (int)std::min<long long>(per_sm, (n + sms - 1) / sms);
+        const double waves = full > 4.0 ? full + 0.5 : std::ceil(full);
+        double t = waves * (kItem + c * (deep ? 2.6 : 0.75 + 0.2 * m));
+        if (faces) t = std::max(t, kItem + c * face_plane + 0.5 * t);
+        if (t < best_t) {
+            best_t = t;
+            best = c;
+        }
+        if (full > 24.0) break;  // shorter items only add halo planes
+    }
+    return best;
+}
+
+// The work list. Items are ordered longest first (an item on a face counting double): CTAs are
+// dispatched in item order, so the short items of the droplet's poles fill the last wave instead of
+// trailing it; among items of one length the plane chunk is slowest (CTAs resident together share
+// halo planes in L2). *active: the cells of the grid inside the items' tiles (read once per step).
+inline std::vector<int4> tiled_items(const TiledPlan& plan, int chunk, long long* active) {
+    struct Item {
+        int4 t;
+        int cost;
+    };
+    std::vector<Item> items;
+    long long act = 0;
+    tiled_each_item(plan, chunk, [&](int j0, int k0, int first, int end, bool face, int rows) {
+        items.push_back(Item{make_int4(j0, k0, first, end), (end - first) * (face ? 2 : 1)});
+        act += (long long)rows * (std::min(plan.Nz, k0 + tiled::TK) - std::max(0, k0)) * (end - first);
+    });
+    std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
+        if (a.cost != b.cost) return a.cost > b.cost;
+        if (a.t.z != b.t.z) return a.t.z < b.t.z;
+        if (a.t.x != b.t.x) return a.t.x < b.t.x;
+        return a.t.y < b.t.y;
+    });
+    std::vector<int4> out;
+    for (const Item& i : items) out.push_back(i.t);
+    if (active) *active = act;
+    return out;
 }
 
 inline int tiled_default_chunk() {
     int chunk = tiled::CHUNK;
-    if (const char* e = getenv("LDG_QSR_CHUNK")) chunk = std::min(4096, std::max(8, atoi(e)));
+    if (const char* e = getenv("LDG_QSR_CHUNK")) chunk = std::min(4096, std::max(1, atoi(e)));
     return chunk;
 }
 
-inline int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int Nz, int sj, long long si, long long sc) {
+inline int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int Nz, int sj, long long si, long long sc,
+                        bool L2) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
         void* fn = nullptr;
@@ -815,7 +752,7 @@ inline int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int 
     }
     cuuint64_t dims[4] = {(cuuint64_t)Nz, (cuuint64_t)Ny, (cuuint64_t)Nx, 5};
     cuuint64_t strides[3] = {(cuuint64_t)sj * 4, (cuuint64_t)si * 4, (cuuint64_t)sc * 4};
-    cuuint32_t box[4] = {tiled::RW, tiled::ROWS, 1, 5};
+    cuuint32_t box[4] = {tiled::RW, (cuuint32_t)(L2 ? tiled::Tile<true>::ROWS : tiled::Tile<false>::ROWS), 1, 5};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void*)base, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -827,18 +764,48 @@ inline int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int 
     return LDG_OK;
 }
 
-// Uploads the work list for chunks of `chunk` planes.
-inline int tiled_plan_rechunk(TiledPlan& plan, int chunk) {
+// Work items and their planes' row masks on the device. `inst` and `rec` are set for droplet `inst`
+// whose masks start at record rec0; returns the number of records through *n_rec.
+inline void tiled_device_items(const std::vector<int4>& list, int inst, int rec0, std::vector<tiled::TileItem>& out,
+                               int* n_rec) {
+    int rec = rec0;
+    for (const int4& t : list) {
+        out.push_back(tiled::TileItem{t.x, t.y, t.z, t.w, inst, rec, 0, 0});
+        rec += t.w - t.z;
+    }
+    *n_rec = rec - rec0;
+}
+inline int tiled_masks(const TiledPlan& plan, const tiled::TileItem* d_items, int n_items, bool L2,
+                       tiled::RowMask* d_masks) {
+    if (n_items == 0) return LDG_OK;
+    tiled::k_tile_masks<<<n_items, tiled::TK * tiled::TJ>>>(d_items, plan.flags, plan.Nx, plan.Ny, plan.Nz, plan.sj,
+                                                            plan.si, L2 ? 2 : 1, d_masks);
+    LDG_LAUNCHED("k_tile_masks");
+    return LDG_OK;
+}
+
+// Uploads the work list for items of at most `cap` planes (tiled_length).
+inline int tiled_plan_rechunk(TiledPlan& plan, int cap) {
+    const int chunk = tiled_length({&plan}, cap, plan.deep);
     long long active = 0;
     const std::vector<int4> items = tiled_items(plan, chunk, &active);
     plan.active_cells = active;
     if (plan.items) cudaFree(plan.items);
+    if (plan.masks) cudaFree(plan.masks);
     plan.items = nullptr;
+    plan.masks = nullptr;
     plan.n_items = (int)items.size();
     plan.chunk = chunk;
     if (plan.n_items > 0) {
-        LDG_CUDA(cudaMalloc(&plan.items, items.size() * sizeof(int4)));
-        LDG_CUDA(cudaMemcpy(plan.items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+        std::vector<tiled::TileItem> dev;
+        int n_rec = 0;
+        tiled_device_items(items, 0, 0, dev, &n_rec);
+        LDG_CUDA(cudaMalloc(&plan.items, dev.size() * sizeof(dev[0])));
+        LDG_CUDA(cudaMemcpy(plan.items, dev.data(), dev.size() * sizeof(dev[0]), cudaMemcpyHostToDevice));
+        LDG_CUDA(cudaMalloc(&plan.masks, (size_t)n_rec * tiled::MASK_BYTES));
+        int rc = tiled_masks(plan, plan.items, plan.n_items, plan.L2, plan.masks);
+        if (rc) return rc;
+        LDG_CUDA(cudaStreamSynchronize(nullptr));
     }
     std::vector<int4> planes;
     for (const int4& t : items)
@@ -855,10 +822,14 @@ inline int tiled_plan_rechunk(TiledPlan& plan, int chunk) {
 
 // Builds the work list from the host classification and encodes the two tensor maps.
 inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, long long si, const uint8_t* fl,
-                            const float* buf0, const float* buf1, long long sc) {
+                            const uint8_t* d_flags, const float* buf0, const float* buf1, long long sc, bool L2, bool L3) {
     using namespace tiled;
     plan = TiledPlan{};
-    plan.Nz = Nz;
+    plan.deep = L2 || L3;
+    plan.Nx = Nx; plan.Ny = Ny; plan.Nz = Nz;
+    plan.sj = sj; plan.si = si;
+    plan.flags = d_flags;
+    plan.L2 = L2;
     const int ntj = (Ny + TJ - 1) / TJ;
     long long written = 0;
     for (int jt = 0; jt < ntj; ++jt) {
@@ -878,6 +849,7 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
                         ++written;
                     }
         if (imax < 0) continue;
+        b.face = b.j0 < (L2 ? 2 : 1) || b.j0 + b.rows > Ny - (L2 ? 2 : 1);
         b.ib = imin;
         b.ie = imax + 1;
         b.kmin.assign(kmin.begin() + imin, kmin.begin() + imax + 1);
@@ -889,75 +861,59 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
     if (rc) return rc;
     LDG_CUDA(cudaMalloc(&plan.err, sizeof(int)));
     LDG_CUDA(cudaMemset(plan.err, 0, sizeof(int)));
-    rc = tiled_encode(&plan.tmap[0], buf0, Nx, Ny, Nz, sj, si, sc);
+    rc = tiled_encode(&plan.tmap[0], buf0, Nx, Ny, Nz, sj, si, sc, L2);
     if (rc) return rc;
-    rc = tiled_encode(&plan.tmap[1], buf1, Nx, Ny, Nz, sj, si, sc);
+    rc = tiled_encode(&plan.tmap[1], buf1, Nx, Ny, Nz, sj, si, sc, L2);
     if (rc) return rc;
     plan.bufs[0] = buf0;
     plan.bufs[1] = buf1;
-    plan.smem_bytes[0] = tile_smem_bytes<false>();
-    plan.smem_bytes[1] = tile_smem_bytes<true>();
-    plan.smem_bytes[2] = tile_smem_bytes<true, true>();
     plan.ok = true;
     return LDG_OK;
 }
 
 template <bool L2, bool L3, bool N, bool R, bool K>
-inline int tiled_launch_t(const TiledPlan& plan, int which, float* out, const uint8_t* flags, const QsrConst& P,
-                          cudaStream_t st, const float* lo_in, float* lo_out) {
+inline int tiled_launch_t(const TiledPlan& plan, int which, float* out, const QsrConst& P, cudaStream_t st,
+                          const float* lo_in, float* lo_out) {
     using namespace tiled;
-    const size_t smem = plan.smem_bytes[(L2 || L3) ? 1 : 0];
+    const auto k = k_step_tiled<L2, L3, N, R, K>;
+    constexpr size_t smem = tile_smem_bytes<L2>();
     static bool configured = false;
     if (!configured) {
-        LDG_CUDA(cudaFuncSetAttribute(k_step_tiled<L2, L3, N, R, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+        LDG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured = true;
     }
     if (plan.n_items == 0) return LDG_OK;
-    if (tiled_use_pair(plan)) {
-        const size_t smem2 = plan.smem_bytes[2];
-        static bool configured_pair = false;
-        if (!configured_pair) {
-            LDG_CUDA(cudaFuncSetAttribute(k_step_tiled_pair<L2, L3, N, R, K>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-            configured_pair = true;
-        }
-        k_step_tiled_pair<L2, L3, N, R, K><<<plan.n_items, PAIR_THREADS, smem2, st>>>(plan.tmap[which], out, flags,
-                                                                                     plan.items, P, plan.err, lo_in,
-                                                                                     lo_out);
-        return LDG_OK;
-    }
-    k_step_tiled<L2, L3, N, R, K><<<plan.n_items, THREADS, smem, st>>>(plan.tmap[which], out, flags, plan.items, P,
-                                                                       plan.err, lo_in, lo_out);
+    LDG_CUDA(launch_pdl(k, dim3((unsigned)plan.n_items), THREADS, smem, st, plan.tmap[which], plan.bufs[which], out,
+                        (const RowMask*)plan.masks, (const TileItem*)plan.items, P, plan.err, lo_in, lo_out));
     return LDG_OK;
 }
 
 template <bool R, bool K>
-inline int tiled_dispatch(const TiledPlan& plan, int which, float* out, const uint8_t* flags, const QsrConst& P,
+inline int tiled_dispatch(const TiledPlan& plan, int which, float* out, const QsrConst& P,
                           bool L2, bool L3, bool noise, cudaStream_t st, const float* lo_in, float* lo_out) {
     const int key = (L2 ? 1 : 0) | (L3 ? 2 : 0) | (noise ? 4 : 0);
     switch (key) {
-        case 0: return tiled_launch_t<false, false, false, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
-        case 1: return tiled_launch_t<true, false, false, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
-        case 2: return tiled_launch_t<false, true, false, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
-        case 3: return tiled_launch_t<true, true, false, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
-        case 4: return tiled_launch_t<false, false, true, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
-        case 5: return tiled_launch_t<true, false, true, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
-        case 6: return tiled_launch_t<false, true, true, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
-        default: return tiled_launch_t<true, true, true, R, K>(plan, which, out, flags, P, st, lo_in, lo_out);
+        case 0: return tiled_launch_t<false, false, false, R, K>(plan, which, out, P, st, lo_in, lo_out);
+        case 1: return tiled_launch_t<true, false, false, R, K>(plan, which, out, P, st, lo_in, lo_out);
+        case 2: return tiled_launch_t<false, true, false, R, K>(plan, which, out, P, st, lo_in, lo_out);
+        case 3: return tiled_launch_t<true, true, false, R, K>(plan, which, out, P, st, lo_in, lo_out);
+        case 4: return tiled_launch_t<false, false, true, R, K>(plan, which, out, P, st, lo_in, lo_out);
+        case 5: return tiled_launch_t<true, false, true, R, K>(plan, which, out, P, st, lo_in, lo_out);
+        case 6: return tiled_launch_t<false, true, true, R, K>(plan, which, out, P, st, lo_in, lo_out);
+        default: return tiled_launch_t<true, true, true, R, K>(plan, which, out, P, st, lo_in, lo_out);
     }
 }
 
 // One step through the tiled kernel. `in` must be one of the two planned buffers. With lo_out
 // set (explicit steps only) the step uses compensated storage: lo_in / lo_out are the low
 // words of the input and output buffers.
-inline int tiled_step(const TiledPlan& plan, const float* in, float* out, const uint8_t* flags, const QsrConst& P,
+inline int tiled_step(const TiledPlan& plan, const float* in, float* out, const QsrConst& P,
                       bool L2, bool L3, bool noise, bool rhs, cudaStream_t st, const float* lo_in = nullptr,
                       float* lo_out = nullptr) {
     const int which = (in == plan.bufs[0]) ? 0 : 1;
-    if (rhs) return tiled_dispatch<true, false>(plan, which, out, flags, P, L2, L3, noise, st, nullptr, nullptr);
-    if (lo_out) return tiled_dispatch<false, true>(plan, which, out, flags, P, L2, L3, noise, st, lo_in, lo_out);
-    return tiled_dispatch<false, false>(plan, which, out, flags, P, L2, L3, noise, st, nullptr, nullptr);
+    if (rhs) return tiled_dispatch<true, false>(plan, which, out, P, L2, L3, noise, st, nullptr, nullptr);
+    if (lo_out) return tiled_dispatch<false, true>(plan, which, out, P, L2, L3, noise, st, lo_in, lo_out);
+    return tiled_dispatch<false, false>(plan, which, out, P, L2, L3, noise, st, nullptr, nullptr);
 }
 
 // Reads and clears the device error word (LDG_OK when no bounded wait gave up).
@@ -976,6 +932,7 @@ inline int tiled_check(const TiledPlan& plan, cudaStream_t st) {
 
 inline void tiled_plan_free(TiledPlan& plan) {
     if (plan.items) cudaFree(plan.items);
+    if (plan.masks) cudaFree(plan.masks);
     if (plan.plane_items) cudaFree(plan.plane_items);
     cudaFree(plan.err);
     plan = TiledPlan{};
