@@ -1,8 +1,14 @@
 // Periodic bulk LdG solver (KZM_bulk_ldg drop-in): device kernels and the kzm_* C ABI.
 //
-// Device layout: FP32 SoA, x fastest (the reference's flatten order, KZM_bulk_ldg.cu:161-169),
-// rows padded to a multiple of 4 floats. One fused kernel per step: periodic 7-point
-// Laplacian, bulk field, traceless projection, Euler, Philox Langevin noise, optional cap.
+// Device layout: FP32 SoA, x fastest (the reference's flatten order, KZM_bulk_ldg.cu:161-169). Each
+// row carries its periodic neighbours: columns x = -1 and x = Nx hold copies of x = Nx - 1 and x = 0,
+// and each plane has the rows y = -1 and y = Ny, all written by whoever writes the site. A tile with
+// its halo is then one rectangle of memory for any Nx and Ny, which a single TMA box fetches; z wraps
+// by the plane index. One fused kernel per step: periodic 7-point Laplacian, bulk field, traceless
+// projection, Euler, Philox Langevin noise, optional cap.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -13,6 +19,7 @@
 
 #include "ldg_api_common.h"
 #include "ldg_common.cuh"
+#include "sm100_ptx.cuh"
 
 using namespace ldg;
 
@@ -22,15 +29,48 @@ constexpr double kPi = 3.14159265358979323846;
 
 struct KzmConst {
     int Nx, Ny, Nz;
-    int sy;          // row pitch (x fastest)
+    int sy;          // row pitch (x fastest); arrays start at site (0, 0, 0), kPadX columns and one row in
     long long sz;    // plane pitch
     long long sc;    // component pitch
     float ix2, iy2, iz2;
     float lap_c;     // -2 (1/dx^2 + 1/dy^2 + 1/dz^2): centre weight of the Laplacian
+    // both halves equal, for the packed arithmetic: -kappa/da^2, -kappa lap_c, -dt/gamma and the bulk
+    // coefficients
+    F2 mkx, mky, mkz, mk0, mmob;
+    BulkC<F2> K;
     float A, B, C, kappa, mob_dt, qcap, sigma;
     uint32_t key0, key1;
     long long step;
 };
+
+// Columns before x = 0, and the multiple of floats of a row: 32 bytes, so that the rows a warp stores
+// (x0 a multiple of 32) are whole sectors. Rows that cut sectors held the step back more than anything
+// else: the same loads and stores without arithmetic take 164 us a step at 256^3 with rows starting
+// 16 bytes into a sector and 110 us with whole sectors (a plain copy of the field takes 112 us).
+constexpr int kPadX = 8;
+constexpr int kHaloX = 4;  // columns of a TMA box before x0 (the box start stays on 16 bytes)
+
+// Copies of a site on a face of the box in the periodic halo (five values at stride sc).
+__device__ __forceinline__ void store_halo(float* __restrict__ out, const KzmConst& P, int x, int y, long long id,
+                                           const float v[5]) {
+    if (x == 0 || x == P.Nx - 1) {
+        const long long o = id + (x == 0 ? P.Nx : -P.Nx);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) out[m * P.sc + o] = v[m];
+    }
+    if (y == 0 || y == P.Ny - 1) {
+        const long long o = id + (long long)(y == 0 ? P.Ny : -P.Ny) * P.sy;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) out[m * P.sc + o] = v[m];
+    }
+}
+// Writes a site and its halo copies.
+__device__ __forceinline__ void store_site(float* __restrict__ out, const KzmConst& P, int x, int y, long long id,
+                                           const float v[5]) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) out[m * P.sc + id] = v[m];
+    store_halo(out, P, x, y, id, v);
+}
 
 // One periodic step: block (32, 8) over (x, y), grid z over planes (KZM_bulk_ldg.cu:351-469).
 template <bool kNoise>
@@ -86,350 +126,168 @@ __global__ void __launch_bounds__(256) k_kzm_step(const float* __restrict__ q, f
             for (int m = 0; m < 5; ++m) u[m] *= s;
         }
     }
-#pragma unroll
-    for (int m = 0; m < 5; ++m) out[m * P.sc + id] = u[m];
+    store_site(out, P, x, y, id, u);
 }
 
-// The same step as k_kzm_step for a (32 x 8) column tile marching along z over a chunk of
-// planes. Each thread keeps its column's planes z-1, z, z+1 in registers and prefetches
-// z+2 and z+3; the x/y neighbours come from a shared (34 x 10) tile whose halo holds the
-// periodically wrapped values (any N >= 2). Every input value is loaded about once from
-// HBM (halo columns from L2) and every site is written once.
-constexpr int KTX = 32, KTY = 8, KZC = 32;
+// The step over (32 x 8) column tiles marching along z over a chunk of planes: 128 threads, each
+// updating two sites (rows 2w and 2w + 1 of warp w) as one packed FP32 instruction stream (FFMA2 /
+// FADD2 / FMUL2); the noise draw, the cap and the stores are per site. A plane of the tile with its
+// halo (40 columns from x0 - 4, 10 rows, 5 components) is one TMA box in a ring of KNQ slots. A site's
+// centre column is carried in registers (z - 1, z; z + 1 is read when its plane arrives), so a
+// plane is read for its neighbours at its own step only, can be refilled right after it, and costs
+// eight shared loads per component and pair instead of fourteen. The warps march independently: the
+// last one done with a plane issues the load that reuses its slot.
+// With noise it is bound by issue slots (240 instructions a site, 102 of them the draw, at 72 % issue
+// efficiency); without, by HBM (256^3: 5.0 TB/s of the 6.1 that the same loads and stores reach without
+// arithmetic).
+constexpr int KTX = 32, KTY = 8;
+constexpr int KTHREADS = KTX * KTY / 2, KWARPS = KTHREADS / 32;
+constexpr int KROW = KTX + 2 * kHaloX;        // floats per ring row: x0 - 4 .. x0 + 35
+constexpr int KROWS = KTY + 2;
+constexpr int KCSTR = KROW * KROWS;           // floats per component plane
+constexpr int KSLOT = (5 * KCSTR + 31) / 32 * 32;  // floats per slot (128-byte aligned)
+constexpr uint32_t KBYTES = 5 * KCSTR * 4;
+constexpr int KNQ = 5;                        // slots: planes z and z + 1 in use, three in flight
+constexpr int KCTAS = 5;                      // CTAs per SM
+constexpr size_t kRingBytes = (size_t)KNQ * KSLOT * 4 + KNQ * 8 + KNQ * 4 + 4;
+
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(sm100::smem_u32(dst)),
+        "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(0), "r"(sm100::smem_u32(bar))
+        : "memory");
+}
+
 template <bool kNoise>
-__global__ void __launch_bounds__(KTX* KTY) k_kzm_step_tiled(const float* __restrict__ q, float* __restrict__ out,
-                                                             KzmConst P) {
-    __shared__ float s[5][KTY + 2][KTX + 2];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * KTX, y0 = blockIdx.y * KTY, z0 = blockIdx.z * KZC;
-    const int z1 = min(z0 + KZC, P.Nz);
-    const int xr = x0 + tx, yr = y0 + ty;
-    const bool valid = (xr < P.Nx) && (yr < P.Ny);
-    const int x = xr % P.Nx, y = yr % P.Ny;
-    const long long row = (long long)y * P.sy;
-    const long long rowm = (long long)((y0 + P.Ny - 1) % P.Ny) * P.sy;   // halo row y0-1
-    const long long rowp = (long long)((y0 + KTY) % P.Ny) * P.sy;        // halo row y0+KTY
-    const int xm = (x0 + P.Nx - 1) % P.Nx, xp = (x0 + KTX) % P.Nx;       // halo columns
-    // z stays within [-1, 2 Nz) here (Nz >= 2), so one compare-and-add wraps it.
-    auto zw = [&](int z) { return z < 0 ? z + P.Nz : (z >= P.Nz ? z - P.Nz : z); };
-    auto load5 = [&](int z, float v[5]) {
-        const long long o = (long long)zw(z) * P.sz + row + x;
-#pragma unroll
-        for (int m = 0; m < 5; ++m) v[m] = __ldg(q + m * P.sc + o);
+__global__ void __launch_bounds__(KTHREADS, KCTAS)
+    k_kzm_step_ring(const __grid_constant__ CUtensorMap tm, float* __restrict__ out, KzmConst P, int planes,
+                    int* __restrict__ err) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    float* ring = reinterpret_cast<float*>(smem);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(ring + KNQ * KSLOT);
+    unsigned* freed = reinterpret_cast<unsigned*>(bar + KNQ);
+    int* s_abort = reinterpret_cast<int*>(freed + KNQ);
+    const int tid = threadIdx.x, tx = tid & 31, w = tid >> 5;
+    const int x0 = blockIdx.x * KTX, y0 = blockIdx.y * KTY, z0 = blockIdx.z * planes;
+    const int z1 = min(z0 + planes, P.Nz);
+    if (tid == 0) {
+        for (int s = 0; s < KNQ; ++s) {
+            sm100::mbar_init(&bar[s], 1);
+            freed[s] = 0;
+        }
+        sm100::fence_mbar_init();
+        *s_abort = 0;
+    }
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    // Plane p of this chunk (z0 - 1 <= p <= z1) in slot (p - z0 + 1) % KNQ.
+    auto issue = [&](int p, int sl) {
+        if (p > z1) return;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        sm100::mbar_expect_tx(&bar[sl], KBYTES);
+        const int zw = p < 0 ? p + P.Nz : (p >= P.Nz ? p - P.Nz : p);
+        tma_load_4d(ring + sl * KSLOT, &tm, x0 + kPadX - kHaloX, y0, zw, &bar[sl]);
     };
-    float qm[5], qc[5], qp[5], qn[5], qn2[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    load5(z0 - 1, qm);
-    load5(z0, qc);
-    load5(z0 + 1, qp);
-    load5(z0 + 2, qn);
-    const uint32_t cell_base = (uint32_t)(x + P.Nx * y);
-    for (int z = z0; z < z1; ++z) {
-        if (z + 3 < z1 + 1) load5(z + 3, qn2);
-        const long long pz = (long long)zw(z) * P.sz;
-#pragma unroll
-        for (int m = 0; m < 5; ++m) s[m][ty + 1][tx + 1] = qc[m];
-        if (ty == 0) {
-#pragma unroll
-            for (int m = 0; m < 5; ++m) s[m][0][tx + 1] = __ldg(q + m * P.sc + pz + rowm + x);
-        }
-        if (ty == KTY - 1) {
-#pragma unroll
-            for (int m = 0; m < 5; ++m) s[m][KTY + 1][tx + 1] = __ldg(q + m * P.sc + pz + rowp + x);
-        }
+    if (tid == 0)
+        for (int s = 0; s < KNQ; ++s) issue(z0 - 1 + s, s);
+    bool ok = true;
+    uint32_t par = 0;  // parity of the next wait on every slot
+    auto wait_slot = [&](int sl) {
+        const uint32_t ph = (par >> sl) & 1u;
+        par ^= 1u << sl;
+        if (sm100::mbar_try_wait(&bar[sl], ph)) return;
+        const long long t0 = clock64();
+        while (!sm100::mbar_try_wait(&bar[sl], ph))
+            if (*(volatile int*)s_abort || clock64() - t0 > 4000000000ll) {  // about 2 s
+                atomicExch(err, LDG_ERR_TIMEOUT);
+                *(volatile int*)s_abort = 1;
+                ok = false;
+                return;
+            }
+    };
+    // This warp is done with plane p: the last warp refills its slot with plane p + KNQ.
+    auto done = [&](int p, int sl) {
+        __syncwarp();
         if (tx == 0) {
-#pragma unroll
-            for (int m = 0; m < 5; ++m) s[m][ty + 1][0] = __ldg(q + m * P.sc + pz + row + xm);
+            unsigned old;
+            asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
+                         : "=r"(old)
+                         : "r"(sm100::smem_u32(&freed[sl]))
+                         : "memory");
+            if (old % (unsigned)KWARPS == (unsigned)KWARPS - 1u) issue(p + KNQ, sl);
         }
-        if (tx == KTX - 1) {
+    };
+    const int x = x0 + tx, y = y0 + 2 * w;
+    const bool v0 = x < P.Nx && y < P.Ny, v1 = x < P.Nx && y + 1 < P.Ny;
+    const int s_c = (2 * w + 1) * KROW + tx + kHaloX;
+    const bool edge = x == 0 || x == P.Nx - 1 || y == 0 || y >= P.Ny - 2;
+    float* o = out + (long long)z0 * P.sz + (long long)y * P.sy + x;
+    uint32_t cell = (uint32_t)x + (uint32_t)P.Nx * ((uint32_t)y + (uint32_t)P.Ny * (uint32_t)z0);
+    const uint32_t cells_z = (uint32_t)P.Nx * (uint32_t)P.Ny;
+    F2 cm[5], c[5];
+    wait_slot(0);
 #pragma unroll
-            for (int m = 0; m < 5; ++m) s[m][ty + 1][KTX + 1] = __ldg(q + m * P.sc + pz + row + xp);
-        }
-        __syncthreads();
-        if (valid) {
-            float lap[5];
+    for (int m = 0; m < 5; ++m) cm[m] = mk2(ring[m * KCSTR + s_c], ring[m * KCSTR + s_c + KROW]);
+    done(z0 - 1, 0);
+    wait_slot(1);
 #pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                const float c = qc[m];
-                lap[m] = fmaf(P.ix2, s[m][ty + 1][tx + 2] + s[m][ty + 1][tx],
-                              fmaf(P.iy2, s[m][ty + 2][tx + 1] + s[m][ty][tx + 1],
-                                   fmaf(P.iz2, qp[m] + qm[m], P.lap_c * c)));
-            }
-            float h[6];
-            bulk_field(qc, P.A, P.B, P.C, h);
-            h[0] -= P.kappa * lap[0];
-            h[1] -= P.kappa * lap[3];
-            h[2] += P.kappa * (lap[0] + lap[3]);
-            h[3] -= P.kappa * lap[1];
-            h[4] -= P.kappa * lap[2];
-            h[5] -= P.kappa * lap[4];
-            const float corr = (h[0] + h[1] + h[2]) * (1.0f / 3.0f);
-            float u[5] = {qc[0] - P.mob_dt * (h[0] - corr), qc[1] - P.mob_dt * h[3], qc[2] - P.mob_dt * h[4],
-                          qc[3] - P.mob_dt * (h[1] - corr), qc[4] - P.mob_dt * h[5]};
-            if (kNoise) {
-                float g[5];
-                normals5(cell_base + (uint32_t)P.Nx * (uint32_t)P.Ny * (uint32_t)z, 0u, P.step, P.key0, P.key1, g);
-#pragma unroll
-                for (int m = 0; m < 5; ++m) u[m] += P.sigma * g[m];
-            }
-            if (P.qcap > 0.0f) {
-                const float zz = -u[0] - u[3];
-                const float tr = u[0] * u[0] + u[3] * u[3] + zz * zz + 2.0f * (u[1] * u[1] + u[2] * u[2] + u[4] * u[4]);
-                const float qn_ = sqrtf(fmaxf(tr, 0.0f));
-                if (qn_ > P.qcap && qn_ > 0.0f) {
-                    const float sc = P.qcap / qn_;
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) u[m] *= sc;
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < 5; ++m) out[m * P.sc + pz + row + x] = u[m];
-        }
-        __syncthreads();
+    for (int m = 0; m < 5; ++m) c[m] = mk2(ring[KSLOT + m * KCSTR + s_c], ring[KSLOT + m * KCSTR + s_c + KROW]);
+    int sl = 1, sn = 2 % KNQ;  // slots of planes z and z + 1
+    int waited = z0 + 1;       // planes below this one were waited for
+    for (int z = z0; z < z1; ++z, o += P.sz, cell += cells_z) {
+        wait_slot(sn);
+        waited = z + 2;
+        if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp stops or none of it
+        const float* pc = ring + sl * KSLOT + s_c;
+        const float* pn = ring + sn * KSLOT + s_c;
+        F2 h[5], u[5];
+        bulk_field5<F2>(c, P.K, h);
 #pragma unroll
         for (int m = 0; m < 5; ++m) {
-            qm[m] = qc[m];
-            qc[m] = qp[m];
-            qp[m] = qn[m];
-            qn[m] = qn2[m];
+            const float* s = pc + m * KCSTR;
+            const F2 cp = mk2(pn[m * KCSTR], pn[m * KCSTR + KROW]);
+            const F2 sx = mk2(s[1], s[KROW + 1]) + mk2(s[-1], s[KROW - 1]);
+            // row y + 1 of the first site is the second site, and the other way round
+            const F2 sy = mk2(c[m].v.y + s[-KROW], s[2 * KROW] + c[m].v.x);
+            const F2 e = vfma(P.mkx, sx, vfma(P.mky, sy, vfma(P.mkz, cp + cm[m], vfma(P.mk0, c[m], h[m]))));
+            u[m] = vfma(P.mmob, e, c[m]);
+            cm[m] = c[m];
+            c[m] = cp;
         }
-    }
-}
-
-// Asynchronous-copy variant: every plane of the tile plus its periodically wrapped halo is
-// fetched with cp.async (4-byte copies, any wrapped address) into a 5-plane shared ring two
-// planes ahead of use, so no thread waits on a global load inside the plane loop; x, y and z
-// neighbours all come from shared memory; one CTA barrier per plane.
-constexpr int KRING = 5;
-constexpr int KPS = (KTY + 2) * (KTX + 2);  // floats per component plane of the ring
-__device__ __forceinline__ void cp_async4(float* sdst, const float* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(sdst)),
-                 "l"(gsrc)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-template <bool kNoise>
-__global__ void __launch_bounds__(KTX* KTY) k_kzm_step_async(const float* __restrict__ q, float* __restrict__ out,
-                                                             KzmConst P) {
-    extern __shared__ __align__(16) float ring[];  // [KRING][5][KTY+2][KTX+2]
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x0 = blockIdx.x * KTX, y0 = blockIdx.y * KTY, z0 = blockIdx.z * KZC;
-    const int z1 = min(z0 + KZC, P.Nz);
-    const int xr = x0 + tx, yr = y0 + ty;
-    const bool valid = (xr < P.Nx) && (yr < P.Ny);
-    const int x = xr % P.Nx, y = yr % P.Ny;
-    const long long g_c = (long long)y * P.sy + x;
-    const int s_c = (ty + 1) * (KTX + 2) + tx + 1;
-    // Flat copy list: the 5 x (KTY+2) x (KTX+2) ring entries of a plane spread over the CTA's
-    // threads; each thread's (global in-plane offset, shared offset) pairs are the same for every
-    // plane, so they are formed once here (wrapped periodically).
-    constexpr int NE = 5 * KPS;
-    constexpr int PER = (NE + KTX * KTY - 1) / (KTX * KTY);
-    const int tid = ty * KTX + tx;
-    long long goff[PER];
-    int soff[PER];
-#pragma unroll
-    for (int t = 0; t < PER; ++t) {
-        const int e = tid + t * KTX * KTY;
-        const int m = e / KPS, cell = e - m * KPS;
-        const int r = cell / (KTX + 2), cc = cell - r * (KTX + 2);
-        const int gx = (x0 - 1 + cc + P.Nx) % P.Nx, gy = (y0 - 1 + r + P.Ny) % P.Ny;
-        goff[t] = (long long)min(m, 4) * P.sc + (long long)gy * P.sy + gx;
-        soff[t] = e;
-    }
-    auto zw = [&](int z) { return z < 0 ? z + P.Nz : (z >= P.Nz ? z - P.Nz : z); };
-    auto issue = [&](int p) {
-        float* dst = ring + ((p + KRING) % KRING) * NE;
-        const float* src = q + (long long)zw(p) * P.sz;
-#pragma unroll
-        for (int t = 0; t < PER; ++t)
-            if (t < PER - 1 || soff[t] < NE) cp_async4(dst + soff[t], src + goff[t]);
-    };
-    // Prologue: planes z0-1 .. z0+2, one commit group each.
-    for (int p = z0 - 1; p <= z0 + 2; ++p) {
-        issue(p);
-        cp_async_commit();
-    }
-    const uint32_t cell_base = (uint32_t)(x + P.Nx * y);
-    for (int z = z0; z < z1; ++z) {
-        cp_async_wait<1>();  // all groups but the newest (plane z+2): planes z-1 .. z+1 are in
-        __syncthreads();     // every thread's copies visible; every thread done with plane z-2
-        if (z + 3 <= z1) issue(z + 3);  // into the slot of plane z-2
-        cp_async_commit();
-        if (valid) {
-            const float* pm = ring + ((z - 1 + KRING) % KRING) * 5 * KPS;
-            const float* pc = ring + ((z + KRING) % KRING) * 5 * KPS;
-            const float* pp = ring + ((z + 1) % KRING) * 5 * KPS;
-            float c[5], lap[5];
-#pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                const float* s = pc + m * KPS + s_c;
-                c[m] = s[0];
-                // sum_a (Q[+1] + Q[-1]) / da^2 - 2 Q sum_a 1/da^2 as one fused chain
-                lap[m] = fmaf(P.ix2, s[1] + s[-1],
-                              fmaf(P.iy2, s[KTX + 2] + s[-(KTX + 2)],
-                                   fmaf(P.iz2, pp[m * KPS + s_c] + pm[m * KPS + s_c], P.lap_c * c[m])));
-            }
-            float h[6];
-            bulk_field(c, P.A, P.B, P.C, h);
-            h[0] -= P.kappa * lap[0];
-            h[1] -= P.kappa * lap[3];
-            h[2] += P.kappa * (lap[0] + lap[3]);
-            h[3] -= P.kappa * lap[1];
-            h[4] -= P.kappa * lap[2];
-            h[5] -= P.kappa * lap[4];
-            const float corr = (h[0] + h[1] + h[2]) * (1.0f / 3.0f);
-            float u[5] = {c[0] - P.mob_dt * (h[0] - corr), c[1] - P.mob_dt * h[3], c[2] - P.mob_dt * h[4],
-                          c[3] - P.mob_dt * (h[1] - corr), c[4] - P.mob_dt * h[5]};
-            if (kNoise) {
-                float g[5];
-                normals5(cell_base + (uint32_t)P.Nx * (uint32_t)P.Ny * (uint32_t)z, 0u, P.step, P.key0, P.key1, g);
-#pragma unroll
-                for (int m = 0; m < 5; ++m) u[m] += P.sigma * g[m];
-            }
-            if (P.qcap > 0.0f) {
-                const float zz = -u[0] - u[3];
-                const float tr = u[0] * u[0] + u[3] * u[3] + zz * zz + 2.0f * (u[1] * u[1] + u[2] * u[2] + u[4] * u[4]);
-                const float qn_ = sqrtf(fmaxf(tr, 0.0f));
-                if (qn_ > P.qcap && qn_ > 0.0f) {
-                    const float sc = P.qcap / qn_;
-#pragma unroll
-                    for (int m = 0; m < 5; ++m) u[m] *= sc;
-                }
-            }
-            float* o = out + (long long)z * P.sz + g_c;
-#pragma unroll
-            for (int m = 0; m < 5; ++m) o[m * P.sc] = u[m];
-        }
-    }
-    cp_async_wait<0>();  // no copy into this CTA's shared memory outlives it
-}
-
-// Two sites per thread: 128 threads over the same (32 x 8) tile and plane loop as
-// k_kzm_step_async, thread (tx, ty) updating rows ty and ty + 4. For Nx a multiple of 4 (so every
-// row pitch, plane pitch and component pitch is too) each ring row holds the 40 columns
-// x0 - 4 .. x0 + 35 and is fetched as ten 16-byte copies whose sources are 16-byte aligned and
-// either wholly inside the box or wholly wrapped (x0 is a multiple of 32): 500 copies per plane
-// instead of 1700 four-byte ones. The Laplacian, bulk field and update of both sites run as one
-// packed FP32 instruction stream (FFMA2 / FADD2 / FMUL2: per site the same fused operations as
-// the one-site kernel); the noise draw, the cap and the stores stay per site.
-constexpr int KPT = KTX * KTY / 2;
-constexpr int KROW2 = KTX + 8;               // ring row of the two-site kernel: x0 - 4 .. x0 + 35
-constexpr int KPS2 = (KTY + 2) * KROW2;      // floats per component plane
-constexpr size_t kRingBytes2 = (size_t)KRING * 5 * KPS2 * sizeof(float);
-__device__ __forceinline__ void cp_async16(float* sdst, const float* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sdst)),
-                 "l"(gsrc)
-                 : "memory");
-}
-template <bool kNoise>
-__global__ void __launch_bounds__(KPT) k_kzm_step_pair(const float* __restrict__ q, float* __restrict__ out,
-                                                       KzmConst P) {
-    extern __shared__ __align__(16) float ring[];  // [KRING][5][KTY+2][KROW2]
-    constexpr int ROW = KROW2;
-    constexpr int KPS = KPS2;
-    const int tid = threadIdx.x;
-    const int tx = tid & 31, ty = tid >> 5;
-    const int x0 = blockIdx.x * KTX, y0 = blockIdx.y * KTY, z0 = blockIdx.z * KZC;
-    const int z1 = min(z0 + KZC, P.Nz);
-    const int xr = x0 + tx;
-    const int x = xr % P.Nx;
-    bool valid[2];
-    long long g_c[2];
-    uint32_t cell_base[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int yr = y0 + ty + 4 * r;
-        valid[r] = (xr < P.Nx) && (yr < P.Ny);
-        const int y = yr % P.Ny;
-        g_c[r] = (long long)y * P.sy + x;
-        cell_base[r] = (uint32_t)(x + P.Nx * y);
-    }
-    const int s_c = (ty + 1) * ROW + tx + 4;  // row ty; row ty + 4 is 4 * ROW further
-    constexpr int NE = 5 * KPS;               // floats per ring plane
-    constexpr int NCH = NE / 4;               // 16-byte chunks per ring plane
-    constexpr int PER = (NCH + KPT - 1) / KPT;
-    long long goff[PER];
-#pragma unroll
-    for (int t = 0; t < PER; ++t) {
-        const int e = min(tid + t * KPT, NCH - 1);
-        const int m = e / (KPS / 4), rem = e - m * (KPS / 4);
-        const int r = rem / (ROW / 4), c4 = rem - r * (ROW / 4);
-        const int gx = (x0 - 4 + 4 * c4 + P.Nx) % P.Nx, gy = (y0 - 1 + r + P.Ny) % P.Ny;
-        goff[t] = (long long)m * P.sc + (long long)gy * P.sy + gx;
-    }
-    auto zw = [&](int z) { return z < 0 ? z + P.Nz : (z >= P.Nz ? z - P.Nz : z); };
-    auto issue = [&](int p) {
-        float* dst = ring + ((p + KRING) % KRING) * NE;
-        const float* src = q + (long long)zw(p) * P.sz;
-#pragma unroll
-        for (int t = 0; t < PER; ++t)
-            if (t < PER - 1 || tid + t * KPT < NCH) cp_async16(dst + 4 * (tid + t * KPT), src + goff[t]);
-    };
-    for (int p = z0 - 1; p <= z0 + 2; ++p) {
-        issue(p);
-        cp_async_commit();
-    }
-    const bool any_valid = valid[0] || valid[1];
-    for (int z = z0; z < z1; ++z) {
-        cp_async_wait<1>();  // planes z-1 .. z+1 are in
-        __syncthreads();     // every thread's copies visible; every thread done with plane z-2
-        if (z + 3 <= z1) issue(z + 3);
-        cp_async_commit();
-        if (any_valid) {
-            const float* pm = ring + ((z - 1 + KRING) % KRING) * NE + s_c;
-            const float* pc = ring + ((z + KRING) % KRING) * NE + s_c;
-            const float* pp = ring + ((z + 1) % KRING) * NE + s_c;
-            auto at = [](const float* b, int off) { return mk2(b[off], b[off + 4 * ROW]); };
-            F2 c[5], lap[5];
-#pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                const float* sc = pc + m * KPS;
-                c[m] = at(sc, 0);
-                lap[m] = vfma(P.ix2, at(sc, 1) + at(sc, -1),
-                              vfma(P.iy2, at(sc, ROW) + at(sc, -ROW),
-                                   vfma(P.iz2, at(pp + m * KPS, 0) + at(pm + m * KPS, 0), P.lap_c * c[m])));
-            }
-            F2 h[5], u[5];
-            bulk_field5<F2>(c, P.A, P.B, P.C, h);
-#pragma unroll
-            for (int m = 0; m < 5; ++m) u[m] = vfma(-P.mob_dt, vfma(-P.kappa, lap[m], h[m]), c[m]);
-            float v[2][5];
-#pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                v[0][m] = u[m].v.x;
-                v[1][m] = u[m].v.y;
-            }
+        done(z, sl);
+        if (v0) {
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                if (!valid[r]) continue;
+                if (r && !v1) continue;
+                float v[5];
+#pragma unroll
+                for (int m = 0; m < 5; ++m) v[m] = r ? u[m].v.y : u[m].v.x;
                 if (kNoise) {
                     float g[5];
-                    normals5(cell_base[r] + (uint32_t)P.Nx * (uint32_t)P.Ny * (uint32_t)z, 0u, P.step, P.key0,
-                             P.key1, g);
+                    normals5(cell + (r ? (uint32_t)P.Nx : 0u), 0u, P.step, P.key0, P.key1, g);
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) v[r][m] = fmaf(P.sigma, g[m], v[r][m]);
+                    for (int m = 0; m < 5; ++m) v[m] = fmaf(P.sigma, g[m], v[m]);
                 }
-                if (P.qcap > 0.0f) {
-                    const float zz = -v[r][0] - v[r][3];
-                    const float tr = v[r][0] * v[r][0] + v[r][3] * v[r][3] + zz * zz +
-                                     2.0f * (v[r][1] * v[r][1] + v[r][2] * v[r][2] + v[r][4] * v[r][4]);
-                    const float qn_ = sqrtf(fmaxf(tr, 0.0f));
-                    if (qn_ > P.qcap && qn_ > 0.0f) {
-                        const float sc = P.qcap / qn_;
+                if (P.qcap > 0.0f) cap_norm(P.qcap, v);
+                float* d = r ? o + P.sy : o;
 #pragma unroll
-                        for (int m = 0; m < 5; ++m) v[r][m] *= sc;
-                    }
-                }
-                float* o = out + (long long)z * P.sz + g_c[r];
-#pragma unroll
-                for (int m = 0; m < 5; ++m) o[m * P.sc] = v[r][m];
+                for (int m = 0; m < 5; ++m) d[m * P.sc] = v[m];
+                if (edge) store_halo(d, P, x, y + r, 0, v);
             }
         }
+        sl = sn;
+        sn = sn + 1 == KNQ ? 0 : sn + 1;
     }
-    cp_async_wait<0>();  // no copy into this CTA's shared memory outlives it
+    if (!ok)  // after an abort: copies that may be in flight, for a bounded time
+        for (int p = waited; p <= z1; ++p) {
+            const int s = (p - z0 + 1) % KNQ;
+            const long long t0 = clock64();
+            while (!sm100::mbar_try_wait(&bar[s], (par >> s) & 1u) && clock64() - t0 < 40000000ll) {
+            }
+            par ^= 1u << s;
+        }
 }
 
 __global__ void k_kzm_from_aos(const double* __restrict__ aos, float* __restrict__ a, KzmConst P) {
@@ -440,8 +298,10 @@ __global__ void k_kzm_from_aos(const double* __restrict__ aos, float* __restrict
         const int y = (int)(r % P.Ny);
         const int z = (int)(r / P.Ny);
         const long long id = (long long)z * P.sz + (long long)y * P.sy + x;
+        float v[5];
 #pragma unroll
-        for (int m = 0; m < 5; ++m) a[m * P.sc + id] = (float)aos[5 * t + m];
+        for (int m = 0; m < 5; ++m) v[m] = (float)aos[5 * t + m];
+        store_site(a, P, x, y, id, v);
     }
 }
 
@@ -722,16 +582,70 @@ int alloc_or_fail(void** p, size_t bytes) {
     return LDG_OK;
 }
 
+int kzm_encode(CUtensorMap* tm, const float* alloc, const KzmConst& P) {
+    static void* const fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool got = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
+                         q == cudaDriverEntryPointSuccess;
+        return got ? f : nullptr;
+    }();
+    LDG_REQUIRE(fn, LDG_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
+    cuuint64_t dims[4] = {(cuuint64_t)P.sy, (cuuint64_t)P.Ny + 2, (cuuint64_t)P.Nz, 5};
+    cuuint64_t strides[3] = {(cuuint64_t)P.sy * 4, (cuuint64_t)P.sz * 4, (cuuint64_t)P.sc * 4};
+    cuuint32_t box[4] = {KROW, KROWS, 1, 5}, estr[4] = {1, 1, 1, 1};
+    const CUresult r = ((PFN_cuTensorMapEncodeTiled_v12000)fn)(
+        tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(alloc), dims, strides, box, estr,
+        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("kzm: cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
+        return LDG_ERR_CUDA;
+    }
+    return LDG_OK;
+}
+
+// Planes per CTA: the chunk length with the least estimated time. A CTA takes 0.95 us and 0.57 + 0.265 m
+// us per plane (with noise) where m CTAs share its SM; full waves of KCTAS per SM, then the rest.
+// Measured (us per step with noise): 64^3 6.8 / 6.3 / 8.6 / 28.9 at 2 / 4 / 8 / 32 planes (one chunk
+// length of 32 for every grid before: 29.7), 128^3 30.5 / 28.3 / 28.5 / 34.1 at 2 / 4 / 8 / 16 (40.5),
+// 256^3 212 / 190 / 182 / 181 (203); without noise 164 / 142 / 136 / 139 (160).
+// LDG_KZM_PLANES forces a length.
+int kzm_planes(const KzmConst& P) {
+    const int lo = (P.Nz + 65534) / 65535;  // the launch grid's z extent is limited
+    if (const char* e = getenv("LDG_KZM_PLANES")) return std::min(P.Nz, std::max(lo, atoi(e)));
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long tiles = (long long)((P.Nx + KTX - 1) / KTX) * ((P.Ny + KTY - 1) / KTY);
+    const long long slots = (long long)sms * KCTAS;
+    auto cta = [](int c, int m) { return 0.95 + c * (0.57 + 0.265 * m); };
+    int best = lo;
+    double best_t = std::numeric_limits<double>::infinity();
+    for (int c = lo; c <= std::min(P.Nz, 32); ++c) {
+        const long long n = tiles * ((P.Nz + c - 1) / c), rest = n % slots;
+        const double t = (double)(n / slots) * cta(c, KCTAS) + (rest ? cta(c, (int)((rest + sms - 1) / sms)) : 0.0);
+        if (t < best_t) {
+            best_t = t;
+            best = c;
+        }
+    }
+    return best;
+}
+
 }  // namespace
 
 struct kzm_handle {
     kzm_params p{};
     KzmConst base{};
     long long n = 0;
-    float* q[2] = {nullptr, nullptr};
+    float* alloc[2] = {nullptr, nullptr};  // the fields' memory, halo included
+    float* q[2] = {nullptr, nullptr};      // site (0, 0, 0) of component 0
+    CUtensorMap tmap[2];
+    int* err = nullptr;                    // device error word of the bounded waits (after the partials)
+    int planes = 1;                        // planes per CTA of the step kernel
     double* stage = nullptr;
     double4* nf = nullptr;
-    KzmPartial* part = nullptr;
+    KzmPartial* part = nullptr;            // kBlocks + 1 partials, then the error word
     int cur = 0;
     bool uploaded = false;
     cudaStream_t stream = nullptr;
@@ -758,31 +672,55 @@ int kzm_create(const kzm_params* params, kzm_handle** out) {
     cudaGetDevice(&h->device);
     KzmConst& P = h->base;
     P.Nx = p.Nx; P.Ny = p.Ny; P.Nz = p.Nz;
-    P.sy = (p.Nx + 3) & ~3;
-    P.sz = (long long)p.Ny * P.sy;
+    P.sy = kPadX + ((p.Nx + 1 + 7) & ~7);
+    P.sz = (long long)(p.Ny + 2) * P.sy;
     P.sc = (long long)p.Nz * P.sz;
     P.ix2 = (float)(1.0 / (p.dx * p.dx)); P.iy2 = (float)(1.0 / (p.dy * p.dy)); P.iz2 = (float)(1.0 / (p.dz * p.dz));
     P.lap_c = (float)(-2.0 * (1.0 / (p.dx * p.dx) + 1.0 / (p.dy * p.dy) + 1.0 / (p.dz * p.dz)));
     P.kappa = (float)p.kappa;
+    auto both = [](double v) { return F2{make_float2((float)v, (float)v)}; };
+    P.mkx = both(-p.kappa / (p.dx * p.dx)); P.mky = both(-p.kappa / (p.dy * p.dy)); P.mkz = both(-p.kappa / (p.dz * p.dz));
+    P.mk0 = both(2.0 * p.kappa * (1.0 / (p.dx * p.dx) + 1.0 / (p.dy * p.dy) + 1.0 / (p.dz * p.dz)));
     P.qcap = (float)p.q_norm_cap;
     h->n = (long long)p.Nx * p.Ny * p.Nz;
     int rc;
     const size_t fb = (size_t)P.sc * 5 * sizeof(float);
-    if ((rc = alloc_or_fail((void**)&h->q[0], fb)) || (rc = alloc_or_fail((void**)&h->q[1], fb)) ||
-        (rc = alloc_or_fail((void**)&h->part, (kBlocks + 1) * sizeof(KzmPartial)))) {
+    if ((rc = alloc_or_fail((void**)&h->alloc[0], fb)) || (rc = alloc_or_fail((void**)&h->alloc[1], fb)) ||
+        (rc = alloc_or_fail((void**)&h->part, (kBlocks + 2) * sizeof(KzmPartial)))) {
         kzm_destroy(h);
         return rc;
     }
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMemset(h->q[0], 0, fb);
-    if (e == cudaSuccess) e = cudaMemset(h->q[1], 0, fb);
+    h->err = reinterpret_cast<int*>(h->part + kBlocks + 1);
+    for (int b = 0; b < 2; ++b) {
+        if (e == cudaSuccess) e = cudaMemset(h->alloc[b], 0, fb);
+        h->q[b] = h->alloc[b] + P.sy + kPadX;
+    }
+    if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
     if (e != cudaSuccess) {
         set_error(std::string("kzm_create: ") + cudaGetErrorString(e));
         kzm_destroy(h);
         return LDG_ERR_CUDA;
     }
+    for (int b = 0; b < 2; ++b)
+        if ((rc = kzm_encode(&h->tmap[b], h->alloc[b], P))) {
+            kzm_destroy(h);
+            return rc;
+        }
+    h->planes = kzm_planes(P);
     *out = h;
     return LDG_OK;
+}
+
+// Reads and clears the device error word (LDG_OK when no bounded wait gave up); synchronises.
+static int kzm_check(kzm_handle* h) {
+    int e = 0;
+    LDG_CUDA(cudaMemcpyAsync(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    LDG_CUDA(cudaStreamSynchronize(h->stream));
+    if (e == 0) return LDG_OK;
+    LDG_CUDA(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream));
+    set_error("periodic step: a bounded shared-memory pipeline wait gave up");
+    return LDG_ERR_TIMEOUT;
 }
 
 static int kzm_stage(kzm_handle* h) {
@@ -818,8 +756,7 @@ int kzm_download(kzm_handle* h, double* q) {
     h->launches++;
     LDG_LAUNCHED("k_kzm_to_aos");
     LDG_CUDA(cudaMemcpyAsync(q, h->stage, (size_t)h->n * 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    LDG_CUDA(cudaStreamSynchronize(h->stream));
-    return LDG_OK;
+    return kzm_check(h);
 }
 
 int kzm_step(kzm_handle* h, int n_steps, const kzm_step_args* a) {
@@ -832,39 +769,30 @@ int kzm_step(kzm_handle* h, int n_steps, const kzm_step_args* a) {
     KzmConst P = h->base;
     P.A = (float)a->A; P.B = (float)a->B; P.C = (float)a->C;
     P.mob_dt = (float)((1.0 / h->p.gamma) * a->dt);
+    auto both = [](float v) { return F2{make_float2(v, v)}; };
+    P.mmob = both(-P.mob_dt);
+    P.K = BulkC<F2>{both(P.A), both(2.0f * P.C), both(2.0f / 3.0f * P.B), both(P.B), both(-P.B)};
     P.sigma = (float)a->noise_sigma;
     P.key0 = (uint32_t)a->seed;
     P.key1 = (uint32_t)(a->seed >> 32);
-    // Two-site asynchronous-copy kernel by default; LDG_KZM_KERNEL=async selects the one-site
-    // asynchronous-copy kernel, =regs the register-queue tiled kernel, =direct the one-thread-per-
-    // site kernel.
+    // LDG_KZM_KERNEL=direct selects the one-thread-per-site kernel (comparisons).
     const char* ksel = getenv("LDG_KZM_KERNEL");
-    const int kind = !ksel                           ? 3
-                     : std::strcmp(ksel, "direct") == 0 ? 0
-                     : std::strcmp(ksel, "regs") == 0   ? 1
-                     : std::strcmp(ksel, "async") == 0  ? 2
-                                                        : 3;
-    // the two-site kernel's 16-byte copies need every pitch a multiple of 4 floats
-    const int kind_run = (kind == 3 && P.Nx % 4 != 0) ? 2 : kind;
-    dim3 blk(32, 8, 1), grd((P.Nx + 31) / 32, (P.Ny + 7) / 8, P.Nz);
-    dim3 tgrd((P.Nx + KTX - 1) / KTX, (P.Ny + KTY - 1) / KTY, (P.Nz + KZC - 1) / KZC);
-    const size_t ring_bytes = (size_t)KRING * 5 * KPS * sizeof(float);
+    const bool direct = ksel && std::strcmp(ksel, "direct") == 0;
+    const bool noise = a->noise_sigma > 0.0;
+    const dim3 blk(32, 8, 1), grd((P.Nx + 31) / 32, (P.Ny + 7) / 8, P.Nz);
+    const dim3 tgrd((P.Nx + KTX - 1) / KTX, (P.Ny + KTY - 1) / KTY, (P.Nz + h->planes - 1) / h->planes);
     for (int s = 0; s < n_steps; ++s) {
         P.step = a->step_index + s;
-        const bool noise = a->noise_sigma > 0.0;
         const float* in = h->q[h->cur];
         float* outb = h->q[1 - h->cur];
-        if (kind_run == 3) {
-            if (noise) k_kzm_step_pair<true><<<tgrd, KPT, kRingBytes2, h->stream>>>(in, outb, P);
-            else k_kzm_step_pair<false><<<tgrd, KPT, kRingBytes2, h->stream>>>(in, outb, P);
-        } else if (kind_run == 2) {
-            if (noise) k_kzm_step_async<true><<<tgrd, blk, ring_bytes, h->stream>>>(in, outb, P);
-            else k_kzm_step_async<false><<<tgrd, blk, ring_bytes, h->stream>>>(in, outb, P);
-        } else if (kind == 1) {
-            if (noise) k_kzm_step_tiled<true><<<tgrd, blk, 0, h->stream>>>(in, outb, P);
-            else k_kzm_step_tiled<false><<<tgrd, blk, 0, h->stream>>>(in, outb, P);
-        } else if (noise) k_kzm_step<true><<<grd, blk, 0, h->stream>>>(in, outb, P);
-        else k_kzm_step<false><<<grd, blk, 0, h->stream>>>(in, outb, P);
+        if (!direct) {
+            LDG_CUDA(launch_pdl(noise ? k_kzm_step_ring<true> : k_kzm_step_ring<false>, tgrd, KTHREADS, kRingBytes,
+                                h->stream, h->tmap[h->cur], outb, P, h->planes, h->err));
+        } else if (noise) {
+            k_kzm_step<true><<<grd, blk, 0, h->stream>>>(in, outb, P);
+        } else {
+            k_kzm_step<false><<<grd, blk, 0, h->stream>>>(in, outb, P);
+        }
         h->launches++;
         LDG_LAUNCHED("k_kzm_step");
         h->cur = 1 - h->cur;
@@ -894,7 +822,7 @@ int kzm_observe(kzm_handle* h, double A, double B, double C, kzm_observables* o)
     LDG_LAUNCHED("kzm observables");
     KzmPartial R{};
     LDG_CUDA(cudaMemcpyAsync(&R, h->part + kBlocks, sizeof(R), cudaMemcpyDeviceToHost, h->stream));
-    LDG_CUDA(cudaStreamSynchronize(h->stream));
+    if (int rc = kzm_check(h)) return rc;
     const double tv = O.cv * (double)p.Nx * (double)p.Ny * (double)p.Nz;
     const double nan = std::numeric_limits<double>::quiet_NaN();
     o->bulk = R.bulk / tv;
@@ -973,7 +901,7 @@ int kzm_observe_device_noalloc(const kzm_params* params, const double* q, double
                         ", not to the current device " + std::to_string(cur));
     }
     double4* nf = nullptr;
-    KzmPartial* part = nullptr;
+    KzmPartial* part = nullptr;            // kBlocks + 1 partials, then the error word
     int rc = noalloc_scratch(&nf, &part);
     if (rc) return rc;
     KzmObsConst O{};
@@ -1012,7 +940,7 @@ int kzm_destroy(kzm_handle* h) {
     if (!h) return LDG_OK;
     DeviceGuard device_guard(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    cudaFree(h->q[0]); cudaFree(h->q[1]); cudaFree(h->stage); cudaFree(h->nf); cudaFree(h->part);
+    cudaFree(h->alloc[0]); cudaFree(h->alloc[1]); cudaFree(h->stage); cudaFree(h->nf); cudaFree(h->part);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return LDG_OK;

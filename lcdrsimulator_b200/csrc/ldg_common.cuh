@@ -81,10 +81,24 @@ __device__ __forceinline__ void philox4x32(uint32_t c[4], uint32_t k0, uint32_t 
     }
 }
 
-// Uniform in (0, 1] from a 21-bit integer: (x + 1) 2^-21, formed as one fused multiply-add
-// (exact: x is exact in FP32 and the result has at most 22 significant bits).
-__device__ __forceinline__ float u21(uint32_t x) {
-    return fmaf((float)x, 1.0f / 2097152.0f, 1.0f / 2097152.0f);
+// Uniform (x + 1) 2^-21 in (0, 1] from a 21-bit integer x given as x << 2 in bits 2..22 (other bits
+// zero): as the mantissa of a float in [1, 2) it is 1 + x 2^-21, and adding 2^-21 - 1 is exact (the
+// result has at most 22 significant bits). Integer and FMA pipes only: a conversion would take the
+// same pipe as the logarithms, roots and sines of the draw.
+__device__ __forceinline__ float u21(uint32_t x4) {
+    return __uint_as_float(0x3F800000u | x4) + (1.0f / 2097152.0f - 1.0f);
+}
+// Hardware approximations without the subnormal handling of the default forms: every argument of the
+// draw is normal (u >= 2^-21, t >= 1e-30), where both give the same value.
+__device__ __forceinline__ float lg2_ftz(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
 // Five standard normals for (cell, instance, step) from one Philox4x32-7 block: the four
@@ -98,18 +112,18 @@ __device__ __forceinline__ void normals5(uint32_t cell, uint32_t instance, long 
                                          float g[5]) {
     uint32_t c[4] = {cell, instance, (uint32_t)step, (uint32_t)((unsigned long long)step >> 32)};
     philox4x32<kNoiseRounds>(c, k0, k1);
-    constexpr uint32_t M21 = (1u << 21) - 1u;
-    const uint32_t f0 = c[0] & M21, f1 = c[1] & M21, f2 = c[2] & M21, f3 = c[3] & M21;
-    const uint32_t f4 = ((c[0] >> 21) << 10) | (c[1] >> 22);  // 11 + 10 bits
-    const uint32_t f5 = ((c[2] >> 21) << 10) | (c[3] >> 22);
+    constexpr uint32_t M21 = ((1u << 21) - 1u) << 2;  // the fields are formed shifted left by two (u21)
+    const uint32_t f0 = (c[0] << 2) & M21, f1 = (c[1] << 2) & M21, f2 = (c[2] << 2) & M21, f3 = (c[3] << 2) & M21;
+    const uint32_t f4 = ((c[0] >> 9) & 0x7FF000u) | ((c[1] >> 20) & 0xFFCu);  // 11 + 10 bits
+    const uint32_t f5 = ((c[2] >> 9) & 0x7FF000u) | ((c[3] >> 20) & 0xFFCu);
     // angle 2 pi u taken as pi + t with t = 2 pi u - pi in (-pi, pi], where the fast hardware
     // sine/cosine is accurate to ~4e-7: cos(2 pi u) = -cos t, sin(2 pi u) = -sin t
     constexpr float kTwoPi = 6.28318530717958647692f, kPi = 3.14159265358979323846f;
     constexpr float kM2Ln2 = -1.38629436111989061883f;  // -2 ln 2
     // radius sqrt(-2 ln u) = t * rsqrt(t), t = -2 ln 2 log2(u) (the guard keeps t = 0, u = 1, at zero)
     auto radius = [](float u) {
-        const float t = kM2Ln2 * __log2f(u);
-        return t * rsqrtf(fmaxf(t, 1e-30f));
+        const float t = kM2Ln2 * lg2_ftz(u);
+        return t * rsqrt_ftz(fmaxf(t, 1e-30f));
     };
     float s, co;
     float r = radius(u21(f0));
@@ -365,20 +379,27 @@ __device__ __forceinline__ float vset<float>(float a) { return a; }
 // Bulk molecular field of the five stored components (xx, xy, xz, yy, yz). It is traceless as
 // written (tr(Q^2 - I tr Q^2 / 3) = 0 and Qzz = -(Qxx + Qyy)), so the zz entry is never formed;
 // with Qzz eliminated the off-diagonal entries of Q^2 are two products each.
+// Coefficients of the bulk field as values of F: a packed operation takes a pair in registers or
+// in the kernel's parameters, and a scalar would have to be copied into both halves at every use.
 template <class F>
-__device__ __forceinline__ void bulk_field5(const F q[5], float cQ, float cQ2, float cQ3, F h[5]) {
+struct BulkC {
+    F cQ, cQ3x2, c23, cQ2, mcQ2;  // cQ, 2 cQ3, 2/3 cQ2, cQ2, -cQ2
+};
+template <class F>
+__device__ __forceinline__ void bulk_field5(const F q[5], const BulkC<F>& K, F h[5]) {
     const F Qxx = q[0], Qxy = q[1], Qxz = q[2], Qyy = q[3], Qyz = q[4];
     const F s = Qxx + Qyy;  // -Qzz
     const F q2xx = vfma(Qxx, Qxx, vfma(Qxy, Qxy, Qxz * Qxz));
     const F q2yy = vfma(Qyy, Qyy, vfma(Qxy, Qxy, Qyz * Qyz));
-    const F t = vfma(Qyz, Qyz, vfma(Qyy, s, q2xx));         // tr(Q^2) / 2
-    const F cg = vfma(2.0f * cQ3, t, vset<F>(cQ));          // cQ + cQ3 tr(Q^2)
-    const F c23 = (2.0f / 3.0f * cQ2) * t;                  // cQ2 tr(Q^2) / 3
-    h[0] = vfma(cg, Qxx, vfma(-cQ2, q2xx, c23));
-    h[3] = vfma(cg, Qyy, vfma(-cQ2, q2yy, c23));
-    h[1] = vfma(cg, Qxy, -cQ2 * vfma(Qxy, s, Qxz * Qyz));
-    h[2] = vfma(cg, Qxz, cQ2 * vfma(Qxz, Qyy, -(Qxy * Qyz)));
-    h[4] = vfma(cg, Qyz, cQ2 * vfma(Qyz, Qxx, -(Qxy * Qxz)));
+    const F t = vfma(Qyz, Qyz, vfma(Qyy, s, q2xx));  // tr(Q^2) / 2
+    const F cg = vfma(K.cQ3x2, t, K.cQ);             // cQ + cQ3 tr(Q^2)
+    const F c23 = K.c23 * t;                         // cQ2 tr(Q^2) / 3
+    const F m1 = K.mcQ2 * Qxy, m2 = K.mcQ2 * Qxz;
+    h[0] = vfma(cg, Qxx, vfma(K.mcQ2, q2xx, c23));
+    h[3] = vfma(cg, Qyy, vfma(K.mcQ2, q2yy, c23));
+    h[1] = vfma(vfma(K.mcQ2, s, cg), Qxy, m2 * Qyz);    // (Q^2)_xy = Qxy (Qxx + Qyy) + Qxz Qyz
+    h[2] = vfma(vfma(K.cQ2, Qyy, cg), Qxz, m1 * Qyz);   // (Q^2)_xz = Qxy Qyz - Qxz Qyy
+    h[4] = vfma(vfma(K.cQ2, Qxx, cg), Qyz, m1 * Qxz);   // (Q^2)_yz = Qxy Qxz - Qyz Qxx
 }
 
 // What one component contributes to the stencil terms of a cell: undivided first differences
@@ -409,7 +430,9 @@ struct Sten {
 template <bool kL2, bool kL3, bool kLap, bool kFace, class F, class St>
 __device__ __forceinline__ void chem_core(const St& S, const QsrConst& P, const F q[5], F l3on, F mu[5], F lap[5]) {
     F* h = mu;
-    bulk_field5<F>(q, P.cQ, P.cQ2, P.cQ3, h);
+    const BulkC<F> K{vset<F>(P.cQ), vset<F>(2.0f * P.cQ3), vset<F>(2.0f / 3.0f * P.cQ2), vset<F>(P.cQ2),
+                     vset<F>(-P.cQ2)};
+    bulk_field5<F>(q, K, h);
     const float cxx = P.l2w[0], cyy = P.l2w[1], czz = P.l2w[2], cxy = P.l2w[3], cxz = P.l2w[4], cyz = P.l2w[5];
     F gx = vset<F>(P.lx), gy = vset<F>(P.ly), gz = vset<F>(P.lz);
     F gxy{}, gxz{}, gyz{};
