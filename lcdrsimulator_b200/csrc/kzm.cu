@@ -357,118 +357,63 @@ struct KzmObsConst {
 };
 
 // Pass 1 (KZM_bulk_ldg.cu:564-632): bulk and forward-difference elastic energy, |Q|^2 and
-// |grad Q|^2 integrals, nematic (S, n) per site into an FP64 scratch field.
-__global__ void __launch_bounds__(kThreads) k_kzm_obs_sites(const float* __restrict__ q, KzmObsConst O,
+// |grad Q|^2 integrals, nematic (S, n) per site into an FP64 scratch field. kAos: the field is the
+// caller's own (reference layout, AoS FP64, x fastest), else the solver's FP32 arrays. A warp takes a
+// row of sites at a time.
+template <bool kAos, class T>
+__global__ void __launch_bounds__(kThreads) k_kzm_obs_sites(const T* __restrict__ q, KzmObsConst O,
                                                             double4* __restrict__ nf, KzmPartial* __restrict__ part) {
     const KzmConst& P = O.P;
-    const long long n = (long long)P.Nx * P.Ny * P.Nz;
     KzmPartial a{};
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(t % P.Nx);
-        const long long r = t / P.Nx;
-        const int y = (int)(r % P.Ny);
-        const int z = (int)(r / P.Ny);
-        const long long id = (long long)z * P.sz + (long long)y * P.sy + x;
-        const long long px = (long long)z * P.sz + (long long)y * P.sy + ((x + 1) % P.Nx);
-        const long long py = (long long)z * P.sz + (long long)((y + 1) % P.Ny) * P.sy + x;
-        const long long pz = (long long)((z + 1) % P.Nz) * P.sz + (long long)y * P.sy + x;
-        double c[5], d[6][3];
+    const int lane = threadIdx.x & 31;
+    const long long rows = (long long)P.Ny * P.Nz, warps = (long long)gridDim.x * (kThreads / 32);
+    for (long long r = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); r < rows; r += warps) {
+        const int z = (int)(r / P.Ny), y = (int)(r - (long long)z * P.Ny);
+        const int yp = y + 1 == P.Ny ? 0 : y + 1, zp = z + 1 == P.Nz ? 0 : z + 1;
+        auto row = [&](int yy, int zz) {
+            return kAos ? q + 5 * (long long)P.Nx * (yy + (long long)P.Ny * zz) : q + (long long)zz * P.sz + (long long)yy * P.sy;
+        };
+        const T *q0 = row(y, z), *qy = row(yp, z), *qz = row(y, zp);
+        const int step = kAos ? 5 : 1;
+        const long long comp = kAos ? 1 : P.sc;
+        for (int x = lane; x < P.Nx; x += 32) {
+            const long long ox = (long long)step * x, op = (long long)step * (x + 1 == P.Nx ? 0 : x + 1);
+            double c[5], d[6][3];
 #pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            const float* b = q + m * P.sc;
-            c[m] = (double)b[id];
-            d[m][0] = ((double)b[px] - c[m]) * O.ix;
-            d[m][1] = ((double)b[py] - c[m]) * O.iy;
-            d[m][2] = ((double)b[pz] - c[m]) * O.iz;
+            for (int m = 0; m < 5; ++m) {
+                c[m] = (double)q0[m * comp + ox];
+                d[m][0] = ((double)q0[m * comp + op] - c[m]) * O.ix;
+                d[m][1] = ((double)qy[m * comp + ox] - c[m]) * O.iy;
+                d[m][2] = ((double)qz[m * comp + ox] - c[m]) * O.iz;
+            }
+#pragma unroll
+            for (int w = 0; w < 3; ++w) d[5][w] = -(d[0][w] + d[3][w]);
+            const double Qxx = c[0], Qxy = c[1], Qxz = c[2], Qyy = c[3], Qyz = c[4], Qzz = -Qxx - Qyy;
+            const double q2xx = Qxx * Qxx + Qxy * Qxy + Qxz * Qxz;
+            const double q2xy = Qxx * Qxy + Qxy * Qyy + Qxz * Qyz;
+            const double q2xz = Qxx * Qxz + Qxy * Qyz + Qxz * Qzz;
+            const double q2yy = Qxy * Qxy + Qyy * Qyy + Qyz * Qyz;
+            const double q2yz = Qxy * Qxz + Qyy * Qyz + Qyz * Qzz;
+            const double q2zz = Qxz * Qxz + Qyz * Qyz + Qzz * Qzz;
+            const double trQ2 = Qxx * Qxx + Qyy * Qyy + Qzz * Qzz + 2.0 * (Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
+            const double trQ3 = Qxx * q2xx + Qxy * q2xy + Qxz * q2xz + Qxy * q2xy + Qyy * q2yy + Qyz * q2yz +
+                                Qxz * q2xz + Qyz * q2yz + Qzz * q2zz;
+            a.bulk += ((O.A / 2.0) * trQ2 - (O.B / 3.0) * trQ3 + (O.C / 4.0) * trQ2 * trQ2) * O.cv;
+            double g2 = 0.0;
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+                const double s = d[m][0] * d[m][0] + d[m][1] * d[m][1] + d[m][2] * d[m][2];
+                g2 += (m == 1 || m == 2 || m == 4) ? 2.0 * s : s;
+            }
+            a.gint += g2 * O.cv;
+            a.qint += trQ2 * O.cv;
+            const Nematic f = nematic64(c, 1e-12, Nematic{0.0, 1.0, 0.0, 0.0});
+            nf[r * P.Nx + x] = make_double4(f.S, f.nx, f.ny, f.nz);
+            a.S_sum += f.S;
+            a.S_max = fmax(a.S_max, f.S);
         }
-#pragma unroll
-        for (int w = 0; w < 3; ++w) d[5][w] = -(d[0][w] + d[3][w]);
-        const double Qxx = c[0], Qxy = c[1], Qxz = c[2], Qyy = c[3], Qyz = c[4], Qzz = -Qxx - Qyy;
-        const double q2xx = Qxx * Qxx + Qxy * Qxy + Qxz * Qxz;
-        const double q2xy = Qxx * Qxy + Qxy * Qyy + Qxz * Qyz;
-        const double q2xz = Qxx * Qxz + Qxy * Qyz + Qxz * Qzz;
-        const double q2yy = Qxy * Qxy + Qyy * Qyy + Qyz * Qyz;
-        const double q2yz = Qxy * Qxz + Qyy * Qyz + Qyz * Qzz;
-        const double q2zz = Qxz * Qxz + Qyz * Qyz + Qzz * Qzz;
-        const double trQ2 = Qxx * Qxx + Qyy * Qyy + Qzz * Qzz + 2.0 * (Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
-        const double trQ3 = Qxx * q2xx + Qxy * q2xy + Qxz * q2xz + Qxy * q2xy + Qyy * q2yy + Qyz * q2yz +
-                            Qxz * q2xz + Qyz * q2yz + Qzz * q2zz;
-        a.bulk += ((O.A / 2.0) * trQ2 - (O.B / 3.0) * trQ3 + (O.C / 4.0) * trQ2 * trQ2) * O.cv;
-        double g2 = 0.0;
-#pragma unroll
-        for (int m = 0; m < 6; ++m) {
-            const double s = d[m][0] * d[m][0] + d[m][1] * d[m][1] + d[m][2] * d[m][2];
-            g2 += (m == 1 || m == 2 || m == 4) ? 2.0 * s : s;
-        }
-        a.gint += g2 * O.cv;
-        a.elastic += 0.5 * O.kappa * g2 * O.cv;
-        a.qint += trQ2 * O.cv;
-        const Nematic f = nematic64(c, 1e-12, Nematic{0.0, 1.0, 0.0, 0.0});
-        nf[t] = make_double4(f.S, f.nx, f.ny, f.nz);
-        a.S_sum += f.S;
-        a.S_max = fmax(a.S_max, f.S);
     }
-    __shared__ double shd[kThreads / 32];
-    KzmPartial res{};
-    res.bulk = bsum(a.bulk, shd);
-    res.elastic = bsum(a.elastic, shd);
-    res.qint = bsum(a.qint, shd);
-    res.gint = bsum(a.gint, shd);
-    res.S_sum = bsum(a.S_sum, shd);
-    res.S_max = bmax(a.S_max, shd);
-    if (threadIdx.x == 0) part[blockIdx.x] = res;
-}
-
-// Pass 1 on a caller-owned device field in the reference layout (AoS FP64, x fastest).
-__global__ void __launch_bounds__(kThreads) k_kzm_obs_sites_aos(const double* __restrict__ q, KzmObsConst O,
-                                                                double4* __restrict__ nf,
-                                                                KzmPartial* __restrict__ part) {
-    const KzmConst& P = O.P;
-    const long long n = (long long)P.Nx * P.Ny * P.Nz;
-    KzmPartial a{};
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(t % P.Nx);
-        const long long r = t / P.Nx;
-        const int y = (int)(r % P.Ny);
-        const int z = (int)(r / P.Ny);
-        const long long px = (long long)((x + 1) % P.Nx) + (long long)P.Nx * ((long long)y + (long long)P.Ny * z);
-        const long long py = (long long)x + (long long)P.Nx * ((long long)((y + 1) % P.Ny) + (long long)P.Ny * z);
-        const long long pz = (long long)x + (long long)P.Nx * ((long long)y + (long long)P.Ny * ((z + 1) % P.Nz));
-        double c[5], d[6][3];
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            c[m] = q[5 * t + m];
-            d[m][0] = (q[5 * px + m] - c[m]) * O.ix;
-            d[m][1] = (q[5 * py + m] - c[m]) * O.iy;
-            d[m][2] = (q[5 * pz + m] - c[m]) * O.iz;
-        }
-#pragma unroll
-        for (int w = 0; w < 3; ++w) d[5][w] = -(d[0][w] + d[3][w]);
-        const double Qxx = c[0], Qxy = c[1], Qxz = c[2], Qyy = c[3], Qyz = c[4], Qzz = -Qxx - Qyy;
-        const double q2xx = Qxx * Qxx + Qxy * Qxy + Qxz * Qxz;
-        const double q2xy = Qxx * Qxy + Qxy * Qyy + Qxz * Qyz;
-        const double q2xz = Qxx * Qxz + Qxy * Qyz + Qxz * Qzz;
-        const double q2yy = Qxy * Qxy + Qyy * Qyy + Qyz * Qyz;
-        const double q2yz = Qxy * Qxz + Qyy * Qyz + Qyz * Qzz;
-        const double q2zz = Qxz * Qxz + Qyz * Qyz + Qzz * Qzz;
-        const double trQ2 = Qxx * Qxx + Qyy * Qyy + Qzz * Qzz + 2.0 * (Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
-        const double trQ3 = Qxx * q2xx + Qxy * q2xy + Qxz * q2xz + Qxy * q2xy + Qyy * q2yy + Qyz * q2yz +
-                            Qxz * q2xz + Qyz * q2yz + Qzz * q2zz;
-        a.bulk += ((O.A / 2.0) * trQ2 - (O.B / 3.0) * trQ3 + (O.C / 4.0) * trQ2 * trQ2) * O.cv;
-        double g2 = 0.0;
-#pragma unroll
-        for (int m = 0; m < 6; ++m) {
-            const double s = d[m][0] * d[m][0] + d[m][1] * d[m][1] + d[m][2] * d[m][2];
-            g2 += (m == 1 || m == 2 || m == 4) ? 2.0 * s : s;
-        }
-        a.gint += g2 * O.cv;
-        a.elastic += 0.5 * O.kappa * g2 * O.cv;
-        a.qint += trQ2 * O.cv;
-        const Nematic f = nematic64(c, 1e-12, Nematic{0.0, 1.0, 0.0, 0.0});
-        nf[t] = make_double4(f.S, f.nx, f.ny, f.nz);
-        a.S_sum += f.S;
-        a.S_max = fmax(a.S_max, f.S);
-    }
+    a.elastic = 0.5 * O.kappa * a.gint;
     __shared__ double shd[kThreads / 32];
     KzmPartial res{};
     res.bulk = bsum(a.bulk, shd);
@@ -514,29 +459,79 @@ __device__ __forceinline__ int plaquette(const double4& a, const double4& b, con
     return (fabs(s) > cut) ? 2 : 1;
 }
 
-// Pass 2 (KZM_bulk_ldg.cu:634-689): three plaquette orientations per site, line length.
+// The same from sign tests. The doubled angle of a projected director (u, v) is that of
+// D = (u^2 - v^2, 2 u v); around a plaquette the wrapped angle differences add up to 2 pi m with a whole
+// number m, and m counts the edges that pass the angle pi: an edge from the upper half plane (angle
+// in [0, pi]) to the lower one passes it upwards where D_a x D_b > 0, one from the lower to the upper
+// downwards where D_a x D_b < 0. So no angle, root or division is needed, and |m| / 2 > cut decides. An edge whose directors
+// are parallel or antiparallel to 1e-9, where rounding of the angles would decide, and a cut within
+// 1e-9 of 0, 1/2 or 1 take the angles themselves (plaquette above).
+struct Doubled {
+    double x, y, r;  // D and its length u^2 + v^2
+};
+__device__ __forceinline__ Doubled doubled(double u, double v) {
+    const double uu = u * u, vv = v * v;
+    return Doubled{uu - vv, 2.0 * u * v, uu + vv};
+}
+// Signed passage of the angle pi from a to b, or 2 where the signs do not decide.
+__device__ __forceinline__ int passage(const Doubled& a, const Doubled& b) {
+    const double cr = a.x * b.y - a.y * b.x;
+    const bool ha = a.y >= 0.0, hb = b.y >= 0.0;
+    const bool flat = !(fabs(cr) > 1e-9 * (a.r * b.r));
+    if (ha == hb && !(flat && !(a.x * b.x + a.y * b.y > 0.0))) return 0;
+    if (flat) return 2;
+    return ha ? (cr > 0.0 ? 1 : 0) : (cr < 0.0 ? -1 : 0);
+}
+__device__ __forceinline__ int plaquette_signs(const double4& a, const double4& b, const double4& c, const double4& d,
+                                               int plane, double thr, double cut, bool plain_cut) {
+    if (!(isfinite(a.x) && isfinite(b.x) && isfinite(c.x) && isfinite(d.x))) return 0;
+    if (!(a.x > thr && b.x > thr && c.x > thr && d.x > thr)) return 0;
+    auto proj = [plane](const double4& f) {
+        return plane == 0 ? doubled(f.y, f.z) : (plane == 1 ? doubled(f.z, f.w) : doubled(f.y, f.w));
+    };
+    const Doubled A = proj(a), B = proj(b), C = proj(c), E = proj(d);
+    const double lo = fmin(fmin(A.r, B.r), fmin(C.r, E.r));
+    if (plain_cut && lo > 1.001e-16) {
+        const int k0 = passage(A, B), k1 = passage(B, C), k2 = passage(C, E), k3 = passage(E, A);
+        if (k0 != 2 && k1 != 2 && k2 != 2 && k3 != 2) return 0.5 * abs(k0 + k1 + k2 + k3) > cut ? 2 : 1;
+    }
+    return plaquette(a, b, c, d, plane, thr, cut);
+}
+
+// Pass 2 (KZM_bulk_ldg.cu:634-689): three plaquette orientations per site, line length. A warp takes a
+// row of sites at a time.
 __global__ void __launch_bounds__(kThreads) k_kzm_obs_plaq(const double4* __restrict__ nf, KzmObsConst O, double thr,
                                                            double cut, double dx, double dy, double dz,
                                                            KzmPartial* __restrict__ part) {
     const KzmConst& P = O.P;
-    const long long n = (long long)P.Nx * P.Ny * P.Nz;
     KzmPartial a{};
-    auto at = [&](int x, int y, int z) { return nf[(long long)x + (long long)P.Nx * ((long long)y + (long long)P.Ny * z)]; };
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(t % P.Nx);
-        const long long r = t / P.Nx;
-        const int y = (int)(r % P.Ny);
-        const int z = (int)(r / P.Ny);
-        const int xp = (x + 1) % P.Nx, yp = (y + 1) % P.Ny, zp = (z + 1) % P.Nz;
-        const double4 f000 = nf[t], f100 = at(xp, y, z), f110 = at(xp, yp, z), f010 = at(x, yp, z);
-        const double4 f001 = at(x, y, zp), f101 = at(xp, y, zp), f011 = at(x, yp, zp);
-        int res = plaquette(f000, f100, f110, f010, 0, thr, cut);
-        if (res) { a.used++; if (res == 2) { a.defects++; a.line += dz; } }
-        res = plaquette(f000, f010, f011, f001, 1, thr, cut);
-        if (res) { a.used++; if (res == 2) { a.defects++; a.line += dx; } }
-        res = plaquette(f000, f100, f101, f001, 2, thr, cut);
-        if (res) { a.used++; if (res == 2) { a.defects++; a.line += dy; } }
+    unsigned used = 0, n0 = 0, n1 = 0, n2 = 0;
+    const bool plain_cut = cut > 1e-9 && fabs(cut - 0.5) > 1e-9 && fabs(cut - 1.0) > 1e-9;
+    const int lane = threadIdx.x & 31;
+    const long long rows = (long long)P.Ny * P.Nz, warps = (long long)gridDim.x * (kThreads / 32);
+    for (long long r = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); r < rows; r += warps) {
+        const int z = (int)(r / P.Ny), y = (int)(r - (long long)z * P.Ny);
+        const int yp = y + 1 == P.Ny ? 0 : y + 1, zp = z + 1 == P.Nz ? 0 : z + 1;
+        auto row = [&](int yy, int zz) { return nf + (long long)P.Nx * (yy + (long long)P.Ny * zz); };
+        const double4 *r00 = row(y, z), *r10 = row(yp, z), *r01 = row(y, zp), *r11 = row(yp, zp);
+        for (int x = lane; x < P.Nx; x += 32) {
+            const int xp = x + 1 == P.Nx ? 0 : x + 1;
+            const double4 f000 = r00[x], f100 = r00[xp], f010 = r10[x], f001 = r01[x];
+            const double4 f110 = r10[xp], f101 = r01[xp], f011 = r11[x];
+            int res = plaquette_signs(f000, f100, f110, f010, 0, thr, cut, plain_cut);
+            used += res != 0;
+            n0 += res == 2;
+            res = plaquette_signs(f000, f010, f011, f001, 1, thr, cut, plain_cut);
+            used += res != 0;
+            n1 += res == 2;
+            res = plaquette_signs(f000, f100, f101, f001, 2, thr, cut, plain_cut);
+            used += res != 0;
+            n2 += res == 2;
+        }
     }
+    a.used = used;
+    a.defects = (unsigned long long)n0 + n1 + n2;
+    a.line = n0 * dz + n1 * dx + n2 * dy;
     __shared__ double shd[kThreads / 32];
     __shared__ unsigned long long shu[kThreads / 32];
     KzmPartial res{};
@@ -814,7 +809,7 @@ int kzm_observe(kzm_handle* h, double A, double B, double C, kzm_observables* o)
     O.A = A; O.B = B; O.C = C; O.kappa = p.kappa;
     O.cv = p.dx * p.dy * p.dz;
     O.ix = 1.0 / p.dx; O.iy = 1.0 / p.dy; O.iz = 1.0 / p.dz;
-    k_kzm_obs_sites<<<kBlocks, kThreads, 0, h->stream>>>(h->q[h->cur], O, h->nf, h->part);
+    k_kzm_obs_sites<false><<<kBlocks, kThreads, 0, h->stream>>>(h->q[h->cur], O, h->nf, h->part);
     k_kzm_obs_plaq<<<kBlocks, kThreads, 0, h->stream>>>(h->nf, O, p.defects_S_threshold, p.defects_charge_cutoff, p.dx,
                                                        p.dy, p.dz, h->part);
     k_kzm_obs_final<<<1, kThreads, 0, h->stream>>>(h->part, kBlocks, h->part + kBlocks);
@@ -901,7 +896,7 @@ int kzm_observe_device_noalloc(const kzm_params* params, const double* q, double
                         ", not to the current device " + std::to_string(cur));
     }
     double4* nf = nullptr;
-    KzmPartial* part = nullptr;            // kBlocks + 1 partials, then the error word
+    KzmPartial* part = nullptr;
     int rc = noalloc_scratch(&nf, &part);
     if (rc) return rc;
     KzmObsConst O{};
@@ -909,7 +904,7 @@ int kzm_observe_device_noalloc(const kzm_params* params, const double* q, double
     O.A = A; O.B = B; O.C = C; O.kappa = p.kappa;
     O.cv = p.dx * p.dy * p.dz;
     O.ix = 1.0 / p.dx; O.iy = 1.0 / p.dy; O.iz = 1.0 / p.dz;
-    k_kzm_obs_sites_aos<<<kBlocks, kThreads, 0, st>>>(q, O, nf, part);
+    k_kzm_obs_sites<true><<<kBlocks, kThreads, 0, st>>>(q, O, nf, part);
     k_kzm_obs_plaq<<<kBlocks, kThreads, 0, st>>>(nf, O, p.defects_S_threshold, p.defects_charge_cutoff, p.dx, p.dy,
                                                   p.dz, part);
     k_kzm_obs_final<<<1, kThreads, 0, st>>>(part, kBlocks, part + kBlocks);

@@ -697,8 +697,27 @@ __device__ __forceinline__ void euler_update(const QsrConst& P, const float q[5]
 // ---------------------------------------------------------------------------------------
 // FP64 nematic eigen-solver (QSR.cu:191-243): shifted power iteration for the largest
 // eigenvalue, S = 1.5 lambda, director gauge nz >= 0.
+// The reference takes 15 steps n <- M n / |M n| of M = Q + alpha I. Its intermediate norms only scale
+// the vector, so the direction after them is that of M^15 n0 = M^8 M^4 M^2 M n0, by three squarings of
+// a symmetric matrix and four products with one norm at the end: about 150 operations instead of 15
+// roots and 45 divisions. M is taken relative to alpha, so its powers stay in range. The
+// reference's early stop (|M n| < 1e-13) can only come at the first step: alpha bounds the row sums of
+// Q, so M is positive semidefinite and |M n| does not fall from one step to the next.
 // ---------------------------------------------------------------------------------------
 struct Nematic { double S, nx, ny, nz; };
+
+struct Sym3 { double xx, xy, xz, yy, yz, zz; };
+__device__ __forceinline__ Sym3 square(const Sym3& m) {
+    return Sym3{fma(m.xx, m.xx, fma(m.xy, m.xy, m.xz * m.xz)), fma(m.xx, m.xy, fma(m.xy, m.yy, m.xz * m.yz)),
+                fma(m.xx, m.xz, fma(m.xy, m.yz, m.xz * m.zz)), fma(m.xy, m.xy, fma(m.yy, m.yy, m.yz * m.yz)),
+                fma(m.xy, m.xz, fma(m.yy, m.yz, m.yz * m.zz)), fma(m.xz, m.xz, fma(m.yz, m.yz, m.zz * m.zz))};
+}
+__device__ __forceinline__ void apply(const Sym3& m, double v[3]) {
+    const double x = v[0], y = v[1], z = v[2];
+    v[0] = fma(m.xx, x, fma(m.xy, y, m.xz * z));
+    v[1] = fma(m.xy, x, fma(m.yy, y, m.yz * z));
+    v[2] = fma(m.xz, x, fma(m.yz, y, m.zz * z));
+}
 
 __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, Nematic iso) {
     const double Qxx = q[0], Qxy = q[1], Qxz = q[2], Qyy = q[3], Qyz = q[4];
@@ -706,22 +725,31 @@ __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, 
     if (fabs(Qxx) < iso_cut && fabs(Qxy) < iso_cut && fabs(Qxz) < iso_cut && fabs(Qyy) < iso_cut &&
         fabs(Qyz) < iso_cut)
         return iso;
-    double nx = Qxx + Qxy + Qxz, ny = Qxy + Qyy + Qyz, nz = Qxz + Qyz - Qxx - Qyy;
-    const double n0 = sqrt(nx * nx + ny * ny + nz * nz);
-    if (n0 > 1e-12) { nx /= n0; ny /= n0; nz /= n0; }
-    else { nx = 0.0; ny = 0.0; nz = 1.0; }
+    double n[3] = {Qxx + Qxy + Qxz, Qxy + Qyy + Qyz, Qxz + Qyz - Qxx - Qyy};
+    double n2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
+    if (!(n2 > 1e-24)) { n[0] = 0.0; n[1] = 0.0; n[2] = 1.0; n2 = 1.0; }
     const double r1 = fabs(Qxx) + fabs(Qxy) + fabs(Qxz);
     const double r2 = fabs(Qxy) + fabs(Qyy) + fabs(Qyz);
     const double r3 = fabs(Qxz) + fabs(Qyz) + fabs(Qzz);
     const double alpha = fmax(r1, fmax(r2, r3)) + 1e-12;
-    for (int it = 0; it < 15; ++it) {
-        const double ax = Qxx * nx + Qxy * ny + Qxz * nz + alpha * nx;
-        const double ay = Qxy * nx + Qyy * ny + Qyz * nz + alpha * ny;
-        const double az = Qxz * nx + Qyz * ny + Qzz * nz + alpha * nz;
-        const double nn = sqrt(ax * ax + ay * ay + az * az);
-        if (nn < 1e-13) break;
-        nx = ax / nn; ny = ay / nn; nz = az / nn;
+    const double ia = 1.0 / alpha;
+    Sym3 m{fma(Qxx, ia, 1.0), Qxy * ia, Qxz * ia, fma(Qyy, ia, 1.0), Qyz * ia, fma(Qzz, ia, 1.0)};
+    const double n0[3] = {n[0], n[1], n[2]};
+    apply(m, n);
+    double v2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
+    if (v2 * (alpha * alpha) < 1e-26 * n2) {  // |M n| < 1e-13: the direction stays the first one
+        n[0] = n0[0]; n[1] = n0[1]; n[2] = n0[2];
+        v2 = n2;
+    } else {
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            m = square(m);
+            apply(m, n);
+        }
+        v2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
     }
+    const double inv = 1.0 / sqrt(v2);
+    const double nx = n[0] * inv, ny = n[1] * inv, nz = n[2] * inv;
     const double lam = nx * (Qxx * nx + Qxy * ny + Qxz * nz) + ny * (Qxy * nx + Qyy * ny + Qyz * nz) +
                        nz * (Qxz * nx + Qyz * ny + Qzz * nz);
     Nematic r{1.5 * lam, nx, ny, nz};

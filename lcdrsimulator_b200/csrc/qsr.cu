@@ -295,236 +295,137 @@ __global__ void k_nematic_out(const float* __restrict__ a, double* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------
-// FP64 observables. Every block writes one partial; a single-block pass sums the partials
-// in block order, so results do not depend on scheduling.
+// FP64 observables, one launch: the first blocks take the volume sums, the others the slice metrics.
+// Every block writes one partial; the last one to finish adds the partials in block order, so results
+// do not depend on scheduling.
 // ---------------------------------------------------------------------------------------
+enum ObsSum { kBulk, kElastic, kAnch, kRad, kSumS, kEven, kOdd, kXi, kObsSums, kMaxS = kObsSums, kMaxQ, kObsVals };
+enum ObsCount { kRadN, kCoreN, kEvenN, kOddN, kNonfinite, kDefects, kPlaq, kEdges, kObsCounts };
 struct ObsPartial {
-    double bulk, elastic, anch, rad_sum, S_sum, S_max, ce, co, ca, qmax;
-    unsigned long long rad_n, core_n, ce_n, co_n, ca_n, nonfinite;
+    double v[kObsVals];                  // sums, then maxima
+    unsigned long long n[kObsCounts];
 };
 
 struct ObsConst {
     QsrConst P;
-    double ix2dummy;
     double i2x, i2y, i2z;
     double c2, c3, c4;         // bulk energy coefficients (QSR.cu:887-899)
-    double Liso, L1, L2, L3;   // elastic energy selection (QSR.cu:955-987)
-    int all_L_zero;
+    double Liso, L2, L3;       // kappa if L1 = L2 = L3 = 0, else L1 (QSR.cu:955-987)
     double dV, Weff_half;      // cell volume; 0.5*W/delta_eff
     double S_shell;
     double cx, cy, cz, gx, gy, gz;  // FP64 geometry for normals and radial directions (cell units)
     double hx, hy, hz;               // spacing
     int checker_k;
+    int mode;                  // bit 0: defects on slice dk, bit 1: xi proxy on slice xk
+    int dk, xk;
+    double dthr, dcut, xthr;
+    int volume_blocks;
 };
 
-constexpr int kObsThreads = 256;
+constexpr int kObsThreads = 256, kObsWarps = kObsThreads / 32;
+// 128 registers: two blocks per SM. (With the FP64 state of a cell in 156 to 255 registers one block
+// fitted, and 16 reductions with a block barrier each cost as much as the cells of a 64^3 grid.)
+constexpr int kObsPerSM = 2;
+constexpr int kObsVolumeBlocks = 148 * 2 * kObsPerSM, kObsSliceBlocks = 148;
+constexpr size_t kObsBytes = (kObsVolumeBlocks + kObsSliceBlocks + 1) * sizeof(ObsPartial) + sizeof(unsigned);
 
-template <class T>
-__device__ __forceinline__ T block_sum(T v, T* sh) {
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    T r = 0;
-    if (threadIdx.x == 0)
-        for (int x = 0; x < (int)(blockDim.x >> 5); ++x) r += sh[x];
-    return r;  // valid in thread 0
-}
-
-__device__ __forceinline__ double block_max(double v, double* sh) {
-    v = warp_max(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x == 0)
-        for (int x = 0; x < (int)(blockDim.x >> 5); ++x) r = fmax(r, sh[x]);
-    return r;
-}
-
-__global__ void __launch_bounds__(kObsThreads) k_observe_volume(const float* __restrict__ q,
-                                                                const uint8_t* __restrict__ flags, ObsConst O,
-                                                                ObsPartial* __restrict__ part) {
+// Volume terms of cell (i, j, k).
+__device__ __forceinline__ void observe_cell(const float* __restrict__ q, const uint8_t* __restrict__ flags,
+                                             const ObsConst& O, int i, int j, int k, double v[kObsVals],
+                                             unsigned n[kObsCounts]) {
     const QsrConst& P = O.P;
-    const long long n = (long long)P.Nx * P.Ny * P.Nz;
-    ObsPartial a{};
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(t % P.Nz);
-        const long long r = t / P.Nz;
-        const int j = (int)(r % P.Ny);
-        const int i = (int)(r / P.Ny);
-        const long long id = (long long)i * P.si + (long long)j * P.sj + k;
-        const uint8_t f = flags[id];
-        double c[5];
-        bool finite = true;
+    const long long id = (long long)i * P.si + (long long)j * P.sj + k;
+    const uint8_t f = flags[id];
+    const float* b = q + id;
+    double c[5];
+    unsigned bits = 0;
+    bool finite = true;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+        const float x = b[m * P.sc];
+        bits |= __float_as_uint(x);
+        c[m] = (double)x;
+        finite = finite && isfinite(x);
+    }
+    if (!finite) n[kNonfinite]++;
+    const double Qxx = c[0], Qxy = c[1], Qxz = c[2], Qyy = c[3], Qyz = c[4], Qzz = -Qxx - Qyy;
+    const double trQ2 = Qxx * Qxx + Qyy * Qyy + Qzz * Qzz + 2 * (Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
+    v[kMaxQ] = fmax(v[kMaxQ], trQ2);  // squared; the root is taken at the end
+    const bool interior = (i >= 1 && j >= 1 && k >= 1 && i < P.Nx - 1 && j < P.Ny - 1 && k < P.Nz - 1);
+    // Outside the droplet a field that is zero, neighbours included, adds nothing.
+    if (interior && !(f & (kInside | kShell))) {
 #pragma unroll
         for (int m = 0; m < 5; ++m) {
-            c[m] = (double)q[m * P.sc + id];
-            finite = finite && isfinite(c[m]);
+            const float* p = b + m * P.sc;
+            bits |= __float_as_uint(p[P.si]) | __float_as_uint(p[-P.si]) | __float_as_uint(p[P.sj]) |
+                    __float_as_uint(p[-P.sj]) | __float_as_uint(p[1]) | __float_as_uint(p[-1]);
         }
-        if (!finite) a.nonfinite++;
-        {
-            const double zz = -c[0] - c[3];
-            const double tr = c[0] * c[0] + c[3] * c[3] + zz * zz + 2.0 * (c[1] * c[1] + c[2] * c[2] + c[4] * c[4]);
-            a.qmax = fmax(a.qmax, sqrt(fmax(tr, 0.0)));
-        }
-        const bool interior = (i >= 1 && j >= 1 && k >= 1 && i < P.Nx - 1 && j < P.Ny - 1 && k < P.Nz - 1);
-        if (interior) {
-            // computeEnergyKernel (QSR.cu:869-992).
-            const double Qxx = c[0], Qxy = c[1], Qxz = c[2], Qyy = c[3], Qyz = c[4], Qzz = -Qxx - Qyy;
-            const double trQ2 = Qxx * Qxx + Qyy * Qyy + Qzz * Qzz + 2 * (Qxy * Qxy + Qxz * Qxz + Qyz * Qyz);
-            const double a2xx = Qxx * Qxx + Qxy * Qxy + Qxz * Qxz;
-            const double a2xy = Qxx * Qxy + Qxy * Qyy + Qxz * Qyz;
-            const double a2xz = Qxx * Qxz + Qxy * Qyz + Qxz * Qzz;
-            const double a2yy = Qxy * Qxy + Qyy * Qyy + Qyz * Qyz;
-            const double a2yz = Qxy * Qxz + Qyy * Qyz + Qyz * Qzz;
-            const double a2zz = Qxz * Qxz + Qyz * Qyz + Qzz * Qzz;
-            const double trQ3 = Qxx * a2xx + Qyy * a2yy + Qzz * a2zz + 2.0 * (Qxy * a2xy + Qxz * a2xz + Qyz * a2yz);
-            a.bulk += (O.c2 * trQ2 - O.c3 * trQ3 + O.c4 * trQ2 * trQ2) * O.dV;
-            double d[6][3];
-#pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                const float* b = q + m * P.sc + id;
-                d[m][0] = ((double)b[P.si] - (double)b[-P.si]) * O.i2x;
-                d[m][1] = ((double)b[P.sj] - (double)b[-P.sj]) * O.i2y;
-                d[m][2] = ((double)b[1] - (double)b[-1]) * O.i2z;
-            }
-#pragma unroll
-            for (int x = 0; x < 3; ++x) d[5][x] = -(d[0][x] + d[3][x]);
-            auto sq = [&](int m) { return d[m][0] * d[m][0] + d[m][1] * d[m][1] + d[m][2] * d[m][2]; };
-            const double g2 = sq(0) + sq(3) + sq(5) + 2.0 * (sq(1) + sq(2) + sq(4));
-            double fel;
-            if (O.all_L_zero) {
-                fel = 0.5 * O.Liso * g2;
-            } else {
-                const double f1 = 0.5 * O.L1 * g2;
-                const double vx = d[0][0] + d[1][1] + d[2][2];
-                const double vy = d[1][0] + d[3][1] + d[4][2];
-                const double vz = d[2][0] + d[4][1] + d[5][2];
-                const double f2 = 0.5 * O.L2 * (vx * vx + vy * vy + vz * vz);
-                double f3 = 0.0;
-                if (O.L3 != 0.0) {
-                    auto M = [&](int x, int y) {
-                        return d[0][x] * d[0][y] + d[3][x] * d[3][y] + d[5][x] * d[5][y] +
-                               2.0 * (d[1][x] * d[1][y] + d[2][x] * d[2][y] + d[4][x] * d[4][y]);
-                    };
-                    f3 = 0.5 * O.L3 * (Qxx * M(0, 0) + Qyy * M(1, 1) + Qzz * M(2, 2) +
-                                       2.0 * (Qxy * M(0, 1) + Qxz * M(0, 2) + Qyz * M(1, 2)));
-                }
-                fel = f1 + f2 + f3;
-            }
-            a.elastic += fel * O.dV;
-        }
-        const double X = ((double)i - O.cx), Y = ((double)j - O.cy), Z = ((double)k - O.cz);
-        if (f & kAnchor) {
-            // computeAnchoringEnergyKernel (QSR.cu:654-695).
-            const double gx = X * O.gx, gy = Y * O.gy, gz = Z * O.gz;
-            const double gn = sqrt(gx * gx + gy * gy + gz * gz);
-            double nx = 1.0, ny = 0.0, nz = 0.0;
-            if (gn > 0.0) { nx = gx / gn; ny = gy / gn; nz = gz / gn; }
-            const double S = O.S_shell;
-            const double q0xx = S * (nx * nx - 1.0 / 3.0), q0xy = S * (nx * ny), q0xz = S * (nx * nz);
-            const double q0yy = S * (ny * ny - 1.0 / 3.0), q0yz = S * (ny * nz), q0zz = -(q0xx + q0yy);
-            const double dxx = c[0] - q0xx, dxy = c[1] - q0xy, dxz = c[2] - q0xz, dyy = c[3] - q0yy, dyz = c[4] - q0yz;
-            const double dzz = (-c[0] - c[3]) - q0zz;
-            const double diff2 = dxx * dxx + dyy * dyy + dzz * dzz + 2.0 * (dxy * dxy + dxz * dxz + dyz * dyz);
-            a.anch += O.Weff_half * diff2 * O.dV;
-        }
-        if (f & (kRadial | kCore)) {
-            const Nematic nf = nematic64(c, 1e-9, Nematic{0.0, 0.0, 0.0, 1.0});
-            if (f & kRadial) {
-                // computeRadialityKernel (QSR.cu:994-1015): r-hat from the centre.
-                const double px = X * O.hx, py = Y * O.hy, pz = Z * O.hz;
-                const double rr = sqrt(px * px + py * py + pz * pz);
-                double rx = 1.0, ry = 0.0, rz = 0.0;
-                if (rr > 1e-30) { rx = px / rr; ry = py / rr; rz = pz / rr; }
-                a.rad_sum += fabs(nf.nx * rx + nf.ny * ry + nf.nz * rz);
-                a.rad_n++;
-            }
-            if (f & kCore) {
-                a.S_sum += nf.S;
-                a.core_n++;
-                if (isfinite(nf.S)) a.S_max = fmax(a.S_max, nf.S);
-                if (k == O.checker_k && isfinite(nf.S) && nf.S > 0.01) {
-                    // Checkerboard sums on the defect slice (QSR.cu:2845-2868).
-                    a.ca += nf.S; a.ca_n++;
-                    if (((i + j) & 1) == 0) { a.ce += nf.S; a.ce_n++; }
-                    else { a.co += nf.S; a.co_n++; }
-                }
-            }
-        }
+    } else {
+        bits = 1;
     }
-    __shared__ double shd[kObsThreads / 32];
-    __shared__ unsigned long long shu[kObsThreads / 32];
-    ObsPartial res{};
-    res.bulk = block_sum(a.bulk, shd);
-    res.elastic = block_sum(a.elastic, shd);
-    res.anch = block_sum(a.anch, shd);
-    res.rad_sum = block_sum(a.rad_sum, shd);
-    res.S_sum = block_sum(a.S_sum, shd);
-    res.ce = block_sum(a.ce, shd);
-    res.co = block_sum(a.co, shd);
-    res.ca = block_sum(a.ca, shd);
-    res.S_max = block_max(a.S_max, shd);
-    res.qmax = block_max(a.qmax, shd);
-    res.rad_n = block_sum(a.rad_n, shu);
-    res.core_n = block_sum(a.core_n, shu);
-    res.ce_n = block_sum(a.ce_n, shu);
-    res.co_n = block_sum(a.co_n, shu);
-    res.ca_n = block_sum(a.ca_n, shu);
-    res.nonfinite = block_sum(a.nonfinite, shu);
-    if (threadIdx.x == 0) part[blockIdx.x] = res;
-}
-
-__global__ void __launch_bounds__(kObsThreads) k_observe_finalize(const ObsPartial* __restrict__ part, int n,
-                                                                  ObsPartial* __restrict__ out) {
-    ObsPartial a{};
-    for (int b = threadIdx.x; b < n; b += blockDim.x) {
-        const ObsPartial& p = part[b];
-        a.bulk += p.bulk; a.elastic += p.elastic; a.anch += p.anch; a.rad_sum += p.rad_sum; a.S_sum += p.S_sum;
-        a.ce += p.ce; a.co += p.co; a.ca += p.ca;
-        a.S_max = fmax(a.S_max, p.S_max); a.qmax = fmax(a.qmax, p.qmax);
-        a.rad_n += p.rad_n; a.core_n += p.core_n; a.ce_n += p.ce_n; a.co_n += p.co_n; a.ca_n += p.ca_n;
-        a.nonfinite += p.nonfinite;
-    }
-    __shared__ double shd[kObsThreads / 32];
-    __shared__ unsigned long long shu[kObsThreads / 32];
-    ObsPartial r{};
-    r.bulk = block_sum(a.bulk, shd);
-    r.elastic = block_sum(a.elastic, shd);
-    r.anch = block_sum(a.anch, shd);
-    r.rad_sum = block_sum(a.rad_sum, shd);
-    r.S_sum = block_sum(a.S_sum, shd);
-    r.ce = block_sum(a.ce, shd);
-    r.co = block_sum(a.co, shd);
-    r.ca = block_sum(a.ca, shd);
-    r.S_max = block_max(a.S_max, shd);
-    r.qmax = block_max(a.qmax, shd);
-    r.rad_n = block_sum(a.rad_n, shu);
-    r.core_n = block_sum(a.core_n, shu);
-    r.ce_n = block_sum(a.ce_n, shu);
-    r.co_n = block_sum(a.co_n, shu);
-    r.ca_n = block_sum(a.ca_n, shu);
-    r.nonfinite = block_sum(a.nonfinite, shu);
-    if (threadIdx.x == 0) *out = r;
-}
-
-// Slice nematic field (S, nx, ny) for the 2-D defect and xi proxies.
-__global__ void k_slice_nematic(const float* __restrict__ q, QsrConst P, int kz, double* __restrict__ snf) {
-    const long long n = (long long)P.Nx * P.Ny;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(t % P.Ny);
-        const int i = (int)(t / P.Ny);
-        const long long id = (long long)i * P.si + (long long)j * P.sj + kz;
-        double c[5];
+    if (interior && bits != 0) {
+        // computeEnergyKernel (QSR.cu:869-992); tr Q^3 = 3 det Q of a traceless Q
+        const double det = Qxx * (Qyy * Qzz - Qyz * Qyz) - Qxy * (Qxy * Qzz - Qyz * Qxz) + Qxz * (Qxy * Qyz - Qyy * Qxz);
+        v[kBulk] += O.c2 * trQ2 - 3.0 * O.c3 * det + O.c4 * trQ2 * trQ2;
+        double d[5][3];
 #pragma unroll
-        for (int m = 0; m < 5; ++m) c[m] = (double)q[m * P.sc + id];
+        for (int m = 0; m < 5; ++m) {
+            const float* p = b + m * P.sc;
+            d[m][0] = ((double)p[P.si] - (double)p[-P.si]) * O.i2x;
+            d[m][1] = ((double)p[P.sj] - (double)p[-P.sj]) * O.i2y;
+            d[m][2] = ((double)p[1] - (double)p[-1]) * O.i2z;
+        }
+        // M_xy = dQ_kl/dx dQ_kl/dy over all nine entries, dQ_zz = -(dQ_xx + dQ_yy)
+        auto M = [&](int x, int y) {
+            return 2.0 * (d[0][x] * (d[0][y] + 0.5 * d[3][y]) + d[3][x] * (d[3][y] + 0.5 * d[0][y]) + d[1][x] * d[1][y] +
+                          d[2][x] * d[2][y] + d[4][x] * d[4][y]);
+        };
+        const double m00 = M(0, 0), m11 = M(1, 1), m22 = M(2, 2);
+        double fel = 0.5 * O.Liso * (m00 + m11 + m22);
+        if (O.L2 != 0.0) {
+            const double vx = d[0][0] + d[1][1] + d[2][2];
+            const double vy = d[1][0] + d[3][1] + d[4][2];
+            const double vz = d[2][0] + d[4][1] - (d[0][2] + d[3][2]);
+            fel += 0.5 * O.L2 * (vx * vx + vy * vy + vz * vz);
+        }
+        if (O.L3 != 0.0)
+            fel += 0.5 * O.L3 * (Qxx * m00 + Qyy * m11 + Qzz * m22 +
+                                 2.0 * (Qxy * M(0, 1) + Qxz * M(0, 2) + Qyz * M(1, 2)));
+        v[kElastic] += fel;
+    }
+    const double X = ((double)i - O.cx), Y = ((double)j - O.cy), Z = ((double)k - O.cz);
+    if (f & kAnchor) {
+        // computeAnchoringEnergyKernel (QSR.cu:654-695).
+        const double gx = X * O.gx, gy = Y * O.gy, gz = Z * O.gz;
+        const double gn = sqrt(gx * gx + gy * gy + gz * gz);
+        double nx = 1.0, ny = 0.0, nz = 0.0;
+        if (gn > 0.0) { nx = gx / gn; ny = gy / gn; nz = gz / gn; }
+        const double S = O.S_shell;
+        const double q0xx = S * (nx * nx - 1.0 / 3.0), q0xy = S * (nx * ny), q0xz = S * (nx * nz);
+        const double q0yy = S * (ny * ny - 1.0 / 3.0), q0yz = S * (ny * nz), q0zz = -(q0xx + q0yy);
+        const double dxx = Qxx - q0xx, dxy = Qxy - q0xy, dxz = Qxz - q0xz, dyy = Qyy - q0yy, dyz = Qyz - q0yz;
+        const double dzz = Qzz - q0zz;
+        v[kAnch] += dxx * dxx + dyy * dyy + dzz * dzz + 2.0 * (dxy * dxy + dxz * dxz + dyz * dyz);
+    }
+    if (f & (kRadial | kCore)) {
         const Nematic nf = nematic64(c, 1e-9, Nematic{0.0, 0.0, 0.0, 1.0});
-        snf[3 * t + 0] = nf.S;
-        snf[3 * t + 1] = nf.nx;
-        snf[3 * t + 2] = nf.ny;
+        if (f & kRadial) {
+            // computeRadialityKernel (QSR.cu:994-1015): r-hat from the centre.
+            const double px = X * O.hx, py = Y * O.hy, pz = Z * O.hz;
+            const double rr = sqrt(px * px + py * py + pz * pz);
+            v[kRad] += rr > 1e-30 ? fabs(nf.nx * px + nf.ny * py + nf.nz * pz) / rr : fabs(nf.nx);
+            n[kRadN]++;
+        }
+        if (f & kCore) {
+            v[kSumS] += nf.S;
+            n[kCoreN]++;
+            if (isfinite(nf.S)) v[kMaxS] = fmax(v[kMaxS], nf.S);
+            if (k == O.checker_k && isfinite(nf.S) && nf.S > 0.01) {
+                // Checkerboard sums on the defect slice (QSR.cu:2845-2868).
+                if (((i + j) & 1) == 0) { v[kEven] += nf.S; n[kEvenN]++; }
+                else { v[kOdd] += nf.S; n[kOddN]++; }
+            }
+        }
     }
 }
 
@@ -536,86 +437,131 @@ __device__ __forceinline__ double wrap_pi(double x) {
     return x - kPi;
 }
 
-struct SlicePartial {
-    double xi_sum;
-    unsigned long long defects, plaq, edges;
-};
-
-// Plaquette winding (QSR.cu:1114-1176) and wrapped phase-gradient edges (QSR.cu:1042-1106)
-// on one slice, from the slice nematic arrays. mode bit 1: defects, bit 2: xi.
-__global__ void __launch_bounds__(kObsThreads) k_slice_metrics(const double* __restrict__ dnf,
-                                                               const double* __restrict__ xnf, int Nx, int Ny,
-                                                               double dthr, double dcut, double xthr, int mode,
-                                                               SlicePartial* __restrict__ part) {
-    SlicePartial a{};
-    auto ok = [](const double* f, double thr) {
-        return isfinite(f[0]) && isfinite(f[1]) && isfinite(f[2]) && f[0] > thr;
+// Plaquette winding (QSR.cu:1114-1176) and wrapped phase-gradient edges (QSR.cu:1042-1106) of cell
+// (i, j) with its neighbours at i + 1 and j + 1, on the defect and the xi slice.
+__device__ __forceinline__ void observe_slice(const float* __restrict__ q, const ObsConst& O, int i, int j,
+                                              double v[kObsVals], unsigned n[kObsCounts]) {
+    const QsrConst& P = O.P;
+    struct Site {
+        double S, psi;
+        bool fine;
     };
-    auto psi = [](const double* f) { return 2.0 * atan2(f[2], f[1]); };
-    const long long n = (long long)Nx * Ny;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(t % Ny);
-        const int i = (int)(t / Ny);
-        if ((mode & 1) && i < Nx - 1 && j < Ny - 1) {
-            const double* f00 = dnf + 3 * ((long long)i * Ny + j);
-            const double* f10 = dnf + 3 * ((long long)(i + 1) * Ny + j);
-            const double* f11 = dnf + 3 * ((long long)(i + 1) * Ny + j + 1);
-            const double* f01 = dnf + 3 * ((long long)i * Ny + j + 1);
-            if (ok(f00, dthr) && ok(f10, dthr) && ok(f11, dthr) && ok(f01, dthr)) {
-                const double p00 = psi(f00), p10 = psi(f10), p11 = psi(f11), p01 = psi(f01);
-                const double dsum = wrap_pi(p10 - p00) + wrap_pi(p11 - p10) + wrap_pi(p01 - p11) + wrap_pi(p00 - p01);
-                const double s = 0.5 * (dsum * (1.0 / (2.0 * kPi)));
-                a.plaq++;
-                if (fabs(s) > dcut) a.defects++;
+    auto site = [&](int ii, int jj, int k) {
+        double c[5];
+        const long long id = (long long)ii * P.si + (long long)jj * P.sj + k;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) c[m] = (double)q[m * P.sc + id];
+        const Nematic f = nematic64(c, 1e-9, Nematic{0.0, 0.0, 0.0, 1.0});
+        return Site{f.S, 2.0 * atan2(f.ny, f.nx), isfinite(f.S) && isfinite(f.nx) && isfinite(f.ny)};
+    };
+    const bool ip = i < P.Nx - 1, jp = j < P.Ny - 1;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+        const bool dfc = (O.mode & 1) && pass == 0, xi = (O.mode & 2) && (O.xk == O.dk && (O.mode & 1) ? pass == 0 : pass == 1);
+        if (!dfc && !xi) continue;
+        const int k = pass == 0 ? O.dk : O.xk;
+        const Site s00 = site(i, j, k), s10 = ip ? site(i + 1, j, k) : s00, s01 = jp ? site(i, j + 1, k) : s00;
+        if (dfc && ip && jp) {
+            const Site s11 = site(i + 1, j + 1, k);
+            auto ok = [&](const Site& s) { return s.fine && s.S > O.dthr; };
+            if (ok(s00) && ok(s10) && ok(s11) && ok(s01)) {
+                const double dsum = wrap_pi(s10.psi - s00.psi) + wrap_pi(s11.psi - s10.psi) + wrap_pi(s01.psi - s11.psi) +
+                                    wrap_pi(s00.psi - s01.psi);
+                n[kPlaq]++;
+                if (fabs(0.5 * (dsum * (1.0 / (2.0 * kPi)))) > O.dcut) n[kDefects]++;
             }
         }
-        if (mode & 2) {
-            const double* f0 = xnf + 3 * ((long long)i * Ny + j);
-            if (i < Nx - 1) {
-                const double* f1 = xnf + 3 * ((long long)(i + 1) * Ny + j);
-                if (ok(f0, xthr) && ok(f1, xthr)) {
-                    const double d = wrap_pi(psi(f1) - psi(f0));
-                    a.xi_sum += d * d;
-                    a.edges++;
-                }
-            }
-            if (j < Ny - 1) {
-                const double* f1 = xnf + 3 * ((long long)i * Ny + j + 1);
-                if (ok(f0, xthr) && ok(f1, xthr)) {
-                    const double d = wrap_pi(psi(f1) - psi(f0));
-                    a.xi_sum += d * d;
-                    a.edges++;
-                }
-            }
+        if (xi) {
+            auto edge = [&](bool in, const Site& s) {
+                if (!(in && s00.fine && s.fine && s00.S > O.xthr && s.S > O.xthr)) return;
+                const double d = wrap_pi(s.psi - s00.psi);
+                v[kXi] += d * d;
+                n[kEdges]++;
+            };
+            edge(ip, s10);
+            edge(jp, s01);
         }
     }
-    __shared__ double shd[kObsThreads / 32];
-    __shared__ unsigned long long shu[kObsThreads / 32];
-    SlicePartial r{};
-    r.xi_sum = block_sum(a.xi_sum, shd);
-    r.defects = block_sum(a.defects, shu);
-    r.plaq = block_sum(a.plaq, shu);
-    r.edges = block_sum(a.edges, shu);
-    if (threadIdx.x == 0) part[blockIdx.x] = r;
 }
 
-__global__ void k_slice_finalize(const SlicePartial* __restrict__ part, int n, SlicePartial* __restrict__ out) {
-    SlicePartial a{};
-    for (int b = threadIdx.x; b < n; b += blockDim.x) {
-        a.xi_sum += part[b].xi_sum; a.defects += part[b].defects; a.plaq += part[b].plaq; a.edges += part[b].edges;
+// Adds the threads' values of a block in a fixed order; valid in threads 0 .. kObsVals + kObsCounts - 1,
+// which write them to `out`. One block barrier.
+template <class N>
+__device__ __forceinline__ void observe_block(const double v[kObsVals], const N n[kObsCounts], ObsPartial* out) {
+    __shared__ double sv[kObsWarps][kObsVals];
+    __shared__ unsigned long long sn[kObsWarps][kObsCounts];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int m = 0; m < kObsVals; ++m) {
+        const double r = m < kObsSums ? warp_sum(v[m]) : warp_max(v[m]);
+        if (lane == 0) sv[w][m] = r;
     }
-    __shared__ double shd[kObsThreads / 32];
-    __shared__ unsigned long long shu[kObsThreads / 32];
-    SlicePartial r{};
-    r.xi_sum = block_sum(a.xi_sum, shd);
-    r.defects = block_sum(a.defects, shu);
-    r.plaq = block_sum(a.plaq, shu);
-    r.edges = block_sum(a.edges, shu);
-    if (threadIdx.x == 0) *out = r;
+#pragma unroll
+    for (int m = 0; m < kObsCounts; ++m) {
+        const unsigned long long r = warp_sum((unsigned long long)n[m]);
+        if (lane == 0) sn[w][m] = r;
+    }
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t < kObsVals) {
+        double r = 0.0;
+        for (int x = 0; x < kObsWarps; ++x) r = t < kObsSums ? r + sv[x][t] : fmax(r, sv[x][t]);
+        out->v[t] = r;
+    } else if (t < kObsVals + kObsCounts) {
+        unsigned long long r = 0;
+        for (int x = 0; x < kObsWarps; ++x) r += sn[x][t - kObsVals];
+        out->n[t - kObsVals] = r;
+    }
 }
 
-constexpr int kObsBlocks = 148 * 8;
-constexpr int kSliceBlocks = 148;
+__global__ void __launch_bounds__(kObsThreads, kObsPerSM) k_observe(const float* __restrict__ q,
+                                                                    const uint8_t* __restrict__ flags, ObsConst O,
+                                                                    ObsPartial* __restrict__ part,
+                                                                    unsigned* __restrict__ ticket,
+                                                                    ObsPartial* __restrict__ out) {
+    const QsrConst& P = O.P;
+    double v[kObsVals] = {};
+    unsigned n[kObsCounts] = {};
+    if ((int)blockIdx.x < O.volume_blocks) {
+        // A warp takes a row of cells at a time: one division per row instead of two per cell.
+        const int lane = threadIdx.x & 31;
+        const long long rows = (long long)P.Nx * P.Ny, warps = (long long)O.volume_blocks * kObsWarps;
+        for (long long r = (long long)blockIdx.x * kObsWarps + (threadIdx.x >> 5); r < rows; r += warps) {
+            const int i = (int)(r / P.Ny), j = (int)(r - (long long)i * P.Ny);
+            for (int k = lane; k < P.Nz; k += 32) observe_cell(q, flags, O, i, j, k, v, n);
+        }
+        v[kBulk] *= O.dV;
+        v[kElastic] *= O.dV;
+        v[kAnch] *= O.Weff_half * O.dV;
+        v[kMaxQ] = sqrt(v[kMaxQ]);
+    } else {
+        const long long cells = (long long)P.Nx * P.Ny, step = (long long)(gridDim.x - O.volume_blocks) * kObsThreads;
+        for (long long t = (long long)(blockIdx.x - O.volume_blocks) * kObsThreads + threadIdx.x; t < cells; t += step)
+            observe_slice(q, O, (int)(t / P.Ny), (int)(t % P.Ny), v, n);
+    }
+    observe_block(v, n, &part[blockIdx.x]);
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double tv[kObsVals] = {};
+    unsigned long long tn[kObsCounts] = {};
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kObsThreads) {
+#pragma unroll
+        for (int m = 0; m < kObsVals; ++m) {
+            const double x = __ldcg(&part[b].v[m]);
+            tv[m] = m < kObsSums ? tv[m] + x : fmax(tv[m], x);
+        }
+#pragma unroll
+        for (int m = 0; m < kObsCounts; ++m) tn[m] += __ldcg(&part[b].n[m]);
+    }
+    __syncthreads();  // the shared arrays of the first reduction are read
+    observe_block(tv, tn, out);
+    if (threadIdx.x == 0) *ticket = 0;
+}
 
 }  // namespace
 
@@ -635,9 +581,7 @@ struct qsr_handle {
     uint8_t* flags = nullptr;
     double* stage = nullptr;       // FP64 AoS staging (5 or 4 doubles per cell)
     bool stage_shared = false;     // staging owned by an ensemble (shared by its droplets)
-    ObsPartial* opart = nullptr;   // kObsBlocks + 1
-    SlicePartial* spart = nullptr; // kSliceBlocks + 1
-    double* snf = nullptr;         // 2 slices x Nx*Ny x 3
+    ObsPartial* opart = nullptr;   // block partials, the result, then the ticket counter
     TiledPlan tiled{};             // tiled-kernel launch plan
     int cur = 0;
     bool uploaded = false;
@@ -738,10 +682,16 @@ int kernel_choice() {
 
 namespace {
 
-// Enqueues the observables of the current field on stream `st`, with the block results copied
-// to R and SR (host memory; pinned for the copies to be asynchronous).
-int observe_enqueue(qsr_handle* h, const qsr_observe_args* a, cudaStream_t st, ObsPartial* R, SlicePartial* SR,
-                    bool* wd_out, bool* wx_out) {
+// Whether a slice metric was asked for on a slice of the grid.
+bool observe_defects(const qsr_handle* h, const qsr_observe_args* a) {
+    return a->want_defects && a->defects_z_slice >= 0 && a->defects_z_slice < h->p.Nz;
+}
+bool observe_xi(const qsr_handle* h, const qsr_observe_args* a) {
+    return a->want_xi && a->xi_z_slice >= 0 && a->xi_z_slice < h->p.Nz;
+}
+
+// Enqueues the observables of the current field on stream `st`; the result goes to `out` (device).
+int observe_enqueue(qsr_handle* h, const qsr_observe_args* a, cudaStream_t st, ObsPartial* out) {
     const qsr_params& p = h->p;
     ObsConst O{};
     O.P = make_const(h, a->T, a->S_shell, 1.0);
@@ -749,8 +699,8 @@ int observe_enqueue(qsr_handle* h, const qsr_observe_args* a, cudaStream_t st, O
     const double dT = a->T - p.T_star;
     if (p.bulk_modechoice == 1) { O.c2 = (3.0 * p.a * dT) / 2.0; O.c3 = (3.0 * p.b) / 2.0; O.c4 = (9.0 * p.c) / 8.0; }
     else { O.c2 = (3.0 * p.a * dT) / 2.0; O.c3 = (9.0 * p.b) / 2.0; O.c4 = (9.0 * p.c) / 4.0; }
-    O.all_L_zero = (p.L1 == 0.0 && p.L2 == 0.0 && p.L3 == 0.0);
-    O.Liso = p.kappa; O.L1 = p.L1; O.L2 = p.L2; O.L3 = p.L3;
+    O.Liso = (p.L1 == 0.0 && p.L2 == 0.0 && p.L3 == 0.0) ? p.kappa : p.L1;
+    O.L2 = p.L2; O.L3 = p.L3;
     O.dV = p.dx * p.dy * p.dz;
     O.Weff_half = (h->delta_eff > 0.0) ? 0.5 * (p.W / h->delta_eff) : 0.0;
     O.S_shell = a->S_shell;
@@ -762,74 +712,50 @@ int observe_enqueue(qsr_handle* h, const qsr_observe_args* a, cudaStream_t st, O
     O.gz = (p.dz / (h->g.rz * h->g.rz)) / sx;
     O.hx = p.dx; O.hy = p.dy; O.hz = p.dz;
     O.checker_k = std::min(std::max(a->defects_z_slice, 0), p.Nz - 1);
-    const float* q = h->q[h->cur];
-    k_observe_volume<<<kObsBlocks, kObsThreads, 0, st>>>(q, h->flags, O, h->opart);
+    const bool wd = observe_defects(h, a), wx = observe_xi(h, a);
+    O.mode = (wd ? 1 : 0) | (wx ? 2 : 0);
+    O.dk = a->defects_z_slice;
+    O.xk = a->xi_z_slice;
+    O.dthr = a->defects_S_threshold; O.dcut = a->defects_charge_cutoff; O.xthr = a->xi_S_threshold;
+    const long long rows = (long long)p.Nx * p.Ny;
+    O.volume_blocks = grid_blocks(rows, kObsWarps, kObsVolumeBlocks);
+    const int slice = (wd || wx) ? grid_blocks(rows, kObsThreads, kObsSliceBlocks) : 0;
+    ObsPartial* result = h->opart + kObsVolumeBlocks + kObsSliceBlocks;
+    k_observe<<<O.volume_blocks + slice, kObsThreads, 0, st>>>(h->q[h->cur], h->flags, O, h->opart,
+                                                               reinterpret_cast<unsigned*>(result + 1), out ? out : result);
     h->launches++;
-    LDG_LAUNCHED("k_observe_volume");
-    k_observe_finalize<<<1, kObsThreads, 0, st>>>(h->opart, kObsBlocks, h->opart + kObsBlocks);
-    h->launches++;
-    LDG_LAUNCHED("k_observe_finalize");
-    const bool wd = a->want_defects && a->defects_z_slice >= 0 && a->defects_z_slice < p.Nz;
-    const bool wx = a->want_xi && a->xi_z_slice >= 0 && a->xi_z_slice < p.Nz;
-    const long long nxy = (long long)p.Nx * p.Ny;
-    if (wd || wx) {
-        double* dnf = h->snf;
-        double* xnf = h->snf + 3 * nxy;
-        if (wd) {
-            k_slice_nematic<<<grid_blocks(nxy, 256, 148 * 4), 256, 0, st>>>(q, O.P, a->defects_z_slice, dnf);
-            h->launches++;
-        }
-        if (wx) {
-            if (wd && a->xi_z_slice == a->defects_z_slice) {
-                xnf = dnf;
-            } else {
-                k_slice_nematic<<<grid_blocks(nxy, 256, 148 * 4), 256, 0, st>>>(q, O.P, a->xi_z_slice, xnf);
-                h->launches++;
-            }
-        }
-        const int mode = (wd ? 1 : 0) | (wx ? 2 : 0);
-        k_slice_metrics<<<kSliceBlocks, kObsThreads, 0, st>>>(dnf, xnf, p.Nx, p.Ny, a->defects_S_threshold,
-                                                                     a->defects_charge_cutoff, a->xi_S_threshold, mode,
-                                                                     h->spart);
-        k_slice_finalize<<<1, kObsThreads, 0, st>>>(h->spart, kSliceBlocks, h->spart + kSliceBlocks);
-        h->launches += 2;
-        LDG_LAUNCHED("k_slice_metrics");
-    }
-    LDG_CUDA(cudaMemcpyAsync(R, h->opart + kObsBlocks, sizeof(*R), cudaMemcpyDeviceToHost, st));
-    if (wd || wx) LDG_CUDA(cudaMemcpyAsync(SR, h->spart + kSliceBlocks, sizeof(*SR), cudaMemcpyDeviceToHost, st));
-    *wd_out = wd;
-    *wx_out = wx;
+    LDG_LAUNCHED("k_observe");
     return LDG_OK;
 }
 
 // Fills the observables from the reduced block results.
-void observe_finish(const qsr_handle* h, const ObsPartial& R, const SlicePartial& SR, bool wd, bool wx,
-                    qsr_observables* o) {
+void observe_finish(const qsr_handle* h, const qsr_observe_args* a, const ObsPartial& R, qsr_observables* o) {
     const qsr_params& p = h->p;
     const double nan = std::numeric_limits<double>::quiet_NaN();
     std::memset(o, 0, sizeof(*o));
-    o->bulk = R.bulk; o->elastic = R.elastic; o->anchoring = R.anch;
-    o->total = R.bulk + R.elastic + R.anch;
-    o->radiality_count = (long long)R.rad_n;
-    o->radiality = R.rad_n > 0 ? R.rad_sum / (double)R.rad_n : 0.0;
-    o->core_count = (long long)R.core_n;
-    o->avg_S = R.core_n > 0 ? R.S_sum / (double)R.core_n : 0.0;
-    o->max_S = R.S_max;
+    o->bulk = R.v[kBulk]; o->elastic = R.v[kElastic]; o->anchoring = R.v[kAnch];
+    o->total = o->bulk + o->elastic + o->anchoring;
+    o->radiality_count = (long long)R.n[kRadN];
+    o->radiality = R.n[kRadN] > 0 ? R.v[kRad] / (double)R.n[kRadN] : 0.0;
+    o->core_count = (long long)R.n[kCoreN];
+    o->avg_S = R.n[kCoreN] > 0 ? R.v[kSumS] / (double)R.n[kCoreN] : 0.0;
+    o->max_S = R.v[kMaxS];
     o->checker_rel = nan;
-    if (R.S_max >= 0.5 && R.ce_n > 10 && R.co_n > 10 && R.ca_n > 20 && R.ca != 0.0)
-        o->checker_rel = std::fabs(R.ce - R.co) / std::fabs(R.ca);
-    o->defect_count = (long long)SR.defects;
-    o->defect_plaquettes = (long long)SR.plaq;
-    o->defect_density = (wd && SR.plaq > 0) ? (double)SR.defects / (double)SR.plaq : nan;
-    o->xi_edges = (long long)SR.edges;
+    const double all = R.v[kEven] + R.v[kOdd];
+    if (o->max_S >= 0.5 && R.n[kEvenN] > 10 && R.n[kOddN] > 10 && R.n[kEvenN] + R.n[kOddN] > 20 && all != 0.0)
+        o->checker_rel = std::fabs(R.v[kEven] - R.v[kOdd]) / std::fabs(all);
+    o->defect_count = (long long)R.n[kDefects];
+    o->defect_plaquettes = (long long)R.n[kPlaq];
+    o->defect_density = (observe_defects(h, a) && R.n[kPlaq] > 0) ? (double)R.n[kDefects] / (double)R.n[kPlaq] : nan;
+    o->xi_edges = (long long)R.n[kEdges];
     o->xi_grad_proxy = nan;
-    if (wx && SR.edges > 0) {
-        const double ms = SR.xi_sum / (double)SR.edges;
+    if (observe_xi(h, a) && R.n[kEdges] > 0) {
+        const double ms = R.v[kXi] / (double)R.n[kEdges];
         const double inv = (ms > 0.0) ? (1.0 / std::sqrt(ms + 1e-30)) : (1.0 / std::sqrt(1e-30));
         o->xi_grad_proxy = std::min(inv, 0.5 * (double)std::min(p.Nx, p.Ny));
     }
-    o->max_q_norm = R.qmax;
-    o->nonfinite_cells = (long long)R.nonfinite;
+    o->max_q_norm = R.v[kMaxQ];
+    o->nonfinite_cells = (long long)R.n[kNonfinite];
 }
 
 }  // namespace
@@ -908,9 +834,7 @@ int qsr_create(const qsr_params* params, qsr_handle** out) {
     const size_t fbytes = (size_t)h->sc * 5 * sizeof(float);
     if ((rc = alloc_or_fail((void**)&h->q[0], fbytes)) || (rc = alloc_or_fail((void**)&h->q[1], fbytes)) ||
         (rc = alloc_or_fail((void**)&h->flags, (size_t)h->sc)) ||
-        (rc = alloc_or_fail((void**)&h->opart, (kObsBlocks + 1) * sizeof(ObsPartial))) ||
-        (rc = alloc_or_fail((void**)&h->spart, (kSliceBlocks + 1) * sizeof(SlicePartial))) ||
-        (rc = alloc_or_fail((void**)&h->snf, (size_t)2 * p.Nx * p.Ny * 3 * sizeof(double))) ||
+        (rc = alloc_or_fail((void**)&h->opart, kObsBytes)) ||
         (p.compensated && ((rc = alloc_or_fail((void**)&h->lo[0], fbytes)) ||
                            (rc = alloc_or_fail((void**)&h->lo[1], fbytes))))) {
         qsr_destroy(h);
@@ -918,6 +842,7 @@ int qsr_create(const qsr_params* params, qsr_handle** out) {
     }
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMemcpy(h->flags, fl.data(), (size_t)h->sc, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(h->opart, 0, kObsBytes);
     if (e == cudaSuccess) e = cudaMemset(h->q[0], 0, fbytes);
     if (e == cudaSuccess) e = cudaMemset(h->q[1], 0, fbytes);
     if (e == cudaSuccess && h->lo[0]) e = cudaMemset(h->lo[0], 0, fbytes);
@@ -1163,13 +1088,12 @@ int qsr_observe(qsr_handle* h, const qsr_observe_args* a, qsr_observables* o) {
     LDG_REQUIRE(h && a && o, LDG_ERR_ARG, "qsr_observe: null argument");
     DeviceGuard device_guard(h->device);
     ObsPartial R{};
-    SlicePartial SR{};
-    bool wd = false, wx = false;
-    int rc = observe_enqueue(h, a, h->stream, &R, &SR, &wd, &wx);
+    int rc = observe_enqueue(h, a, h->stream, nullptr);
     if (rc) return rc;
-    LDG_CUDA(cudaStreamSynchronize(h->stream));
+    LDG_CUDA(cudaMemcpyAsync(&R, h->opart + kObsVolumeBlocks + kObsSliceBlocks, sizeof(R), cudaMemcpyDeviceToHost,
+                             h->stream));
     if ((rc = tiled_check(h->tiled, h->stream))) return rc;
-    observe_finish(h, R, SR, wd, wx, o);
+    observe_finish(h, a, R, o);
     return LDG_OK;
 }
 
@@ -1252,7 +1176,7 @@ int qsr_destroy(qsr_handle* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     cudaFree(h->q[0]); cudaFree(h->q[1]); cudaFree(h->lo[0]); cudaFree(h->lo[1]); cudaFree(h->rhs); cudaFree(h->flags);
     if (!h->stage_shared) cudaFree(h->stage);
-    cudaFree(h->opart); cudaFree(h->spart); cudaFree(h->snf);
+    cudaFree(h->opart);
     tiled_plan_free(h->tiled);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -1270,7 +1194,7 @@ struct ens_handle {
     ens_params p{};
     int device = -1;                       // the GPU the ensemble was created on
     double* stage = nullptr;               // host-boundary staging shared by all droplets
-    void* obs_host = nullptr;              // pinned block results of ens_observe_all
+    ObsPartial* d_obs = nullptr;           // results of ens_observe_all, one per droplet
     std::vector<qsr_handle*> inst;
     std::vector<ens_instance> desc;
     std::vector<tiled::EnsInstDev> host_inst;
@@ -1696,27 +1620,17 @@ int ens_observe_all(ens_handle* h, const qsr_observe_args* args, qsr_observables
     if (rc) return rc;
     ens_sync_cur(h);
     const size_t n = h->inst.size();
-    if (!h->obs_host) {
-        LDG_CUDA(cudaMallocHost((void**)&h->obs_host, n * (sizeof(ObsPartial) + sizeof(SlicePartial))));
-    }
-    ObsPartial* R = reinterpret_cast<ObsPartial*>(h->obs_host);
-    SlicePartial* SR = reinterpret_cast<SlicePartial*>(R + n);
-    std::vector<char> wd(n), wx(n);
+    // Every droplet's reductions on the ensemble's stream, after its steps; one copy of all results.
+    if (!h->d_obs && (rc = alloc_or_fail((void**)&h->d_obs, n * sizeof(ObsPartial)))) return rc;
+    std::vector<ObsPartial> R(n);
     std::vector<qsr_observe_args> a(n);
     for (size_t i = 0; i < n; ++i) {
         a[i] = args ? args[i] : ens_default_observe_args(h, (int)i);
-        std::memset(&SR[i], 0, sizeof(SlicePartial));
-        bool d = false, x = false;
-        // every droplet's reductions on the ensemble's stream, after its steps
-        if ((rc = observe_enqueue(h->inst[i], &a[i], h->stream, &R[i], &SR[i], &d, &x))) return rc;
-        wd[i] = d;
-        wx[i] = x;
+        if ((rc = observe_enqueue(h->inst[i], &a[i], h->stream, h->d_obs + i))) return rc;
     }
+    LDG_CUDA(cudaMemcpyAsync(R.data(), h->d_obs, n * sizeof(ObsPartial), cudaMemcpyDeviceToHost, h->stream));
     LDG_CUDA(cudaStreamSynchronize(h->stream));
-    for (size_t i = 0; i < n; ++i) {
-        if ((rc = tiled_check(h->inst[i]->tiled, h->stream))) return rc;
-        observe_finish(h->inst[i], R[i], SR[i], wd[i] != 0, wx[i] != 0, &out[i]);
-    }
+    for (size_t i = 0; i < n; ++i) observe_finish(h->inst[i], &a[i], R[i], &out[i]);
     return LDG_OK;
 }
 
@@ -1816,7 +1730,7 @@ int ens_destroy(ens_handle* h) {
     ens_drop_graph(h);
     for (qsr_handle* q : h->inst) qsr_destroy(q);
     cudaFree(h->stage);
-    if (h->obs_host) cudaFreeHost(h->obs_host);
+    cudaFree(h->d_obs);
     cudaFree(h->d_tms); cudaFree(h->d_inst); cudaFree(h->d_items); cudaFree(h->d_masks); cudaFree(h->d_ctl); cudaFree(h->d_err);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
