@@ -166,73 +166,6 @@ __global__ void __launch_bounds__(256) k_jacobi(const float* __restrict__ rhs, c
     for (int m = 0; m < 5; ++m) qn[m * P.sc + id] = o[m];
 }
 
-// The same sweep over the tiles of the explicit step's work list only (tiles holding moving or
-// strongly anchored cells, each over its plane range), writing only moving and strongly anchored
-// cells. Every other cell never changes: it holds the same value in both ping-pong buffers, so
-// the reference's copy of it (QSR.cu:803-810) is already done. One block of 128 threads per
-// visited tile plane (the work list expanded to single planes); each thread updates two
-// neighbouring cells (k and k + 1, k even): the centre, i +- 1 and j +- 1 operands and the
-// right-hand side of both cells are 8-byte loads, the k-neighbours two 4-byte loads. Each cell's
-// arithmetic is the full-box sweep's, operand for operand.
-template <bool kLast>
-__global__ void __launch_bounds__(128) k_jacobi_tiled(const float* __restrict__ rhs, const float* __restrict__ qo,
-                                                       float* __restrict__ qn, const uint8_t* __restrict__ flags,
-                                                       const int4* __restrict__ items, QsrConst P) {
-    const int4 item = items[blockIdx.x];
-    const int i = item.z;
-    const int k = item.y + 2 * (int)(threadIdx.x & 15);  // even (tiles start at k0 = 2 mod 4)
-    const int j = item.x + (int)(threadIdx.x >> 4);
-    if (k < 0 || k >= P.Nz || j >= P.Ny) return;  // the first tile of a row may start at k = -2
-    const long long id = (long long)i * P.si + (long long)j * P.sj + k;
-    const bool has1 = k + 1 < P.Nz;
-    const unsigned f2 = *reinterpret_cast<const unsigned short*>(flags + id);  // both cells' classes
-    const uint8_t f[2] = {(uint8_t)(f2 & 0xffu), has1 ? (uint8_t)(f2 >> 8) : (uint8_t)0};
-    bool wr[2], st[2];
-    const bool ij_face = (j == 0 || j == P.Ny - 1 || i == 0 || i == P.Nx - 1);
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        wr[r] = (f[r] & (kMove | kFixed)) != 0;
-        const bool k_face = (k + r == 0) || (k + r == P.Nz - 1);
-        st[r] = wr[r] && !(kLast && (f[r] & kFixed)) && (f[r] & kMove) && !ij_face && !k_face;
-    }
-    if (!wr[0] && !wr[1]) return;
-    float o[2][5];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-        const float* b = qo + m * P.sc + id;
-        const float2 c = *reinterpret_cast<const float2*>(b);
-        o[0][m] = c.x;
-        o[1][m] = c.y;
-        if (st[0] || st[1]) {  // i and j are interior here (ij_face is false)
-            const float2 xp = __ldg(reinterpret_cast<const float2*>(b + P.si));
-            const float2 xm = __ldg(reinterpret_cast<const float2*>(b - P.si));
-            const float2 yp = __ldg(reinterpret_cast<const float2*>(b + P.sj));
-            const float2 ym = __ldg(reinterpret_cast<const float2*>(b - P.sj));
-            const float km1 = k >= 1 ? __ldg(b - 1) : 0.0f;
-            const float kp2 = k + 2 < P.Nz ? __ldg(b + 2) : 0.0f;
-            const float2 rh = __ldg(reinterpret_cast<const float2*>(rhs + m * P.sc + id));
-            const float s0 = P.ix2 * (xp.x + xm.x) + P.iy2 * (yp.x + ym.x) + P.iz2 * (c.y + km1);
-            const float s1 = P.ix2 * (xp.y + xm.y) + P.iy2 * (yp.y + ym.y) + P.iz2 * (kp2 + c.x);
-            if (st[0]) o[0][m] = (rh.x + P.alpha * s0) * P.jdenom_inv;
-            if (st[1]) o[1][m] = (rh.y + P.alpha * s1) * P.jdenom_inv;
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-        if (kLast && wr[r] && (f[r] & kFixed)) surface_q0(P, i, j, k + r, o[r]);
-    if (wr[0] && wr[1]) {
-#pragma unroll
-        for (int m = 0; m < 5; ++m) *reinterpret_cast<float2*>(qn + m * P.sc + id) = make_float2(o[0][m], o[1][m]);
-    } else {
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-            if (wr[r]) {
-#pragma unroll
-                for (int m = 0; m < 5; ++m) qn[m * P.sc + id + r] = o[r][m];
-            }
-    }
-}
-
 // Host AoS FP64 (reference cell order) <-> device FP32 SoA.
 __global__ void k_aos_to_soa(const double* __restrict__ aos, float* __restrict__ a, float* __restrict__ b,
                              int Nx, int Ny, int Nz, int sj, long long si, long long sc, float* __restrict__ la = nullptr,
@@ -583,6 +516,8 @@ struct qsr_handle {
     bool stage_shared = false;     // staging owned by an ensemble (shared by its droplets)
     ObsPartial* opart = nullptr;   // block partials, the result, then the ticket counter
     TiledPlan tiled{};             // tiled-kernel launch plan
+    TiledPlan sweep{};             // plan of the IMEX sweeps (shares the other one's error word)
+    CUtensorMap rhs_map;
     int cur = 0;
     bool uploaded = false;
     cudaStream_t stream = nullptr;
@@ -776,7 +711,7 @@ int qsr_create(const qsr_params* params, qsr_handle** out) {
     h->p = p;
     cudaGetDevice(&h->device);
     h->g = make_geometry(p);
-    h->sj = (p.Nz + 3) & ~3;
+    h->sj = (p.Nz + 7) & ~7;  // rows of whole 32-byte sectors
     h->si = (long long)p.Ny * h->sj;
     h->sc = (long long)p.Nx * h->si;
     h->ncells = (long long)p.Nx * p.Ny * p.Nz;
@@ -1014,6 +949,9 @@ int qsr_step(qsr_handle* h, int n_steps, const qsr_step_args* a) {
             int rc = alloc_or_fail((void**)&h->rhs, (size_t)h->sc * 5 * sizeof(float));
             if (rc) return rc;
             LDG_CUDA(cudaMemset(h->rhs, 0, (size_t)h->sc * 5 * sizeof(float)));
+            rc = tiled_encode(&h->rhs_map, h->rhs, p.Nx, p.Ny, p.Nz, h->sj, h->si, h->sc, false, false);
+            if (rc == LDG_OK) rc = tiled_sweep_plan(h->tiled, h->sc, h->sweep);
+            if (rc) return rc;
         }
         P.alpha = (float)(a->dt * (1.0 / p.gamma) * a->L_stab);
         const double aj = (a->dt / p.gamma) * a->L_stab;  // QSR.cu:2728
@@ -1052,15 +990,8 @@ int qsr_step(qsr_handle* h, int n_steps, const qsr_step_args* a) {
             for (int it = 0; it < a->jacobi_iters; ++it) {
                 const bool last = (it == a->jacobi_iters - 1);
                 if (tiled) {
-                    if (h->tiled.n_plane_items > 0) {
-                        const int nb = h->tiled.n_plane_items;
-                        if (last)
-                            k_jacobi_tiled<true><<<nb, 128, 0, h->stream>>>(h->rhs, h->q[c], h->q[1 - c], h->flags,
-                                                                             h->tiled.plane_items, P);
-                        else
-                            k_jacobi_tiled<false><<<nb, 128, 0, h->stream>>>(h->rhs, h->q[c], h->q[1 - c], h->flags,
-                                                                              h->tiled.plane_items, P);
-                    }
+                    int rc = tiled_sweep(h->sweep, h->q[c], h->q[1 - c], h->rhs_map, P, last, h->stream);
+                    if (rc) return rc;
                 } else if (last) {
                     k_jacobi<true><<<grd, blk, 0, h->stream>>>(h->rhs, h->q[c], h->q[1 - c], h->flags, P);
                 } else {
@@ -1177,6 +1108,8 @@ int qsr_destroy(qsr_handle* h) {
     cudaFree(h->q[0]); cudaFree(h->q[1]); cudaFree(h->lo[0]); cudaFree(h->lo[1]); cudaFree(h->rhs); cudaFree(h->flags);
     if (!h->stage_shared) cudaFree(h->stage);
     cudaFree(h->opart);
+    h->sweep.err = nullptr;
+    tiled_plan_free(h->sweep);
     tiled_plan_free(h->tiled);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -1250,7 +1183,7 @@ void ens_drop_graph(ens_handle* h) {
 int ens_rechunk(ens_handle* h, int cap) {
     std::vector<const TiledPlan*> plans;
     for (const qsr_handle* q : h->inst) plans.push_back(&q->tiled);
-    const int chunk = tiled_length(plans, cap, h->L2 || h->L3);
+    const int chunk = tiled_length(plans, cap, (h->L2 || h->L3) ? kLoadDeep : kLoadL1);
     std::vector<tiled::TileItem> items;
     std::vector<int> first;   // first item of every instance
     long long active = 0;

@@ -54,31 +54,37 @@ constexpr int TK = 32;               // tile width along k (one warp per row)
 constexpr int TJ = 8;                // tile rows along j
 constexpr int THREADS = TK * TJ / 2;  // two cells per thread: rows 2w and 2w + 1 of warp w
 constexpr int NWARP = THREADS / 32;
-// Halo columns loaded with each plane: the TMA box starts at column k0 - HK, which must be a
-// multiple of 4 floats (16 bytes), so tiles start at k0 = 2 (mod 4) (the first may start at
-// k0 = -2: its two columns outside the grid are zero fill and compute nothing).
-constexpr int HK = 2;
-constexpr int RW = TK + 2 * HK;      // 36 floats per smem row
-
-// What a step with / without the L2 term keeps in shared memory. The L2 term reads two cells out
-// (wide second differences): two halo rows and the planes i-2 .. i+2. Without it the stencil reaches
-// one cell: one halo row and the planes i-1 .. i+1, so the same ring has three planes in flight
-// instead of one, and a plane is 7.2 instead of 8.6 KB (five 128-thread CTAs per SM instead of
-// four): 256^3, R = 115, L1 only 95 -> 88 us a step, 128^3 17 -> 15 us.
-template <bool kL2>
+// What the kernels keep of a plane in shared memory. The L2 term reads two cells out (wide second
+// differences): two halo rows and the planes i-2 .. i+2. Without it the stencil reaches one cell: one
+// halo row and the planes i-1 .. i+1, so a ring has more planes in flight.
+// A TMA box starts at column k0 - HK, which must be a multiple of 4 floats (16 bytes). Without L2 the
+// tiles start on 8 floats and HK is 4: every row a warp stores is made of whole 32-byte sectors (rows
+// are padded to 8 floats). Stores that cut sectors bound the L1-only step: the same loads and stores
+// without arithmetic took 164 us with cut and 110 us with whole sectors on a 256^3 box. With L2, a
+// plane of 40 columns would let only three blocks share an SM, and that step is bound by
+// arithmetic: its tiles start at k0 = 2 (mod 4) with HK = 2 (the first may start at k0 = -2: columns
+// outside the grid are zero fill and compute nothing).
+// A sweep's slot also holds the tile of the right-hand side.
+enum Mode { kStep, kRhs, kSweep, kSweepLast };  // explicit step; IMEX right-hand side; Jacobi sweep, the last one
+template <bool kL2, int kMode = kStep>
 struct Tile {
+    static constexpr bool kHasRhs = kMode >= kSweep;
     static constexpr int H = kL2 ? 2 : 1;             // halo rows and planes read on each side
+    static constexpr int HK = kL2 ? 2 : 4;            // halo columns
+    static constexpr int RW = TK + 2 * HK;            // floats per shared row
     static constexpr int ROWS = TJ + 2 * H;
     static constexpr int CSTR = RW * ROWS;            // floats per component plane
     static constexpr int PLANE = 5 * CSTR;            // floats per plane (all components)
-    // floats per ring slot: the plane, then its row masks; 128-byte aligned
-    static constexpr int SLOT = (PLANE + 4 * TJ + 31) / 32 * 32;
-    static constexpr uint32_t BYTES = PLANE * 4;
+    static constexpr int RHS = (PLANE + 31) / 32 * 32;            // right-hand side (128-byte aligned)
+    static constexpr int MASKS = kHasRhs ? RHS + 5 * TK * TJ : PLANE;
+    static constexpr int SLOT = (MASKS + 4 * TJ + 31) / 32 * 32;  // floats per ring slot (128-byte aligned)
+    static constexpr uint32_t BYTES = PLANE * 4, RHS_BYTES = kHasRhs ? 5 * TK * TJ * 4 : 0;
+    // ring slots: planes i-H .. i+H are read at plane i, the rest are in flight
+    static constexpr int NQ = kL2 ? 6 : (kHasRhs ? 4 : 5);
 };
-constexpr int NQ = 6;  // ring slots: planes i-H .. i+H are read at plane i, the rest are in flight
 // CTAs per SM the register budget is set for.
-template <bool kL2, bool kL3>
-__host__ __device__ constexpr int ctas() { return kL2 || kL3 ? 4 : 5; }
+template <bool kL2, bool kL3, int kMode = kStep>
+__host__ __device__ constexpr int ctas() { return kL2 || kL3 || kMode >= kSweep ? 4 : 5; }
 
 // What a warp does with one row of 32 cells of one plane, one bit per cell. They are formed once per
 // work list from the cell classes and travel through the ring with their plane (one bulk copy on
@@ -168,7 +174,7 @@ struct SmemQ {
     const float* pl[5];
     int off;
     __device__ __forceinline__ float operator()(int c, int di, int dj, int dk) const {
-        return pl[di + 2][off + dj * RW + dk + c * Tile<kL2>::CSTR];
+        return pl[di + 2][off + dj * Tile<kL2>::RW + dk + c * Tile<kL2>::CSTR];
     }
 };
 // The same with runtime offsets (face cells): the plane is picked from the five by selects.
@@ -177,7 +183,7 @@ struct SmemQRt {
     int off;
     __device__ __forceinline__ float operator()(int c, int di, int dj, int dk) const {
         const float* s = di == 0 ? pl[2] : (di > 0 ? (di == 1 ? pl[3] : pl[4]) : (di == -1 ? pl[1] : pl[0]));
-        return s[off + dj * RW + dk + c * Tile<true>::CSTR];
+        return s[off + dj * Tile<true>::RW + dk + c * Tile<true>::CSTR];
     }
 };
 // Face cells without the L2 term read the field itself: the shifted second difference of a cell on
@@ -204,7 +210,7 @@ __device__ __forceinline__ void chem_face(const SmemQ<kL2>& A, int row, const fl
         SmemQRt R;
 #pragma unroll
         for (int d = 0; d < 5; ++d) R.pl[d] = A.pl[d];
-        R.off = A.off + row * RW;
+        R.off = A.off + row * Tile<kL2>::RW;
         const FaceOne<kL2, kL3, SmemQRt> S{R, x, y, z};
         chem_core<kL2, kL3, kLap, true, float>(S, P, q, inner ? 1.0f : 0.0f, mu, lap);
     } else {
@@ -223,19 +229,20 @@ struct TileSmem {
     int* s_item;        // work item broadcast (persistent kernel)
 };
 
-template <bool kL2>
+template <bool kL2, int kMode = kStep>
 __device__ __forceinline__ TileSmem tile_smem(unsigned char* raw) {
+    using G = Tile<kL2, kMode>;
     TileSmem S;
     S.sq = reinterpret_cast<float*>(raw);
-    S.bar = reinterpret_cast<uint64_t*>(S.sq + NQ * Tile<kL2>::SLOT);
-    S.freed = reinterpret_cast<unsigned*>(S.bar + NQ);
-    S.s_abort = reinterpret_cast<int*>(S.freed + NQ);
+    S.bar = reinterpret_cast<uint64_t*>(S.sq + G::NQ * G::SLOT);
+    S.freed = reinterpret_cast<unsigned*>(S.bar + G::NQ);
+    S.s_abort = reinterpret_cast<int*>(S.freed + G::NQ);
     S.s_item = S.s_abort + 1;
     return S;
 }
-template <bool kL2>
+template <bool kL2, int kMode = kStep>
 __host__ __device__ constexpr size_t tile_smem_bytes() {
-    return (size_t)NQ * (Tile<kL2>::SLOT * 4 + 8 + 4) + 16;
+    return (size_t)Tile<kL2, kMode>::NQ * (Tile<kL2, kMode>::SLOT * 4 + 8 + 4) + 16;
 }
 
 // A warp's arrival on a slot counter: returns the count before it (acquire-release at CTA
@@ -255,15 +262,19 @@ __device__ __forceinline__ unsigned arrive_freed(unsigned* ctr) {
 // packed (FFMA2 / FADD2 / FMUL2) instruction stream, and adjacent rows share operands (the centre of
 // one is a j-neighbour of the other). kComp: compensated storage (explicit steps only): the low words
 // of the input cells are read from lo_in and the new low words written to lo_out.
-template <bool kL2, bool kL3, bool kNoise, bool kRHS, bool kComp = false>
+template <bool kL2, bool kL3, bool kNoise, int kMode, bool kComp = false>
 __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float* __restrict__ qin,
                                              float* __restrict__ qout, const RowMask* __restrict__ masks, int j0,
                                              int k0, int ib, int ie, const QsrConst& P, const TileSmem& S,
                                              uint32_t& phase, int* __restrict__ err,
                                              const float* __restrict__ lo_in = nullptr,
-                                             float* __restrict__ lo_out = nullptr) {
-    constexpr int H = Tile<kL2>::H, SLOT = Tile<kL2>::SLOT, PLANE = Tile<kL2>::PLANE;
+                                             float* __restrict__ lo_out = nullptr,
+                                             const CUtensorMap* tm_rhs = nullptr) {
+    using G = Tile<kL2, kMode>;
+    constexpr int H = G::H, SLOT = G::SLOT, NQ = G::NQ, RW = G::RW;
+    constexpr bool kRHS = kMode == kRhs, kJacobi = kMode >= kSweep;
     static_assert(NQ > 2 * H + 1, "the ring holds planes i - H .. i + H and at least one in flight");
+    static_assert(!kJacobi || !kL2, "a sweep reaches one cell");
     float* sq = S.sq;
     uint64_t* bar = S.bar;
     const int base = ib - H;  // first plane this item loads; slots and phases count from it
@@ -279,9 +290,12 @@ __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float*
             const bool own = p >= ib && p < ie;
             float* dst = sq + sl * SLOT;
             fence_proxy_async();
-            mbar_expect_tx(b, Tile<kL2>::BYTES + (own ? MASK_BYTES : 0u));
-            tma_load_4d(dst, tm, k0 - HK, j0 - H, p, 0, b);
-            if (own) bulk_load(dst + PLANE, masks + (size_t)(p - ib) * TJ, MASK_BYTES, b);
+            mbar_expect_tx(b, G::BYTES + (own ? MASK_BYTES + G::RHS_BYTES : 0u));
+            tma_load_4d(dst, tm, k0 - G::HK, j0 - H, p, 0, b);
+            if (own) {
+                bulk_load(dst + G::MASKS, masks + (size_t)(p - ib) * TJ, MASK_BYTES, b);
+                if (kJacobi) tma_load_4d(dst + G::RHS, tm_rhs, k0, j0, p, 0, b);
+            }
         } else {
             mbar_arrive(b);
         }
@@ -305,7 +319,7 @@ __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float*
     const int issued_end = ie + NQ - H;
     const int j = j0 + 2 * w, k = k0 + kl;
     const uint32_t bit = 1u << kl;
-    const int off = (2 * w + H) * RW + kl + HK;
+    const int off = (2 * w + H) * RW + kl + G::HK;
     long long id = (long long)ib * P.si + (long long)j * P.sj + k;  // row j; row j + 1 is P.sj further
     // Shared-memory planes i-H .. i+H of the current step, rolled forward by one plane per step.
     const float* qpl[5];
@@ -319,7 +333,7 @@ __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float*
         waited_end = i + H + 1;
         if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp stops or none of it
         // The masks are read again after the chemical potential: eight registers fewer live across it.
-        const uint32_t mk = su32(qpl[2] + PLANE) + 2 * w * sizeof(RowMask);
+        const uint32_t mk = su32(qpl[2] + G::MASKS) + 2 * w * sizeof(RowMask);
         uint4 m0 = lds_u4(mk), m1 = lds_u4(mk + sizeof(RowMask));
         if ((m0.x | m1.x) != 0u || (!kRHS && (m0.y | m1.y) != 0u)) {
             SmemQ<kL2> A;
@@ -329,40 +343,55 @@ __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float*
             F2 c[5], mu[5], lap[5];
 #pragma unroll
             for (int m = 0; m < 5; ++m) c[m] = mk2(A(m, 0, 0, 0), A(m, 0, 1, 0));
-            if ((m0.w | m1.w) == 0u) {
-                const InteriorPair<kL2, kL3, SmemQ<kL2>> St{A};
-                chem_core<kL2, kL3, kRHS, false, F2>(St, P, c, F2{}, mu, lap);
+            // the chemical potential, then the new values of both cells (compensated storage keeps the potential)
+            if constexpr (kJacobi) {
+                // (I - alpha Lap) Q = rhs with the centre term on the left (QSR.cu:786-849); cells on a grid face hold
+                const float* rh = qpl[2] + G::RHS + 2 * w * TK + kl;
+                const uint32_t up0 = m0.x & ~m0.w & bit, up1 = m1.x & ~m1.w & bit;
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+                    const F2 sx = mk2(A(m, 1, 0, 0), A(m, 1, 1, 0)) + mk2(A(m, -1, 0, 0), A(m, -1, 1, 0));
+                    const F2 sy = mk2(c[m].v.y + A(m, 0, -1, 0), A(m, 0, 2, 0) + c[m].v.x);
+                    const F2 sz = mk2(A(m, 0, 0, 1), A(m, 0, 1, 1)) + mk2(A(m, 0, 0, -1), A(m, 0, 1, -1));
+                    const F2 r = mk2(rh[m * TK * TJ], rh[m * TK * TJ + TK]);
+                    const F2 v = P.jdenom_inv * vfma(P.alpha, vfma(P.ix2, sx, vfma(P.iy2, sy, P.iz2 * sz)), r);
+                    mu[m] = mk2(up0 ? v.v.x : c[m].v.x, up1 ? v.v.y : c[m].v.y);
+                }
             } else {
+                if ((m0.w | m1.w) == 0u) {
+                    const InteriorPair<kL2, kL3, SmemQ<kL2>> St{A};
+                    chem_core<kL2, kL3, kRHS, false, F2>(St, P, c, F2{}, mu, lap);
+                } else {
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    float cr[5], mr[5], lr[5];
+                    for (int r = 0; r < 2; ++r) {
+                        float cr[5], mr[5], lr[5];
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) cr[m] = mr[m] = lr[m] = r ? c[m].v.y : c[m].v.x;
-                    if ((r ? m1.x : m0.x) & bit) chem_face<kL2, kL3, kRHS>(A, r, qin, P, i, j + r, k, cr, mr, lr);
+                        for (int m = 0; m < 5; ++m) cr[m] = mr[m] = lr[m] = r ? c[m].v.y : c[m].v.x;
+                        if ((r ? m1.x : m0.x) & bit) chem_face<kL2, kL3, kRHS>(A, r, qin, P, i, j + r, k, cr, mr, lr);
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) {
-                        (r ? mu[m].v.y : mu[m].v.x) = mr[m];
-                        if (kRHS) (r ? lap[m].v.y : lap[m].v.x) = lr[m];
+                        for (int m = 0; m < 5; ++m) {
+                            (r ? mu[m].v.y : mu[m].v.x) = mr[m];
+                            if (kRHS) (r ? lap[m].v.y : lap[m].v.x) = lr[m];
+                        }
                     }
                 }
-            }
-            m0 = lds_u4(mk);
-            m1 = lds_u4(mk + sizeof(RowMask));
-            if ((m0.z | m1.z) != 0u) {  // weak-anchoring penalty (QSR.cu:623-652)
-                float Qa[5], Qb[5];
-                surface_q0(P, i, j, k, Qa);
-                surface_q0(P, i, j + 1, k, Qb);
-                const F2 wf = mk2((m0.z & bit) ? P.Weff : 0.0f, (m1.z & bit) ? P.Weff : 0.0f);
+                m0 = lds_u4(mk);
+                m1 = lds_u4(mk + sizeof(RowMask));
+                if ((m0.z | m1.z) != 0u) {  // weak-anchoring penalty (QSR.cu:623-652)
+                    float Qa[5], Qb[5];
+                    surface_q0(P, i, j, k, Qa);
+                    surface_q0(P, i, j + 1, k, Qb);
+                    const F2 wf = mk2((m0.z & bit) ? P.Weff : 0.0f, (m1.z & bit) ? P.Weff : 0.0f);
 #pragma unroll
-                for (int m = 0; m < 5; ++m) mu[m] = vfma(wf, c[m] - mk2(Qa[m], Qb[m]), mu[m]);
-            }
-            F2 u[5];
-            if (kRHS) {
+                    for (int m = 0; m < 5; ++m) mu[m] = vfma(wf, c[m] - mk2(Qa[m], Qb[m]), mu[m]);
+                }
+                if (kRHS) {
 #pragma unroll
-                for (int m = 0; m < 5; ++m) u[m] = vfma(-P.alpha, lap[m], vfma(-P.mob_dt, mu[m], c[m]));
-            } else if (!kComp) {
+                    for (int m = 0; m < 5; ++m) mu[m] = vfma(-P.alpha, lap[m], vfma(-P.mob_dt, mu[m], c[m]));
+                } else if (!kComp) {
 #pragma unroll
-                for (int m = 0; m < 5; ++m) u[m] = vfma(-P.mob_dt, mu[m], c[m]);
+                    for (int m = 0; m < 5; ++m) mu[m] = vfma(-P.mob_dt, mu[m], c[m]);
+                }
             }
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
@@ -372,8 +401,10 @@ __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float*
                 const long long ir = id + (r ? P.sj : 0);
                 float o[5];
 #pragma unroll
-                for (int m = 0; m < 5; ++m) o[m] = r ? u[m].v.y : u[m].v.x;
-                if (fixed) {
+                for (int m = 0; m < 5; ++m) o[m] = r ? mu[m].v.y : mu[m].v.x;
+                if (kJacobi) {
+                    if (kMode == kSweepLast && fixed) surface_q0(P, i, j + r, k, o);
+                } else if (fixed) {
                     surface_q0(P, i, j + r, k, o);
                     if (kComp) {
 #pragma unroll
@@ -437,10 +468,10 @@ __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float*
     return ok;
 }
 
-template <bool kL2>
+template <bool kL2, int kMode = kStep>
 __device__ __forceinline__ void tile_smem_init(const TileSmem& S) {
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NQ; ++s) {
+        for (int s = 0; s < Tile<kL2, kMode>::NQ; ++s) {
             mbar_init(&S.bar[s], 1);
             S.freed[s] = 0;
         }
@@ -451,7 +482,7 @@ __device__ __forceinline__ void tile_smem_init(const TileSmem& S) {
 }
 
 // Single grid: one work item per CTA.
-template <bool kL2, bool kL3, bool kNoise, bool kRHS, bool kComp = false>
+template <bool kL2, bool kL3, bool kNoise, int kMode, bool kComp = false>
 __global__ void __launch_bounds__(THREADS, ctas<kL2, kL3>())
     k_step_tiled(const __grid_constant__ CUtensorMap tm_in, const float* __restrict__ qin, float* __restrict__ qout,
                  const RowMask* __restrict__ masks, const TileItem* __restrict__ items, QsrConst P,
@@ -463,8 +494,33 @@ __global__ void __launch_bounds__(THREADS, ctas<kL2, kL3>())
     uint32_t phase = 0;
     pdl_wait();
     pdl_trigger();
-    process_tile<kL2, kL3, kNoise, kRHS, kComp>(&tm_in, qin, qout, masks + (size_t)e.rec * TJ, e.j0, e.k0, e.ib, e.ie,
-                                                P, S, phase, err, lo_in, lo_out);
+    process_tile<kL2, kL3, kNoise, kMode, kComp>(&tm_in, qin, qout, masks + (size_t)e.rec * TJ, e.j0, e.k0, e.ib, e.ie,
+                                                 P, S, phase, err, lo_in, lo_out);
+}
+
+// One Jacobi sweep of (I - alpha Lap) Q = rhs over the changing cells, the field through the same plane
+// ring as the step's (one load per value) and the right-hand side's tile beside it. Bound by HBM: at
+// 256^3, R = 120, a sweep takes 105 us (135 with one block per tile plane and its loads from global
+// memory) and moves 616 MB, 438 MB of them needed: the rest are the tiles' idle cells and halo planes
+// that fell out of L2. Tried and slower or no faster: four sweeps per pass in overlapping patches (2.8 ms
+// for 25 against 2.7: 2.7 to 4.3 times the cells), the right-hand side by plain loads a plane ahead
+// (3.0 ms), a ring of its own for it (2.7 ms). Every other cell never changes:
+// it holds the same value in both ping-pong buffers, so the reference's copy of it (QSR.cu:803-810) is
+// already done. The last sweep applies the strong-anchoring rewrite (QSR.cu:851-867).
+template <int kMode>
+__global__ void __launch_bounds__(THREADS, ctas<false, false, kMode>())
+    k_sweep_tiled(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_rhs,
+                  float* __restrict__ qout, const RowMask* __restrict__ masks, const TileItem* __restrict__ items,
+                  QsrConst P, int* __restrict__ err) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const TileSmem S = tile_smem<false, kMode>(smem_raw);
+    tile_smem_init<false, kMode>(S);
+    const TileItem e = items[blockIdx.x];
+    uint32_t phase = 0;
+    pdl_wait();
+    pdl_trigger();
+    process_tile<false, false, false, kMode>(&tm_in, nullptr, qout, masks + (size_t)e.rec * TJ, e.j0, e.k0, e.ib, e.ie,
+                                             P, S, phase, err, nullptr, nullptr, &tm_rhs);
 }
 
 // Row masks of a work list: one block per item, one warp per tile row, a ballot per plane. `lo` is
@@ -575,7 +631,7 @@ __global__ void __launch_bounds__(THREADS, ctas<kL2, kL3>())
             P.S_shell = (float)D.S_custom;
         }
         P.step = step;
-        process_tile<kL2, kL3, kNoise, false>(tms + 2 * e.inst + which, D.q[which], D.q[1 - which],
+        process_tile<kL2, kL3, kNoise, kStep>(tms + 2 * e.inst + which, D.q[which], D.q[1 - which],
                                               masks + (size_t)e.rec * TJ, e.j0, e.k0, e.ib, e.ie, P, S, phase, err);
     }
     if (threadIdx.x == 0) {
@@ -600,6 +656,7 @@ struct TiledBand {
     std::vector<int> kmin, kmax;
 };
 
+enum Load { kLoadL1, kLoadDeep, kLoadSweep };  // L1-only step; step with L2 or L3; Jacobi sweep
 struct TiledPlan {
     bool ok = false;
     long long active_cells = 0;   // cells inside visited tiles at the current chunk (read once per step)
@@ -612,9 +669,7 @@ struct TiledPlan {
     int Nx = 0, Ny = 0, sj = 0;
     long long si = 0;
     bool L2 = false;              // the kernels take the L2 term (halo, interior distance)
-    bool deep = false;            // the L2 or the L3 term
-    int n_plane_items = 0;
-    int4* plane_items = nullptr;  // the same tiles one plane each (j0, k0, i, i + 1): IMEX sweeps
+    Load load = kLoadL1;          // what the kernels do (tiled_length)
     int Nz = 0;
     std::vector<TiledBand> bands; // host: the changing cells' extent per row band and plane
     int* err = nullptr;           // device error word
@@ -623,8 +678,8 @@ struct TiledPlan {
 };
 
 // Calls emit(j0, k0, first, last + 1, face) for every work item of chunks of `chunk` planes. In each
-// row band and plane chunk the k tiles start at the first changing cell (rounded down to the 4-float
-// TMA alignment) instead of at multiples of TK, and each tile's plane range is cut to the planes
+// row band and plane chunk the k tiles start at the first changing cell (rounded down to the tiles'
+// alignment) instead of at multiples of TK, and each tile's plane range is cut to the planes
 // whose changing cells reach it: every changing cell lies in exactly one item, and fewer idle lanes
 // are visited than with a fixed tile grid. `face`: the item has changing cells next to a grid face.
 template <class Emit>
@@ -641,7 +696,7 @@ inline void tiled_each_item(const TiledPlan& plan, int chunk, Emit emit) {
                     kmax = std::max(kmax, b.kmax[p - b.ib]);
                 }
             if (kmax < 0) continue;
-            for (int k0 = ((kmin - 2) & ~3) + 2; k0 <= kmax; k0 += TK) {
+            for (int k0 = plan.L2 ? ((kmin - 2) & ~3) + 2 : kmin & ~7; k0 <= kmax; k0 += TK) {
                 int first = -1, last = -1;
                 bool face = false;
                 for (int p = ib; p < ie; ++p) {
@@ -669,7 +724,7 @@ inline void tiled_each_item(const TiledPlan& plan, int chunk, Emit emit) {
 // fifth on (longest items first evens them out). An item on a face takes twice as long per plane.
 // Measured against it (64^3, R = 28, L1: 4.8 us at 1 plane, 17.1 at 16; 128^3: 13.9 us at 6, 20.2
 // at 16; 96^3 with L2 and L3: 15.1 us at 4, 24.8 at 16; 256^3: 8 to 16 within 2 %).
-inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, bool deep) {
+inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Load load) {
     static const int sms = [] {
         int dev = 0, n = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -678,8 +733,8 @@ inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, boo
         return n;
     }();
     if (cap < 8) return cap;
-    const int per_sm = deep ? 4 : 5;
-    const double kItem = deep ? 1.3 : 1.0, face_plane = deep ? 5.3 : 2.0;
+    const int per_sm = load == kLoadL1 ? 5 : 4;
+    const double kItem = load == kLoadDeep ? 1.3 : 1.0, face_plane = load == kLoadDeep ? 5.3 : 2.0;
     int best = cap;
     double best_t = std::numeric_limits<double>::infinity();
     for (int c : {cap, 6, 4, 3, 2, 1}) {
@@ -693,7 +748,7 @@ inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, boo
         const double full = (double)n / ((double)sms * per_sm);
         const int m = (int)std::min<long long>(per_sm, (n + sms - 1) / sms);
         const double waves = full > 4.0 ? full + 0.5 : std::ceil(full);
-        double t = waves * (kItem + c * (deep ? 2.6 : 0.75 + 0.2 * m));
+        double t = waves * (kItem + c * (load == kLoadDeep ? 2.6 : load == kLoadL1 ? 0.75 + 0.2 * m : 0.6 + 0.35 * m));
         if (faces) t = std::max(t, kItem + c * face_plane + 0.5 * t);
         if (t < best_t) {
             best_t = t;
@@ -737,8 +792,9 @@ inline int tiled_default_chunk() {
     return chunk;
 }
 
+// Tensor map of a field: boxes of a tile with its halo, or of the tile alone.
 inline int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int Nz, int sj, long long si, long long sc,
-                        bool L2) {
+                        bool L2, bool halo = true) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
         void* fn = nullptr;
@@ -752,13 +808,15 @@ inline int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int 
     }
     cuuint64_t dims[4] = {(cuuint64_t)Nz, (cuuint64_t)Ny, (cuuint64_t)Nx, 5};
     cuuint64_t strides[3] = {(cuuint64_t)sj * 4, (cuuint64_t)si * 4, (cuuint64_t)sc * 4};
-    cuuint32_t box[4] = {tiled::RW, (cuuint32_t)(L2 ? tiled::Tile<true>::ROWS : tiled::Tile<false>::ROWS), 1, 5};
+    using namespace tiled;
+    const int w = L2 ? Tile<true>::RW : Tile<false>::RW, r = L2 ? Tile<true>::ROWS : Tile<false>::ROWS;
+    cuuint32_t box[4] = {(cuuint32_t)(halo ? w : TK), (cuuint32_t)(halo ? r : TJ), 1, 5};
     cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void*)base, dims, strides, box, estr,
+    CUresult res = encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void*)base, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        set_error("cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
+    if (res != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed: " + std::to_string((int)res));
         return LDG_ERR_CUDA;
     }
     return LDG_OK;
@@ -786,7 +844,7 @@ inline int tiled_masks(const TiledPlan& plan, const tiled::TileItem* d_items, in
 
 // Uploads the work list for items of at most `cap` planes (tiled_length).
 inline int tiled_plan_rechunk(TiledPlan& plan, int cap) {
-    const int chunk = tiled_length({&plan}, cap, plan.deep);
+    const int chunk = tiled_length({&plan}, cap, plan.load);
     long long active = 0;
     const std::vector<int4> items = tiled_items(plan, chunk, &active);
     plan.active_cells = active;
@@ -807,16 +865,6 @@ inline int tiled_plan_rechunk(TiledPlan& plan, int cap) {
         if (rc) return rc;
         LDG_CUDA(cudaStreamSynchronize(nullptr));
     }
-    std::vector<int4> planes;
-    for (const int4& t : items)
-        for (int i = t.z; i < t.w; ++i) planes.push_back(make_int4(t.x, t.y, i, i + 1));
-    if (plan.plane_items) cudaFree(plan.plane_items);
-    plan.plane_items = nullptr;
-    plan.n_plane_items = (int)planes.size();
-    if (plan.n_plane_items > 0) {
-        LDG_CUDA(cudaMalloc(&plan.plane_items, planes.size() * sizeof(int4)));
-        LDG_CUDA(cudaMemcpy(plan.plane_items, planes.data(), planes.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    }
     return LDG_OK;
 }
 
@@ -825,7 +873,7 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
                             const uint8_t* d_flags, const float* buf0, const float* buf1, long long sc, bool L2, bool L3) {
     using namespace tiled;
     plan = TiledPlan{};
-    plan.deep = L2 || L3;
+    plan.load = (L2 || L3) ? kLoadDeep : kLoadL1;
     plan.Nx = Nx; plan.Ny = Ny; plan.Nz = Nz;
     plan.sj = sj; plan.si = si;
     plan.flags = d_flags;
@@ -871,7 +919,7 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
     return LDG_OK;
 }
 
-template <bool L2, bool L3, bool N, bool R, bool K>
+template <bool L2, bool L3, bool N, int R, bool K>
 inline int tiled_launch_t(const TiledPlan& plan, int which, float* out, const QsrConst& P, cudaStream_t st,
                           const float* lo_in, float* lo_out) {
     using namespace tiled;
@@ -888,7 +936,7 @@ inline int tiled_launch_t(const TiledPlan& plan, int which, float* out, const Qs
     return LDG_OK;
 }
 
-template <bool R, bool K>
+template <int R, bool K>
 inline int tiled_dispatch(const TiledPlan& plan, int which, float* out, const QsrConst& P,
                           bool L2, bool L3, bool noise, cudaStream_t st, const float* lo_in, float* lo_out) {
     const int key = (L2 ? 1 : 0) | (L3 ? 2 : 0) | (noise ? 4 : 0);
@@ -911,9 +959,51 @@ inline int tiled_step(const TiledPlan& plan, const float* in, float* out, const 
                       bool L2, bool L3, bool noise, bool rhs, cudaStream_t st, const float* lo_in = nullptr,
                       float* lo_out = nullptr) {
     const int which = (in == plan.bufs[0]) ? 0 : 1;
-    if (rhs) return tiled_dispatch<true, false>(plan, which, out, P, L2, L3, noise, st, nullptr, nullptr);
-    if (lo_out) return tiled_dispatch<false, true>(plan, which, out, P, L2, L3, noise, st, lo_in, lo_out);
-    return tiled_dispatch<false, false>(plan, which, out, P, L2, L3, noise, st, nullptr, nullptr);
+    if (rhs) return tiled_dispatch<tiled::kRhs, false>(plan, which, out, P, L2, L3, noise, st, nullptr, nullptr);
+    if (lo_out) return tiled_dispatch<tiled::kStep, true>(plan, which, out, P, L2, L3, noise, st, lo_in, lo_out);
+    return tiled_dispatch<tiled::kStep, false>(plan, which, out, P, L2, L3, noise, st, nullptr, nullptr);
+}
+
+// The sweeps' plan of the same grid: the step's changing cells, cut to the sweeps' own item length and
+// encoded for one-cell stencils.
+inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan& plan) {
+    plan = TiledPlan{};
+    plan.Nx = step.Nx; plan.Ny = step.Ny; plan.Nz = step.Nz;
+    plan.sj = step.sj; plan.si = step.si;
+    plan.flags = step.flags;
+    plan.bands = step.bands;
+    plan.err = step.err;
+    plan.load = kLoadSweep;
+    int rc = tiled_plan_rechunk(plan, tiled_default_chunk());
+    for (int b = 0; b < 2 && rc == LDG_OK; ++b) {
+        plan.bufs[b] = step.bufs[b];
+        rc = tiled_encode(&plan.tmap[b], step.bufs[b], step.Nx, step.Ny, step.Nz, step.sj, step.si, sc, false);
+    }
+    plan.ok = rc == LDG_OK;
+    return rc;
+}
+
+// One Jacobi sweep: field `in` (one of the planned buffers) to `out`. tm_rhs: the right-hand side's map.
+template <int kMode>
+inline int tiled_sweep_t(const TiledPlan& plan, const float* in, float* out, const CUtensorMap& tm_rhs, const QsrConst& P,
+                         cudaStream_t st) {
+    using namespace tiled;
+    constexpr size_t smem = tile_smem_bytes<false, kMode>();
+    static bool configured = false;
+    if (!configured) {
+        LDG_CUDA(cudaFuncSetAttribute(k_sweep_tiled<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured = true;
+    }
+    if (plan.n_items == 0) return LDG_OK;
+    LDG_CUDA(launch_pdl(k_sweep_tiled<kMode>, dim3((unsigned)plan.n_items), THREADS, smem, st,
+                        plan.tmap[in == plan.bufs[0] ? 0 : 1], tm_rhs, out, (const RowMask*)plan.masks,
+                        (const TileItem*)plan.items, P, plan.err));
+    return LDG_OK;
+}
+inline int tiled_sweep(const TiledPlan& plan, const float* in, float* out, const CUtensorMap& tm_rhs, const QsrConst& P,
+                       bool last, cudaStream_t st) {
+    return last ? tiled_sweep_t<tiled::kSweepLast>(plan, in, out, tm_rhs, P, st)
+                : tiled_sweep_t<tiled::kSweep>(plan, in, out, tm_rhs, P, st);
 }
 
 // Reads and clears the device error word (LDG_OK when no bounded wait gave up).
@@ -933,7 +1023,6 @@ inline int tiled_check(const TiledPlan& plan, cudaStream_t st) {
 inline void tiled_plan_free(TiledPlan& plan) {
     if (plan.items) cudaFree(plan.items);
     if (plan.masks) cudaFree(plan.masks);
-    if (plan.plane_items) cudaFree(plan.plane_items);
     cudaFree(plan.err);
     plan = TiledPlan{};
 }
