@@ -218,6 +218,17 @@ int sg_conv3d_wgrad(const sg_conv_shape* s, const void* x, const void* dy, float
 /* wf[Ci][26 - t][Co] = w[Co][t][Ci]: the data gradient of a layer is sg_conv3d_fwd of the
  * output gradient with wf and the shape's Ci and Co exchanged. */
 int sg_conv3d_flip_weights(const sg_conv_shape* s, const void* w, void* wf, void* stream);
+/* Activation and bias gradients of a layer in one pass over its output gradient gy (FP32 or BF16,
+ * nvox voxels x C channels): g = BF16(gy * (y > 0 ? 1 : 0.01)) (y NULL: no mask; g NULL: sums only)
+ * and db[c] = sum of g over the voxels. ws: sg_conv3d_act_grad_ws(nvox, C) doubles of device memory. */
+long long sg_conv3d_act_grad_ws(long long nvox, int C);
+int sg_conv3d_act_grad(long long nvox, int C, const void* y, const void* gy, int fp32, void* g, float* db, double* ws,
+                       void* stream);
+/* All gradients of a layer in one call: dx (NULL: not wanted), dw and db from its input x, weights w, output y
+ * (NULL: no activation) and output gradient gy (fp32: of FP32, else BF16). ws: sg_conv3d_bwd_ws bytes, 256-byte aligned. */
+long long sg_conv3d_bwd_ws(const sg_conv_shape* s);
+int sg_conv3d_bwd(const sg_conv_shape* s, const void* x, const void* w, const void* y, const void* gy, int fp32, void* dx,
+                  float* dw, float* db, void* ws, void* stream);
 /* Reads and clears the conv kernels' device error word (LDG_ERR_TIMEOUT when a bounded
  * pipeline wait gave up); synchronises `stream`. */
 int sg_check(void* stream);

@@ -36,6 +36,10 @@ namespace {
 
 constexpr int BM = 128;     // UMMA M
 constexpr int STAGES = 4;
+// Stages of the weight gradient: three leave room for one more CTA per SM than four, and all the
+// CTAs of a launch run at once (32 -> 32 channels, 64^3 x 4: 0.247 ms with four, 0.205 with three).
+constexpr int WG_STAGES = 3;
+constexpr int kWgFixed = 8;  // a weight-gradient CTA's start and atomics, in K boxes
 constexpr int KV = 64;      // voxels per weight-gradient K stage
 
 struct BoxDims {
@@ -50,7 +54,7 @@ struct FwdArgs {
     int act;       // 0 identity, 1 leaky ReLU (slope 0.01)
     int out_f32;
     int ksteps;    // 27 * cchunks
-    int cchunks;   // Ci / CK
+    int cs;        // output channels of a CTA: Co / gridDim.y
     uint32_t tmem_cols;
 };
 
@@ -82,7 +86,7 @@ __global__ void __launch_bounds__(128, 1)
     constexpr uint32_t A_BYTES = BM * ROW;
     constexpr uint32_t SWZ = swizzle_code(ROW);
     constexpr uint32_t SBO = 8 * ROW;            // 8-row core-matrix group stride
-    const uint32_t B_BYTES = (uint32_t)a.Co * ROW;
+    const uint32_t B_BYTES = (uint32_t)a.cs * ROW;
     const uint32_t B_STRIDE = (B_BYTES + 1023u) & ~1023u;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -93,9 +97,10 @@ __global__ void __launch_bounds__(128, 1)
     uint64_t* done = empty + STAGES;
     uint32_t* tslot = (uint32_t*)(done + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     int x0, y0, z0, n0;
     box_origin(a.b, blockIdx.x, x0, y0, z0, n0);
+    const int co0 = (int)blockIdx.y * a.cs;
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -114,27 +119,38 @@ __global__ void __launch_bounds__(128, 1)
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    if (tid == 0) {
+    bool ok = true;
+    if (warp == 0) {
         // TMA producer
-        int issued = 0;
+        int issued = 0, tap = 0, cc = 0, dx = -1, dy = -1, dz = -1;  // tap = 9 (dz + 1) + 3 (dy + 1) + dx + 1
         for (int ks = 0; ks < a.ksteps; ++ks) {
             const int s = ks % STAGES;
             if (ks >= STAGES && !mbar_wait(&empty[s], ((ks / STAGES) - 1) & 1)) {
                 atomicExch(err, LDG_ERR_TIMEOUT);
                 break;
             }
-            const int tap = ks / a.cchunks, cc = ks - tap * a.cchunks;
-            const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-            mbar_expect_tx(&full[s], (uint32_t)a.b.rows * ROW + B_BYTES);
-            tma_load_5d(sA + s * A_BYTES, &tmx, cc * CK, x0 + dx, y0 + dy, z0 + dz, n0, &full[s]);
-            tma_load_3d(sB + s * B_STRIDE, &tmw, cc * CK, tap, 0, &full[s]);
+            if (elect_one()) {
+                mbar_expect_tx(&full[s], (uint32_t)a.b.rows * ROW + B_BYTES);
+                tma_load_5d(sA + s * A_BYTES, &tmx, cc, x0 + dx, y0 + dy, z0 + dz, n0, &full[s]);
+                tma_load_3d(sB + s * B_STRIDE, &tmw, cc, tap, co0, &full[s]);
+            }
+            __syncwarp();
             issued = ks + 1;
+            cc += CK;
+            if (cc == a.Ci) {
+                cc = 0;
+                ++tap;
+                if (++dx == 2) {
+                    dx = -1;
+                    if (++dy == 2) { dy = -1; ++dz; }
+                }
+            }
         }
         for (int ks = (issued > STAGES ? issued - STAGES : 0); ks < issued; ++ks)
             if (!mbar_wait(&full[ks % STAGES], (ks / STAGES) & 1)) atomicExch(err, LDG_ERR_TIMEOUT);
-    } else if (tid == 32) {
+    } else if (warp == 1) {
         // MMA issuer
-        const uint32_t idesc = idesc_bf16(BM, a.Co, false, false);
+        const uint32_t idesc = idesc_bf16(BM, a.cs, false, false);
         for (int ks = 0; ks < a.ksteps; ++ks) {
             const int s = ks % STAGES;
             if (!mbar_wait(&full[s], (ks / STAGES) & 1)) {
@@ -143,16 +159,23 @@ __global__ void __launch_bounds__(128, 1)
             }
             tc_fence_after();
             const uint32_t a0 = smem_u32(sA + s * A_BYTES), b0 = smem_u32(sB + s * B_STRIDE);
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < CK / 16; ++k)
-                umma_bf16(tmem, smem_desc(a0 + k * 32, 16, SBO, SWZ), smem_desc(b0 + k * 32, 16, SBO, SWZ), idesc,
-                          (ks | k) != 0 ? 1u : 0u);
-            umma_commit(&empty[s]);
+                for (int k = 0; k < CK / 16; ++k)
+                    umma_bf16(tmem, smem_desc(a0 + k * 32, 16, SBO, SWZ), smem_desc(b0 + k * 32, 16, SBO, SWZ), idesc,
+                              (ks | k) != 0 ? 1u : 0u);
+                umma_commit(&empty[s]);
+            }
+            __syncwarp();
         }
-        umma_commit(done);
+        if (elect_one()) umma_commit(done);
+        __syncwarp();
+        ok = mbar_wait(done, 0);
     }
     // Epilogue: row m of the accumulator is output voxel m of the box; warp w owns lanes 32w..32w+31.
-    bool ok = mbar_wait(done, 0);
+    // The other lanes of the two working warps stand at a warp barrier until here: polling `done`
+    // from them held up the producing and the issuing lane of the same warp at every stage.
+    __syncwarp();
     ok = __syncthreads_and(ok) != 0;
     tc_fence_after();
     if (!ok && tid == 0) atomicExch(err, LDG_ERR_TIMEOUT);
@@ -163,14 +186,14 @@ __global__ void __launch_bounds__(128, 1)
     const bool inside = ok && m < a.b.rows && x < a.W && yy < a.H && z < a.D && n < a.N;
     const long long vox = (((long long)n * a.D + z) * a.H + yy) * a.W + x;
     const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-    for (int c0 = 0; c0 < a.Co; c0 += 16) {
+    for (int c0 = 0; c0 < a.cs; c0 += 16) {
         float v[16];
         tmem_ld16(trow + (uint32_t)c0, v);
         if (!inside) continue;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = act_apply(v[i] + (bias ? bias[c0 + i] : 0.0f), a.act);
+        for (int i = 0; i < 16; ++i) v[i] = act_apply(v[i] + (bias ? bias[co0 + c0 + i] : 0.0f), a.act);
         if (a.out_f32) {
-            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(y) + vox * a.Co + c0);
+            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(y) + vox * a.Co + co0 + c0);
 #pragma unroll
             for (int q = 0; q < 4; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         } else {
@@ -180,7 +203,7 @@ __global__ void __launch_bounds__(128, 1)
                 __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
                 p[q] = *reinterpret_cast<uint32_t*>(&h);
             }
-            uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(y) + vox * a.Co + c0);
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(y) + vox * a.Co + co0 + c0);
             dst[0] = make_uint4(p[0], p[1], p[2], p[3]);
             dst[1] = make_uint4(p[4], p[5], p[6], p[7]);
         }
@@ -213,13 +236,13 @@ __global__ void __launch_bounds__(128, 1)
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sA = base;
-    unsigned char* sB = base + STAGES * A_BYTES;
-    uint64_t* full = (uint64_t*)(sB + STAGES * B_STRIDE);
-    uint64_t* empty = full + STAGES;
-    uint64_t* done = empty + STAGES;
+    unsigned char* sB = base + WG_STAGES * A_BYTES;
+    uint64_t* full = (uint64_t*)(sB + WG_STAGES * B_STRIDE);
+    uint64_t* empty = full + WG_STAGES;
+    uint64_t* done = empty + WG_STAGES;
     uint32_t* tslot = (uint32_t*)(done + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     // Row block of this CTA: 128 rows of (tap, ci).
     const bool wide = a.Ci > BM;                       // Ci = 256: two tiles per tap
     const int tap_base = wide ? (int)(blockIdx.x >> 1) : (int)blockIdx.x * (BM / a.Ci);
@@ -230,15 +253,24 @@ __global__ void __launch_bounds__(128, 1)
 
     // A atoms of this tile that hold a real tap (rows of taps >= 27 are left unloaded and
     // their accumulator rows are discarded).
+    // Channel and tap shift of each atom, worked out once: the one producing thread is a serial
+    // chain, and with the divisions inside it the loads of a box were issued more slowly than
+    // they arrived (64^3 x 4 volumes, 32 channels: 0.79 ms with the divisions, 0.39 ms
+    // without; 0.26 ms with the whole warp in the loop and one elected lane issuing, where operands
+    // stay uniform; 0.20 ms with WG_STAGES).
     int natom_a_valid = 0;
+    int aci[NATOM_A], adx[NATOM_A], ady[NATOM_A], adz[NATOM_A];
+#pragma unroll
     for (int j = 0; j < NATOM_A; ++j) {
         const int row0 = j * ACA;
         const int tap = wide ? tap_base : tap_base + row0 / a.Ci;
-        if (tap < 27) ++natom_a_valid;
+        if (tap < 27) natom_a_valid = j + 1;  // taps grow with j
+        aci[j] = wide ? ci_base + row0 : row0 % a.Ci;
+        adz[j] = tap / 9 - 1, ady[j] = (tap / 3) % 3 - 1, adx[j] = tap % 3 - 1;
     }
 
     if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < WG_STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
@@ -250,7 +282,7 @@ __global__ void __launch_bounds__(128, 1)
     // inside the row under the swizzle).
     if (a.b.rows < KV) {
         const uint32_t za = (uint32_t)(KV - a.b.rows) * ROWA, zb = (uint32_t)(KV - a.b.rows) * ROWB;
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < WG_STAGES; ++s) {
             for (int j = 0; j < NATOM_A; ++j) {
                 uint4* p = reinterpret_cast<uint4*>(sA + s * A_BYTES + j * ATOM_A + (uint32_t)a.b.rows * ROWA);
                 for (uint32_t q = tid; q < za / 16; q += blockDim.x) p[q] = make_uint4(0, 0, 0, 0);
@@ -271,50 +303,67 @@ __global__ void __launch_bounds__(128, 1)
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    if (tid == 0) {
-        int issued = 0;
+    bool ok = true;
+    if (warp == 0) {
+        int issued = 0, vx, vy, vz, vn;
+        box_origin(a.b, kb0, vx, vy, vz, vn);
+        int s = 0;
+        uint32_t phase = 1;  // of the stage's previous release
         for (int st = 0; st < nsteps; ++st) {
-            const int s = st % STAGES;
-            if (st >= STAGES && !mbar_wait(&empty[s], ((st / STAGES) - 1) & 1)) {
+            if (st >= WG_STAGES && !mbar_wait(&empty[s], phase)) {
                 atomicExch(err, LDG_ERR_TIMEOUT);
                 break;
             }
-            int vx, vy, vz, vn;
-            box_origin(a.b, kb0 + st, vx, vy, vz, vn);
-            mbar_expect_tx(&full[s], (uint32_t)(natom_a_valid * ACA + a.Co) * (uint32_t)a.b.rows * 2u);
-            for (int j = 0; j < NATOM_A; ++j) {
-                const int row0 = j * ACA;
-                const int tap = wide ? tap_base : tap_base + row0 / a.Ci;
-                const int ci = wide ? ci_base + row0 : row0 % a.Ci;
-                if (tap >= 27) continue;
-                const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                tma_load_5d(sA + s * A_BYTES + j * ATOM_A, &tmx, ci, vx + dx, vy + dy, vz + dz, vn, &full[s]);
+            if (elect_one()) {
+                mbar_expect_tx(&full[s], (uint32_t)(natom_a_valid * ACA + a.Co) * (uint32_t)a.b.rows * 2u);
+#pragma unroll
+                for (int j = 0; j < NATOM_A; ++j)
+                    if (j < natom_a_valid)
+                        tma_load_5d(sA + s * A_BYTES + j * ATOM_A, &tmx, aci[j], vx + adx[j], vy + ady[j], vz + adz[j],
+                                    vn, &full[s]);
+                for (int j = 0; j < natom_b; ++j)
+                    tma_load_5d(sB + s * B_STRIDE + j * ATOM_B, &tmdy, j * ACB, vx, vy, vz, vn, &full[s]);
             }
-            for (int j = 0; j < natom_b; ++j)
-                tma_load_5d(sB + s * B_STRIDE + j * ATOM_B, &tmdy, j * ACB, vx, vy, vz, vn, &full[s]);
+            __syncwarp();
             issued = st + 1;
+            if (++s == WG_STAGES) s = 0, phase ^= 1u;
+            // next box, x fastest (a division per box here cost more than the box's matrix products)
+            if ((vx += a.b.bx) >= a.b.tx * a.b.bx) {
+                vx = 0;
+                if ((vy += a.b.by) >= a.b.ty * a.b.by) {
+                    vy = 0;
+                    if ((vz += a.b.bz) >= a.b.tz * a.b.bz) { vz = 0; vn += a.b.bn; }
+                }
+            }
         }
-        for (int st = (issued > STAGES ? issued - STAGES : 0); st < issued; ++st)
-            if (!mbar_wait(&full[st % STAGES], (st / STAGES) & 1)) atomicExch(err, LDG_ERR_TIMEOUT);
-    } else if (tid == 32) {
+        for (int st = (issued > WG_STAGES ? issued - WG_STAGES : 0); st < issued; ++st)
+            if (!mbar_wait(&full[st % WG_STAGES], (st / WG_STAGES) & 1)) atomicExch(err, LDG_ERR_TIMEOUT);
+    } else if (warp == 1) {
         const uint32_t idesc = idesc_bf16(BM, a.Co, true, true);
+        int s = 0;
+        uint32_t phase = 0;
         for (int st = 0; st < nsteps; ++st) {
-            const int s = st % STAGES;
-            if (!mbar_wait(&full[s], (st / STAGES) & 1)) {
+            if (!mbar_wait(&full[s], phase)) {
                 atomicExch(err, LDG_ERR_TIMEOUT);
                 break;
             }
             tc_fence_after();
             const uint32_t a0 = smem_u32(sA + s * A_BYTES), b0 = smem_u32(sB + s * B_STRIDE);
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < KV / 16; ++k)
-                umma_bf16(tmem, smem_desc(a0 + k * 2 * SBOA, ATOM_A, SBOA, SWZA),
-                          smem_desc(b0 + k * 2 * SBOB, ATOM_B, SBOB, SWZB), idesc, (st | k) != 0 ? 1u : 0u);
-            umma_commit(&empty[s]);
+                for (int k = 0; k < KV / 16; ++k)
+                    umma_bf16(tmem, smem_desc(a0 + k * 2 * SBOA, ATOM_A, SBOA, SWZA),
+                              smem_desc(b0 + k * 2 * SBOB, ATOM_B, SBOB, SWZB), idesc, (st | k) != 0 ? 1u : 0u);
+                umma_commit(&empty[s]);
+            }
+            __syncwarp();
+            if (++s == WG_STAGES) s = 0, phase ^= 1u;
         }
-        umma_commit(done);
+        if (elect_one()) umma_commit(done);
+        __syncwarp();
+        ok = mbar_wait(done, 0);
     }
-    bool ok = mbar_wait(done, 0);
+    __syncwarp();  // see k_conv3d_fwd
     ok = __syncthreads_and(ok) != 0;
     tc_fence_after();
     if (!ok && tid == 0) atomicExch(err, LDG_ERR_TIMEOUT);
@@ -338,16 +387,123 @@ __global__ void __launch_bounds__(128, 1)
     }
 }
 
-// w[co][t][ci] -> wf[ci][26 - t][co]: the data gradient is the forward convolution of the
-// output gradient with these weights.
-__global__ void k_flip_weights(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wf, int Ci, int Co) {
-    const long long n = (long long)Co * 27 * Ci;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int ci = (int)(i % Ci);
-        const int t = (int)((i / Ci) % 27);
-        const int co = (int)(i / ((long long)Ci * 27));
-        wf[((long long)ci * 27 + (26 - t)) * Co + co] = w[i];
+// ---------------------------------------------------------------------------------------
+// Activation mask of the output gradient and bias gradient, one pass
+// ---------------------------------------------------------------------------------------
+// g = gy * (y > 0 ? 1 : slope) in gy's type (FP32 or BF16; the slope is rounded to it), rounded
+// to BF16; part[block][c] = sum over the block's voxels of g[., c]. Bound by memory: it reads y
+// and gy and writes g once, where the same as separate elementwise operations and a reduction
+// moved the field eleven times through FP32 temporaries (64^3 x 4, 32 channels: 331 us; 35 us here,
+// 201 MB at 5.7 TB/s). A thread keeps eight
+// channels, so the sums need no exchange until the block's end; they are kept in FP64.
+template <typename T, bool kMask>
+__global__ void __launch_bounds__(256)
+    k_act_grad(const T* __restrict__ y, const T* __restrict__ gy, __nv_bfloat16* __restrict__ g, double* __restrict__ part,
+               long long nvox, int C) {
+    extern __shared__ double s_part[];  // [256][8]
+    const int lanes = C / 8, per = 256 / lanes, used = per * lanes;  // threads per voxel, voxels per pass
+    const int tid = threadIdx.x, c8 = tid % lanes;
+    const float slope = sizeof(T) == 2 ? __bfloat162float(__float2bfloat16_rn(0.01f)) : 0.01f;
+    double acc[8] = {};
+    if (tid < used)
+        for (long long v = (long long)blockIdx.x * per + tid / lanes; v < nvox; v += (long long)gridDim.x * per) {
+            const long long o = v * C + c8 * 8;
+            float a[8], m[8];
+            if constexpr (sizeof(T) == 2) {
+                const uint4 q = *reinterpret_cast<const uint4*>(gy + o);
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    a[2 * i] = __uint_as_float(w[i] << 16), a[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+                if constexpr (kMask) {
+                    const uint4 p = *reinterpret_cast<const uint4*>(y + o);
+                    const uint32_t u[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        m[2 * i] = __uint_as_float(u[i] << 16), m[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+                }
+            } else {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float4 q = *reinterpret_cast<const float4*>(gy + o + 4 * h);
+                    a[4 * h] = q.x, a[4 * h + 1] = q.y, a[4 * h + 2] = q.z, a[4 * h + 3] = q.w;
+                    if constexpr (kMask) {
+                        const float4 p = *reinterpret_cast<const float4*>(y + o + 4 * h);
+                        m[4 * h] = p.x, m[4 * h + 1] = p.y, m[4 * h + 2] = p.z, m[4 * h + 3] = p.w;
+                    }
+                }
+            }
+            uint32_t r[4];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if constexpr (kMask) a[i] = m[i] > 0.0f ? a[i] : a[i] * slope;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(a[2 * i], a[2 * i + 1]);
+                r[i] = *reinterpret_cast<const uint32_t*>(&h);
+                acc[2 * i] += (double)__uint_as_float(r[i] << 16);
+                acc[2 * i + 1] += (double)__uint_as_float(r[i] & 0xffff0000u);
+            }
+            if (g) *reinterpret_cast<uint4*>(g + o) = make_uint4(r[0], r[1], r[2], r[3]);
+        }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s_part[tid * 8 + i] = acc[i];
+    __syncthreads();
+    for (int c = tid; c < C; c += 256) {
+        double t = 0.0;
+        for (int k = 0; k < per; ++k) t += s_part[(k * lanes + c / 8) * 8 + c % 8];
+        part[(long long)blockIdx.x * C + c] = t;
     }
+}
+
+// db[c] = sum over the blocks of part[block][c]; one block of 32 x 8 threads per 8 channels
+__global__ void __launch_bounds__(256) k_act_grad_sum(const double* __restrict__ part, float* __restrict__ db, int blocks, int C) {
+    __shared__ double s[256];
+    const int c = blockIdx.x * 8 + (threadIdx.x & 7);
+    double t = 0.0;
+    for (int b = threadIdx.x >> 3; b < blocks; b += 32) t += part[(long long)b * C + c];
+    s[threadIdx.x] = t;
+    __syncthreads();
+    for (int h = 128; h >= 8; h >>= 1) {
+        if (threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
+        __syncthreads();
+    }
+    if (threadIdx.x < 8) db[c] = (float)s[threadIdx.x];
+}
+
+int act_grad_blocks(long long nvox, int C) {
+    const long long per = 256 / (C / 8);
+    return (int)std::max(1LL, std::min<long long>((nvox + 4 * per - 1) / (4 * per), 148 * 8));
+}
+
+template <typename T>
+int launch_act_grad(long long nvox, int C, const void* y, const void* gy, void* g, float* db, double* ws, cudaStream_t st) {
+    const int blocks = act_grad_blocks(nvox, C);
+    const size_t smem = 256 * 8 * sizeof(double);
+    if (y)
+        k_act_grad<T, true><<<blocks, 256, smem, st>>>((const T*)y, (const T*)gy, (__nv_bfloat16*)g, ws, nvox, C);
+    else
+        k_act_grad<T, false><<<blocks, 256, smem, st>>>(nullptr, (const T*)gy, (__nv_bfloat16*)g, ws, nvox, C);
+    LDG_LAUNCHED("k_act_grad");
+    k_act_grad_sum<<<C / 8, 256, 0, st>>>(ws, db, blocks, C);
+    LDG_LAUNCHED("k_act_grad_sum");
+    return LDG_OK;
+}
+
+// w[co][t][ci] -> wf[ci][26 - t][co]: the data gradient is the forward convolution of the
+// output gradient with these weights. A 32 x 32 tile of (co, ci) of one tap is turned in shared
+// memory, so that both sides move whole sectors (element by element the writes were 2 bytes to a
+// sector: 18 us at 256 x 256 channels, 4 us now).
+__global__ void __launch_bounds__(256)
+    k_flip_weights(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wf, int Ci, int Co) {
+    __shared__ __nv_bfloat16 tile[32][34];
+    const int t = blockIdx.x, ci0 = blockIdx.y * 32, co0 = blockIdx.z * 32;
+    const int a = threadIdx.x & 31, b = threadIdx.x >> 5;
+    for (int r = b; r < 32; r += 8)
+        if (co0 + r < Co && ci0 + a < Ci) tile[r][a] = w[((long long)(co0 + r) * 27 + t) * Ci + ci0 + a];
+    __syncthreads();
+    for (int r = b; r < 32; r += 8)
+        if (ci0 + r < Ci && co0 + a < Co) wf[((long long)(ci0 + r) * 27 + 26 - t) * Co + co0 + a] = tile[a][r];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -427,13 +583,13 @@ int encode_act(CUtensorMap* tm, const void* p, const sg_conv_shape& s, int C, in
     return LDG_OK;
 }
 
-// Weight map [Co][27][Ci]: dims (Ci, 27, Co), box (ck, 1, Co).
-int encode_w(CUtensorMap* tm, const void* p, int Ci, int Co, int ck) {
+// Weight map [Co][27][Ci]: dims (Ci, 27, Co), box (ck, 1, cs).
+int encode_w(CUtensorMap* tm, const void* p, int Ci, int Co, int ck, int cs) {
     auto enc = encoder();
     LDG_REQUIRE(enc, LDG_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
     cuuint64_t dims[3] = {(cuuint64_t)Ci, 27, (cuuint64_t)Co};
     cuuint64_t strides[2] = {(cuuint64_t)Ci * 2, (cuuint64_t)Ci * 2 * 27};
-    cuuint32_t box[3] = {(cuuint32_t)ck, 1, (cuuint32_t)Co};
+    cuuint32_t box[3] = {(cuuint32_t)ck, 1, (cuuint32_t)cs};
     cuuint32_t es[3] = {1, 1, 1};
     CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dims, strides, box, es,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(ck * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -471,20 +627,28 @@ int launch_fwd(const sg_conv_shape& s, const void* x, const void* w, const float
     a.b = make_box(s.N, s.D, s.H, s.W, BM);
     a.act = act;
     a.out_f32 = f32;
-    a.cchunks = s.Ci / CK;
-    a.ksteps = 27 * a.cchunks;
-    a.tmem_cols = tmem_cols_for(s.Co);
+    a.ksteps = 27 * (s.Ci / CK);
+    const long long tiles = (long long)a.b.tx * a.b.ty * a.b.tz * a.b.tn;
+    LDG_REQUIRE(tiles < (1LL << 31), LDG_ERR_ARG, "conv3d: too many tiles");
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // Where the tiles leave most SMs idle, a tile's output channels are shared out over CTAs (no
+    // fewer than 64 each: every CTA loads the whole input tile). 256 -> 256 channels on 8^3 x 8 has
+    // 32 tiles: 42 us undivided, 25 in four.
+    int slices = 1;
+    while (tiles * slices * 2 <= sms && s.Co % (slices * 32) == 0 && s.Co / (slices * 2) >= 64) slices *= 2;
+    a.cs = s.Co / slices;
+    a.tmem_cols = tmem_cols_for(a.cs);
     CUtensorMap tmx, tmw;
     int rc = encode_act(&tmx, x, s, s.Ci, CK, a.b);
     if (rc) return rc;
-    rc = encode_w(&tmw, w, s.Ci, s.Co, CK);
+    rc = encode_w(&tmw, w, s.Ci, s.Co, CK, a.cs);
     if (rc) return rc;
-    const size_t b_stride = ((size_t)s.Co * CK * 2 + 1023) & ~(size_t)1023;
+    const size_t b_stride = ((size_t)a.cs * CK * 2 + 1023) & ~(size_t)1023;
     const size_t smem = 1024 + STAGES * ((size_t)BM * CK * 2 + b_stride) + (2 * STAGES + 1) * 8 + 16;
     LDG_CUDA(cudaFuncSetAttribute(k_conv3d_fwd<CK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const long long tiles = (long long)a.b.tx * a.b.ty * a.b.tz * a.b.tn;
-    LDG_REQUIRE(tiles < (1LL << 31), LDG_ERR_ARG, "conv3d: too many tiles");
-    k_conv3d_fwd<CK><<<(unsigned)tiles, 128, smem, st>>>(tmx, tmw, y, bias, a, g_err);
+    k_conv3d_fwd<CK><<<dim3((unsigned)tiles, (unsigned)slices), 128, smem, st>>>(tmx, tmw, y, bias, a, g_err);
     LDG_LAUNCHED("k_conv3d_fwd");
     g_launches++;
     return LDG_OK;
@@ -498,14 +662,6 @@ int launch_wgrad(const sg_conv_shape& s, const void* x, const void* dy, float* d
     a.nkb = (long long)a.b.tx * a.b.ty * a.b.tz * a.b.tn;
     a.tmem_cols = tmem_cols_for(s.Co);
     const int mtiles = (s.Ci > BM) ? 27 * (s.Ci / BM) : (27 + (BM / s.Ci) - 1) / (BM / s.Ci);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // Split K so the grid covers every SM about twice; at least 8 K boxes per CTA.
-    long long splits = std::max(1LL, (2LL * sms + mtiles - 1) / mtiles);
-    splits = std::min(splits, std::max(1LL, a.nkb / 8));
-    a.kb_per_cta = (int)((a.nkb + splits - 1) / splits);
-    splits = (a.nkb + a.kb_per_cta - 1) / a.kb_per_cta;
     CUtensorMap tmx, tmdy;
     BoxDims bk = a.b;
     int rc = encode_act(&tmx, x, s, s.Ci, ACA, bk);
@@ -513,8 +669,27 @@ int launch_wgrad(const sg_conv_shape& s, const void* x, const void* dy, float* d
     rc = encode_act(&tmdy, dy, s, s.Co, ACB, bk);
     if (rc) return rc;
     const size_t b_stride = ((size_t)s.Co * KV * 2 + 1023) & ~(size_t)1023;
-    const size_t smem = 1024 + STAGES * ((size_t)BM * KV * 2 + b_stride) + (2 * STAGES + 1) * 8 + 16;
+    const size_t smem = 1024 + WG_STAGES * ((size_t)BM * KV * 2 + b_stride) + (2 * WG_STAGES + 1) * 8 + 16;
     LDG_CUDA(cudaFuncSetAttribute(k_conv3d_wgrad<ACA, ACB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int dev = 0, sms = 148, per_sm = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    LDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv3d_wgrad<ACA, ACB>, 128, smem));
+    const long long slots = (long long)sms * std::max(1, std::min(per_sm, 512 / (int)a.tmem_cols));
+    // Split K so the grid covers every SM about twice; at least 8 K boxes per CTA.
+    long long splits = std::max(1LL, (2LL * sms + mtiles - 1) / mtiles);
+    splits = std::min(splits, std::max(1LL, a.nkb / 8));
+    // Small volumes (at most 64 boxes a CTA) are split up to twice as often where that takes
+    // fewer or shorter waves: 256 -> 256 channels, 8^3 x 8, is 324 CTAs in 148 places otherwise. A
+    // split is never coarser, since a longer accumulation loses precision.
+    const long long coarse = splits;
+    long long best = -1;
+    for (long long c = coarse; c <= 2 * coarse && (c == coarse || (a.nkb + coarse - 1) / coarse <= 64); ++c) {
+        const long long boxes = (a.nkb + c - 1) / c, waves = (mtiles * ((a.nkb + boxes - 1) / boxes) + slots - 1) / slots;
+        if (best < 0 || waves * (boxes + kWgFixed) < best) best = waves * (boxes + kWgFixed), splits = c;
+    }
+    a.kb_per_cta = (int)((a.nkb + splits - 1) / splits);
+    splits = (a.nkb + a.kb_per_cta - 1) / a.kb_per_cta;
     LDG_CUDA(cudaMemsetAsync(dw, 0, (size_t)s.Co * 27 * s.Ci * sizeof(float), st));
     dim3 grid((unsigned)mtiles, (unsigned)splits);
     k_conv3d_wgrad<ACA, ACB><<<grid, 128, smem, st>>>(tmx, tmdy, dw, a, g_err);
@@ -566,14 +741,72 @@ int sg_conv3d_wgrad(const sg_conv_shape* s, const void* x, const void* dy, float
 int sg_conv3d_flip_weights(const sg_conv_shape* s, const void* w, void* wf, void* stream) {
     clear_error();
     LDG_REQUIRE(s && w && wf, LDG_ERR_ARG, "sg_conv3d_flip_weights: null argument");
-    const long long n = (long long)s->Co * 27 * s->Ci;
-    const int blocks = (int)std::min<long long>((n + 255) / 256, 148 * 8);
-    k_flip_weights<<<std::max(blocks, 1), 256, 0, (cudaStream_t)stream>>>(
+    LDG_REQUIRE(s->Ci >= 1 && s->Co >= 1 && s->Co <= 65535 * 32 && s->Ci <= 65535 * 32, LDG_ERR_ARG,
+                "sg_conv3d_flip_weights: channels out of range");
+    const dim3 grid(27, (unsigned)((s->Ci + 31) / 32), (unsigned)((s->Co + 31) / 32));
+    k_flip_weights<<<grid, 256, 0, (cudaStream_t)stream>>>(
         static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(wf), s->Ci, s->Co);
     LDG_LAUNCHED("k_flip_weights");
     std::lock_guard<std::mutex> lk(g_mu);
     g_launches++;
     return LDG_OK;
+}
+
+// Doubles of scratch that sg_conv3d_act_grad needs.
+long long sg_conv3d_act_grad_ws(long long nvox, int C) {
+    return (C >= 16 && C <= 256 && C % 16 == 0 && nvox >= 1) ? (long long)act_grad_blocks(nvox, C) * C : 0;
+}
+
+// g = BF16(gy * leaky-ReLU mask of y) (y null: no mask; g null: sums only), db = channel sums of g.
+int sg_conv3d_act_grad(long long nvox, int C, const void* y, const void* gy, int fp32, void* g, float* db, double* ws,
+                       void* stream) {
+    clear_error();
+    LDG_REQUIRE(nvox >= 1 && C >= 16 && C <= 256 && C % 16 == 0, LDG_ERR_ARG,
+                "sg_conv3d_act_grad: channels must be a multiple of 16 in [16, 256], and the volume not empty");
+    LDG_REQUIRE(gy && db && ws, LDG_ERR_ARG, "sg_conv3d_act_grad: null pointer");
+    LDG_REQUIRE((((uintptr_t)y | (uintptr_t)gy | (uintptr_t)g) & 15) == 0, LDG_ERR_ARG,
+                "sg_conv3d_act_grad: pointers must be 16-byte aligned");
+    const int rc = fp32 ? launch_act_grad<float>(nvox, C, y, gy, g, db, ws, (cudaStream_t)stream)
+                        : launch_act_grad<__nv_bfloat16>(nvox, C, y, gy, g, db, ws, (cudaStream_t)stream);
+    if (rc) return rc;
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_launches += 2;
+    return LDG_OK;
+}
+
+// Bytes of scratch that sg_conv3d_bwd needs, 256-byte aligned parts: g, the flipped weights, partial sums.
+static size_t bwd_part(size_t b) { return (b + 255) & ~(size_t)255; }
+long long sg_conv3d_bwd_ws(const sg_conv_shape* s) {
+    const long long nvox = (long long)s->N * s->D * s->H * s->W;
+    return (long long)(bwd_part((size_t)nvox * s->Co * 2) + bwd_part((size_t)s->Ci * 27 * s->Co * 2)) +
+           sg_conv3d_act_grad_ws(nvox, s->Co) * (long long)sizeof(double);
+}
+
+// All gradients of a layer, from its input x, weights w, output y (null: no activation) and output
+// gradient gy, in one call (dx null: not wanted): on small volumes the four separate calls took
+// longer to make than their kernels to run.
+int sg_conv3d_bwd(const sg_conv_shape* s, const void* x, const void* w, const void* y, const void* gy, int fp32, void* dx,
+                  float* dw, float* db, void* ws, void* stream) {
+    clear_error();
+    int rc = check_shape(s, "sg_conv3d_bwd");
+    if (rc) return rc;
+    LDG_REQUIRE(x && w && gy && dw && db && ws, LDG_ERR_ARG, "sg_conv3d_bwd: null pointer");
+    const long long nvox = (long long)s->N * s->D * s->H * s->W;
+    unsigned char* p = static_cast<unsigned char*>(ws);
+    void* g = p;
+    void* wf = p += bwd_part((size_t)nvox * s->Co * 2);
+    double* part = reinterpret_cast<double*>(p + bwd_part((size_t)s->Ci * 27 * s->Co * 2));
+    const bool same = !y && !fp32;  // the output gradient as it is
+    if ((rc = sg_conv3d_act_grad(nvox, s->Co, y, gy, fp32, same ? nullptr : g, db, part, stream))) return rc;
+    const void* go = same ? gy : g;
+    if (dx) {
+        if ((rc = sg_conv3d_flip_weights(s, w, wf, stream))) return rc;
+        sg_conv_shape t = *s;
+        t.Ci = s->Co;
+        t.Co = s->Ci;
+        if ((rc = sg_conv3d_fwd(&t, go, wf, nullptr, dx, 0, 0, stream))) return rc;
+    }
+    return sg_conv3d_wgrad(s, x, go, dw, stream);
 }
 
 // Reads and clears the device error word of the conv kernels (synchronises the stream).

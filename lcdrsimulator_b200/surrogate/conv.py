@@ -30,6 +30,12 @@ def _lib():
         L.sg_conv3d_fwd.argtypes = [C.POINTER(SgShape), vp, vp, vp, vp, C.c_int, C.c_int, vp]
         L.sg_conv3d_wgrad.argtypes = [C.POINTER(SgShape), vp, vp, vp, vp]
         L.sg_conv3d_flip_weights.argtypes = [C.POINTER(SgShape), vp, vp, vp]
+        L.sg_conv3d_act_grad_ws.argtypes = [C.c_longlong, C.c_int]
+        L.sg_conv3d_act_grad_ws.restype = C.c_longlong
+        L.sg_conv3d_act_grad.argtypes = [C.c_longlong, C.c_int, vp, vp, C.c_int, vp, vp, vp, vp]
+        L.sg_conv3d_bwd_ws.argtypes = [C.POINTER(SgShape)]
+        L.sg_conv3d_bwd_ws.restype = C.c_longlong
+        L.sg_conv3d_bwd.argtypes = [C.POINTER(SgShape), vp, vp, vp, vp, C.c_int, vp, vp, vp, vp, vp]
         L.sg_check.argtypes = [vp]
         L.sg_launch_count.restype = C.c_longlong
         _bound = True
@@ -89,6 +95,55 @@ def flip_weights(w: torch.Tensor) -> torch.Tensor:
     return wf
 
 
+def _plain(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _act_grad(y: torch.Tensor | None, gy: torch.Tensor):
+    """(g, db): g = BF16(gy * leaky-ReLU mask of y) (y None: no mask), db its FP32 channel sums."""
+    gy = _plain(gy)
+    if y is not None:
+        y = _plain(y)
+    Co = gy.shape[-1]
+    nvox = gy.numel() // Co
+    g = torch.empty(gy.shape, dtype=torch.bfloat16, device=gy.device)
+    db = torch.empty((Co,), dtype=torch.float32, device=gy.device)
+    L = _lib()
+    ws = torch.empty((L.sg_conv3d_act_grad_ws(nvox, Co),), dtype=torch.float64, device=gy.device)
+    _check(L.sg_conv3d_act_grad(nvox, Co, y.data_ptr() if y is not None else None, gy.data_ptr(),
+                                int(gy.dtype == torch.float32), g.data_ptr(), db.data_ptr(), ws.data_ptr(),
+                                _stream()), "sg_conv3d_act_grad")
+    return g, db
+
+
+def conv3d_bwd(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor | None, gy: torch.Tensor, x_grad: bool = True):
+    """(dx, dw, db) of y = act(conv3d(x, w) + bias) (y None: no activation; dx None without x_grad)."""
+    N, D, H, W, Ci = x.shape
+    Co = w.shape[0]
+    _require(x, torch.bfloat16, (N, D, H, W, Ci), "x")
+    _require(w, torch.bfloat16, (Co, 27, Ci), "w")
+    # without a mask a BF16 gradient is read by the convolutions as it is
+    gy = gy.contiguous() if y is None and gy.dtype == torch.bfloat16 else _plain(gy)
+    if gy.dtype not in (torch.bfloat16, torch.float32):
+        raise ValueError(f"gy: expected BF16 or FP32, got {gy.dtype}")
+    _require(gy, gy.dtype, (N, D, H, W, Co), "gy")
+    if y is not None:
+        y = _plain(y)  # a saved-tensor hook may hand back another layout
+        _require(y, gy.dtype, (N, D, H, W, Co), "y")
+    dev = x.device
+    dx = torch.empty(x.shape, dtype=torch.bfloat16, device=dev) if x_grad else None
+    dw = torch.empty((Co, 27, Ci), dtype=torch.float32, device=dev)
+    db = torch.empty((Co,), dtype=torch.float32, device=dev)
+    s = SgShape(N, D, H, W, Ci, Co)
+    L = _lib()
+    ws = torch.empty((L.sg_conv3d_bwd_ws(C.byref(s)),), dtype=torch.uint8, device=dev)
+    _check(L.sg_conv3d_bwd(C.byref(s), x.data_ptr(), w.data_ptr(), y.data_ptr() if y is not None else None,
+                           gy.data_ptr(), int(gy.dtype == torch.float32), dx.data_ptr() if x_grad else None,
+                           dw.data_ptr(), db.data_ptr(), ws.data_ptr(), _stream()), "sg_conv3d_bwd")
+    return dx, dw, db
+
+
 def check(stream=None):
     _check(_lib().sg_check(C.c_void_p(stream if stream is not None else torch.cuda.current_stream().cuda_stream)),
            "sg_check")
@@ -102,7 +157,8 @@ class Conv3dFunction(torch.autograd.Function):
     """3x3x3 convolution, stride 1, zero padding 1, with bias and optional leaky ReLU (slope 0.01).
 
     Forward, data gradient (forward of the flipped weights) and weight gradient all run on the
-    tcgen05 kernels; only the activation mask and the bias gradient (a channel sum) use torch.
+    tcgen05 kernels; the activation mask and the bias gradient (a channel sum) are one pass
+    over the output gradient, or torch operations where a graph of the backward is recorded.
     """
 
     @staticmethod
@@ -117,7 +173,9 @@ class Conv3dFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, wb, y = ctx.saved_tensors
-        g = gy
+        if not torch.is_grad_enabled():
+            return *conv3d_bwd(x, wb, y if ctx.act == 1 else None, gy, ctx.x_grad), None, None
+        g = gy  # create_graph: the bias gradient stays differentiable
         if ctx.act == 1:
             g = g * torch.where(y > 0, 1.0, 0.01).to(g.dtype)
         g = g.to(torch.bfloat16).contiguous()
