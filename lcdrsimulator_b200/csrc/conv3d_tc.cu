@@ -10,6 +10,8 @@
 //   K-major, exactly as the UMMA descriptors read them. One thread issues tcgen05.mma into a
 //   TMEM accumulator of 128 lanes x Co columns; the epilogue reads TMEM with tcgen05.ld and
 //   applies bias and leaky ReLU before the BF16 (or FP32) store.
+//   Narrow layers on long volumes march along z instead, loading each shifted plane once for the
+//   three taps along z that read it.
 // Weight gradient:
 //   GEMM M = 128 rows of (tap, ci), N = Co, K = voxels, both operands MN-major (channels are
 //   contiguous per voxel): the A tile stacks 128/Ci taps of the shifted input, the B tile is
@@ -75,6 +77,28 @@ __device__ __forceinline__ void box_origin(const BoxDims& b, long long t, int& x
 
 __device__ __forceinline__ float act_apply(float v, int act) { return (act == 1 && v < 0.0f) ? 0.01f * v : v; }
 
+// Bias, activation and store of 16 channels c.. of a voxel, at element o of y.
+__device__ __forceinline__ void store16(void* __restrict__ y, const float* __restrict__ bias, float* v, long long o, int c,
+                                        int act, int f32) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = act_apply(v[i] + (bias ? bias[c + i] : 0.0f), act);
+    if (f32) {
+        float4* dst = reinterpret_cast<float4*>(static_cast<float*>(y) + o);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+        uint32_t p[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+            p[q] = *reinterpret_cast<uint32_t*>(&h);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(y) + o);
+        dst[0] = make_uint4(p[0], p[1], p[2], p[3]);
+        dst[1] = make_uint4(p[4], p[5], p[6], p[7]);
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // Forward / data-gradient kernel
 // ---------------------------------------------------------------------------------------
@@ -125,7 +149,7 @@ __global__ void __launch_bounds__(128, 1)
         int issued = 0, tap = 0, cc = 0, dx = -1, dy = -1, dz = -1;  // tap = 9 (dz + 1) + 3 (dy + 1) + dx + 1
         for (int ks = 0; ks < a.ksteps; ++ks) {
             const int s = ks % STAGES;
-            if (ks >= STAGES && !mbar_wait(&empty[s], ((ks / STAGES) - 1) & 1)) {
+            if (ks >= STAGES && !mbar_wait_warp(&empty[s], ((ks / STAGES) - 1) & 1)) {
                 atomicExch(err, LDG_ERR_TIMEOUT);
                 break;
             }
@@ -147,13 +171,13 @@ __global__ void __launch_bounds__(128, 1)
             }
         }
         for (int ks = (issued > STAGES ? issued - STAGES : 0); ks < issued; ++ks)
-            if (!mbar_wait(&full[ks % STAGES], (ks / STAGES) & 1)) atomicExch(err, LDG_ERR_TIMEOUT);
+            if (!mbar_wait_warp(&full[ks % STAGES], (ks / STAGES) & 1)) atomicExch(err, LDG_ERR_TIMEOUT);
     } else if (warp == 1) {
         // MMA issuer
         const uint32_t idesc = idesc_bf16(BM, a.cs, false, false);
         for (int ks = 0; ks < a.ksteps; ++ks) {
             const int s = ks % STAGES;
-            if (!mbar_wait(&full[s], (ks / STAGES) & 1)) {
+            if (!mbar_wait_warp(&full[s], (ks / STAGES) & 1)) {
                 atomicExch(err, LDG_ERR_TIMEOUT);
                 break;
             }
@@ -170,7 +194,7 @@ __global__ void __launch_bounds__(128, 1)
         }
         if (elect_one()) umma_commit(done);
         __syncwarp();
-        ok = mbar_wait(done, 0);
+        ok = mbar_wait_warp(done, 0);
     }
     // Epilogue: row m of the accumulator is output voxel m of the box; warp w owns lanes 32w..32w+31.
     // The other lanes of the two working warps stand at a warp barrier until here: polling `done`
@@ -190,24 +214,160 @@ __global__ void __launch_bounds__(128, 1)
         float v[16];
         tmem_ld16(trow + (uint32_t)c0, v);
         if (!inside) continue;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = act_apply(v[i] + (bias ? bias[co0 + c0 + i] : 0.0f), a.act);
-        if (a.out_f32) {
-            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(y) + vox * a.Co + co0 + c0);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        } else {
-            uint32_t p[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-                p[q] = *reinterpret_cast<uint32_t*>(&h);
+        store16(y, bias, v, vox * a.Co + co0 + c0, co0 + c0, a.act, a.out_f32);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, a.tmem_cols);
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// Forward / data gradient of narrow layers: a march along z
+// ---------------------------------------------------------------------------------------
+// With few channels k_conv3d_fwd is bound by reading each input box 27 times from L2 (64^3 x 4
+// volumes, 32 -> 32 channels: 2.3 GB in 0.163 ms). Here a CTA keeps all 27 weight slices in shared
+// memory and marches a 128-voxel (x, y) tile along z: each of a plane's nine (dy, dx)-shifted boxes
+// is loaded once and multiplied for the three output planes that it belongs to, in three of four
+// TMEM accumulators, while four warps store the plane that is complete (0.108 ms). An output takes its
+// taps in the order of k_conv3d_fwd (dz outermost), so the results are the same bits.
+struct MarchArgs {
+    int D, H, W, Co, bx, by, tx, ty;
+    int zlen, act, out_f32;
+    uint32_t acc_cols, tmem_cols;  // columns of an accumulator, and of the four
+};
+
+template <int CK>
+__global__ void __launch_bounds__(192, 1)
+    k_conv3d_march(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw, void* __restrict__ y,
+                   const float* __restrict__ bias, MarchArgs a, int* __restrict__ err) {
+    constexpr int MS = CK == 64 ? 4 : 6;  // stages
+    constexpr uint32_t ROW = CK * 2, A_BYTES = BM * ROW, SWZ = swizzle_code(ROW), SBO = 8 * ROW;
+    const uint32_t B_BYTES = (uint32_t)a.Co * ROW, B_STRIDE = (B_BYTES + 1023u) & ~1023u;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* sA = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* sB = sA + MS * A_BYTES;
+    uint64_t* full = (uint64_t*)(sB + 27 * B_STRIDE);
+    uint64_t* empty = full + MS;
+    uint64_t* acc_full = empty + MS;    // [4] an accumulator holds its whole output plane
+    uint64_t* acc_empty = acc_full + 4; // [4] its plane has been read
+    uint64_t* wfull = acc_empty + 4;
+    uint64_t* done = wfull + 1;
+    uint32_t* tslot = (uint32_t*)(done + 1);
+
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int x0 = (int)(blockIdx.x % a.tx) * a.bx, y0 = (int)(blockIdx.x / a.tx) * a.by;
+    const int n0 = (int)blockIdx.z, z0 = (int)blockIdx.y * a.zlen;
+    const int z1 = min(z0 + a.zlen, a.D);  // output planes [z0, z1)
+    const int nplanes = z1 - z0 + 2;       // input planes z0 - 1 .. z1 (zeros outside the volume)
+
+    if (tid == 0) {
+        for (int s = 0; s < MS; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 4; ++s) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 128);
+        }
+        mbar_init(wfull, 1);
+        mbar_init(done, 1);
+        fence_mbar_init();
+    }
+    if (warp == 0) {
+        __syncwarp();
+        tmem_alloc(tslot, a.tmem_cols);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+
+    bool ok = true;
+    if (warp == 0) {
+        if (elect_one()) {
+            mbar_expect_tx(wfull, 27 * B_BYTES);
+            for (int t = 0; t < 27; ++t) tma_load_3d(sB + t * B_STRIDE, &tmw, 0, t, 0, wfull);
+        }
+        __syncwarp();
+        int s = 0, issued = 0;
+        uint32_t phase = 1;
+        for (int p = 0; p < nplanes && ok; ++p)
+            for (int t = 0; t < 9; ++t) {
+                if (issued >= MS && !(ok = mbar_wait_warp(&empty[s], phase))) break;
+                if (elect_one()) {
+                    mbar_expect_tx(&full[s], A_BYTES);
+                    tma_load_5d(sA + s * A_BYTES, &tmx, 0, x0 + t % 3 - 1, y0 + t / 3 - 1, z0 - 1 + p, n0, &full[s]);
+                }
+                __syncwarp();
+                ++issued;
+                if (++s == MS) s = 0, phase ^= 1u;
             }
-            uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(y) + vox * a.Co + co0 + c0);
-            dst[0] = make_uint4(p[0], p[1], p[2], p[3]);
-            dst[1] = make_uint4(p[4], p[5], p[6], p[7]);
+        // the loads in flight land before the block may end
+        for (int k = (issued > MS ? issued - MS : 0); k < issued; ++k)
+            if (!mbar_wait_warp(&full[k % MS], (k / MS) & 1)) ok = false;
+        if (!mbar_wait_warp(wfull, 0)) ok = false;
+    } else if (warp == 1) {
+        const uint32_t idesc = idesc_bf16(BM, a.Co, false, false);
+        const uint32_t b00 = smem_u32(sB);
+        int s = 0;
+        uint32_t phase = 0;
+        ok = mbar_wait_warp(wfull, 0);
+        for (int p = 0; p < nplanes && ok; ++p) {
+            // input plane p of the march is dz = +1 of output p - 2, 0 of p - 1, -1 of p
+            if (p >= 4 && p < z1 - z0) {
+                if (!(ok = mbar_wait_warp(&acc_empty[p & 3], ((p >> 2) - 1) & 1))) break;
+                tc_fence_after();
+            }
+            for (int t = 0; t < 9; ++t) {
+                if (!(ok = mbar_wait_warp(&full[s], phase))) break;
+                tc_fence_after();
+                const uint32_t a0 = smem_u32(sA + s * A_BYTES);
+                if (elect_one()) {
+#pragma unroll
+                    for (int dz = 0; dz < 3; ++dz) {  // dz + 1 of the tap
+                        const int o = p - dz;
+                        if (o < 0 || o >= z1 - z0) continue;
+                        const uint32_t b0 = b00 + (uint32_t)(9 * dz + t) * B_STRIDE, d = tmem + (uint32_t)(o & 3) * a.acc_cols;
+#pragma unroll
+                        for (int k = 0; k < CK / 16; ++k)
+                            umma_bf16(d, smem_desc(a0 + k * 32, 16, SBO, SWZ), smem_desc(b0 + k * 32, 16, SBO, SWZ), idesc,
+                                      (dz | t | k) != 0 ? 1u : 0u);
+                    }
+                    umma_commit(&empty[s]);
+                    if (t == 8 && p >= 2) umma_commit(&acc_full[(p - 2) & 3]);
+                }
+                __syncwarp();
+                if (++s == MS) s = 0, phase ^= 1u;
+            }
+        }
+        if (elect_one()) umma_commit(done);
+        __syncwarp();
+        if (!mbar_wait_warp(done, 0)) ok = false;
+    } else {
+        // warp w reads the TMEM lanes 32 (w & 3) ..: row m of the tile is voxel (m % bx, m / bx)
+        const int m = (warp & 3) * 32 + (tid & 31);
+        const int x = x0 + m % a.bx, yy = y0 + m / a.bx;
+        const bool inside = x < a.W && yy < a.H;
+        for (int o = 0; o < z1 - z0; ++o) {
+            if (!(ok = mbar_wait_warp(&acc_full[o & 3], (o >> 2) & 1))) break;
+            tc_fence_after();
+            const long long vox = (((long long)n0 * a.D + z0 + o) * a.H + yy) * a.W + x;
+            const uint32_t trow = tmem + (uint32_t)(o & 3) * a.acc_cols + ((uint32_t)((warp & 3) * 32) << 16);
+            for (int c0 = 0; c0 < a.Co; c0 += 16) {
+                float v[16];
+                __syncwarp();
+                tmem_ld16(trow + (uint32_t)c0, v);
+                if (inside) store16(y, bias, v, vox * a.Co + c0, c0, a.act, a.out_f32);
+            }
+            tc_fence_before();
+            mbar_arrive(&acc_empty[o & 3]);
         }
     }
+    __syncwarp();
+    if (!ok) atomicExch(err, LDG_ERR_TIMEOUT);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -310,7 +470,7 @@ __global__ void __launch_bounds__(128, 1)
         int s = 0;
         uint32_t phase = 1;  // of the stage's previous release
         for (int st = 0; st < nsteps; ++st) {
-            if (st >= WG_STAGES && !mbar_wait(&empty[s], phase)) {
+            if (st >= WG_STAGES && !mbar_wait_warp(&empty[s], phase)) {
                 atomicExch(err, LDG_ERR_TIMEOUT);
                 break;
             }
@@ -337,13 +497,13 @@ __global__ void __launch_bounds__(128, 1)
             }
         }
         for (int st = (issued > WG_STAGES ? issued - WG_STAGES : 0); st < issued; ++st)
-            if (!mbar_wait(&full[st % WG_STAGES], (st / WG_STAGES) & 1)) atomicExch(err, LDG_ERR_TIMEOUT);
+            if (!mbar_wait_warp(&full[st % WG_STAGES], (st / WG_STAGES) & 1)) atomicExch(err, LDG_ERR_TIMEOUT);
     } else if (warp == 1) {
         const uint32_t idesc = idesc_bf16(BM, a.Co, true, true);
         int s = 0;
         uint32_t phase = 0;
         for (int st = 0; st < nsteps; ++st) {
-            if (!mbar_wait(&full[s], phase)) {
+            if (!mbar_wait_warp(&full[s], phase)) {
                 atomicExch(err, LDG_ERR_TIMEOUT);
                 break;
             }
@@ -361,7 +521,7 @@ __global__ void __launch_bounds__(128, 1)
         }
         if (elect_one()) umma_commit(done);
         __syncwarp();
-        ok = mbar_wait(done, 0);
+        ok = mbar_wait_warp(done, 0);
     }
     __syncwarp();  // see k_conv3d_fwd
     ok = __syncthreads_and(ok) != 0;
@@ -619,6 +779,47 @@ int check_shape(const sg_conv_shape* s, const char* who) {
     return LDG_OK;
 }
 
+// The march along z where it is the shorter one: the tile is one plane of 128 voxels, the weights
+// and the stages fit in shared memory, four accumulators fit in TMEM. Lengths are compared in boxes
+// loaded per SM: 27 for each tile of k_conv3d_fwd against nine for each plane of a march, two
+// planes more than it stores, and 27 for its weights (a CTA alone on an SM waits more: x 1.3).
+template <int CK>
+int try_march(const sg_conv_shape& s, const void* x, const void* w, const float* bias, void* y, int act, int f32,
+              const BoxDims& b, int sms, cudaStream_t st, bool& taken) {
+    taken = false;
+    const size_t b_stride = ((size_t)s.Co * CK * 2 + 1023) & ~(size_t)1023;
+    constexpr int MS = CK == 64 ? 4 : 6;  // stages
+    const size_t smem = 1024 + MS * (size_t)BM * CK * 2 + 27 * b_stride + (2 * MS + 10) * 8 + 16;
+    const uint32_t acc = tmem_cols_for(s.Co);
+    if (s.Ci != CK || b.bx * b.by != BM || smem > 227 * 1024 || acc * 4 > 512 || s.N > 65535) return LDG_OK;
+    const long long cols = (long long)b.tx * b.ty * s.N;
+    double best = 27.0 * (double)((cols * s.D + sms - 1) / sms);
+    int zlen = 0;
+    for (int zs = 1; zs <= s.D && zs <= 65535; ++zs) {
+        const int len = (s.D + zs - 1) / zs;
+        const long long k = (cols * ((s.D + len - 1) / len) + sms - 1) / sms;
+        const double t = ((len + 3) * 9 + 27) * std::max((double)k, 1.3);
+        if (t < best) best = t, zlen = len;
+    }
+    if (!zlen) return LDG_OK;
+    MarchArgs a{};
+    a.D = s.D; a.H = s.H; a.W = s.W; a.Co = s.Co;
+    a.bx = b.bx; a.by = b.by; a.tx = b.tx; a.ty = b.ty;
+    a.zlen = zlen; a.act = act; a.out_f32 = f32;
+    a.acc_cols = acc; a.tmem_cols = 4 * acc;
+    CUtensorMap tmx, tmw;
+    int rc = encode_act(&tmx, x, s, CK, CK, b);
+    if (rc) return rc;
+    if ((rc = encode_w(&tmw, w, CK, s.Co, CK, s.Co))) return rc;
+    LDG_CUDA(cudaFuncSetAttribute(k_conv3d_march<CK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)(b.tx * b.ty), (unsigned)((s.D + zlen - 1) / zlen), (unsigned)s.N);
+    k_conv3d_march<CK><<<grid, 192, smem, st>>>(tmx, tmw, y, bias, a, g_err);
+    LDG_LAUNCHED("k_conv3d_march");
+    g_launches++;
+    taken = true;
+    return LDG_OK;
+}
+
 template <int CK>
 int launch_fwd(const sg_conv_shape& s, const void* x, const void* w, const float* bias, void* y, int act, int f32,
                cudaStream_t st) {
@@ -633,6 +834,9 @@ int launch_fwd(const sg_conv_shape& s, const void* x, const void* w, const float
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    bool taken = false;
+    int rc = try_march<CK>(s, x, w, bias, y, act, f32, a.b, sms, st, taken);
+    if (rc || taken) return rc;
     // Where the tiles leave most SMs idle, a tile's output channels are shared out over CTAs (no
     // fewer than 64 each: every CTA loads the whole input tile). 256 -> 256 channels on 8^3 x 8 has
     // 32 tiles: 42 us undivided, 25 in four.
@@ -641,7 +845,7 @@ int launch_fwd(const sg_conv_shape& s, const void* x, const void* w, const float
     a.cs = s.Co / slices;
     a.tmem_cols = tmem_cols_for(a.cs);
     CUtensorMap tmx, tmw;
-    int rc = encode_act(&tmx, x, s, s.Ci, CK, a.b);
+    rc = encode_act(&tmx, x, s, s.Ci, CK, a.b);
     if (rc) return rc;
     rc = encode_w(&tmw, w, s.Ci, s.Co, CK, a.cs);
     if (rc) return rc;

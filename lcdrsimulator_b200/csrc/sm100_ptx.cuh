@@ -26,6 +26,9 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -48,6 +51,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
         if (mbar_try_wait(b, parity)) return true;
         if (globaltimer_ns() - t0 > kWaitNs) return false;
     }
+}
+
+// The same by a converged warp, with one answer for all its lanes (elections and aligned
+// instructions follow, so no lane may leave alone).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* b, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(b, parity)) != 0;
 }
 
 // True in one lane of a converged warp, the same lane each time.

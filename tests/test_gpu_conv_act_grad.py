@@ -45,3 +45,23 @@ def test_backward_in_one_call_is_its_parts(shape, act, fp32):
     want = conv.conv3d_wgrad(x, g)
     assert float((dw - want).abs().max()) <= 1e-5 * float(want.abs().max())
     conv.check()
+
+
+@pytest.mark.parametrize("shape", [(2, 64, 64, 64, 32, 32), (3, 37, 45, 50, 16, 48), (2, 64, 64, 64, 64, 32),
+                                   (4, 33, 32, 32, 16, 128), (1, 70, 130, 126, 32, 16)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_planes_of_a_long_volume_are_those_of_thin_ones(shape, fp32):
+    """A plane needs three input planes: the march along z gives the bits of the tile kernel on a 3-plane volume."""
+    from lcdrsimulator_b200.surrogate import conv
+    N, D, H, W, Ci, Co = shape
+    gen = torch.Generator().manual_seed(Ci * Co + D)
+    x = torch.randn((N, D, H, W, Ci), generator=gen).to(torch.bfloat16).cuda()
+    w = (torch.randn((Co, 27, Ci), generator=gen) * 0.05).to(torch.bfloat16).cuda()
+    b = torch.randn((Co,), generator=gen).cuda()
+    y = conv.conv3d_fwd(x, w, b, 1, fp32)
+    for z in sorted({0, 1, D // 2 - 1, D // 2, D // 2 + 1, D - 2, D - 1}):
+        thin = torch.zeros((N, 3, H, W, Ci), dtype=torch.bfloat16, device="cuda")
+        lo, hi = max(z - 1, 0), min(z + 2, D)
+        thin[:, lo - z + 1:hi - z + 1] = x[:, lo:hi]
+        assert torch.equal(y[:, z], conv.conv3d_fwd(thin, w, b, 1, fp32)[:, 1])
+    conv.check()
