@@ -880,28 +880,38 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
     plan.L2 = L2;
     const int ntj = (Ny + TJ - 1) / TJ;
     long long written = 0;
+    std::vector<TiledBand> bands(ntj);
+    for (TiledBand& b : bands) {  // no allocation inside the parallel loop
+        b.kmin.assign(Nx, INT32_MAX);
+        b.kmax.assign(Nx, -1);
+    }
+    // the bands are independent; with one thread the creation of a 256^3 solver took 77 ms, 34-61 with sixteen
+#pragma omp parallel for reduction(+ : written) schedule(dynamic) if (sc > (1 << 18))
     for (int jt = 0; jt < ntj; ++jt) {
-        TiledBand b;
+        TiledBand& b = bands[jt];
         b.j0 = jt * TJ;
         b.rows = std::min(Ny, (jt + 1) * TJ) - b.j0;
-        std::vector<int> kmin(Nx, INT32_MAX), kmax(Nx, -1);
         int imin = Nx, imax = -1;
         for (int i = 0; i < Nx; ++i)
             for (int j = b.j0; j < b.j0 + b.rows; ++j)
                 for (int k = 0; k < Nz; ++k)
                     if (fl[(size_t)i * si + (size_t)j * sj + k] & (kMove | kFixed)) {
-                        kmin[i] = std::min(kmin[i], k);
-                        kmax[i] = std::max(kmax[i], k);
+                        b.kmin[i] = std::min(b.kmin[i], k);
+                        b.kmax[i] = std::max(b.kmax[i], k);
                         imin = std::min(imin, i);
                         imax = std::max(imax, i);
                         ++written;
                     }
-        if (imax < 0) continue;
         b.face = b.j0 < (L2 ? 2 : 1) || b.j0 + b.rows > Ny - (L2 ? 2 : 1);
         b.ib = imin;
         b.ie = imax + 1;
-        b.kmin.assign(kmin.begin() + imin, kmin.begin() + imax + 1);
-        b.kmax.assign(kmax.begin() + imin, kmax.begin() + imax + 1);
+    }
+    for (TiledBand& b : bands) {
+        if (b.ie <= b.ib) continue;
+        b.kmin.erase(b.kmin.begin() + b.ie, b.kmin.end());
+        b.kmin.erase(b.kmin.begin(), b.kmin.begin() + b.ib);
+        b.kmax.erase(b.kmax.begin() + b.ie, b.kmax.end());
+        b.kmax.erase(b.kmax.begin(), b.kmax.begin() + b.ib);
         plan.bands.push_back(std::move(b));
     }
     plan.written_cells = written;
