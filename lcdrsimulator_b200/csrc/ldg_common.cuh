@@ -703,6 +703,11 @@ __device__ __forceinline__ void euler_update(const QsrConst& P, const float q[5]
 // roots and 45 divisions. M is taken relative to alpha, so its powers stay in range. The
 // reference's early stop (|M n| < 1e-13) can only come at the first step: alpha bounds the row sums of
 // Q, so M is positive semidefinite and |M n| does not fall from one step to the next.
+// Where that stop comes, or where the start vector lies almost at right angles to the largest eigenvector, the 15
+// normalised steps themselves are taken. The row sums of a negative uniaxial order along (1, 1, 1), or of a negative Q_xy
+// alone, are the eigenvector to -alpha, which M shrinks by 1e-12 / alpha: the steps hold on to it, while of M^15 n0
+// only rounding is left (NaN, or another eigenvector). |M^15 n0|^2 < 1e-6 |n0|^2 decides: M^15 does not shrink
+// the largest eigenvector's share of n0, so every start vector with more than 1e-3 of it stays on the fast way.
 // ---------------------------------------------------------------------------------------
 struct Nematic { double S, nx, ny, nz; };
 
@@ -717,6 +722,24 @@ __device__ __forceinline__ void apply(const Sym3& m, double v[3]) {
     v[0] = fma(m.xx, x, fma(m.xy, y, m.xz * z));
     v[1] = fma(m.xy, x, fma(m.yy, y, m.yz * z));
     v[2] = fma(m.xz, x, fma(m.yz, y, m.zz * z));
+}
+
+// The 15 normalised steps (QSR.cu:213-224), from the row sums n or the z axis. Out of line: cells take it rarely.
+inline __device__ __noinline__ void nematic_steps(double Qxx, double Qxy, double Qxz, double Qyy, double Qyz,
+                                                  double alpha, double n[3]) {
+    const double Qzz = -Qxx - Qyy;
+    double nx = n[0], ny = n[1], nz = n[2];
+    const double n0 = sqrt(nx * nx + ny * ny + nz * nz);
+    nx /= n0; ny /= n0; nz /= n0;
+    for (int it = 0; it < 15; ++it) {
+        const double ax = Qxx * nx + Qxy * ny + Qxz * nz + alpha * nx;
+        const double ay = Qxy * nx + Qyy * ny + Qyz * nz + alpha * ny;
+        const double az = Qxz * nx + Qyz * ny + Qzz * nz + alpha * nz;
+        const double nn = sqrt(ax * ax + ay * ay + az * az);
+        if (nn < 1e-13) break;
+        nx = ax / nn; ny = ay / nn; nz = az / nn;
+    }
+    n[0] = nx; n[1] = ny; n[2] = nz;
 }
 
 __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, Nematic iso) {
@@ -736,19 +759,19 @@ __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, 
     Sym3 m{fma(Qxx, ia, 1.0), Qxy * ia, Qxz * ia, fma(Qyy, ia, 1.0), Qyz * ia, fma(Qzz, ia, 1.0)};
     const double n0[3] = {n[0], n[1], n[2]};
     apply(m, n);
-    double v2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
-    if (v2 * (alpha * alpha) < 1e-26 * n2) {  // |M n| < 1e-13: the direction stays the first one
-        n[0] = n0[0]; n[1] = n0[1]; n[2] = n0[2];
-        v2 = n2;
-    } else {
+    const double v1 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            m = square(m);
-            apply(m, n);
-        }
-        v2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
+    for (int p = 0; p < 3; ++p) {
+        m = square(m);
+        apply(m, n);
     }
-    const double inv = 1.0 / sqrt(v2);
+    const double v2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
+    double inv = 1.0 / sqrt(v2);
+    if (v2 < 1e-6 * n2 || v1 * (alpha * alpha) < 1e-26 * n2) {
+        n[0] = n0[0]; n[1] = n0[1]; n[2] = n0[2];
+        nematic_steps(Qxx, Qxy, Qxz, Qyy, Qyz, alpha, n);
+        inv = 1.0;
+    }
     const double nx = n[0] * inv, ny = n[1] * inv, nz = n[2] * inv;
     const double lam = nx * (Qxx * nx + Qxy * ny + Qxz * nz) + ny * (Qxy * nx + Qyy * ny + Qyz * nz) +
                        nz * (Qxz * nx + Qyz * ny + Qzz * nz);
