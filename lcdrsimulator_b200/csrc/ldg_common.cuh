@@ -724,13 +724,15 @@ __device__ __forceinline__ void apply(const Sym3& m, double v[3]) {
     v[2] = fma(m.xz, x, fma(m.yz, y, m.zz * z));
 }
 
-// The 15 normalised steps (QSR.cu:213-224), from the row sums n or the z axis. Out of line: cells take it rarely.
-inline __device__ __noinline__ void nematic_steps(double Qxx, double Qxy, double Qxz, double Qyy, double Qyz,
-                                                  double alpha, double n[3]) {
+// The 15 normalised steps (QSR.cu:203-224). Out of line, and from the tensor alone: cells take it rarely, and the
+// callers' registers decide how many blocks share an SM.
+inline __device__ __noinline__ double3 nematic_steps(double Qxx, double Qxy, double Qxz, double Qyy, double Qyz,
+                                                     double alpha) {
     const double Qzz = -Qxx - Qyy;
-    double nx = n[0], ny = n[1], nz = n[2];
+    double nx = Qxx + Qxy + Qxz, ny = Qxy + Qyy + Qyz, nz = Qxz + Qyz - Qxx - Qyy;
     const double n0 = sqrt(nx * nx + ny * ny + nz * nz);
-    nx /= n0; ny /= n0; nz /= n0;
+    if (n0 > 1e-12) { nx /= n0; ny /= n0; nz /= n0; }
+    else { nx = 0.0; ny = 0.0; nz = 1.0; }
     for (int it = 0; it < 15; ++it) {
         const double ax = Qxx * nx + Qxy * ny + Qxz * nz + alpha * nx;
         const double ay = Qxy * nx + Qyy * ny + Qyz * nz + alpha * ny;
@@ -739,7 +741,7 @@ inline __device__ __noinline__ void nematic_steps(double Qxx, double Qxy, double
         if (nn < 1e-13) break;
         nx = ax / nn; ny = ay / nn; nz = az / nn;
     }
-    n[0] = nx; n[1] = ny; n[2] = nz;
+    return make_double3(nx, ny, nz);
 }
 
 __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, Nematic iso) {
@@ -757,7 +759,6 @@ __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, 
     const double alpha = fmax(r1, fmax(r2, r3)) + 1e-12;
     const double ia = 1.0 / alpha;
     Sym3 m{fma(Qxx, ia, 1.0), Qxy * ia, Qxz * ia, fma(Qyy, ia, 1.0), Qyz * ia, fma(Qzz, ia, 1.0)};
-    const double n0[3] = {n[0], n[1], n[2]};
     apply(m, n);
     const double v1 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
 #pragma unroll
@@ -768,8 +769,8 @@ __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, 
     const double v2 = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
     double inv = 1.0 / sqrt(v2);
     if (v2 < 1e-6 * n2 || v1 * (alpha * alpha) < 1e-26 * n2) {
-        n[0] = n0[0]; n[1] = n0[1]; n[2] = n0[2];
-        nematic_steps(Qxx, Qxy, Qxz, Qyy, Qyz, alpha, n);
+        const double3 v = nematic_steps(Qxx, Qxy, Qxz, Qyy, Qyz, alpha);
+        n[0] = v.x; n[1] = v.y; n[2] = v.z;
         inv = 1.0;
     }
     const double nx = n[0] * inv, ny = n[1] * inv, nz = n[2] * inv;
