@@ -766,7 +766,7 @@ int kzm_step(kzm_handle* h, int n_steps, const kzm_step_args* a) {
     P.mob_dt = (float)((1.0 / h->p.gamma) * a->dt);
     auto both = [](float v) { return F2{make_float2(v, v)}; };
     P.mmob = both(-P.mob_dt);
-    P.K = BulkC<F2>{both(P.A), both(2.0f * P.C), both(2.0f / 3.0f * P.B), both(P.B), both(-P.B)};
+    P.K = BulkC<F2>{both(P.A), both(2.0f * P.C), both(-1.0f / 3.0f * P.B), both(P.B), both(-P.B)};
     P.sigma = (float)a->noise_sigma;
     P.key0 = (uint32_t)a->seed;
     P.key1 = (uint32_t)(a->seed >> 32);

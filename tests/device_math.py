@@ -28,3 +28,11 @@ def nematic(lib, q, iso_cut=1e-9):
     out = np.empty((len(q), 4))
     lib.dm_nematic(ptr(q), C.c_longlong(len(q)), C.c_double(iso_cut), ptr(out))
     return out
+
+
+def chem(lib, q, dx, e, packed):
+    """Chemical potential of an FP32 field (5, n, n, n) on cells 2 .. n - 3, e = (L1, L2, L3, cQ, cQ2, cQ3)."""
+    n = q.shape[1]
+    mu = np.full(q.shape, np.nan, dtype=np.float32)
+    lib.dm_chem(ptr(q), n, C.c_double(dx), ptr(np.asarray(e, dtype=np.float64)), int(packed), ptr(mu))
+    return mu

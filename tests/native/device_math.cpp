@@ -39,7 +39,89 @@ using std::min;
 
 using namespace ldg;
 
+namespace {
+
+// FP32 field of n^3 cells, component-major, centred on a cell.
+struct Cell {
+    const float* q;
+    int n, i, j, k;
+    float operator()(int c, int di, int dj, int dk) const {
+        const long long o = ((long long)(i + di) * n + j + dj) * n + k + dk, m = (long long)n * n * n;
+        return c < 5 ? q[c * m + o] : -(q[o] + q[3 * m + o]);
+    }
+};
+struct Divergence {
+    const Cell& A;
+    const QsrConst& P;
+    float operator()(int c, int di, int dj, int dk) const {
+        float D[3];
+        dcol_at<false>(A, P, A.i, A.j, A.k, di, dj, dk, D);
+        return D[c];
+    }
+};
+
+QsrConst constants(double dx, const double e[6]) {  // L1, L2, L3, cQ, cQ2, cQ3
+    QsrConst P{};
+    const double ix2 = 1 / (dx * dx), i2 = 1 / (2 * dx);
+    P.ix2 = P.iy2 = P.iz2 = (float)ix2;
+    P.i2x = P.i2y = P.i2z = (float)i2;
+    P.ix = P.iy = P.iz = (float)(1 / dx);
+    P.i4xy = P.i4xz = P.i4yz = (float)(ix2 / 4);
+    P.Liso = (float)e[0], P.L2 = (float)e[1], P.L3 = (float)e[2];
+    P.cQ = (float)e[3], P.cQ2 = (float)e[4], P.cQ3 = (float)e[5];
+    P.lap_c = (float)(-6 * ix2);
+    P.L2i2x = P.L2i2y = P.L2i2z = (float)(e[1] * i2);
+    P.lx = P.ly = P.lz = (float)(e[0] * ix2);
+    for (int m = 0; m < 6; ++m) {
+        P.l3m[m] = (float)(0.5 * e[2] * i2 * i2);
+        P.l2w[m] = (float)(e[1] * i2 * i2);
+        P.l3d[m] = (float)(e[2] * i2 * i2);
+    }
+    for (int m = 0; m < 3; ++m) P.l3s[m] = (float)(e[2] * ix2), P.l3c[m] = (float)(2 * e[2] * i2 * i2);
+    return P;
+}
+
+template <bool kL2, bool kL3>
+void chem(const float* q, int n, const QsrConst& P, bool packed, float* mu) {
+    const long long m = (long long)n * n * n;
+    for (int i = 2; i < n - 2; ++i)
+        for (int j = 2; j < n - 3; j += 2)
+            for (int k = 2; k < n - 2; ++k) {
+                const long long o = ((long long)i * n + j) * n + k;
+                if (packed) {
+                    const Cell A{q, n, i, j, k};
+                    F2 c[5], r[5], lap[5];
+                    for (int x = 0; x < 5; ++x) c[x] = mk2(A(x, 0, 0, 0), A(x, 0, 1, 0));
+                    const InteriorPair<kL2, kL3, Cell> S{A};
+                    chem_core<kL2, kL3, false, false, F2>(S, P, c, F2{}, r, lap);
+                    for (int x = 0; x < 5; ++x) mu[x * m + o] = r[x].v.x, mu[x * m + o + n] = r[x].v.y;
+                } else {
+                    for (int y = 0; y < 2; ++y) {
+                        const Cell A{q, n, i, j + y, k};
+                        const Divergence D{A, P};
+                        float c[5], r[5], lap[5];
+                        for (int x = 0; x < 5; ++x) c[x] = A(x, 0, 0, 0);
+                        chem_potential<kL2, kL3, false>(A, D, P, i, j + y, k, c, false, r, lap);
+                        for (int x = 0; x < 5; ++x) mu[x * m + o + y * n] = r[x];
+                    }
+                }
+            }
+}
+
+}  // namespace
+
 extern "C" {
+
+// Chemical potential of the interior cells of an n^3 field; packed: the step kernels' two-cell form, else the
+// term-by-term form of the one-thread-per-cell kernel.
+void dm_chem(const float* q, int n, double dx, const double* e, int packed, float* mu) {
+    const QsrConst P = constants(dx, e);
+    const bool l2 = e[1] != 0.0, l3 = e[2] != 0.0;
+    if (l2 && l3) chem<true, true>(q, n, P, packed, mu);
+    else if (l2) chem<true, false>(q, n, P, packed, mu);
+    else if (l3) chem<false, true>(q, n, P, packed, mu);
+    else chem<false, false>(q, n, P, packed, mu);
+}
 
 // S and director of n tensors (five stored components each).
 void dm_nematic(const double* q, long long n, double iso_cut, double* out) {
