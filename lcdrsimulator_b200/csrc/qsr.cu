@@ -1183,7 +1183,7 @@ void ens_drop_graph(ens_handle* h) {
 int ens_rechunk(ens_handle* h, int cap) {
     std::vector<const TiledPlan*> plans;
     for (const qsr_handle* q : h->inst) plans.push_back(&q->tiled);
-    const int chunk = tiled_length(plans, cap, (h->L2 || h->L3) ? kLoadDeep : kLoadL1);
+    const int chunk = tiled_length(plans, cap, (h->L2 || h->L3) ? kLoadDeep : kLoadL1, h->L2);
     std::vector<tiled::TileItem> items;
     std::vector<int> first;   // first item of every instance
     long long active = 0;
@@ -1192,7 +1192,7 @@ int ens_rechunk(ens_handle* h, int cap) {
         long long a = 0;
         int nr = 0;
         first.push_back((int)items.size());
-        tiled_device_items(tiled_items(h->inst[n]->tiled, chunk, &a), (int)n, recs, items, &nr);
+        tiled_device_items(tiled_items(h->inst[n]->tiled, chunk, h->L2, &a), (int)n, recs, items, &nr);
         recs += nr;
         active += a;
     }

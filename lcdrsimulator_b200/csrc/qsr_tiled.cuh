@@ -677,15 +677,16 @@ struct TiledPlan {
     const float* bufs[2] = {nullptr, nullptr};
 };
 
-// Calls emit(j0, k0, first, last + 1, face) for every work item of chunks of `chunk` planes. In each
-// row band and plane chunk the k tiles start at the first changing cell (rounded down to the tiles'
+// Calls emit(j0, k0, first, last + 1, face, rows) for every work item of chunks of `chunk` planes. `L2` says which kernel
+// takes the list, and with it where its tiles may start (Tile): an ensemble's kernel has the L2 term when any of its
+// droplets has, so that a droplet's own plan.L2 does not decide. In each row band and plane chunk the k tiles start at the first changing cell (rounded down to the tiles'
 // alignment) instead of at multiples of TK, and each tile's plane range is cut to the planes
 // whose changing cells reach it: every changing cell lies in exactly one item, and fewer idle lanes
 // are visited than with a fixed tile grid. `face`: the item has changing cells next to a grid face.
 template <class Emit>
-inline void tiled_each_item(const TiledPlan& plan, int chunk, Emit emit) {
+inline void tiled_each_item(const TiledPlan& plan, int chunk, bool L2, Emit emit) {
     using namespace tiled;
-    const int lo_d = plan.L2 ? 2 : 1;
+    const int lo_d = L2 ? 2 : 1;
     for (const TiledBand& b : plan.bands) {
         for (int ib = b.ib; ib < b.ie; ib += chunk) {
             const int ie = std::min(b.ie, ib + chunk);
@@ -696,7 +697,7 @@ inline void tiled_each_item(const TiledPlan& plan, int chunk, Emit emit) {
                     kmax = std::max(kmax, b.kmax[p - b.ib]);
                 }
             if (kmax < 0) continue;
-            for (int k0 = plan.L2 ? ((kmin - 2) & ~3) + 2 : kmin & ~7; k0 <= kmax; k0 += TK) {
+            for (int k0 = L2 ? ((kmin - 2) & ~3) + 2 : kmin & ~7; k0 <= kmax; k0 += TK) {
                 int first = -1, last = -1;
                 bool face = false;
                 for (int p = ib; p < ie; ++p) {
@@ -724,7 +725,7 @@ inline void tiled_each_item(const TiledPlan& plan, int chunk, Emit emit) {
 // fifth on (longest items first evens them out). An item on a face takes twice as long per plane.
 // Measured against it (64^3, R = 28, L1: 4.8 us at 1 plane, 17.1 at 16; 128^3: 13.9 us at 6, 20.2
 // at 16; 96^3 with L2 and L3: 15.1 us at 4, 24.8 at 16; 256^3: 8 to 16 within 2 %).
-inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Load load) {
+inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Load load, bool L2) {
     static const int sms = [] {
         int dev = 0, n = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -741,7 +742,7 @@ inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Loa
         long long n = 0;
         bool faces = false;
         for (const TiledPlan* p : plans)
-            tiled_each_item(*p, c, [&](int, int, int, int, bool f, int) {
+            tiled_each_item(*p, c, L2, [&](int, int, int, int, bool f, int) {
                 ++n;
                 faces = faces || f;
             });
@@ -763,14 +764,14 @@ inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Loa
 // dispatched in item order, so the short items of the droplet's poles fill the last wave instead of
 // trailing it; among items of one length the plane chunk is slowest (CTAs resident together share
 // halo planes in L2). *active: the cells of the grid inside the items' tiles (read once per step).
-inline std::vector<int4> tiled_items(const TiledPlan& plan, int chunk, long long* active) {
+inline std::vector<int4> tiled_items(const TiledPlan& plan, int chunk, bool L2, long long* active) {
     struct Item {
         int4 t;
         int cost;
     };
     std::vector<Item> items;
     long long act = 0;
-    tiled_each_item(plan, chunk, [&](int j0, int k0, int first, int end, bool face, int rows) {
+    tiled_each_item(plan, chunk, L2, [&](int j0, int k0, int first, int end, bool face, int rows) {
         items.push_back(Item{make_int4(j0, k0, first, end), (end - first) * (face ? 2 : 1)});
         act += (long long)rows * (std::min(plan.Nz, k0 + tiled::TK) - std::max(0, k0)) * (end - first);
     });
@@ -844,9 +845,9 @@ inline int tiled_masks(const TiledPlan& plan, const tiled::TileItem* d_items, in
 
 // Uploads the work list for items of at most `cap` planes (tiled_length).
 inline int tiled_plan_rechunk(TiledPlan& plan, int cap) {
-    const int chunk = tiled_length({&plan}, cap, plan.load);
+    const int chunk = tiled_length({&plan}, cap, plan.load, plan.L2);
     long long active = 0;
-    const std::vector<int4> items = tiled_items(plan, chunk, &active);
+    const std::vector<int4> items = tiled_items(plan, chunk, plan.L2, &active);
     plan.active_cells = active;
     if (plan.items) cudaFree(plan.items);
     if (plan.masks) cudaFree(plan.masks);
