@@ -571,6 +571,7 @@ __global__ void __launch_bounds__(kThreads) k_kzm_obs_final(const KzmPartial* __
 int alloc_or_fail(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();
         set_error(std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
         return LDG_ERR_NOMEM;
     }

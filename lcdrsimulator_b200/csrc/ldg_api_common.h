@@ -13,11 +13,13 @@ namespace ldg {
 void set_error(const std::string& msg);
 void clear_error();
 
-// Checks a CUDA call; on failure records the message and returns LDG_ERR_CUDA from the caller.
+// Checks a CUDA call; on failure records the message and returns LDG_ERR_CUDA from the caller. The runtime's own record
+// of the failure is taken back, or the check of the next launch would report it.
 #define LDG_CUDA(call)                                                                          \
     do {                                                                                        \
         cudaError_t e__ = (call);                                                               \
         if (e__ != cudaSuccess) {                                                               \
+            (void)cudaGetLastError();                                                           \
             ::ldg::set_error(std::string(#call) + ": " + cudaGetErrorString(e__));              \
             return LDG_ERR_CUDA;                                                                \
         }                                                                                       \

@@ -574,6 +574,7 @@ QsrConst make_const(const qsr_handle* h, double T, double S_shell, double dt) {
 int alloc_or_fail(void** ptr, size_t bytes) {
     cudaError_t e = cudaMalloc(ptr, bytes);
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();
         set_error(std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
         return LDG_ERR_NOMEM;
     }
