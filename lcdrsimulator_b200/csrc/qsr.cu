@@ -946,13 +946,23 @@ int qsr_step(qsr_handle* h, int n_steps, const qsr_step_args* a) {
     // The reference falls back to the explicit update when the stabiliser is inactive (QSR.cu:2721).
     const bool imex = a->semi_implicit && a->L_stab > 0.0 && a->jacobi_iters > 0;
     if (imex) {
-        if (!h->rhs) {
-            int rc = alloc_or_fail((void**)&h->rhs, (size_t)h->sc * 5 * sizeof(float));
+        if (!h->sweep.ok) {
+            // all of it or nothing: the next call starts again where this one fails
+            const size_t bytes = (size_t)h->sc * 5 * sizeof(float);
+            float* rhs = nullptr;
+            int rc = alloc_or_fail((void**)&rhs, bytes);
             if (rc) return rc;
-            LDG_CUDA(cudaMemset(h->rhs, 0, (size_t)h->sc * 5 * sizeof(float)));
-            rc = tiled_encode(&h->rhs_map, h->rhs, p.Nx, p.Ny, p.Nz, h->sj, h->si, h->sc, false, false);
+            if (cudaMemset(rhs, 0, bytes) != cudaSuccess) {
+                set_error("qsr_step: clearing the right-hand side failed");
+                rc = LDG_ERR_CUDA;
+            }
+            if (rc == LDG_OK) rc = tiled_encode(&h->rhs_map, rhs, p.Nx, p.Ny, p.Nz, h->sj, h->si, h->sc, false, false);
             if (rc == LDG_OK) rc = tiled_sweep_plan(h->tiled, h->sc, h->sweep);
-            if (rc) return rc;
+            if (rc) {
+                cudaFree(rhs);
+                return rc;
+            }
+            h->rhs = rhs;
         }
         P.alpha = (float)(a->dt * (1.0 / p.gamma) * a->L_stab);
         const double aj = (a->dt / p.gamma) * a->L_stab;  // QSR.cu:2728
@@ -1109,8 +1119,7 @@ int qsr_destroy(qsr_handle* h) {
     cudaFree(h->q[0]); cudaFree(h->q[1]); cudaFree(h->lo[0]); cudaFree(h->lo[1]); cudaFree(h->rhs); cudaFree(h->flags);
     if (!h->stage_shared) cudaFree(h->stage);
     cudaFree(h->opart);
-    h->sweep.err = nullptr;
-    tiled_plan_free(h->sweep);
+    tiled_sweep_free(h->sweep);
     tiled_plan_free(h->tiled);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;

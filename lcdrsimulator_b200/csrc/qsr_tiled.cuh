@@ -975,8 +975,20 @@ inline int tiled_step(const TiledPlan& plan, const float* in, float* out, const 
     return tiled_dispatch<tiled::kStep, false>(plan, which, out, P, L2, L3, noise, st, nullptr, nullptr);
 }
 
+inline void tiled_plan_free(TiledPlan& plan) {
+    if (plan.items) cudaFree(plan.items);
+    if (plan.masks) cudaFree(plan.masks);
+    cudaFree(plan.err);
+    plan = TiledPlan{};
+}
+// A sweep plan shares the step plan's error word.
+inline void tiled_sweep_free(TiledPlan& plan) {
+    plan.err = nullptr;
+    tiled_plan_free(plan);
+}
+
 // The sweeps' plan of the same grid: the step's changing cells, cut to the sweeps' own item length and
-// encoded for one-cell stencils.
+// encoded for one-cell stencils. On failure the plan is empty again.
 inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan& plan) {
     plan = TiledPlan{};
     plan.Nx = step.Nx; plan.Ny = step.Ny; plan.Nz = step.Nz;
@@ -991,6 +1003,7 @@ inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan
         rc = tiled_encode(&plan.tmap[b], step.bufs[b], step.Nx, step.Ny, step.Nz, step.sj, step.si, sc, false);
     }
     plan.ok = rc == LDG_OK;
+    if (rc) tiled_sweep_free(plan);
     return rc;
 }
 
@@ -1013,6 +1026,7 @@ inline int tiled_sweep_t(const TiledPlan& plan, const float* in, float* out, con
 }
 inline int tiled_sweep(const TiledPlan& plan, const float* in, float* out, const CUtensorMap& tm_rhs, const QsrConst& P,
                        bool last, cudaStream_t st) {
+    LDG_REQUIRE(plan.ok, LDG_ERR_STATE, "Jacobi sweep: no plan");
     return last ? tiled_sweep_t<tiled::kSweepLast>(plan, in, out, tm_rhs, P, st)
                 : tiled_sweep_t<tiled::kSweep>(plan, in, out, tm_rhs, P, st);
 }
@@ -1029,13 +1043,6 @@ inline int tiled_check(const TiledPlan& plan, cudaStream_t st) {
         return LDG_ERR_TIMEOUT;
     }
     return LDG_OK;
-}
-
-inline void tiled_plan_free(TiledPlan& plan) {
-    if (plan.items) cudaFree(plan.items);
-    if (plan.masks) cudaFree(plan.masks);
-    cudaFree(plan.err);
-    plan = TiledPlan{};
 }
 
 }  // namespace ldg
