@@ -1188,8 +1188,8 @@ void ens_drop_graph(ens_handle* h) {
     h->graph_steps = 0;
 }
 
-// Work list of all instances split into chunks of `chunk` planes (instance-major, so CTAs that
-// run together share halo planes of one droplet in L2), and the persistent grid size.
+// Work list of all instances for items of at most `cap` planes (instance-major, so CTAs that run together share halo
+// planes of one droplet in L2), and the persistent grid size. On failure the ensemble is as before.
 int ens_rechunk(ens_handle* h, int cap) {
     std::vector<const TiledPlan*> plans;
     for (const qsr_handle* q : h->inst) plans.push_back(&q->tiled);
@@ -1207,23 +1207,6 @@ int ens_rechunk(ens_handle* h, int cap) {
         active += a;
     }
     first.push_back((int)items.size());
-    h->active = active;
-    if (h->d_items) cudaFree(h->d_items);
-    if (h->d_masks) cudaFree(h->d_masks);
-    h->d_items = nullptr;
-    h->d_masks = nullptr;
-    h->n_items = (int)items.size();
-    if (h->n_items > 0) {
-        int rc = alloc_or_fail((void**)&h->d_items, items.size() * sizeof(items[0]));
-        if (!rc) rc = alloc_or_fail((void**)&h->d_masks, (size_t)recs * tiled::MASK_BYTES);
-        if (rc) return rc;
-        LDG_CUDA(cudaMemcpy(h->d_items, items.data(), items.size() * sizeof(items[0]), cudaMemcpyHostToDevice));
-        for (size_t n = 0; n < h->inst.size(); ++n)
-            if ((rc = tiled_masks(h->inst[n]->tiled, h->d_items + first[n], first[n + 1] - first[n], h->L2, h->d_masks)))
-                return rc;
-        LDG_CUDA(cudaStreamSynchronize(nullptr));
-    }
-    h->chunk = chunk;
     const EnsKernel k = ens_kernel(h->L2, h->L3, h->noise);
     LDG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
     int dev = 0, sms = 0, per_sm = 0;
@@ -1231,8 +1214,23 @@ int ens_rechunk(ens_handle* h, int cap) {
     LDG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     LDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tiled::THREADS, h->smem));
     LDG_REQUIRE(per_sm > 0, LDG_ERR_CUDA, "ensemble: step kernel does not fit on an SM");
+    DeviceList now;
+    const int rc = tiled_list_make(items, recs, now, [&](const DeviceList& d) -> int {
+        for (size_t n = 0; n < h->inst.size(); ++n)
+            if (int e = tiled_masks(h->inst[n]->tiled, d.items + first[n], first[n + 1] - first[n], h->L2, d.masks))
+                return e;
+        return LDG_OK;
+    });
+    if (rc) return rc;
+    ens_drop_graph(h);  // it launches the old list
+    DeviceList old{h->d_items, h->d_masks};
+    tiled_list_free(old);
+    h->d_items = now.items;
+    h->d_masks = now.masks;
+    h->n_items = (int)items.size();
+    h->active = active;
+    h->chunk = chunk;
     h->grid = std::max(1, std::min(sms * per_sm, h->n_items));
-    ens_drop_graph(h);
     return LDG_OK;
 }
 
@@ -1647,9 +1645,13 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
     }
     cudaStreamSynchronize(h->stream);
     for (float* b : backup) cudaFree(b);
-    if (rc != LDG_OK) return rc;
+    {
+        const std::string msg = ldg_last_error();
+        const int e = ens_set_step(h, step0);
+        if (rc != LDG_OK) set_error(msg);
+        if (rc != LDG_OK || (rc = e)) return rc;
+    }
     if ((rc = ens_rechunk(h, best))) return rc;
-    if ((rc = ens_set_step(h, step0))) return rc;
     if ((rc = ens_build_graph(h))) return rc;
     if (chosen_chunk) *chosen_chunk = best;
     return LDG_OK;

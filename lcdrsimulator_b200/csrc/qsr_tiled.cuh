@@ -843,29 +843,55 @@ inline int tiled_masks(const TiledPlan& plan, const tiled::TileItem* d_items, in
     return LDG_OK;
 }
 
-// Uploads the work list for items of at most `cap` planes (tiled_length).
+// A work list on the device. It is made in full before it takes the place of another, so that a plan keeps a
+// list that can be launched where making a new one fails.
+struct DeviceList {
+    tiled::TileItem* items = nullptr;
+    tiled::RowMask* masks = nullptr;
+};
+inline void tiled_list_free(DeviceList& d) {
+    cudaFree(d.items);
+    cudaFree(d.masks);
+    d = DeviceList{};
+}
+// Uploads `items` (n_rec planes in all) and forms their masks by `form`, which launches on the default stream.
+template <class Form>
+inline int tiled_list_make(const std::vector<tiled::TileItem>& items, int n_rec, DeviceList& d, Form form) {
+    d = DeviceList{};
+    if (items.empty()) return LDG_OK;
+    auto make = [&]() -> int {
+        LDG_CUDA(cudaMalloc(&d.items, items.size() * sizeof(items[0])));
+        LDG_CUDA(cudaMalloc(&d.masks, (size_t)n_rec * tiled::MASK_BYTES));
+        LDG_CUDA(cudaMemcpy(d.items, items.data(), items.size() * sizeof(items[0]), cudaMemcpyHostToDevice));
+        const int rc = form(d);
+        if (rc) return rc;
+        LDG_CUDA(cudaStreamSynchronize(nullptr));
+        return LDG_OK;
+    };
+    const int rc = make();
+    if (rc) tiled_list_free(d);
+    return rc;
+}
+
+// Uploads the work list for items of at most `cap` planes (tiled_length). On failure the plan is as before.
 inline int tiled_plan_rechunk(TiledPlan& plan, int cap) {
     const int chunk = tiled_length({&plan}, cap, plan.load, plan.L2);
     long long active = 0;
-    const std::vector<int4> items = tiled_items(plan, chunk, plan.L2, &active);
-    plan.active_cells = active;
-    if (plan.items) cudaFree(plan.items);
-    if (plan.masks) cudaFree(plan.masks);
-    plan.items = nullptr;
-    plan.masks = nullptr;
+    std::vector<tiled::TileItem> items;
+    int n_rec = 0;
+    tiled_device_items(tiled_items(plan, chunk, plan.L2, &active), 0, 0, items, &n_rec);
+    DeviceList now;
+    const int rc = tiled_list_make(items, n_rec, now, [&](const DeviceList& d) {
+        return tiled_masks(plan, d.items, (int)items.size(), plan.L2, d.masks);
+    });
+    if (rc) return rc;
+    DeviceList old{plan.items, plan.masks};
+    tiled_list_free(old);
+    plan.items = now.items;
+    plan.masks = now.masks;
     plan.n_items = (int)items.size();
+    plan.active_cells = active;
     plan.chunk = chunk;
-    if (plan.n_items > 0) {
-        std::vector<tiled::TileItem> dev;
-        int n_rec = 0;
-        tiled_device_items(items, 0, 0, dev, &n_rec);
-        LDG_CUDA(cudaMalloc(&plan.items, dev.size() * sizeof(dev[0])));
-        LDG_CUDA(cudaMemcpy(plan.items, dev.data(), dev.size() * sizeof(dev[0]), cudaMemcpyHostToDevice));
-        LDG_CUDA(cudaMalloc(&plan.masks, (size_t)n_rec * tiled::MASK_BYTES));
-        int rc = tiled_masks(plan, plan.items, plan.n_items, plan.L2, plan.masks);
-        if (rc) return rc;
-        LDG_CUDA(cudaStreamSynchronize(nullptr));
-    }
     return LDG_OK;
 }
 

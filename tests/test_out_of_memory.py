@@ -1,10 +1,12 @@
 """Calls after one that ran out of device memory, on a runtime whose n-th allocation fails: the failing call returns an
 error, a later one starts again, and no launch gets memory that is not there."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import fake_gpu
-from lcdrsimulator_b200 import LdgError, QSRSolver
+from lcdrsimulator_b200 import EnsembleSolver, LdgError, QSRSolver
 
 STEP = dict(T=302.0, S_shell=0.6, dt=1.6e-10)
 IMEX = dict(semi_implicit=True, L_stab=6e-12, jacobi_iters=3)
@@ -55,3 +57,47 @@ def test_imex_after_a_failed_set_up(fake, L2):
                     assert g.is_live(x.arg[3]) and g.is_live(x.arg[4])
             assert g.live() == before
         assert failed == 3  # right-hand side, items, masks
+
+
+def test_steps_after_a_failed_autotune(fake):
+    with fake_gpu.use(fake) as g, solver() as s:
+        failed = 0
+        for n in range(1, 40):
+            g.fail_malloc(n)
+            try:
+                s.autotune(trial_steps=1, **STEP)
+            except LdgError:
+                failed += 1
+            g.fail_malloc(0)
+            start = g.count()
+            s.step(1, **STEP)
+            (step,) = g.launches("k_step_tiled", start)
+            assert g.is_live(step.arg[3]) and g.is_live(step.arg[4])
+        assert failed >= 5  # the field's copy and at least two lists
+
+
+def test_ensemble_steps_after_a_failed_autotune(fake):
+    instances = [dict(N=40, droplet_radius_cells=13.0, T_high=310.0, T_low=300.0), dict(N=33)]
+    with fake_gpu.use(fake) as g, EnsembleSolver(instances, L1=6e-12) as s:
+        s.initial_fields()
+        s.step(3)
+        ctl = g.launches("k_step_ensemble")[-1].arg[5]
+        device_step = C.c_longlong.from_address(ctl + 8)  # EnsCtl: next, done, step
+        failed = 0
+        for n in range(1, 40):
+            device_step.value = -1  # as trials that ran would leave it: another step than the host's
+            g.fail_malloc(n)
+            try:
+                s.autotune(trial_steps=1)
+            except LdgError:
+                failed += 1
+            g.fail_malloc(0)
+            assert device_step.value == s.step_index
+            start = g.count()
+            s.step(33)  # one replayed graph and one launch
+            assert s.step_index == 3 + 33 * n
+            launched = g.launches("k_step_ensemble", start)
+            for x in launched:
+                assert g.is_live(x.arg[2]) and g.is_live(x.arg[3]) and g.is_live(x.arg[5])
+            assert launched
+        assert failed >= 6
