@@ -125,7 +125,8 @@ int qsr_observe(qsr_handle* h, const qsr_observe_args* args, qsr_observables* ou
 int qsr_nematic(qsr_handle* h, double* s_n4);
 /* Tile autotuner: times each candidate work-item length (planes per tile item) for trial_steps
  * steps with the given step arguments on the uploaded field and keeps the fastest; the field and
- * the launch count are restored afterwards. No counterpart in the reference (fixed launch shapes). */
+ * the launch count are restored afterwards. chosen_chunk: the length in use (a short work list cuts its
+ * candidates). No counterpart in the reference (fixed launch shapes). */
 int qsr_autotune(qsr_handle* h, const qsr_step_args* args, int trial_steps, int* chosen_chunk);
 int qsr_sync(qsr_handle* h);
 /* The handle's CUDA stream (a cudaStream_t), for timing with events. */
@@ -188,7 +189,7 @@ int ens_observe_all(ens_handle* h, const qsr_observe_args* args, qsr_observables
 long long ens_step_index(const ens_handle* h);
 int ens_geometry(const ens_handle* h, int instance, qsr_geometry_info* out);
 /* Times each candidate work-item length (planes per tile item) for trial_steps steps and keeps
- * the fastest; the fields and the step index are restored afterwards. */
+ * the fastest; the fields and the step index are restored afterwards. chosen_chunk: the length in use. */
 int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk);
 long long ens_cells(const ens_handle* h);           /* total box cells of all instances    */
 long long ens_active_cells(const ens_handle* h);    /* cells in visited tiles, all instances */

@@ -1058,7 +1058,8 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
     LDG_CUDA(cudaMemcpyAsync(backup, h->q[cur0], fbytes, cudaMemcpyDeviceToDevice, h->stream));
     if (h->lo[0]) LDG_CUDA(cudaMemcpyAsync(backup + h->sc * 5, h->lo[cur0], fbytes, cudaMemcpyDeviceToDevice, h->stream));
     const int candidates[] = {8, 12, 16, 24, 32, 48, 64};
-    int best = 0;
+    int best = h->tiled.chunk;  // lengths in use: on a short list several candidates are cut to the same one
+    std::vector<int> tried;
     float best_ms = std::numeric_limits<float>::infinity();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
@@ -1068,7 +1069,9 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
     qsr_step_args t = *a;
     for (int c : candidates) {
         if (rc) break;
-        if ((rc = tiled_plan_rechunk(h->tiled, c))) break;
+        if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{c, false}))) break;
+        if (std::find(tried.begin(), tried.end(), h->tiled.chunk) != tried.end()) continue;
+        tried.push_back(h->tiled.chunk);
         if ((rc = qsr_step(h, 2, &t))) break;
         cudaEventRecord(e0, h->stream);
         if ((rc = qsr_step(h, trial_steps, &t))) break;
@@ -1080,7 +1083,7 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
         }
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) { best_ms = ms; best = c; }
+        if (ms < best_ms) { best_ms = ms; best = h->tiled.chunk; }
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -1095,7 +1098,7 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
     h->launches = launches0;
     if (rc == LDG_OK) rc = tiled_check(h->tiled, h->stream);
     if (rc) return rc;
-    if ((rc = tiled_plan_rechunk(h->tiled, best))) return rc;
+    if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{best, true}))) return rc;
     if (chosen_chunk) *chosen_chunk = best;
     return LDG_OK;
 }
@@ -1188,12 +1191,13 @@ void ens_drop_graph(ens_handle* h) {
     h->graph_steps = 0;
 }
 
-// Work list of all instances for items of at most `cap` planes (instance-major, so CTAs that run together share halo
+// Work list of all instances for items of that length (instance-major, so CTAs that run together share halo
 // planes of one droplet in L2), and the persistent grid size. On failure the ensemble is as before.
-int ens_rechunk(ens_handle* h, int cap) {
+int ens_rechunk(ens_handle* h, ItemLength len) {
     std::vector<const TiledPlan*> plans;
     for (const qsr_handle* q : h->inst) plans.push_back(&q->tiled);
-    const int chunk = tiled_length(plans, cap, (h->L2 || h->L3) ? kLoadDeep : kLoadL1, h->L2);
+    const int chunk = len.exact ? len.planes
+                                : tiled_length(plans, len.planes, (h->L2 || h->L3) ? kLoadDeep : kLoadL1, h->L2);
     std::vector<tiled::TileItem> items;
     std::vector<int> first;   // first item of every instance
     long long active = 0;
@@ -1450,7 +1454,7 @@ int ens_create(const ens_params* params, int n_instances, const ens_instance* in
         ens_destroy(h);
         return LDG_ERR_CUDA;
     }
-    if ((rc = ens_rechunk(h, tiled_default_chunk())) || (rc = ens_set_step(h, 0)) || (rc = ens_build_graph(h))) {
+    if ((rc = ens_rechunk(h, tiled_default_length())) || (rc = ens_set_step(h, 0)) || (rc = ens_build_graph(h))) {
         const std::string msg = ldg_last_error();
         ens_destroy(h);
         set_error(msg);
@@ -1607,7 +1611,8 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
         }
     }
     const int candidates[] = {8, 12, 16, 24, 32, 48, 64};
-    int best = h->chunk;
+    int best = h->chunk;  // lengths in use: on a short list several candidates are cut to the same one
+    std::vector<int> tried;
     float best_ms = std::numeric_limits<float>::infinity();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (rc == LDG_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) {
@@ -1616,7 +1621,9 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
     }
     for (int c : candidates) {
         if (rc != LDG_OK) break;
-        if ((rc = ens_rechunk(h, c))) break;
+        if ((rc = ens_rechunk(h, ItemLength{c, false}))) break;
+        if (std::find(tried.begin(), tried.end(), h->chunk) != tried.end()) continue;
+        tried.push_back(h->chunk);
         for (int s = 0; s < 2 && rc == LDG_OK; ++s) rc = ens_launch(h);
         if (rc) break;
         cudaEventRecord(e0, h->stream);
@@ -1631,7 +1638,7 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
         h->launches += 2 + trial_steps;
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) { best_ms = ms; best = c; }
+        if (ms < best_ms) { best_ms = ms; best = h->chunk; }
         if ((rc = ens_check(h))) break;
     }
     if (e0) cudaEventDestroy(e0);
@@ -1651,7 +1658,7 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
         if (rc != LDG_OK) set_error(msg);
         if (rc != LDG_OK || (rc = e)) return rc;
     }
-    if ((rc = ens_rechunk(h, best))) return rc;
+    if ((rc = ens_rechunk(h, ItemLength{best, true}))) return rc;
     if ((rc = ens_build_graph(h))) return rc;
     if (chosen_chunk) *chosen_chunk = best;
     return LDG_OK;

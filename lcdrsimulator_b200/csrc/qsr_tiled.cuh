@@ -716,9 +716,8 @@ inline void tiled_each_item(const TiledPlan& plan, int chunk, bool L2, Emit emit
     }
 }
 
-// Planes per work item. `cap` is the length asked for (the default, or a length the autotuner
-// tries); a list too short to fill the GPU at that length is cut further, by this estimate of a
-// step's time in microseconds: with n items on `slots` CTA slots,
+// Planes per work item. `cap` is the longest (the default, or a length the autotuner tries); a list too short to fill
+// the GPU at that length is cut further, by this estimate of a step's time in microseconds: with n items on `slots` CTA slots,
 //     waves(n) * (kItem + c * kPlane),
 // kItem the first planes' way to shared memory, kPlane a plane of a CTA while its SM is shared (L1
 // only: 0.95 us alone to 1.75 us with five CTAs; with L2 / L3 2.6 us), waves fractional from the
@@ -733,12 +732,12 @@ inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Loa
             return 148;
         return n;
     }();
-    if (cap < 8) return cap;
     const int per_sm = load == kLoadL1 ? 5 : 4;
     const double kItem = load == kLoadDeep ? 1.3 : 1.0, face_plane = load == kLoadDeep ? 5.3 : 2.0;
     int best = cap;
     double best_t = std::numeric_limits<double>::infinity();
     for (int c : {cap, 6, 4, 3, 2, 1}) {
+        if (c > cap) continue;
         long long n = 0;
         bool faces = false;
         for (const TiledPlan* p : plans)
@@ -787,10 +786,15 @@ inline std::vector<int4> tiled_items(const TiledPlan& plan, int chunk, bool L2, 
     return out;
 }
 
-inline int tiled_default_chunk() {
-    int chunk = tiled::CHUNK;
-    if (const char* e = getenv("LDG_QSR_CHUNK")) chunk = std::min(4096, std::max(1, atoi(e)));
-    return chunk;
+// Length of the work items asked for: at most `planes` (tiled_length), or exactly.
+struct ItemLength {
+    int planes;
+    bool exact;
+};
+// LDG_QSR_CHUNK sets the length exactly.
+inline ItemLength tiled_default_length() {
+    if (const char* e = getenv("LDG_QSR_CHUNK")) return ItemLength{std::min(4096, std::max(1, atoi(e))), true};
+    return ItemLength{tiled::CHUNK, false};
 }
 
 // Tensor map of a field: boxes of a tile with its halo, or of the tile alone.
@@ -873,9 +877,9 @@ inline int tiled_list_make(const std::vector<tiled::TileItem>& items, int n_rec,
     return rc;
 }
 
-// Uploads the work list for items of at most `cap` planes (tiled_length). On failure the plan is as before.
-inline int tiled_plan_rechunk(TiledPlan& plan, int cap) {
-    const int chunk = tiled_length({&plan}, cap, plan.load, plan.L2);
+// Uploads the work list for items of that length. On failure the plan is as before.
+inline int tiled_plan_rechunk(TiledPlan& plan, ItemLength len) {
+    const int chunk = len.exact ? len.planes : tiled_length({&plan}, len.planes, plan.load, plan.L2);
     long long active = 0;
     std::vector<tiled::TileItem> items;
     int n_rec = 0;
@@ -942,7 +946,7 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
         plan.bands.push_back(std::move(b));
     }
     plan.written_cells = written;
-    int rc = tiled_plan_rechunk(plan, tiled_default_chunk());
+    int rc = tiled_plan_rechunk(plan, tiled_default_length());
     if (rc) return rc;
     LDG_CUDA(cudaMalloc(&plan.err, sizeof(int)));
     LDG_CUDA(cudaMemset(plan.err, 0, sizeof(int)));
@@ -1023,7 +1027,7 @@ inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan
     plan.bands = step.bands;
     plan.err = step.err;
     plan.load = kLoadSweep;
-    int rc = tiled_plan_rechunk(plan, tiled_default_chunk());
+    int rc = tiled_plan_rechunk(plan, tiled_default_length());
     for (int b = 0; b < 2 && rc == LDG_OK; ++b) {
         plan.bufs[b] = step.bufs[b];
         rc = tiled_encode(&plan.tmap[b], step.bufs[b], step.Nx, step.Ny, step.Nz, step.sj, step.si, sc, false);

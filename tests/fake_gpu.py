@@ -26,6 +26,7 @@ class Launch:
     def __init__(self, lib, i):
         self.name = lib.fk_name(i).decode()
         self.device = lib.fk_device(i)
+        self.grid = lib.fk_grid(i)  # blocks along x
         self.arg = [lib.fk_arg(i, a) for a in range(10)]
 
 

@@ -16,6 +16,7 @@ namespace {
 struct Launch {
     std::string name;
     int device;
+    unsigned grid;
     uint64_t arg[10];  // the first eight bytes of each argument (where the kernel has as many)
 };
 std::map<const void*, std::string> g_names;
@@ -39,10 +40,11 @@ int args_of(const std::string& n) {
     if (has("k_sweep_tiled") || has("k_step_ensemble")) return 7;
     return 0;
 }
-cudaError_t launch(const void* f, size_t smem, cudaStream_t st, void** args) {
+cudaError_t launch(const void* f, dim3 grid, size_t smem, cudaStream_t st, void** args) {
     Launch l{};
     l.name = g_names.count(f) ? g_names[f] : "?";
     l.device = g_device;
+    l.grid = grid.x;
     for (int i = 0; i < args_of(l.name); ++i) {
         const bool wide = !(l.name.find("k_tile_masks") != std::string::npos && i >= 2 && i <= 7 && i != 6) &&
                           !(l.name.find("k_step_ensemble") != std::string::npos && i == 4);
@@ -71,6 +73,7 @@ int fk_live() { return (int)g_live.size(); }
 int fk_is_live(void* p) { return (int)g_live.count(p); }
 int fk_launches() { return (int)g_launches.size(); }
 const char* fk_name(int i) { return g_launches[i].name.c_str(); }
+unsigned fk_grid(int i) { return g_launches[i].grid; }
 int fk_device(int i) { return g_launches[i].device; }
 uint64_t fk_arg(int i, int a) { return g_launches[i].arg[a]; }
 void fk_elapsed(const float* ms, int n) { g_elapsed.assign(ms, ms + n); }
@@ -97,11 +100,11 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* st)
     *g = c.grid, *b = c.block, *smem = c.smem, *(cudaStream_t*)st = c.stream;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t smem, cudaStream_t st) {
-    return launch(f, smem, st, args);
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3, void** args, size_t smem, cudaStream_t st) {
+    return launch(f, grid, smem, st, args);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
-    return launch(f, c->dynamicSmemBytes, c->stream, args);
+    return launch(f, c->gridDim, c->dynamicSmemBytes, c->stream, args);
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
     if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) g_smem[{f, g_device}] = v;
