@@ -36,6 +36,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdint>
@@ -525,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, ctas<false, false, kMode>())
 
 // Row masks of a work list: one block per item, one warp per tile row, a ballot per plane. `lo` is
 // the distance from a face from which the interior stencils hold (2 with the L2 term, else 1).
-inline __global__ void __launch_bounds__(TK* TJ) k_tile_masks(const TileItem* __restrict__ items,
+static __global__ void __launch_bounds__(TK* TJ) k_tile_masks(const TileItem* __restrict__ items,
                                                               const uint8_t* __restrict__ flags, int Nx, int Ny, int Nz,
                                                               int sj, long long si, int lo, RowMask* __restrict__ masks) {
     const TileItem e = items[blockIdx.x];
@@ -724,7 +725,7 @@ inline void tiled_each_item(const TiledPlan& plan, int chunk, bool L2, Emit emit
 // fifth on (longest items first evens them out). An item on a face takes twice as long per plane.
 // Measured against it (64^3, R = 28, L1: 4.8 us at 1 plane, 17.1 at 16; 128^3: 13.9 us at 6, 20.2
 // at 16; 96^3 with L2 and L3: 15.1 us at 4, 24.8 at 16; 256^3: 8 to 16 within 2 %).
-inline int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Load load, bool L2) {
+static int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Load load, bool L2) {
     static const int sms = [] {
         int dev = 0, n = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -798,7 +799,7 @@ inline ItemLength tiled_default_length() {
 }
 
 // Tensor map of a field: boxes of a tile with its halo, or of the tile alone.
-inline int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int Nz, int sj, long long si, long long sc,
+static int tiled_encode(CUtensorMap* tm, const float* base, int Nx, int Ny, int Nz, int sj, long long si, long long sc,
                         bool L2, bool halo = true) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
@@ -960,17 +961,27 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
     return LDG_OK;
 }
 
+// Raises a kernel's shared-memory limit on the current device. The limit belongs to the device: `done` holds one bit for
+// each device (of the first 64) that has it, so that it is set once on each.
+template <class Kernel>
+inline int tiled_smem_limit(Kernel k, size_t smem, std::atomic<unsigned long long>& done) {
+    int dev = 0;
+    LDG_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (done.load(std::memory_order_relaxed) & bit) return LDG_OK;
+    LDG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    done.fetch_or(bit, std::memory_order_relaxed);
+    return LDG_OK;
+}
+
 template <bool L2, bool L3, bool N, int R, bool K>
-inline int tiled_launch_t(const TiledPlan& plan, int which, float* out, const QsrConst& P, cudaStream_t st,
+static int tiled_launch_t(const TiledPlan& plan, int which, float* out, const QsrConst& P, cudaStream_t st,
                           const float* lo_in, float* lo_out) {
     using namespace tiled;
     const auto k = k_step_tiled<L2, L3, N, R, K>;
     constexpr size_t smem = tile_smem_bytes<L2>();
-    static bool configured = false;
-    if (!configured) {
-        LDG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> devices{0};
+    if (int rc = tiled_smem_limit(k, smem, devices)) return rc;
     if (plan.n_items == 0) return LDG_OK;
     LDG_CUDA(launch_pdl(k, dim3((unsigned)plan.n_items), THREADS, smem, st, plan.tmap[which], plan.bufs[which], out,
                         (const RowMask*)plan.masks, (const TileItem*)plan.items, P, plan.err, lo_in, lo_out));
@@ -1039,15 +1050,12 @@ inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan
 
 // One Jacobi sweep: field `in` (one of the planned buffers) to `out`. tm_rhs: the right-hand side's map.
 template <int kMode>
-inline int tiled_sweep_t(const TiledPlan& plan, const float* in, float* out, const CUtensorMap& tm_rhs, const QsrConst& P,
+static int tiled_sweep_t(const TiledPlan& plan, const float* in, float* out, const CUtensorMap& tm_rhs, const QsrConst& P,
                          cudaStream_t st) {
     using namespace tiled;
     constexpr size_t smem = tile_smem_bytes<false, kMode>();
-    static bool configured = false;
-    if (!configured) {
-        LDG_CUDA(cudaFuncSetAttribute(k_sweep_tiled<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = true;
-    }
+    static std::atomic<unsigned long long> devices{0};
+    if (int rc = tiled_smem_limit(k_sweep_tiled<kMode>, smem, devices)) return rc;
     if (plan.n_items == 0) return LDG_OK;
     LDG_CUDA(launch_pdl(k_sweep_tiled<kMode>, dim3((unsigned)plan.n_items), THREADS, smem, st,
                         plan.tmap[in == plan.bufs[0] ? 0 : 1], tm_rhs, out, (const RowMask*)plan.masks,

@@ -10,7 +10,14 @@ import lcdrsimulator_b200 as ldg
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
+_built = None
+
+
 def build(out_dir):
+    """The library's path; one copy for the process."""
+    global _built
+    if _built is not None:
+        return _built
     from lcdrsimulator_b200.build import LIB, LIB_SOURCES, _host_cxx, _nvcc, build as build_lib
     build_lib()
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
@@ -19,6 +26,7 @@ def build(out_dir):
     subprocess.run([_host_cxx(), "-O1", "-std=c++17", "-shared", "-fPIC", "-I", cuda,
                     os.path.join(HERE, "native", "fake_cudart.cpp"), *objs, "-Wl,-Bsymbolic", "-Wl,--no-undefined",
                     "-lgomp", "-o", so], check=True)
+    _built = so
     return so
 
 
