@@ -680,8 +680,13 @@ int ensure_err() {
     LDG_CUDA(cudaGetDevice(&dev));
     LDG_REQUIRE(dev >= 0 && dev < kMaxDevices, LDG_ERR_ARG, "conv3d: device index out of range");
     if (!g_err_dev[dev]) {
-        LDG_CUDA(cudaMalloc(&g_err_dev[dev], sizeof(int)));
-        LDG_CUDA(cudaMemset(g_err_dev[dev], 0, sizeof(int)));
+        int* word = nullptr;
+        LDG_CUDA(cudaMalloc(&word, sizeof(int)));
+        cudaError_t e = cudaMemset(word, 0, sizeof(int));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // callers' streams do not wait for the default one
+        if (e != cudaSuccess) cudaFree(word);
+        LDG_CUDA(e);
+        g_err_dev[dev] = word;
     }
     g_err = g_err_dev[dev];
     return LDG_OK;
@@ -1023,7 +1028,8 @@ int sg_check(void* stream) {
     LDG_CUDA(cudaMemcpyAsync(&e, g_err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     LDG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     if (e) {
-        LDG_CUDA(cudaMemset(g_err, 0, sizeof(int)));
+        LDG_CUDA(cudaMemsetAsync(g_err, 0, sizeof(int), (cudaStream_t)stream));
+        LDG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
         set_error("conv3d: a bounded pipeline wait gave up");
         return LDG_ERR_TIMEOUT;
     }

@@ -689,10 +689,11 @@ int kzm_create(const kzm_params* params, kzm_handle** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     h->err = reinterpret_cast<int*>(h->part + kBlocks + 1);
     for (int b = 0; b < 2; ++b) {
-        if (e == cudaSuccess) e = cudaMemset(h->alloc[b], 0, fb);
+        // on the handle's stream, as all later work: nothing orders the default stream against it
+        if (e == cudaSuccess) e = cudaMemsetAsync(h->alloc[b], 0, fb, h->stream);
         h->q[b] = h->alloc[b] + P.sy + kPadX;
     }
-    if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->err, 0, sizeof(int), h->stream);
     if (e != cudaSuccess) {
         set_error(std::string("kzm_create: ") + cudaGetErrorString(e));
         kzm_destroy(h);

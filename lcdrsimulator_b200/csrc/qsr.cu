@@ -777,19 +777,26 @@ int qsr_create(const qsr_params* params, qsr_handle** out) {
         return rc;
     }
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMemcpy(h->flags, fl.data(), (size_t)h->sc, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(h->opart, 0, kObsBytes);
-    if (e == cudaSuccess) e = cudaMemset(h->q[0], 0, fbytes);
-    if (e == cudaSuccess) e = cudaMemset(h->q[1], 0, fbytes);
-    if (e == cudaSuccess && h->lo[0]) e = cudaMemset(h->lo[0], 0, fbytes);
-    if (e == cudaSuccess && h->lo[1]) e = cudaMemset(h->lo[1], 0, fbytes);
+    // On the handle's stream, as all later work: it is non-blocking, so nothing would order a default-stream
+    // operation before that work, and a late one would clear what has been written since.
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h->flags, fl.data(), (size_t)h->sc, cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->opart, 0, kObsBytes, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->q[0], 0, fbytes, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->q[1], 0, fbytes, h->stream);
+    if (e == cudaSuccess && h->lo[0]) e = cudaMemsetAsync(h->lo[0], 0, fbytes, h->stream);
+    if (e == cudaSuccess && h->lo[1]) e = cudaMemsetAsync(h->lo[1], 0, fbytes, h->stream);
     if (e != cudaSuccess) {
         set_error(std::string("qsr_create: ") + cudaGetErrorString(e));
         qsr_destroy(h);
         return LDG_ERR_CUDA;
     }
     rc = tiled_plan_build(h->tiled, p.Nx, p.Ny, p.Nz, h->sj, h->si, fl.data(), h->flags, h->q[0], h->q[1],
-                          h->sc, p.L2 != 0.0, p.L3 != 0.0);
+                          h->sc, p.L2 != 0.0, p.L3 != 0.0, h->stream);
+    // an ensemble works on its droplets from a stream of its own
+    if (rc == LDG_OK && cudaStreamSynchronize(h->stream) != cudaSuccess) {
+        set_error("qsr_create: clearing the fields failed");
+        rc = LDG_ERR_CUDA;
+    }
     if (rc != LDG_OK) {
         qsr_destroy(h);
         return rc;
@@ -952,12 +959,12 @@ int qsr_step(qsr_handle* h, int n_steps, const qsr_step_args* a) {
             float* rhs = nullptr;
             int rc = alloc_or_fail((void**)&rhs, bytes);
             if (rc) return rc;
-            if (cudaMemset(rhs, 0, bytes) != cudaSuccess) {
+            if (cudaMemsetAsync(rhs, 0, bytes, h->stream) != cudaSuccess) {
                 set_error("qsr_step: clearing the right-hand side failed");
                 rc = LDG_ERR_CUDA;
             }
             if (rc == LDG_OK) rc = tiled_encode(&h->rhs_map, rhs, p.Nx, p.Ny, p.Nz, h->sj, h->si, h->sc, false, false);
-            if (rc == LDG_OK) rc = tiled_sweep_plan(h->tiled, h->sc, h->sweep);
+            if (rc == LDG_OK) rc = tiled_sweep_plan(h->tiled, h->sc, h->sweep, h->stream);
             if (rc) {
                 cudaFree(rhs);
                 return rc;
@@ -1069,7 +1076,7 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
     qsr_step_args t = *a;
     for (int c : candidates) {
         if (rc) break;
-        if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{c, false}))) break;
+        if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{c, false}, h->stream))) break;
         if (std::find(tried.begin(), tried.end(), h->tiled.chunk) != tried.end()) continue;
         tried.push_back(h->tiled.chunk);
         if ((rc = qsr_step(h, 2, &t))) break;
@@ -1098,7 +1105,7 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
     h->launches = launches0;
     if (rc == LDG_OK) rc = tiled_check(h->tiled, h->stream);
     if (rc) return rc;
-    if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{best, true}))) return rc;
+    if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{best, true}, h->stream))) return rc;
     if (chosen_chunk) *chosen_chunk = best;
     return LDG_OK;
 }
@@ -1219,9 +1226,10 @@ int ens_rechunk(ens_handle* h, ItemLength len) {
     LDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tiled::THREADS, h->smem));
     LDG_REQUIRE(per_sm > 0, LDG_ERR_CUDA, "ensemble: step kernel does not fit on an SM");
     DeviceList now;
-    const int rc = tiled_list_make(items, recs, now, [&](const DeviceList& d) -> int {
+    const int rc = tiled_list_make(items, recs, h->stream, now, [&](const DeviceList& d) -> int {
         for (size_t n = 0; n < h->inst.size(); ++n)
-            if (int e = tiled_masks(h->inst[n]->tiled, d.items + first[n], first[n + 1] - first[n], h->L2, d.masks))
+            if (int e = tiled_masks(h->inst[n]->tiled, d.items + first[n], first[n + 1] - first[n], h->L2, d.masks,
+                                    h->stream))
                 return e;
         return LDG_OK;
     });
@@ -1445,10 +1453,12 @@ int ens_create(const ens_params* params, int n_instances, const ens_instance* in
         ens_destroy(h);
         return rc;
     }
-    e = cudaMemcpy(h->d_tms, tms.data(), tms.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(h->d_tms, tms.data(), tms.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpy(h->d_inst, h->host_inst.data(), h->host_inst.size() * sizeof(EnsInstDev), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(h->d_err, 0, sizeof(int));
+        e = cudaMemcpyAsync(h->d_inst, h->host_inst.data(), h->host_inst.size() * sizeof(EnsInstDev),
+                            cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) {
         set_error(std::string("ens_create: ") + cudaGetErrorString(e));
         ens_destroy(h);

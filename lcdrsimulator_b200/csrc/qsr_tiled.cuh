@@ -840,9 +840,9 @@ inline void tiled_device_items(const std::vector<int4>& list, int inst, int rec0
     *n_rec = rec - rec0;
 }
 inline int tiled_masks(const TiledPlan& plan, const tiled::TileItem* d_items, int n_items, bool L2,
-                       tiled::RowMask* d_masks) {
+                       tiled::RowMask* d_masks, cudaStream_t st) {
     if (n_items == 0) return LDG_OK;
-    tiled::k_tile_masks<<<n_items, tiled::TK * tiled::TJ>>>(d_items, plan.flags, plan.Nx, plan.Ny, plan.Nz, plan.sj,
+    tiled::k_tile_masks<<<n_items, tiled::TK * tiled::TJ, 0, st>>>(d_items, plan.flags, plan.Nx, plan.Ny, plan.Nz, plan.sj,
                                                             plan.si, L2 ? 2 : 1, d_masks);
     LDG_LAUNCHED("k_tile_masks");
     return LDG_OK;
@@ -859,19 +859,19 @@ inline void tiled_list_free(DeviceList& d) {
     cudaFree(d.masks);
     d = DeviceList{};
 }
-// Uploads `items` (n_rec planes in all) and forms their masks by `form`, which launches on the default stream.
+// Uploads `items` (n_rec planes in all) and forms their masks by `form`, both on `st` and complete on return.
 template <class Form>
-inline int tiled_list_make(const std::vector<tiled::TileItem>& items, int n_rec, DeviceList& d, Form form) {
+inline int tiled_list_make(const std::vector<tiled::TileItem>& items, int n_rec, cudaStream_t st, DeviceList& d,
+                           Form form) {
     d = DeviceList{};
     if (items.empty()) return LDG_OK;
     auto make = [&]() -> int {
         LDG_CUDA(cudaMalloc(&d.items, items.size() * sizeof(items[0])));
         LDG_CUDA(cudaMalloc(&d.masks, (size_t)n_rec * tiled::MASK_BYTES));
-        LDG_CUDA(cudaMemcpy(d.items, items.data(), items.size() * sizeof(items[0]), cudaMemcpyHostToDevice));
+        LDG_CUDA(cudaMemcpyAsync(d.items, items.data(), items.size() * sizeof(items[0]), cudaMemcpyHostToDevice, st));
         const int rc = form(d);
-        if (rc) return rc;
-        LDG_CUDA(cudaStreamSynchronize(nullptr));
-        return LDG_OK;
+        LDG_CUDA(cudaStreamSynchronize(st));
+        return rc;
     };
     const int rc = make();
     if (rc) tiled_list_free(d);
@@ -879,15 +879,15 @@ inline int tiled_list_make(const std::vector<tiled::TileItem>& items, int n_rec,
 }
 
 // Uploads the work list for items of that length. On failure the plan is as before.
-inline int tiled_plan_rechunk(TiledPlan& plan, ItemLength len) {
+inline int tiled_plan_rechunk(TiledPlan& plan, ItemLength len, cudaStream_t st) {
     const int chunk = len.exact ? len.planes : tiled_length({&plan}, len.planes, plan.load, plan.L2);
     long long active = 0;
     std::vector<tiled::TileItem> items;
     int n_rec = 0;
     tiled_device_items(tiled_items(plan, chunk, plan.L2, &active), 0, 0, items, &n_rec);
     DeviceList now;
-    const int rc = tiled_list_make(items, n_rec, now, [&](const DeviceList& d) {
-        return tiled_masks(plan, d.items, (int)items.size(), plan.L2, d.masks);
+    const int rc = tiled_list_make(items, n_rec, st, now, [&](const DeviceList& d) {
+        return tiled_masks(plan, d.items, (int)items.size(), plan.L2, d.masks, st);
     });
     if (rc) return rc;
     DeviceList old{plan.items, plan.masks};
@@ -900,9 +900,10 @@ inline int tiled_plan_rechunk(TiledPlan& plan, ItemLength len) {
     return LDG_OK;
 }
 
-// Builds the work list from the host classification and encodes the two tensor maps.
+// Builds the work list from the host classification and encodes the two tensor maps. The device's part runs on `st`, which
+// the caller's later work uses or waits for (a default-stream operation has no order against a non-blocking stream).
 inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, long long si, const uint8_t* fl,
-                            const uint8_t* d_flags, const float* buf0, const float* buf1, long long sc, bool L2, bool L3) {
+                            const uint8_t* d_flags, const float* buf0, const float* buf1, long long sc, bool L2, bool L3, cudaStream_t st) {
     using namespace tiled;
     plan = TiledPlan{};
     plan.load = (L2 || L3) ? kLoadDeep : kLoadL1;
@@ -947,10 +948,10 @@ inline int tiled_plan_build(TiledPlan& plan, int Nx, int Ny, int Nz, int sj, lon
         plan.bands.push_back(std::move(b));
     }
     plan.written_cells = written;
-    int rc = tiled_plan_rechunk(plan, tiled_default_length());
+    int rc = tiled_plan_rechunk(plan, tiled_default_length(), st);
     if (rc) return rc;
     LDG_CUDA(cudaMalloc(&plan.err, sizeof(int)));
-    LDG_CUDA(cudaMemset(plan.err, 0, sizeof(int)));
+    LDG_CUDA(cudaMemsetAsync(plan.err, 0, sizeof(int), st));
     rc = tiled_encode(&plan.tmap[0], buf0, Nx, Ny, Nz, sj, si, sc, L2);
     if (rc) return rc;
     rc = tiled_encode(&plan.tmap[1], buf1, Nx, Ny, Nz, sj, si, sc, L2);
@@ -1030,7 +1031,7 @@ inline void tiled_sweep_free(TiledPlan& plan) {
 
 // The sweeps' plan of the same grid: the step's changing cells, cut to the sweeps' own item length and
 // encoded for one-cell stencils. On failure the plan is empty again.
-inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan& plan) {
+inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan& plan, cudaStream_t st) {
     plan = TiledPlan{};
     plan.Nx = step.Nx; plan.Ny = step.Ny; plan.Nz = step.Nz;
     plan.sj = step.sj; plan.si = step.si;
@@ -1038,7 +1039,7 @@ inline int tiled_sweep_plan(const TiledPlan& step, const long long sc, TiledPlan
     plan.bands = step.bands;
     plan.err = step.err;
     plan.load = kLoadSweep;
-    int rc = tiled_plan_rechunk(plan, tiled_default_length());
+    int rc = tiled_plan_rechunk(plan, tiled_default_length(), st);
     for (int b = 0; b < 2 && rc == LDG_OK; ++b) {
         plan.bufs[b] = step.bufs[b];
         rc = tiled_encode(&plan.tmap[b], step.bufs[b], step.Nx, step.Ny, step.Nz, step.sj, step.si, sc, false);

@@ -34,7 +34,7 @@ def step_list(g, s):
     return longest(x.arg[4], x.grid)
 
 
-# every candidate is cut to one length; some are; none
+# lists of one and of several lengths
 @pytest.mark.parametrize("N,R", [(40, 14.0), (128, 58.0), (200, 98.0)])
 def test_autotune_returns_the_length_in_use(fake, N, R):
     with fake_gpu.use(fake) as g, solver(N, R) as s:
