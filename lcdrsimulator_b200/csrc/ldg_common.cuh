@@ -789,7 +789,9 @@ __device__ __forceinline__ Nematic nematic64(const double q[5], double iso_cut, 
 // Programmatic dependent launch (launch_pdl): a kernel is put on the SMs while its predecessor in the
 // stream drains, sets itself up, and waits in pdl_wait until the predecessor's writes are complete;
 // pdl_trigger then lets its own successor be put in place. Every access to data that an earlier
-// kernel writes comes after pdl_wait.
+// kernel writes comes after pdl_wait, and is an ordinary load: the data changes during the kernel's
+// lifetime, so neither __ldg nor a const __restrict__ pointer may be used for it (their read-only loads
+// may be taken before the wait).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -188,13 +188,13 @@ struct SmemQRt {
     }
 };
 // Face cells without the L2 term read the field itself: the shifted second difference of a cell on
-// a face reaches two cells in, one more than the one-cell halo holds.
+// a face reaches two cells in, one more than the one-cell halo holds. Plain loads (pdl_wait).
 struct GlobQRt {
     const float* q;  // component 0 of the cell
     long long sc, si;
     int sj;
     __device__ __forceinline__ float operator()(int c, int di, int dj, int dk) const {
-        return __ldg(q + c * sc + di * si + (long long)dj * sj + dk);
+        return q[c * sc + di * si + (long long)dj * sj + dk];
     }
 };
 
@@ -264,12 +264,11 @@ __device__ __forceinline__ unsigned arrive_freed(unsigned* ctr) {
 // one is a j-neighbour of the other). kComp: compensated storage (explicit steps only): the low words
 // of the input cells are read from lo_in and the new low words written to lo_out.
 template <bool kL2, bool kL3, bool kNoise, int kMode, bool kComp = false>
-__device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float* __restrict__ qin,
+__device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float* qin,
                                              float* __restrict__ qout, const RowMask* __restrict__ masks, int j0,
                                              int k0, int ib, int ie, const QsrConst& P, const TileSmem& S,
                                              uint32_t& phase, int* __restrict__ err,
-                                             const float* __restrict__ lo_in = nullptr,
-                                             float* __restrict__ lo_out = nullptr,
+                                             const float* lo_in = nullptr, float* __restrict__ lo_out = nullptr,
                                              const CUtensorMap* tm_rhs = nullptr) {
     using G = Tile<kL2, kMode>;
     constexpr int H = G::H, SLOT = G::SLOT, NQ = G::NQ, RW = G::RW;
@@ -415,7 +414,7 @@ __device__ __forceinline__ bool process_tile(const CUtensorMap* tm, const float*
                     float lo[5], cr[5], mr[5];
 #pragma unroll
                     for (int m = 0; m < 5; ++m) {
-                        lo[m] = __ldg(lo_in + m * P.sc + ir);
+                        lo[m] = lo_in[m * P.sc + ir];
                         cr[m] = r ? c[m].v.y : c[m].v.x;
                         mr[m] = r ? mu[m].v.y : mu[m].v.x;
                     }
@@ -485,9 +484,9 @@ __device__ __forceinline__ void tile_smem_init(const TileSmem& S) {
 // Single grid: one work item per CTA.
 template <bool kL2, bool kL3, bool kNoise, int kMode, bool kComp = false>
 __global__ void __launch_bounds__(THREADS, ctas<kL2, kL3>())
-    k_step_tiled(const __grid_constant__ CUtensorMap tm_in, const float* __restrict__ qin, float* __restrict__ qout,
+    k_step_tiled(const __grid_constant__ CUtensorMap tm_in, const float* qin, float* __restrict__ qout,
                  const RowMask* __restrict__ masks, const TileItem* __restrict__ items, QsrConst P,
-                 int* __restrict__ err, const float* __restrict__ lo_in, float* __restrict__ lo_out) {
+                 int* __restrict__ err, const float* lo_in, float* __restrict__ lo_out) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const TileSmem S = tile_smem<kL2>(smem_raw);
     tile_smem_init<kL2>(S);
