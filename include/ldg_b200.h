@@ -123,10 +123,10 @@ int qsr_observe(qsr_handle* h, const qsr_observe_args* args, qsr_observables* ou
 /* Replaces computeNematicFieldKernel + D2H (QSR.cu:1017-1025, 2816-2821): 4 doubles per
  * cell (S, nx, ny, nz) in the host cell order. */
 int qsr_nematic(qsr_handle* h, double* s_n4);
-/* Tile autotuner: times each candidate work-item length (planes per tile item) for trial_steps
- * steps with the given step arguments on the uploaded field and keeps the fastest; the field and
- * the launch count are restored afterwards. chosen_chunk: the length in use (a short work list cuts its
- * candidates). No counterpart in the reference (fixed launch shapes). */
+/* Tile autotuner: times each candidate for the longest work item (planes per tile item; a work list too short
+ * for it is cut further) for trial_steps steps with the given step arguments on the uploaded field and keeps
+ * the fastest, which chosen_chunk receives; candidates that give the same list are timed once. The field and
+ * the launch count are restored afterwards. No counterpart in the reference (fixed launch shapes). */
 int qsr_autotune(qsr_handle* h, const qsr_step_args* args, int trial_steps, int* chosen_chunk);
 int qsr_sync(qsr_handle* h);
 /* The handle's CUDA stream (a cudaStream_t), for timing with events. */
@@ -188,8 +188,7 @@ int ens_observe(ens_handle* h, int instance, const qsr_observe_args* args, qsr_o
 int ens_observe_all(ens_handle* h, const qsr_observe_args* args, qsr_observables* out);
 long long ens_step_index(const ens_handle* h);
 int ens_geometry(const ens_handle* h, int instance, qsr_geometry_info* out);
-/* Times each candidate work-item length (planes per tile item) for trial_steps steps and keeps
- * the fastest; the fields and the step index are restored afterwards. chosen_chunk: the length in use. */
+/* As qsr_autotune, for all droplets; the fields and the step index are restored afterwards. */
 int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk);
 long long ens_cells(const ens_handle* h);           /* total box cells of all instances    */
 long long ens_active_cells(const ens_handle* h);    /* cells in visited tiles, all instances */

@@ -263,7 +263,7 @@ class QSRSolver:
         return o.as_dict()
 
     def autotune(self, T, S_shell, dt, trial_steps=10, **kw) -> int:
-        """Picks the tiled kernel's work-item length for these step arguments (field restored)."""
+        """Picks the longest work item of the tiled kernel for these step arguments (field restored)."""
         a = self.step_args(T, S_shell, dt, **kw)
         c = C.c_int(0)
         _check(load_library().qsr_autotune(self._h, C.byref(a), int(trial_steps), C.byref(c)), "qsr_autotune")

@@ -1065,8 +1065,8 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
     LDG_CUDA(cudaMemcpyAsync(backup, h->q[cur0], fbytes, cudaMemcpyDeviceToDevice, h->stream));
     if (h->lo[0]) LDG_CUDA(cudaMemcpyAsync(backup + h->sc * 5, h->lo[cur0], fbytes, cudaMemcpyDeviceToDevice, h->stream));
     const int candidates[] = {8, 12, 16, 24, 32, 48, 64};
-    int best = h->tiled.chunk;  // lengths in use: on a short list several candidates are cut to the same one
-    std::vector<int> tried;
+    int best = candidates[0];
+    std::vector<int> tried;  // lengths in use: on a short list several candidates are cut to the same one
     float best_ms = std::numeric_limits<float>::infinity();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
@@ -1090,7 +1090,7 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
         }
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) { best_ms = ms; best = h->tiled.chunk; }
+        if (ms < best_ms) { best_ms = ms; best = c; }
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -1105,7 +1105,7 @@ int qsr_autotune(qsr_handle* h, const qsr_step_args* a, int trial_steps, int* ch
     h->launches = launches0;
     if (rc == LDG_OK) rc = tiled_check(h->tiled, h->stream);
     if (rc) return rc;
-    if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{best, true}, h->stream))) return rc;
+    if ((rc = tiled_plan_rechunk(h->tiled, ItemLength{best, false}, h->stream))) return rc;
     if (chosen_chunk) *chosen_chunk = best;
     return LDG_OK;
 }
@@ -1621,8 +1621,8 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
         }
     }
     const int candidates[] = {8, 12, 16, 24, 32, 48, 64};
-    int best = h->chunk;  // lengths in use: on a short list several candidates are cut to the same one
-    std::vector<int> tried;
+    int best = candidates[0];
+    std::vector<int> tried;  // lengths in use: on a short list several candidates are cut to the same one
     float best_ms = std::numeric_limits<float>::infinity();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (rc == LDG_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) {
@@ -1648,7 +1648,7 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
         h->launches += 2 + trial_steps;
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_ms) { best_ms = ms; best = h->chunk; }
+        if (ms < best_ms) { best_ms = ms; best = c; }
         if ((rc = ens_check(h))) break;
     }
     if (e0) cudaEventDestroy(e0);
@@ -1668,7 +1668,7 @@ int ens_autotune(ens_handle* h, int trial_steps, int* chosen_chunk) {
         if (rc != LDG_OK) set_error(msg);
         if (rc != LDG_OK || (rc = e)) return rc;
     }
-    if ((rc = ens_rechunk(h, ItemLength{best, true}))) return rc;
+    if ((rc = ens_rechunk(h, ItemLength{best, false}))) return rc;
     if ((rc = ens_build_graph(h))) return rc;
     if (chosen_chunk) *chosen_chunk = best;
     return LDG_OK;

@@ -1,5 +1,5 @@
-"""Work-item lengths: what autotuning returns is the length in use, a length is timed once, and LDG_QSR_CHUNK is that
-length on lists of any size (CPU, on a runtime that records launches)."""
+"""Work-item lengths: autotuning keeps the list of its fastest trial, times a list once and returns the longest item that it
+allowed, and LDG_QSR_CHUNK is the length on lists of any size (CPU, on a runtime that records launches)."""
 import ctypes as C
 
 import numpy as np
@@ -34,25 +34,37 @@ def step_list(g, s):
     return longest(x.arg[4], x.grid)
 
 
+CANDIDATES = (8, 12, 16, 24, 32, 48, 64)
+
+
 # lists of one and of several lengths
 @pytest.mark.parametrize("N,R", [(40, 14.0), (128, 58.0), (200, 98.0)])
-def test_autotune_returns_the_length_in_use(fake, N, R):
+@pytest.mark.parametrize("ms", [[5.0, 4.0, 3.0, 3.5, 6.0, 6.0, 6.0], [1.0, 4.0, 4.0, 4.0, 4.0, 4.0, 4.0]])
+def test_autotune_keeps_the_fastest_list(fake, N, R, ms):
     with fake_gpu.use(fake) as g, solver(N, R) as s:
-        g.elapsed([5.0, 4.0, 3.0, 3.5, 6.0, 6.0, 6.0])
+        g.elapsed(ms)
         start = g.count()
         got = s.autotune(trial_steps=1, **STEP)
-        trials = g.launches("k_step_tiled", start)
-        assert got == step_list(g, s)
-        assert len(trials) % 3 == 0 and len(trials) // 3 == len({x.grid for x in trials})  # one trial per list
+        lists = [x.grid for x in g.launches("k_step_tiled", start)][::3]  # two steps before each timed one
+        assert len(lists) == len(set(lists))  # one trial per list
+        start = g.count()
+        longest_item = step_list(g, s)
+        (step,) = g.launches("k_step_tiled", start)
+        assert step.grid == lists[int(np.argmin(ms[:len(lists)]))]
+        assert got in CANDIDATES and longest_item <= got
 
 
-def test_ensemble_autotune_returns_the_length_in_use(fake):
+def test_ensemble_autotune_times_a_list_once(fake):
     with fake_gpu.use(fake) as g, EnsembleSolver([dict(N=40, droplet_radius_cells=13.0), dict(N=33)], L1=6e-12) as s:
         s.initial_fields()
+        start = g.count()
         got = s.autotune(trial_steps=1)
+        lists = [x.arg[4] for x in g.launches("k_step_ensemble", start)]
+        trials = lists[:len(lists) - 32:3]  # the captured graph of 32 steps comes last
+        assert len(trials) == len(set(trials))
         s.step(1)
         x = g.launches("k_step_ensemble")[-1]
-        assert got == longest(x.arg[2], x.arg[4])
+        assert got in CANDIDATES and longest(x.arg[2], x.arg[4]) <= got
 
 
 @pytest.mark.parametrize("planes", [1, 5, 8, 16, 20])
