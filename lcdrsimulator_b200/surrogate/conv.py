@@ -122,14 +122,16 @@ def conv3d_bwd(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor | None, gy: tor
     N, D, H, W, Ci = x.shape
     Co = w.shape[0]
     _require(x, torch.bfloat16, (N, D, H, W, Ci), "x")
-    _require(w, torch.bfloat16, (Co, 27, Ci), "w")
+    if x_grad:  # nothing else reads the weights
+        _require(w, torch.bfloat16, (Co, 27, Ci), "w")
     # without a mask a BF16 gradient is read by the convolutions as it is
     gy = gy.contiguous() if y is None and gy.dtype == torch.bfloat16 else _plain(gy)
     if gy.dtype not in (torch.bfloat16, torch.float32):
         raise ValueError(f"gy: expected BF16 or FP32, got {gy.dtype}")
     _require(gy, gy.dtype, (N, D, H, W, Co), "gy")
     if y is not None:
-        y = _plain(y)  # a saved-tensor hook may hand back another layout
+        # a saved-tensor hook may hand back another layout or type; only the signs count
+        y = _plain(y if y.dtype == gy.dtype else (y > 0).to(gy.dtype))
         _require(y, gy.dtype, (N, D, H, W, Co), "y")
     dev = x.device
     dx = torch.empty(x.shape, dtype=torch.bfloat16, device=dev) if x_grad else None
