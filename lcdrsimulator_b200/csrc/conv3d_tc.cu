@@ -986,6 +986,7 @@ int sg_conv3d_act_grad(long long nvox, int C, const void* y, const void* gy, int
 // Bytes of scratch that sg_conv3d_bwd needs, 256-byte aligned parts: g, the flipped weights, partial sums.
 static size_t bwd_part(size_t b) { return (b + 255) & ~(size_t)255; }
 long long sg_conv3d_bwd_ws(const sg_conv_shape* s) {
+    if (!s || s->N < 1 || s->D < 1 || s->H < 1 || s->W < 1 || s->Ci < 1 || s->Co < 1) return 0;
     const long long nvox = (long long)s->N * s->D * s->H * s->W;
     return (long long)(bwd_part((size_t)nvox * s->Co * 2) + bwd_part((size_t)s->Ci * 27 * s->Co * 2)) +
            sg_conv3d_act_grad_ws(nvox, s->Co) * (long long)sizeof(double);
