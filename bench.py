@@ -441,7 +441,12 @@ def run_reference_arm(args, w):
     if rank != 0:
         return 0
     from oracle.oracle import RefCPU
-    ref = RefCPU()
+    try:
+        ref = RefCPU()
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's QSR.cpp is not built here (its sources "
+                          f"are absent): no {os.path.relpath(str(e), ROOT)}"}), flush=True)
+        return 0
     op, q, dt, S_shell = _reference_problem(w, args.ref_grid)
     cells = op.Nx * op.Ny * op.Nz
     if args.warmup > 0:
