@@ -137,9 +137,9 @@ __global__ void __launch_bounds__(256) k_kzm_step(const float* __restrict__ q, f
 // plane is read for its neighbours at its own step only, can be refilled right after it, and costs
 // eight shared loads per component and pair instead of fourteen. The warps march independently: the
 // last one done with a plane issues the load that reuses its slot.
-// With noise it is bound by issue slots (240 instructions a site, 102 of them the draw, at 72 % issue
-// efficiency); without, by HBM (256^3: 5.0 TB/s of the 6.1 that the same loads and stores reach without
-// arithmetic).
+// With noise it is bound by issue slots (234 instructions a site, 101 of them the draw, at 70 % issue
+// efficiency); without, by HBM and the wait for planes (256^3: 4.4 TB/s of the 6.1 that the same loads and stores
+// reach without arithmetic).
 constexpr int KTX = 32, KTY = 8;
 constexpr int KTHREADS = KTX * KTY / 2, KWARPS = KTHREADS / 32;
 constexpr int KROW = KTX + 2 * kHaloX;        // floats per ring row: x0 - 4 .. x0 + 35
@@ -603,9 +603,11 @@ int kzm_encode(CUtensorMap* tm, const float* alloc, const KzmConst& P) {
 
 // Planes per CTA: the chunk length with the least estimated time. A CTA takes 0.95 us and 0.57 + 0.265 m
 // us per plane (with noise) where m CTAs share its SM; full waves of KCTAS per SM, then the rest.
-// Measured (us per step with noise): 64^3 6.8 / 6.3 / 8.6 / 28.9 at 2 / 4 / 8 / 32 planes (one chunk
-// length of 32 for every grid before: 29.7), 128^3 30.5 / 28.3 / 28.5 / 34.1 at 2 / 4 / 8 / 16 (40.5),
-// 256^3 212 / 190 / 182 / 181 (203); without noise 164 / 142 / 136 / 139 (160).
+// Measured, us a step with chunks of 2 / 4 / 8 / 16 / 32 planes and of the length chosen (32 planes in every grid before,
+// with the kernel of then: 28.7, 40, 208 with noise, 20.5, 29.5, 176 without):
+//     64^3  with noise   7.1   6.5   9.2  16.4  30.9   7.1     without   5.7   5.0   7.0  12.2  22.5   5.7
+//     128^3             30.9  28.9  29.1  35.5  37.4  28.2              27.1  24.2  24.6  29.3  26.4  25.0
+//     256^3            214   192   180   182   188   187               179   156   146   146   151   152
 // LDG_KZM_PLANES forces a length.
 int kzm_planes(const KzmConst& P) {
     const int lo = (P.Nz + 65534) / 65535;  // the launch grid's z extent is limited

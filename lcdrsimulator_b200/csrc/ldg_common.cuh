@@ -24,7 +24,7 @@ enum : uint8_t {
 // FP32 SoA: component c of cell (i, j, k) lives at q[c*sc + i*si + j*sj + k].
 struct QsrConst {
     int Nx, Ny, Nz;
-    int sj;          // row pitch (>= Nz, multiple of 4)
+    int sj;          // row pitch (>= Nz, multiple of 8)
     long long si;    // plane pitch = Ny*sj
     long long sc;    // component pitch = Nx*si
     float ix2, iy2, iz2;        // 1/d^2
@@ -380,8 +380,8 @@ __device__ __forceinline__ float vset<float>(float a) { return a; }
 // written (tr(Q^2 - I tr Q^2 / 3) = 0 and Qzz = -(Qxx + Qyy)), so the zz entry is never formed;
 // with Qzz eliminated the off-diagonal entries of Q^2 are two products each. The diagonal entries of
 // Q^2 - I tr Q^2 / 3 are formed from their own products, (q2xx - 2 u) / 3 and (q2yy - 2 w) / 3, before they meet
-// cQ2: taking q2xx and tr Q^2 / 3 to cQ2 apart needs four operations less (4 of 371 instructions a cell) and rounded
-// 1.25 to 1.3 times as much as the six-entry form above at S = 0.5; this one rounds 0.78 times as much.
+// cQ2: taking q2xx and tr Q^2 / 3 to cQ2 apart needs four operations less and rounded 1.25 to 1.3 times as much as
+// the six-entry form above at S = 0.5; this one rounds 0.78 times as much.
 // Coefficients of the bulk field as values of F: a packed operation takes a pair in registers or
 // in the kernel's parameters, and a scalar would have to be copied into both halves at every use.
 template <class F>
@@ -427,7 +427,8 @@ struct Sten {
 //  * the centre terms -2 Q of the L1 and L3 sums are collected per entry;
 //  * the many small terms of L2, M_ab and D.grad are summed apart and meet the bulk and L1 terms once: added one by
 //    one, and with the centre terms of the wide differences collected too, they rounded 1.1 to 1.3 times as much
-//    as the term-by-term form (chem_potential) does, this way 0.75 to 0.99 times.
+//    as the term-by-term form (chem_potential) does, this way 0.75 to 0.99 times, for 1 to 2 % of a step with all
+//    terms (256^3, R = 120: 144.9 -> 146.6 us).
 // The L2 term d_a D_b is sum_k S_ak(Q_kb) / (4 da dk): the wide second difference for k = a, four
 // corners for k != a. With kFace the stencils hold the reference's one-sided forms (QSR.cu:245-371)
 // in the same undivided units and l3on is 0 for a cell on a face (no L3 term there, QSR.cu:474-621).

@@ -18,13 +18,14 @@
 // no changing cell are never visited (host-built work list). The same per-tile routine drives a
 // persistent, work-stealing ensemble kernel over many droplets.
 //
-// What bounds it. With L2 and L3 the issue slots and the FMA pipe: 418 instructions per visited
-// cell at 65 % issue efficiency, 184 of them on the FMA pipe. L1 only: the loads and stores (a 256^3
-// step with its arithmetic left out takes 87 of 89 us). A grid of few tiles: the serial march of one
-// item (about 1 us per plane), hence tiled_length, and the launch gap, hence the programmatic
-// dependent launches (2 us a step). Per step, one work-list length for all before -> now, 256^3 with
-// all terms 168 -> 142 us, 64^3 L1 only 16.4 -> 4.7 us, 32^3 15.3 -> 4.1 us, 101 x 90 x 117 touching
-// its faces with all terms 68 -> 21 us.
+// What bounds it. With L2 and L3 the issue slots: 372 instructions per visited cell at 61 % issue
+// efficiency, 170 of them on the FMA pipe, which is busy 48 % of the time. L1 only: the loads and stores (182
+// instructions a cell at 55 %, the warps wait for their planes; a 256^3 step with its arithmetic left out
+// took 87 of 89 us). A grid of few tiles: the serial march of one item (about 1 us per plane), hence
+// tiled_length, and the launch gap, hence the programmatic dependent launches (2 us a step). Per step, one
+// work-list length for all before -> now: 256^3, R = 120, with all terms 168 -> 147 us, L1 only (R = 115)
+// 101 -> 76 us, 64^3 16.4 -> 5.1 us, 32^3 14.4 -> 3.0 us, 101 x 90 x 117 touching its faces with all terms
+// 61.5 -> 17.5 us, with compensated storage 67.6 -> 21.3 us.
 //
 // mbarrier waits are bounded: on timeout the kernel records LDG_ERR_TIMEOUT in a device
 // word, waits (bounded) for its own TMA loads and returns.
@@ -722,8 +723,12 @@ inline void tiled_each_item(const TiledPlan& plan, int chunk, bool L2, Emit emit
 // kItem the first planes' way to shared memory, kPlane a plane of a CTA while its SM is shared (L1
 // only: 0.95 us alone to 1.75 us with five CTAs; with L2 / L3 2.6 us), waves fractional from the
 // fifth on (longest items first evens them out). An item on a face takes twice as long per plane.
-// Measured against it (64^3, R = 28, L1: 4.8 us at 1 plane, 17.1 at 16; 128^3: 13.9 us at 6, 20.2
-// at 16; 96^3 with L2 and L3: 15.1 us at 4, 24.8 at 16; 256^3: 8 to 16 within 2 %).
+// Measured against it, us a step with items of 1 / 2 / 3 / 4 / 6 / 8 / 16 planes and of the length chosen:
+//     64^3, R = 28, L1              5.2   5.1   5.4   6.3   7.8   9.4  16.8   5.2
+//     128^3, R = 58, L1            18.8  15.6  14.9  15.7  16.8  15.9  20.0  15.7
+//     96^3, R = 42, L2 and L3      15.7  15.2  16.2  14.4  19.0  15.6  23.2  15.7
+//     256^3, R = 120, L2 and L3   219   170   159   152   147   145   144   147
+//     256^3, R = 115, L1          131    95    85    80    77    75    78    76
 static int tiled_length(const std::vector<const TiledPlan*>& plans, int cap, Load load, bool L2) {
     static const int sms = [] {
         int dev = 0, n = 0;
